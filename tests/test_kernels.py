@@ -361,6 +361,32 @@ def test_linear_rows_do_not_depend_on_the_batch():
     assert torch.equal(full[41:42], one)
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (7, 33), (130, 96), (64, 100), (1183, 260), (1184, 770), (9471, 36), (9472, 61), (768, 3072)])
+def test_float32_products_of_few_and_of_many_rows_form_one_sum(N, K):
+    """The kernels for up to 1, 4, 8 and 16 rows and the tiles for more, at the edges of what each takes: every element within
+    the rounding of its K products (each of the K + 8 additions may lose 2^-24 of the sum of magnitudes), rows beyond M
+    untouched, and a row's result the same bits whatever shares its call."""
+    from vlrf_b200.csrc import ops
+    x, w, b, res = randn(133, K, seed=61), randn(N, K, seed=62), randn(N, seed=63), randn(133, N, seed=64)
+    want = x.double() @ w.double().T + b.double() + res.double()
+    bound = (K + 11) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs() + res.double().abs())
+    xd, wd, bd = x.to(DEV), w.to(DEV), b.to(DEV)
+    full = torch.empty(133, N, device=DEV)
+    ops.linear(xd, wd, bd, full, residual=res.to(DEV))
+    assert ((full.cpu().double() - want).abs() <= bound).all()
+    for first, rows in ((0, 1), (132, 1), (5, 2), (9, 4), (64, 5), (60, 8), (17, 9), (100, 16), (101, 17), (3, 64), (40, 65)):
+        some = torch.full((rows + 1, N), float("nan"), device=DEV)
+        some[:rows] = res[first:first + rows].to(DEV)
+        ops.linear(xd[first:first + rows].contiguous(), wd, bd, some, residual=some, rows=rows)
+        assert torch.equal(some[:rows], full[first:first + rows]), (first, rows)
+        assert torch.isnan(some[rows]).all()
+    odd = torch.empty(5 * K + 1, device=DEV)[1:].view(5, K)              # rows that do not begin on 16 bytes
+    odd.copy_(xd[:5])
+    some = torch.empty(5, N, device=DEV)
+    ops.linear(odd, wd, bd, some, residual=res[:5].to(DEV))
+    assert torch.equal(some, full[:5])
+
+
 # ------------------------------------------------------------------------------------------------
 def paged(k, v, n_blocks, order_seed, dtype):
     """Put [H, C, dh] keys and values of one sequence into a pool with scattered blocks; unused pool

@@ -5,8 +5,15 @@
 // refuse.  W is kept [out, in] with `in` contiguous, so the product is the reference's
 // linear(x, W) = x · Wᵀ (include/model/compute.hpp:64-68) with bias (include/model/attention.hpp:103-105),
 // activation (include/model/feedforward.hpp:54-76) and residual (include/model/transformer_block.hpp:153,158)
-// applied in the epilogue.  Each output element accumulates over K in the same order whatever M
-// is, so a row's result does not depend on how many rows share the call.
+// applied in the epilogue.
+//
+// A row's result does not depend on how many rows share the call: every kernel for a type forms an element's sum in
+// one order.  In float32 that order is: K in PARTS = 8 runs of equal length (`part_length`), each a chain of FMAs in the
+// order of k, the eight sums added in their order.  The parts are what a few rows are spread over the GPU by (a chain of
+// all K terms in one thread took 104 us a product at 4 rows, whatever its size):
+//   up to 16 rows    gemm_f32_rows_kernel: a thread per (column, part); bound by streaming W once
+//   more rows        gemm_f32_tile_kernel: 64 x 64 tiles, the eight parts of a tile one CTA each of a cluster; bound by FMAs
+// bfloat16 operands take gemm_simt_kernel (shapes outside the tensor-core kernels' rules: rare and small).
 #include "common.cuh"
 
 namespace {
@@ -68,6 +75,268 @@ gemm_simt_kernel(const IT* __restrict__ X, const IT* __restrict__ W, const float
         }
     }
 }
+// ---- float32 ------------------------------------------------------------------------------------------------------------
+
+constexpr int PARTS = 8;
+constexpr int KB = 32;                 // numbers of k a stage of a ring holds, per part
+constexpr int KPITCH = KB + 4;         // … and their pitch in shared memory: neighbours start one 16-byte bank group apart
+
+__host__ __device__ inline int part_length(int K) { return ((K + PARTS - 1) / PARTS + 3) & ~3; }
+
+template <int BYTES> __device__ __forceinline__ void cp_async_zfill(float* dst, const float* src, bool take) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int n = take ? BYTES : 0;    // (nothing is read where n is 0; the rest of the destination becomes zero)
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// KB numbers of row `row` from column k0 on into dst, zeros from column `end` on and for rows that are not there.  VEC: the
+// rows begin on 16 bytes and k0, end are multiples of 4.  `lane` of the `lanes` threads that share the work.
+template <bool VEC> __device__ __forceinline__ void stage_piece(float* dst, const float* base, size_t ld, int row, int rows, int k0, int end, int piece) {
+    constexpr int W = VEC ? 4 : 1;
+    const int k = k0 + piece * W;
+    const bool take = row < rows && k < end;
+    cp_async_zfill<W * 4>(dst + piece * W, take ? base + (size_t)row * ld + k : base, take);
+}
+
+__device__ __forceinline__ float fma4(const float4& a, const float4& b, float acc) {
+    acc = fmaf(a.x, b.x, acc);
+    acc = fmaf(a.y, b.y, acc);
+    acc = fmaf(a.z, b.z, acc);
+    return fmaf(a.w, b.w, acc);
+}
+
+__device__ __forceinline__ void f32_finish(float v, const float* bias, const float* residual, float* Y, int m, int n, int ldy, int act) {
+    if (bias) v += bias[n];
+    v = apply_act_rt(v, act);
+    if (residual) v += residual[(size_t)m * ldy + n];
+    Y[(size_t)m * ldy + n] = v;
+}
+
+// Up to R rows.  A CTA owns C columns; thread (part p, column c) runs the chain of its part for all rows.  W and x arrive
+// through a ring of STAGES stages of KB numbers of every part (`cp.async`, coalesced along k); the first stages of W are
+// asked for before the kernel ahead has ended.  A warp holds several columns of few parts, so that its reads of x are one
+// wavefront each; R and C trade reads of x for CTAs.  N x K at 4 rows, weights from memory (one chain a thread before): 2,304 x 768
+// 58 -> 4.1 us, 768 x 3,072 232 -> 7.3 us, 50,257 x 768 201 -> 33 us (4.7 TB/s); at 1 row the last is 25 us (6.2 TB/s); at 16 rows
+// 59 -> 6.2, 235 -> 19 and 205 -> 63 us.
+template <int R, int C> __host__ __device__ constexpr int rows_stage_floats() { return PARTS * C * KPITCH + PARTS * (R * KPITCH + 4); }
+
+template <int R, int C, int STAGES, bool VEC>
+__global__ void __launch_bounds__(C * PARTS)
+gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias, const float* residual,
+                     float* Y, int M, int N, int K, int ldx, int ldy, int act) {
+    extern __shared__ __align__(16) float ring[];
+    constexpr int STAGE = rows_stage_floats<R, C>(), THREADS_R = C * PARTS, PIECES = VEC ? KB / 4 : KB;
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, c = tid % C, p = tid / C, n0 = blockIdx.x * C;
+    const int len = part_length(K), n_chunks = (min(len, K) + KB - 1) / KB;
+    auto load_w = [&](int chunk) {
+        float* at = ring + (chunk % STAGES) * STAGE;
+        for (int i = tid; i < PARTS * C * PIECES; i += THREADS_R) {
+            const int piece = i % PIECES, cc = i / PIECES % C, pp = i / (PIECES * C);
+            stage_piece<VEC>(at + (pp * C + cc) * KPITCH, W, K, n0 + cc, N, pp * len + chunk * KB, min(K, (pp + 1) * len), piece);
+        }
+    };
+    auto load_x = [&](int chunk) {
+        float* at = ring + (chunk % STAGES) * STAGE + PARTS * C * KPITCH;
+        for (int i = tid; i < PARTS * R * PIECES; i += THREADS_R) {
+            const int piece = i % PIECES, r = i / PIECES % R, pp = i / (PIECES * R);
+            stage_piece<VEC>(at + pp * (R * KPITCH + 4) + r * KPITCH, X, ldx, r, M, pp * len + chunk * KB, min(K, (pp + 1) * len), piece);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s)
+        if (s < n_chunks) load_w(s);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < n_chunks) load_x(s);
+        cp_async_commit();
+    }
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                                   // the stage is here, and the one before it has been read by everyone
+        if (chunk + STAGES - 1 < n_chunks) {
+            load_w(chunk + STAGES - 1);
+            load_x(chunk + STAGES - 1);
+        }
+        cp_async_commit();
+        const float* at = ring + (chunk % STAGES) * STAGE;
+        const float4* w4 = (const float4*)(at + (p * C + c) * KPITCH);
+        const float4* x4 = (const float4*)(at + PARTS * C * KPITCH + p * (R * KPITCH + 4));
+#pragma unroll
+        for (int k = 0; k < KB / 4; ++k) {
+            const float4 w = w4[k];
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r] = fma4(x4[r * (KPITCH / 4) + k], w, acc[r]);
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    float* sums = ring;                                    // [part][row][column]
+#pragma unroll
+    for (int r = 0; r < R; ++r) sums[(p * R + r) * C + c] = acc[r];
+    __syncthreads();
+    for (int i = tid; i < R * C; i += THREADS_R) {
+        const int r = i / C, n = n0 + i % C;
+        if (r >= M || n >= N) continue;
+        float v = sums[i];
+#pragma unroll
+        for (int pp = 1; pp < PARTS; ++pp) v += sums[pp * R * C + i];
+        f32_finish(v, bias, residual, Y, r, n, ldy, act);
+    }
+}
+
+// Many rows.  The PARTS CTAs of a cluster multiply one 64 x 64 tile, each over its part of K (128 threads, 8 x 4 elements a
+// thread read four k at a time: 12 shared-memory wavefronts for 128 FMA instructions of a warp, so the FMAs bound it); then
+// each adds the eight sums of 8 of the tile's rows out of its neighbours' shared memory, in the order of the parts.  N x K at 64, 240
+// and 1,000 rows (tiles of 64 x 64 over all of K, 4 x 4 elements a thread, before): 768 x 3,072 242, 222, 324 -> 25, 51, 146 us;
+// 2,304 x 768 62, 57, 149 -> 16, 34, 116 us; 50,257 x 768 230, 793, 3,053 -> 156, 609, 2,422 us (32 TFLOP/s).
+constexpr int TILE = 64, TILE_STAGES = 3, TILE_THREADS = 128, TILE_STAGE = 2 * TILE * KPITCH, SUM_PITCH = TILE + 4;
+constexpr int TILE_SMEM = TILE_STAGES * TILE_STAGE * 4;
+static_assert(TILE * SUM_PITCH * 4 <= TILE_SMEM, "a tile of sums takes the ring's place");
+
+template <bool VEC>
+__global__ void __launch_bounds__(TILE_THREADS)
+gemm_f32_tile_kernel(const float* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias, const float* residual,
+                     float* Y, int M, int N, int K, int ldx, int ldy, int act) {
+    extern __shared__ __align__(16) float ring[];
+    constexpr int PIECES = VEC ? KB / 4 : KB;
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, part = blockIdx.x % PARTS;
+    const int n0 = blockIdx.x / PARTS * TILE, m0 = blockIdx.y * TILE;
+    // warps 2 (rows) x 2 (columns); a thread's rows are mg + 8 i, its columns ng + 16 j: a warp's reads then fall on
+    // neighbouring rows, one bank group apart
+    const int lane = tid & 31, warp = tid >> 5;
+    const int mg = (warp >> 1) * 4 + (lane >> 3), ng = (warp & 1) * 8 + (lane & 7);
+    const int len = part_length(K), first = part * len, end = min(K, first + len);
+    const int n_chunks = max(0, (end - first + KB - 1) / KB);
+    auto load = [&](int chunk, bool weights) {
+        float* at = ring + (chunk % TILE_STAGES) * TILE_STAGE + (weights ? TILE * KPITCH : 0);
+        for (int i = tid; i < TILE * PIECES; i += TILE_THREADS) {
+            const int piece = i % PIECES, r = i / PIECES;
+            if (weights) stage_piece<VEC>(at + r * KPITCH, W, K, n0 + r, N, first + chunk * KB, end, piece);
+            else stage_piece<VEC>(at + r * KPITCH, X, ldx, m0 + r, M, first + chunk * KB, end, piece);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < TILE_STAGES - 1; ++s)
+        if (s < n_chunks) load(s, true);
+    pdl_wait();
+#pragma unroll
+    for (int s = 0; s < TILE_STAGES - 1; ++s) {
+        if (s < n_chunks) load(s, false);
+        cp_async_commit();
+    }
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        cp_async_wait<TILE_STAGES - 2>();
+        __syncthreads();
+        if (chunk + TILE_STAGES - 1 < n_chunks) {
+            load(chunk + TILE_STAGES - 1, true);
+            load(chunk + TILE_STAGES - 1, false);
+        }
+        cp_async_commit();
+        const float* at = ring + (chunk % TILE_STAGES) * TILE_STAGE;
+        const float4* a4 = (const float4*)(at + mg * KPITCH);
+        const float4* b4 = (const float4*)(at + TILE * KPITCH + ng * KPITCH);
+#pragma unroll
+        for (int k = 0; k < KB / 4; ++k) {
+            float4 b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = b4[j * 16 * (KPITCH / 4) + k];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float4 a = a4[i * 8 * (KPITCH / 4) + k];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma4(a, b[j], acc[i][j]);
+            }
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    float* sums = ring;                                    // [row][column] of this part
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sums[(mg + 8 * i) * SUM_PITCH + ng + 16 * j] = acc[i][j];
+    cluster_sync_all();
+    {
+        const int r = part * (TILE / PARTS) + tid / 16, col = tid % 16 * 4;      // 8 rows of 16 pieces of 4: one a thread
+        const uint32_t own = (uint32_t)__cvta_generic_to_shared(sums + r * SUM_PITCH + col);
+        float4 v = ld_cluster_f32x4(own, 0);
+#pragma unroll
+        for (int pp = 1; pp < PARTS; ++pp) {
+            const float4 u = ld_cluster_f32x4(own, pp);
+            v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+        }
+        const int m = m0 + r, n = n0 + col;
+        if (m < M) {
+            if (n < N) f32_finish(v.x, bias, residual, Y, m, n, ldy, act);
+            if (n + 1 < N) f32_finish(v.y, bias, residual, Y, m, n + 1, ldy, act);
+            if (n + 2 < N) f32_finish(v.z, bias, residual, Y, m, n + 2, ldy, act);
+            if (n + 3 < N) f32_finish(v.w, bias, residual, Y, m, n + 3, ldy, act);
+        }
+    }
+    cluster_sync_relaxed();                                // nobody leaves while a neighbour still reads its sums
+}
+
+template <int R, int C, int STAGES, bool VEC>
+int launch_f32_rows(const float* X, const float* W, const float* bias, const float* residual, float* Y, int M, int N, int K, int ldx, int ldy,
+                    int act, cudaStream_t stream) {
+    constexpr size_t smem = (size_t)STAGES * rows_stage_floats<R, C>() * 4;
+    static_assert(smem <= 227 * 1024 && STAGES * rows_stage_floats<R, C>() >= PARTS * R * C, "shared memory");
+    auto kern = gemm_f32_rows_kernel<R, C, STAGES, VEC>;
+    static bool raised = false;
+    if (!raised && smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        raised = true;
+    }
+    launch_chained(kern, dim3((N + C - 1) / C), dim3(C * PARTS), smem, stream, X, W, bias, residual, Y, M, N, K, ldx, ldy, act);
+    return vlrf_check_launch("gemm_f32_rows");
+}
+
+// Columns a CTA: as few as leave every SM a CTA (4 below 8 x 148 columns), 32 where even those make two waves (a head over
+// a vocabulary), so that x is read from L2 less often.
+template <int R, bool VEC>
+int launch_f32_rows_for(const float* X, const float* W, const float* bias, const float* residual, float* Y, int M, int N, int K, int ldx, int ldy,
+                        int act, cudaStream_t stream) {
+    constexpr int S = R <= 8 ? 5 : 4;
+    if (N < 8 * 148) return launch_f32_rows<R, 4, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    if (N < 2 * 32 * 148) return launch_f32_rows<R, 8, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    return launch_f32_rows<R, 32, 2, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+}
+
+// Rows a thread: the next instantiation up.  Tiles from 17 rows on: at 16 the rows kernel wins at every shape above (6.2 against 15.5
+// us at 64 rows of 2,304 x 768, which is what a tile costs at 17 rows too), and its registers hold 16 sums.
+template <bool VEC>
+int launch_f32(const float* X, const float* W, const float* bias, const float* residual, float* Y, int M, int N, int K, int ldx, int ldy, int act,
+               cudaStream_t stream) {
+    if (M == 1) return launch_f32_rows_for<1, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    if (M <= 4) return launch_f32_rows_for<4, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    if (M <= 8) return launch_f32_rows_for<8, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    if (M <= 16) return launch_f32_rows_for<16, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    auto kern = gemm_f32_tile_kernel<VEC>;
+    static bool raised = false;
+    if (!raised) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
+        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %d bytes of shared memory: %s", TILE_SMEM, cudaGetErrorString(e));
+        raised = true;
+    }
+    const dim3 grid((unsigned)((N + TILE - 1) / TILE * PARTS), (unsigned)((M + TILE - 1) / TILE));
+    launch_chained_cluster(kern, grid, dim3(TILE_THREADS), TILE_SMEM, dim3(PARTS), stream, X, W, bias, residual, Y, M, N, K, ldx, ldy, act);
+    return vlrf_check_launch("gemm_f32_tile");
+}
 }  // namespace
 
 extern "C" int vlrf_gemm_simt(const void* X, const void* W, const float* bias, const float* residual,
@@ -82,8 +351,12 @@ extern "C" int vlrf_gemm_simt(const void* X, const void* W, const float* bias, c
 #define LAUNCH(IT, OT)                                                                                  \
     gemm_simt_kernel<IT, OT><<<grid, THREADS, 0, stream>>>((const IT*)X, (const IT*)W, bias, residual, \
                                                            (OT*)Y, M, N, K, ldx, ldy, act)
-    if (in_dtype == VLRF_F32 && out_dtype == VLRF_F32) LAUNCH(float, float);
-    else if (in_dtype == VLRF_BF16 && out_dtype == VLRF_F32) LAUNCH(__nv_bfloat16, float);
+    if (in_dtype == VLRF_F32 && out_dtype == VLRF_F32) {
+        const bool vec = K % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)X | (uintptr_t)W) % 16 == 0;
+        return vec ? launch_f32<true>((const float*)X, (const float*)W, bias, residual, (float*)Y, M, N, K, ldx, ldy, act, stream)
+                   : launch_f32<false>((const float*)X, (const float*)W, bias, residual, (float*)Y, M, N, K, ldx, ldy, act, stream);
+    }
+    if (in_dtype == VLRF_BF16 && out_dtype == VLRF_F32) LAUNCH(__nv_bfloat16, float);
     else if (in_dtype == VLRF_BF16 && out_dtype == VLRF_BF16) LAUNCH(__nv_bfloat16, __nv_bfloat16);
     else return vlrf_fail(VLRF_ERR_INVALID_ARG, "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 #undef LAUNCH
