@@ -240,3 +240,49 @@ def test_recurrence_in_steps_of_every_parity(Hs, P, N, G, taps, ng):
     for i in range(3):
         close(torch.cat(got[i]), want[i], 3e-5, f"sequence {i}")
     assert torch.isnan(state[[1, 3, 5]]).all()
+
+
+@pytest.mark.parametrize("d,groups,rows", [(128, 1, 1), (384, 3, 300), (2048, 4, 9), (4096, 8, 3), (4096, 32, 297), (4608, 9, 2), (640, 1, 5)])
+def test_gated_norm_with_rows_in_registers(d, groups, rows):
+    """The kernel for whole warps' worth of columns, at the edges of its quads a thread, beside the one for any row (which a column
+    that is not on 16 bytes asks for): both within float32 rounding of the plain formula, and of one another."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(d + groups)
+    y, z, w = torch.randn(rows, d, generator=g), 2.0 * torch.randn(rows, d, generator=g), torch.randn(d, generator=g)
+    want = 0.7 * plain.group_rms_norm(y.double() * plain.silu(z.double()), w.double(), groups, 1e-5)
+    for off in (8, 9):                                       # 9: the gate's columns do not begin on 16 bytes
+        proj = torch.full((rows, d + 12), float("nan"))
+        proj[:, off:off + d] = z
+        for dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 2.0 ** -8)):
+            out = torch.full((rows + 1, d + 4), float("nan"), dtype=dtype, device=DEV)
+            ops.ssd_gate_norm(dev(y), dev(proj), off, dev(w), groups, 1e-5, 0.7, out[:, :d], rows)
+            close(out[:rows, :d].float().cpu(), want, tol, f"gate at {off}")
+            assert torch.isnan(out[rows]).all() and torch.isnan(out[:, d:]).all()
+
+
+@pytest.mark.parametrize("S,d", [(1, 4), (2, 128), (4, 1024), (4, 1000), (5, 2048), (8, 4096), (8, 4100), (9, 256)])
+def test_streams_with_rows_in_registers(S, d):
+    """Embedding, write and read of rows that the kernels hold in registers (up to 8 streams of 4,096 numbers) and just beyond."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(S * d)
+    T = 5
+    x, y, w = torch.randn(T, S, d, generator=g), torch.randn(T, d, generator=g), torch.randn(d, generator=g)
+    mix, b, a = torch.randn(S, S, generator=g), torch.randn(S, generator=g), torch.randn(S, generator=g)
+    want_x = torch.einsum("sj,tsd->tjd", mix.double(), x.double()) + b.double()[None, :, None] * y.double()[:, None]
+    want_h = plain.rms_norm(torch.einsum("s,tsd->td", a.double(), want_x), w.double(), 1e-5)
+    for dtype, tol in ((torch.float32, 3e-6), (torch.bfloat16, 2.0 ** -8)):
+        xd = dev(x.reshape(T, S * d))
+        h = torch.full((T + 1, d), float("nan"), dtype=dtype, device=DEV)
+        ops.streams_write_read(xd, S, dev(mix), dev(b), dev(y), dev(a), dev(w), 1e-5, h, T)
+        close(xd.cpu().reshape(T, S, d), want_x, 3e-6, "streams")
+        close(h[:T].float().cpu(), want_h, tol, "read behind the write")
+        assert torch.isnan(h[T].float()).all()
+        rows = torch.tensor([3, 0, 3], dtype=torch.int32, device=DEV)
+        some = torch.full((3, d), float("nan"), dtype=dtype, device=DEV)
+        ops.streams_read_norm(xd, S, None, dev(w), 1e-5, some, rows)
+        close(some.float().cpu(), plain.rms_norm(want_x.sum(1)[[3, 0, 3]], w.double(), 1e-5), tol, "sum of the streams")
+        table = torch.randn(11, d, generator=g).to(dtype)
+        e, err = torch.full((3, S * d), float("nan"), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.embed_streams(table.to(DEV), torch.tensor([10, 0, 4], dtype=torch.int32, device=DEV), e, S, 1.5, err)
+        close(e.cpu().reshape(3, S, d), (1.5 * table.double()[[10, 0, 4]])[:, None].repeat(1, S, 1), 3e-7, "embedding")
+        assert int(err.item()) == 0

@@ -165,6 +165,7 @@ __device__ __forceinline__ float gelu_erf_f(float x) {
 __device__ __forceinline__ float relu2_f(float x) { const float r = fmaxf(x, 0.f); return r * r; }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
+__device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 // x · sigmoid(x) for results that are rounded to bfloat16 anyway
 __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 template <int ACT> __device__ __forceinline__ float apply_act(float x) {
