@@ -286,3 +286,73 @@ def test_streams_with_rows_in_registers(S, d):
         ops.embed_streams(table.to(DEV), torch.tensor([10, 0, 4], dtype=torch.int32, device=DEV), e, S, 1.5, err)
         close(e.cpu().reshape(3, S, d), (1.5 * table.double()[[10, 0, 4]])[:, None].repeat(1, S, 1), 3e-7, "embedding")
         assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("Hs,P,N,G", [(4, 64, 64, 1), (8, 64, 64, 2), (3, 20, 16, 3), (10, 132, 32, 2), (2, 128, 128, 1), (5, 4, 128, 1)])
+def test_recurrence_in_chunks(Hs, P, N, G):
+    """Runs at the edges of the chunks and of their blocks of 16, from zero and from kept states in both copies, a padding row and
+    NaN-poisoned neighbours; heads that forget within a token and heads that keep everything.  The chunked kernels may be as far from
+    the plain float64 recurrence as the token-by-token kernel is, or within 2^-21 of the largest result: an operand in three
+    bfloat16 parts and the six products of parts are good to 2^-23, and a sum's roundings add.  (Measured: 1.3e-7 to 2.0e-7 of the
+    largest result, token by token 4.5e-7 to 1.2e-6.)"""
+    import types
+
+    from vlrf_b200.csrc import ops
+    from vlrf_b200.parts.context import Workspace
+    g = torch.Generator().manual_seed(Hs * 1000 + P * 10 + N)
+    inner, channels = Hs * P, Hs * P + 2 * G * N
+    lens, pos0, slots = [64, 1, 65, 130, 15, 200, 17], [0, 3, 4, 7, 0, 128, 1], [6, 0, 3, 5, 1, 8, 2]
+    rand = lambda *shape: torch.randn(*shape, generator=g)   # noqa: E731
+    dt_bias, a_log, D = rand(Hs), torch.linspace(-6.0, 2.5, Hs), rand(Hs)
+    state_row = Hs * N * P + 8
+    kept = {s: rand(Hs, N, P) if p else torch.zeros(Hs, N, P) for s, p in zip(slots, pos0)}
+    state = torch.full((10, 2, state_row), float("nan"))
+    for s, p in zip(slots, pos0):
+        state[s, p & 1, :Hs * N * P] = kept[s].flatten()
+    rows, seq_slot, seq_start, seq_pos0, want, ends = [], [], [0], [], [], {}
+    for i, (n, p, s) in enumerate(zip(lens, pos0, slots)):
+        xbc, dt = rand(n, channels), rand(n, Hs) * 2.0
+        x, B, C = (t.double() for t in (xbc[:, :inner].reshape(n, Hs, P), xbc[:, inner:inner + G * N].reshape(n, G, N), xbc[:, inner + G * N:].reshape(n, G, N)))
+        step = plain.softplus(dt.double() + dt_bias.double())
+        B, C = (t.repeat_interleave(Hs // G, 1) for t in (B, C))
+        S, y = kept[s].double().clone(), torch.empty(n, Hs, P, dtype=torch.float64)
+        for t in range(n):
+            S = torch.exp(-torch.exp(a_log.double()) * step[t])[:, None, None] * S + (step[t][:, None] * B[t])[:, :, None] * x[t][:, None, :]
+            y[t] = (S * C[t][:, :, None]).sum(1) + D.double()[:, None] * x[t]
+        want.append(y.reshape(n, inner)); ends[s] = S
+        rows.append((xbc, dt)); seq_slot.append(s); seq_pos0.append(p); seq_start.append(seq_start[-1] + n)
+        if i == 2:                                                      # a padding row between two sequences
+            rows.append((torch.full((1, channels), float("nan")), torch.full((1, Hs), float("nan"))))
+            seq_slot.append(-1); seq_pos0.append(0); seq_start.append(seq_start[-1] + 1)
+    T = seq_start[-1]
+    xbc, proj = dev(torch.cat([r[0] for r in rows])), dev(torch.cat([torch.cat([rand(r[1].shape[0], 3), r[1]], 1) for r in rows]))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)   # noqa: E731
+    ctx = types.SimpleNamespace(n_tokens=T, n_seqs=len(seq_slot), seq_slot=i32(seq_slot), seq_start=i32(seq_start), seq_pos0=i32(seq_pos0),
+                                max_new=max(lens), ws=Workspace(torch.device(DEV)), act_dtype=torch.bfloat16)
+    ctx.max_new = ops.SSD_CHUNKS_MIN_RUN                              # (the rule asks for longer runs than this test's)
+    assert ops.ssd_chunks_takes(torch.bfloat16, ctx, Hs, G, N, P, channels, state_row)
+    assert not ops.ssd_chunks_takes(torch.float32, ctx, Hs, G, N, P, channels, state_row)
+    ctx.max_new = max(lens)
+    keep = torch.ones(T, dtype=torch.bool)
+    for s, a in zip(seq_slot, seq_start):
+        if s < 0:
+            keep[a] = False
+    want, off = torch.cat(want), {}
+    for chunked in (False, True):
+        st, y = state.to(DEV), torch.full((T, inner), float("nan"), device=DEV)
+        if chunked:
+            ops.ssd_chunks(xbc, proj, 3, dev(dt_bias), dev(a_log), dev(D), st, ctx, y, Hs, G, N, P)
+        else:
+            ops.ssd_scan(xbc, proj, 3, dev(dt_bias), dev(a_log), dev(D), st, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, ctx.n_seqs, Hs, G, N, P,
+                         ctx.max_new)
+        y, st = y.cpu(), st.cpu()
+        assert torch.isnan(y[~keep]).all() and torch.isfinite(y[keep]).all()
+        off[chunked] = [float((y[keep].double() - want).norm() / want.norm()), float((y[keep].double() - want).abs().max() / want.abs().max())]
+        for s, p, n in zip(slots, pos0, lens):
+            close(st[s, (p + n) & 1, :Hs * N * P].reshape(Hs, N, P), ends[s], 1e-5, f"state of slot {s}")
+            if n & 1:
+                assert torch.equal(st[s, p & 1, :Hs * N * P], state[s, p & 1, :Hs * N * P])
+        assert torch.isnan(st[[4, 7, 9]]).all() and torch.isnan(st[:, :, Hs * N * P:]).all()
+    print(f"heads {Hs} of {N} x {P}: token by token {off[False]}, in chunks {off[True]}")
+    for a, b in zip(off[True], off[False]):
+        assert a <= max(1.5 * b, 2.0 ** -21), off

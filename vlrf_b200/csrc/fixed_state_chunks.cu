@@ -19,36 +19,12 @@
 // [slots][2][state_row], head by head [V][K], read from the copy of the parity of the position at the step's start and written to
 // that of its end.
 #include "common.cuh"
+#include "chunk_mma.cuh"
 
 namespace {
 constexpr int FC = 64;                              // tokens of a chunk
 constexpr int FC_MAX_K = 256;
 
-__device__ __forceinline__ uint32_t fc_sm(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-// 16 bytes, or zeros where there is nothing
-__device__ __forceinline__ void fc_cp16(void* dst, const void* src, bool there) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(fc_sm(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void fc_ldsm(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void fc_ldsm_t(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void fc_ldsm_t2(uint32_t& r0, uint32_t& r1, uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-__device__ __forceinline__ void fc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// two numbers as the sum of two pairs of bfloat16
-__device__ __forceinline__ void fc_split(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(x - __low2float(h), y - __high2float(h));
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-}
 // a^n by squaring, n ≥ 0
 __device__ __forceinline__ float fc_power(float a, int n) {
     float r = 1.f;

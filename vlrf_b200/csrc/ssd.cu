@@ -19,7 +19,8 @@
 //                   column, a warp per slice of rows, the state in registers; the inputs of 16 tokens at a time arrive in
 //                   shared memory by `cp.async` a batch ahead, B and C are read from there by every lane alike; the
 //                   C-weighted sums of the slices meet in shared memory once per batch;
-//                   serves prompts and single tokens alike, with the same arithmetic in the same order
+//                   serves prompts and single tokens alike, with the same arithmetic in the same order (long prompts of the
+//                   bfloat16 engine go to state_chunks.cu)
 //   ssd_gate_norm   y · (z·sigmoid(z)), RMS norm in equal groups, weight, a factor; rounded to the activation dtype
 #include "common.cuh"
 
