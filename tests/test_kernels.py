@@ -61,6 +61,24 @@ def test_layernorm(out_dtype, tol, d, eps):
     assert rel_err(out2.float().cpu(), want[rows.long()]) < tol
 
 
+@pytest.mark.parametrize("d", [4, 768, 1024, 1028, 2048, 2052])
+@pytest.mark.parametrize("n", [1, 3, 7, 9])
+def test_layernorm_of_few_rows(n, d):
+    """Down to one row, at the edges of the widths that a warp keeps in registers; and from a place that is not on 16 bytes."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(n * d)
+    x, gamma, beta = torch.randn(n, d, generator=g) * 3 + 1, torch.randn(d, generator=g), torch.randn(d, generator=g)
+    want = torch.nn.functional.layer_norm(x.double(), (d,), gamma.double(), beta.double(), 1e-5)
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-2)):
+        for off in (0, 1):
+            flat = torch.zeros(n * d + 1, device=DEV)
+            xd = flat[off:off + n * d].view(n, d)
+            xd.copy_(x)
+            out = torch.full((n, d), float("nan"), dtype=dtype, device=DEV)
+            ops.layernorm(xd, gamma.to(DEV), beta.to(DEV), 1e-5, out)
+            assert float((out.double().cpu() - want).abs().max()) <= tol * float(want.abs().max()), (dtype, off)
+
+
 def test_layernorm_small_variance_uses_eps():
     from vlrf_b200.csrc import ops
     x = torch.full((2, 64), 3.0) + randn(2, 64, seed=8) * 1e-4
