@@ -458,3 +458,28 @@ def test_cache_rows_of_a_step_as_plain_matrices():
         assert int(err.item()) == 0
         assert torch.equal(oc[:5].cpu(), rows[pos[:5], :C]) and torch.equal(orr[:5].cpu(), rows[pos[:5], C:])
         assert float(oc[5].float().abs().max()) == 0.0 and float(orr[5].float().abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("width,top", [(4, 1), (21, 3), (512, 8), (516, 9), (1028, 2), (2048, 32)])
+def test_weighted_sum_of_experts_at_the_edges_of_its_quads(width, top):
+    """Widths around the 512 columns of a CTA (and one that is not of whole quads), and experts around the eight that are asked for
+    together, with and without each of the other terms, against float64 sums."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(width + top)
+    T = 5
+    eo, so, res = (torch.randn(n, width, generator=g) for n in (T * top, T, T))
+    h = torch.randn(T, width, generator=g).bfloat16()
+    row_of = torch.randperm(T * top, generator=g).reshape(T, top).int()
+    ids, wts, gate = torch.zeros(T, top, dtype=torch.int32), torch.rand(T, top, generator=g), torch.rand(T, 1, generator=g)
+    row_of[0, 0], ids[0, 0] = -1, -2                      # returns its input
+    row_of[1, top - 1], ids[1, top - 1] = -1, -1          # chose nothing
+    terms = torch.where((row_of >= 0)[..., None], eo.double()[row_of.clamp_min(0)], torch.where((ids == -2)[..., None], h.double()[:, None], 0.0))
+    for with_h, with_w, with_so, with_gate in ((True, True, True, True), (True, True, False, False), (False, False, True, False)):
+        t = terms if with_h else torch.where((row_of >= 0)[..., None], terms, 0.0)
+        want = (t * (wts.double()[..., None] if with_w else 1.0)).sum(1) + res.double()
+        if with_so:
+            want = want + (gate.double() if with_gate else 1.0) * so.double()
+        y = res.cuda()
+        ops.moe_combine(eo.cuda(), row_of.cuda(), wts.cuda() if with_w else None, top, so.cuda() if with_so else None, gate.cuda() if with_gate else None,
+                        y, T, residual=y, ids=ids.cuda() if with_h else None, h=h.cuda() if with_h else None)
+        close(y, want, 1e-6, f"{with_h} {with_w} {with_so}")

@@ -246,6 +246,58 @@ moe_combine_kernel(const float* __restrict__ expert_out, int width, const int* _
         y[(size_t)t * width + i] = s;
     }
 }
+
+// four numbers from a row of either type
+__device__ __forceinline__ float4 moe_quad(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 moe_quad(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// The same for rows of whole quads on 16-byte boundaries: a thread has four numbers of a token and asks for all it adds before it adds
+// any (the experts of a token eight at a time); the row is dealt to CTAs of 128 threads.  The kernel above waits for every term of
+// every 128 numbers in turn, in one CTA a token: 12 us for 16 tokens of 1,024 inside a decode step, whatever there is to read, and
+// 33 us for 1,928 of 2,048 with four experts; here 3.1 us, and 20 us, bound by the 110 MB of rows.
+template <typename HT>
+__global__ void __launch_bounds__(128)
+moe_combine_quads_kernel(const float* __restrict__ expert_out, int width, const int* __restrict__ row_of, const float* __restrict__ wts,
+                         int top, const float* __restrict__ shared_out, const float* __restrict__ gate, const float* residual,
+                         float* y, const int* __restrict__ ids, const HT* __restrict__ h) {
+    pdl_wait();                 // chained launch: nothing is read before the kernels ahead have finished
+    pdl_launch_dependents();
+    const int t = blockIdx.x, i = 4 * (blockIdx.y * 128 + threadIdx.x);
+    if (i >= width) return;
+    constexpr int AHEAD = 8;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const size_t at = (size_t)t * width + i;
+    const float4 so = shared_out != nullptr ? moe_quad(shared_out + at) : zero;
+    const float g = shared_out != nullptr && gate != nullptr ? gate[t] : 1.f;
+    const float4 res = residual != nullptr ? moe_quad(residual + at) : zero;
+    float4 s = zero;
+    for (int j0 = 0; j0 < top; j0 += AHEAD) {
+        float4 e[AHEAD];
+        float w[AHEAD];
+        bool there[AHEAD];
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j) {
+            const size_t pair = (size_t)t * top + j0 + j;
+            const int row = j0 + j < top ? row_of[pair] : -1;
+            const bool self = j0 + j < top && row < 0 && ids != nullptr && ids[pair] == -2;      // an expert that returns its input
+            there[j] = row >= 0 || self;
+            w[j] = there[j] && wts != nullptr ? wts[pair] : 1.f;
+            e[j] = row >= 0 ? moe_quad(expert_out + (size_t)row * width + i) : self ? moe_quad(h + at) : zero;
+        }
+#pragma unroll
+        for (int j = 0; j < AHEAD; ++j)
+            if (there[j]) {
+                s.x = fmaf(w[j], e[j].x, s.x); s.y = fmaf(w[j], e[j].y, s.y); s.z = fmaf(w[j], e[j].z, s.z); s.w = fmaf(w[j], e[j].w, s.w);
+            }
+    }
+    if (shared_out != nullptr) { s.x += g * so.x; s.y += g * so.y; s.z += g * so.z; s.w += g * so.w; }
+    if (residual != nullptr) { s.x += res.x; s.y += res.y; s.z += res.z; s.w += res.w; }
+    *reinterpret_cast<float4*>(y + at) = s;
+}
 }  // namespace
 
 extern "C" int vlrf_moe_route(const float* z, int ld_z, int E, int top, int shared_gate, const int* tok_slot, int* ids,
@@ -302,6 +354,16 @@ extern "C" int vlrf_moe_combine(const float* expert_out, int width, const int* r
     VLRF_REQUIRE(wts != nullptr || ids == nullptr, "moe_combine: experts that return their input need weights");
     VLRF_REQUIRE((ids == nullptr) == (h == nullptr), "moe_combine: experts that return their input need ids and the input rows");
     if (T == 0) return VLRF_OK;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(expert_out) | reinterpret_cast<uintptr_t>(shared_out) | reinterpret_cast<uintptr_t>(residual) |
+                          reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(h);
+    const dim3 quads(T, (width / 4 + 127) / 128);
+    if (width % 4 == 0 && (all & 15) == 0 && quads.y <= 65535 && (h == nullptr || h_dtype == VLRF_BF16 || h_dtype == VLRF_F32)) {
+        if (h != nullptr && h_dtype == VLRF_BF16)
+            launch_chained(moe_combine_quads_kernel<__nv_bfloat16>, quads, dim3(128), (size_t)(0), stream, expert_out, width, row_of, wts, top, shared_out, gate, residual, y, ids, (const __nv_bfloat16*)h);
+        else
+            launch_chained(moe_combine_quads_kernel<float>, quads, dim3(128), (size_t)(0), stream, expert_out, width, row_of, wts, top, shared_out, gate, residual, y, ids, (const float*)h);
+        return vlrf_check_launch("moe_combine");
+    }
     if (h != nullptr && h_dtype == VLRF_BF16)
         launch_chained(moe_combine_kernel<__nv_bfloat16>, dim3(T), dim3(128), (size_t)(0), stream, expert_out, width, row_of, wts, top, shared_out, gate, residual, y, ids, (const __nv_bfloat16*)h);
     else if (h == nullptr || h_dtype == VLRF_F32)
