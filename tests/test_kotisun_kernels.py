@@ -356,3 +356,35 @@ def test_recurrence_in_chunks(Hs, P, N, G):
     print(f"heads {Hs} of {N} x {P}: token by token {off[False]}, in chunks {off[True]}")
     for a, b in zip(off[True], off[False]):
         assert a <= max(1.5 * b, 2.0 ** -21), off
+
+
+@pytest.mark.parametrize("taps", [1, 2, 4, 5])
+def test_convolution_over_runs(taps):
+    """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a
+    padding row.  Sums of at most five products and x·sigmoid(x) in float32."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(taps)
+    channels, ld, off = 130, 200, 7
+    lens, pos0, slots = [1, 16, 17, 33, 1, 2], [5, 0, 4, 0, 0, 2], [2, 0, 4, 1, -1, 3]
+    w, bias = torch.randn(channels, taps, generator=g), torch.randn(channels, generator=g)
+    for some in ((0, 1, 4, 5), (0, 1, 2, 3, 4, 5)):            # all runs at most 16 tokens, or not
+        n = [lens[i] for i in some]
+        start = torch.tensor([0] + list(torch.tensor(n).cumsum(0)), dtype=torch.int32)
+        proj = torch.randn(int(start[-1]), ld, generator=g)
+        row = (taps - 1) * channels + 3
+        state = torch.randn(5, 2, row, generator=g)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)   # noqa: E731
+        st, out = state.to(DEV), torch.full((int(start[-1]), channels), float("nan"), device=DEV)
+        pos = [pos0[i] for i in some]
+        ops.ssd_conv(dev(proj), off, dev(w), dev(bias), st, 3, i32([slots[i] for i in some]), start.to(DEV), i32(pos), out, len(some), max(n))
+        for j, i in enumerate(some):
+            a, b = int(start[j]), int(start[j + 1])
+            if slots[i] < 0:
+                assert torch.isnan(out[a:b]).all()
+                continue
+            kept = state[slots[i], pos0[i] & 1, 3:].reshape(taps - 1, channels).double()
+            u = torch.cat([kept, proj[a:b, off:off + channels].double()])
+            want = torch.stack([(u[t:t + taps] * w.double().T).sum(0) + bias.double() for t in range(b - a)])
+            close(out[a:b], want * torch.sigmoid(want), 3e-6, f"run {i}")
+            if taps > 1:
+                close(st[slots[i], (pos0[i] + b - a) & 1, 3:], u[len(u) - (taps - 1):].reshape(-1), 1e-7, f"kept inputs of run {i}")
