@@ -388,3 +388,39 @@ def test_convolution_over_runs(taps):
             close(out[a:b], want * torch.sigmoid(want), 3e-6, f"run {i}")
             if taps > 1:
                 close(st[slots[i], (pos0[i] + b - a) & 1, 3:], u[len(u) - (taps - 1):].reshape(-1), 1e-7, f"kept inputs of run {i}")
+
+
+@pytest.mark.parametrize("H,G,dk,dv,rot,interleaved,maps,norm", [
+    (16, 4, 64, 96, 32, False, 1, None), (3, 1, 12, 4, 8, False, 1, None), (2, 2, 128, 128, 128, False, 2, None), (5, 5, 20, 8, 12, True, 1, None),
+    (4, 2, 8, 4, 0, False, 1, None), (3, 3, 16, 12, 4, True, 2, None), (17, 3, 64, 64, 32, False, 1, "head"), (2, 1, 96, 20, 0, True, 1, "head")])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rotation_and_append_of_aligned_rows(H, G, dk, dv, rot, interleaved, maps, norm, dtype):
+    """Rows on 16-byte boundaries (quads of entries a thread) against the same rows one number further (pairs): queries, keys and
+    values, with a padding row, a token whose block is missing, and a layer that keeps no keys.  Both work out an entry from the
+    same two products; which of them is fused into the sum may differ, by a rounding of float32, and then of bfloat16."""
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(H * 100 + dk)
+    T, nq, nk = 5, H * maps * dk, G * maps * dk
+    rows = torch.randn(T, nq + nk + G * dv, generator=g)
+    freq = dev(torch.rand(rot // 2, generator=g)) if rot else None
+    slots, pos = dev(torch.tensor([0, 1, -1, 1, 0]), torch.int32), dev(torch.tensor([3, 64, 5, 1000, 127]), torch.int32)
+    table = dev(torch.tensor([[2, 0], [3, 1]] if T else []), torch.int32)
+    weights = dict(norm=norm, q_norm=dev(torch.randn(dk, generator=g)), k_norm=dev(torch.randn(dk, generator=g)), eps=1e-5) if norm else {}
+    got = []
+    for shift in (4, 3):
+        wide = torch.full((T, rows.shape[1] + 8 + (-rows.shape[1]) % 4), float("nan"))
+        wide[:, shift:shift + rows.shape[1]] = rows
+        wide = dev(wide)
+        for write in (True, False):
+            q = torch.full((T, nq), 7.0, dtype=dtype, device=DEV)
+            k, v = torch.full((4, G, 64, maps * dk), 7.0, dtype=dtype, device=DEV), torch.full((4, G, 64, dv), 7.0, dtype=dtype, device=DEV)
+            err = torch.zeros(1, dtype=torch.int32, device=DEV)
+            ops.qkv_rope_append(wide[:, shift:shift + rows.shape[1]], 0, nq, nq + nk, freq, rot, q, k, v, table, slots, pos, T, H, G, dk, dv, write,
+                                err, interleaved=interleaved, magnitude=1.25, maps=maps, **weights)
+            assert (int(err.item()) != 0) == write                      # position 1,000 has no block
+            got.append([t.double().cpu() for t in (q, k, v)])
+    for a, b in zip(got[:2], got[2:]):
+        for x, y in zip(a, b):
+            assert float((x - y).abs().max()) <= (1e-6 if dtype == torch.float32 else 2.0 ** -8) * max(1.0, float(y.abs().max()))
+            assert torch.equal(x == 7.0, y == 7.0)
+    assert (got[0][0][2] == 7.0).all() and (got[1][1] == 7.0).all() and (got[0][1] != 7.0).any()
