@@ -483,3 +483,16 @@ def test_weighted_sum_of_experts_at_the_edges_of_its_quads(width, top):
         ops.moe_combine(eo.cuda(), row_of.cuda(), wts.cuda() if with_w else None, top, so.cuda() if with_so else None, gate.cuda() if with_gate else None,
                         y, T, residual=y, ids=ids.cuda() if with_h else None, h=h.cuda() if with_h else None)
         close(y, want, 1e-6, f"{with_h} {with_w} {with_so}")
+
+
+@pytest.mark.parametrize("counts,N,K", [([2] * 16, 264, 128), ([33] + [0] * 15, 130 + 6, 192), ([10] * 10, 128, 64), ([31, 33, 64, 0, 1], 200, 320),
+                                        ([241] * 8, 1736, 64), ([0] * 1021 + [10, 11], 16, 16)])
+def test_products_per_group_by_the_rows_of_a_group(counts, N, K):
+    """Tiles of 16, 32 and 64 rows with the weights as the 128-row operand (groups of fewer and of more rows than a tile among them), 256
+    columns a tile, and as many groups as the table of tiles holds."""
+    test_products_per_group_on_the_tensor_cores(counts, N, K)
+
+
+@pytest.mark.parametrize("M,H,N,K", [(16, 16, 256, 64), (17, 3, 136, 72), (33, 2, 128, 256), (65, 4, 320, 64), (2, 700, 8, 8)])
+def test_products_per_head_of_few_rows(M, H, N, K):
+    test_products_per_head_on_the_tensor_cores(M, H, N, K)

@@ -59,7 +59,8 @@ struct TcKvScatter {
 // `offsets` (device, G + 1 entries) the groups are consecutive row ranges (experts over rows sorted by expert); without,
 // every group takes all `rows` rows (heads, each with columns of its own).  The row tiles of all groups are listed in
 // shared memory once the kernel ahead has finished (it wrote the offsets); a tile never spans two groups, rows beyond
-// its group's end are computed and not stored, and columns of W beyond N (the next group's rows) likewise.
+// its group's end are computed and not stored, and columns of W beyond N (the next group's rows) likewise.  With SWAP as well,
+// a row tile has BN rows.
 constexpr int TC_GR_TAB = 1024;      // row tiles of all groups together
 struct TcGroups {
     const int* offsets; int G, x_gs, y_gs, rows;
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(TC_THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                     const float* __restrict__ bias, const float* residual, OT* Y, int M, int N, int K, int ldy,
                     int act, TcKvScatter kv, int* __restrict__ dev_err, long long* trace, TcGroups gr = TcGroups{}) {
-    static_assert(!(GR && SWAP), "groups keep the roles of the operands");
+    constexpr int GR_ROWS = SWAP ? BN : TC_BM;                       // rows of a group's tile
     __shared__ int gr_m0[GR ? TC_GR_TAB : 1], gr_end[GR ? TC_GR_TAB : 1], gr_g[GR ? TC_GR_TAB : 1];
     __shared__ int gr_count;
     extern __shared__ unsigned char tc_raw[];
@@ -105,9 +106,22 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     const int n_kb = (K + KA * TC_BK - 1) / (KA * TC_BK);             // stages of K (atoms behind K's end are read as zeros)
     // tiles: not swapped — 128 rows of X by BN rows of W, neighbours in N first (they share the rows of X in
     // L2); swapped — 128 rows of W by all rows of X
-    const int tiles_n = SWAP ? 1 : (N + BN - 1) / BN;
+    const int tiles_n = SWAP ? (GR ? (N + TC_BM - 1) / TC_BM : 1) : (N + BN - 1) / BN;
     int n_tiles = SWAP ? (N + TC_BM - 1) / TC_BM : tiles_n * ((M + TC_BM - 1) / TC_BM);
-    if (GR) n_tiles = 0;                                            // known once the groups' rows are (below)
+    if (GR) n_tiles = gr.offsets == nullptr ? tiles_n * gr.G * ((gr.rows + GR_ROWS - 1) / GR_ROWS) : 0;    // (with offsets: known below)
+    // the first rows of a tile's two operands, the column at which it begins to read X, and its group's row tile
+    auto place = [&](int tile, int& a_row, int& b_row, int& xk0) {
+        if (GR) {
+            const int rt = tile / tiles_n, tn = tile - rt * tiles_n, w_row = gr_g[rt] * N + tn * (SWAP ? TC_BM : BN);
+            xk0 = gr_g[rt] * gr.x_gs;
+            a_row = SWAP ? w_row : gr_m0[rt];
+            b_row = SWAP ? gr_m0[rt] : w_row;
+        } else {
+            xk0 = 0;
+            a_row = SWAP ? tile * TC_BM : (tile / tiles_n) * TC_BM;
+            b_row = SWAP ? 0 : (tile % tiles_n) * BN;
+        }
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { tbar_init(&full[s], 1); tbar_init(&empty[s], 1); }
@@ -128,30 +142,44 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     // The weights do not depend on the kernel ahead: the first tile's weight operand (the 128-row one when the
     // roles are exchanged, else the BN-row one) is requested for as many k blocks as the ring holds before the
     // wait; the rows of X follow after it.
+    if (GR && gr.offsets == nullptr) {             // every group has all rows: nothing to wait for
+        const int each = (gr.rows + GR_ROWS - 1) / GR_ROWS;
+        for (int i = threadIdx.x; i < gr.G * each; i += TC_THREADS) { gr_m0[i] = i % each * GR_ROWS; gr_end[i] = gr.rows; gr_g[i] = i / each; }
+        __syncthreads();
+    }
     const int early = (int)blockIdx.x < n_tiles ? min(STAGES, n_kb) : 0;
-    if (warp == 8 && lane == 0) {
-        const int tile = blockIdx.x;
-        const int m0 = SWAP ? tile * TC_BM : (tile / tiles_n) * TC_BM, n0 = SWAP ? 0 : (tile % tiles_n) * BN;
+    if (warp == 8 && lane == 0 && early > 0) {
+        int a_row, b_row, xk0;
+        place(blockIdx.x, a_row, b_row, xk0);
         for (int kb = 0; kb < early; ++kb) {
             tbar_expect_tx(&full[kb], A_BYTES + B_BYTES);
 #pragma unroll
             for (int a = 0; a < KA; ++a) {
-                if (SWAP) tma_load_2d(a_tiles + (size_t)kb * A_BYTES + a * A_ATOM, &tmap_x, (kb * KA + a) * TC_BK, m0, &full[kb]);
-                else tma_load_2d(b_tiles + (size_t)kb * B_BYTES + a * B_ATOM, &tmap_w, (kb * KA + a) * TC_BK, n0, &full[kb]);
+                if (SWAP) tma_load_2d(a_tiles + (size_t)kb * A_BYTES + a * A_ATOM, &tmap_x, (kb * KA + a) * TC_BK, a_row, &full[kb]);
+                else tma_load_2d(b_tiles + (size_t)kb * B_BYTES + a * B_ATOM, &tmap_w, (kb * KA + a) * TC_BK, b_row, &full[kb]);
             }
         }
     }
     pdl_launch_dependents();
     pdl_wait();                                    // X (and the residual) come from the kernel before
     if (threadIdx.x == 0) VLRF_TRACE(trace, 3, (int)blockIdx.x, 1);
-    if (GR) {
-        if (threadIdx.x == 0) {
-            int n = 0;
-            for (int g = 0; g < gr.G; ++g) {
-                const int lo = gr.offsets ? gr.offsets[g] : 0, hi = gr.offsets ? gr.offsets[g + 1] : gr.rows;
-                for (int r = lo; r < hi && n < TC_GR_TAB; r += TC_BM) { gr_m0[n] = r; gr_end[n] = hi; gr_g[n] = g; ++n; }
+    if (GR && gr.offsets != nullptr) {
+        // a lane per group (32 groups at a time): its rows, and where its tiles begin among all tiles
+        if (warp == 0) {
+            int before = 0;
+            for (int g0 = 0; g0 < gr.G; g0 += 32) {
+                const int g = g0 + lane, lo = g < gr.G ? gr.offsets[g] : 0, hi = g < gr.G ? gr.offsets[g + 1] : 0;
+                const int mine = hi > lo ? (hi - lo + GR_ROWS - 1) / GR_ROWS : 0;
+                int upto = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += v; }
+                for (int i = 0; i < mine; ++i) {
+                    const int n = before + upto - mine + i;
+                    if (n < TC_GR_TAB) { gr_m0[n] = lo + i * GR_ROWS; gr_end[n] = hi; gr_g[n] = g; }
+                }
+                before += __shfl_sync(0xffffffffu, upto, 31);
             }
-            gr_count = n;
+            if (lane == 0) gr_count = min(before, TC_GR_TAB);
         }
         __syncthreads();
         n_tiles = tiles_n * gr_count;
@@ -161,17 +189,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         if (lane == 0) {
             uint32_t kc = 0;                       // k-blocks requested so far, over all tiles
             for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x) {
-                const int m0 = GR ? gr_m0[tile / tiles_n] : (SWAP ? tile * TC_BM : (tile / tiles_n) * TC_BM);
-                const int xk0 = GR ? gr_g[tile / tiles_n] * gr.x_gs : 0;                    // the group's columns of X
-                const int n0 = (SWAP ? 0 : (tile % tiles_n) * BN) + (GR ? gr_g[tile / tiles_n] * N : 0);   // rows of the stacked W
+                int a_row, b_row, xk0;
+                place(tile, a_row, b_row, xk0);
                 for (int kb = 0; kb < n_kb; ++kb, ++kc) {
                     const int s = kc % STAGES;
                     const uint32_t use = kc / STAGES;
                     if ((int)kc < early) {         // the weight half of this stage is already on its way
 #pragma unroll
                         for (int a = 0; a < KA; ++a) {
-                            if (SWAP) tma_load_2d(b_tiles + (size_t)s * B_BYTES + a * B_ATOM, &tmap_w, (kb * KA + a) * TC_BK, n0, &full[s]);
-                            else tma_load_2d(a_tiles + (size_t)s * A_BYTES + a * A_ATOM, &tmap_x, (kb * KA + a) * TC_BK, m0, &full[s]);
+                            if (SWAP) tma_load_2d(b_tiles + (size_t)s * B_BYTES + a * B_ATOM, &tmap_w, xk0 + (kb * KA + a) * TC_BK, b_row, &full[s]);
+                            else tma_load_2d(a_tiles + (size_t)s * A_BYTES + a * A_ATOM, &tmap_x, xk0 + (kb * KA + a) * TC_BK, a_row, &full[s]);
                         }
                         continue;
                     }
@@ -179,8 +206,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     tbar_expect_tx(&full[s], A_BYTES + B_BYTES);
 #pragma unroll
                     for (int a = 0; a < KA; ++a) {
-                        tma_load_2d(a_tiles + (size_t)s * A_BYTES + a * A_ATOM, &tmap_x, xk0 + (kb * KA + a) * TC_BK, m0, &full[s]);
-                        tma_load_2d(b_tiles + (size_t)s * B_BYTES + a * B_ATOM, &tmap_w, (kb * KA + a) * TC_BK, n0, &full[s]);
+                        tma_load_2d(a_tiles + (size_t)s * A_BYTES + a * A_ATOM, &tmap_x, (SWAP ? 0 : xk0) + (kb * KA + a) * TC_BK, a_row, &full[s]);
+                        tma_load_2d(b_tiles + (size_t)s * B_BYTES + a * B_ATOM, &tmap_w, (SWAP ? xk0 : 0) + (kb * KA + a) * TC_BK, b_row, &full[s]);
                     }
                 }
             }
@@ -220,6 +247,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         uint32_t tc = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++tc) {
             const uint32_t b = tc & 1;
+            // (SWAP without groups: m0 is the first column of Y, as W has the 128 rows; with groups: the first row, as without SWAP)
             const int m0 = GR ? gr_m0[tile / tiles_n] : (SWAP ? tile * TC_BM : (tile / tiles_n) * TC_BM);
             const int n0 = SWAP ? 0 : (tile % tiles_n) * BN;
             const int m_lim = GR ? gr_end[tile / tiles_n] : M;     // rows of the tile beyond it are not stored
@@ -242,7 +270,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + b * ACC_STRIDE + ((uint32_t)(q * 32) << 16);
             if (SWAP) {
-                const int n = m0 + q * 32 + lane;             // this thread's output column = row of W
+                const int n = (GR ? (tile % tiles_n) * TC_BM : m0) + q * 32 + lane;             // this thread's output column = row of W
+                const int r0 = GR ? m0 : 0;                   // the tile's first row of Y
                 const float bv = (bias && n < N) ? bias[n] : 0.f;
                 constexpr int PER_HALF = BN >= 32 ? BN / 2 : BN;     // with 16 columns only the first half works
                 if (BN >= 32 || half == 0) {
@@ -261,11 +290,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                                 constexpr int ACT = decltype(act_c)::value;
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) {
-                                    const int m = c0 + j;
-                                    if (m < M) {
+                                    const int m = r0 + c0 + j;
+                                    if (m < m_lim) {
                                         float x = apply_act_const<OT, ACT>(__uint_as_float(r[j]) + bv);
                                         if (residual) x += residual[(size_t)m * ldy + n];
-                                        ElemIO<OT>::store(Y + (size_t)m * ldy + n, x);
+                                        ElemIO<OT>::store(Yt + (size_t)m * ldy + n, x);
                                     }
                                 }
                             };
@@ -532,30 +561,43 @@ extern "C" int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias
 
 // ---- a weight matrix per group: experts over rows sorted by expert, or heads with columns of their own --------------
 namespace {
-template <int BN, int STAGES, typename OT>
+// Rows of a group's tile.  Few rows a group (a decode step's experts and heads): W is the 128-row operand and a tile has as many rows as
+// twice the average group fills (16, 32 or 64), so that a tile brings the weights and little else through the ring; with 128 rows of X beside
+// them, nearly all of other groups or none, it brought as many bytes again and filled half the ring with them (16 experts of 2,048 x 1,024 with 2 rows
+// each 24.1 -> 13.6 us inside a decode step, its down product 13.7 -> 8.3 us).  Heads' rows are known: the tile that takes them all.
+int gr_tile_rows(int rows, int G, bool by_offsets) {
+    const long long fill = by_offsets ? (2ll * rows + G - 1) / G : rows;
+    const int each = fill <= 16 ? 16 : fill <= 32 ? 32 : fill <= 64 ? 64 : TC_BM;
+    return by_offsets && (rows + each - 1) / each + G > TC_GR_TAB ? TC_BM : each;             // (the table holds so many)
+}
+long long gr_row_tiles(int rows, int G, bool by_offsets) {       // at most: one partly filled tile a group beyond the rows' own
+    const int each = gr_tile_rows(rows, G, by_offsets), n = (rows + each - 1) / each;
+    return by_offsets ? (long long)n + G : (long long)G * n;
+}
+
+template <int BN, int STAGES, typename OT, bool SWAP>
 int launch_tc_groups(const void* X, int ldx, const void* W, void* Y, int ldy, const TcGroups& gr, int N, int K, int act, int* dev_err,
                      cudaStream_t stream) {
-    CUtensorMap tx, tw;
+    CUtensorMap tx, tw;      // the rows of X, the rows of W
     const long long x_cols = gr.offsets ? K : (long long)(gr.G - 1) * gr.x_gs + K;
-    int st = vlrf_make_tmap_bf16(X, gr.rows, x_cols, ldx, TC_BM, TC_BK, &tx);
+    int st = vlrf_make_tmap_bf16(X, gr.rows, x_cols, ldx, SWAP ? BN : TC_BM, TC_BK, &tx);
     if (st != VLRF_OK) return st;
-    st = vlrf_make_tmap_bf16(W, (long long)gr.G * N, K, K, BN, TC_BK, &tw);
+    st = vlrf_make_tmap_bf16(W, (long long)gr.G * N, K, K, SWAP ? TC_BM : BN, TC_BK, &tw);
     if (st != VLRF_OK) return st;
     const size_t smem = 1024 + (size_t)STAGES * tc_atoms(BN) * (TC_BM * TC_BK * 2 + BN * TC_BK * 2) + (2 * STAGES + 4) * 8 + 16;
-    auto kern = gemm_tcgen05_kernel<BN, STAGES, OT, false, true>;
+    auto kern = gemm_tcgen05_kernel<BN, STAGES, OT, SWAP, true>;
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm_tcgen05_groups: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
         raised = true;
     }
-    // row tiles: at most one partly filled tile a group beyond the rows' own
-    const long long row_tiles = gr.offsets ? (gr.rows + TC_BM - 1) / TC_BM + gr.G : (long long)gr.G * ((gr.rows + TC_BM - 1) / TC_BM);
-    const long long tiles = row_tiles * ((N + BN - 1) / BN);
+    const int w_tile = SWAP ? TC_BM : BN;
+    const long long tiles = gr_row_tiles(gr.rows, gr.G, gr.offsets != nullptr) * ((N + w_tile - 1) / w_tile);
     const int sms = sm_count_cached();
     dim3 grid((unsigned)(tiles < sms ? tiles : sms));
-    cudaError_t e = launch_chained(kern, grid, dim3(TC_THREADS), smem, stream, tx, tw, (const float*)nullptr, (const float*)nullptr,
-                                   (OT*)Y, gr.rows, N, K, ldy, act, TcKvScatter{}, dev_err, vlrf_trace_buffer(), gr);
+    cudaError_t e = launch_chained(kern, grid, dim3(TC_THREADS), smem, stream, SWAP ? tw : tx, SWAP ? tx : tw, (const float*)nullptr,
+                                   (const float*)nullptr, (OT*)Y, gr.rows, N, K, ldy, act, TcKvScatter{}, dev_err, vlrf_trace_buffer(), gr);
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm_tcgen05_groups: %s", cudaGetErrorString(e));
     return vlrf_check_launch("gemm_tcgen05_groups");
 }
@@ -565,8 +607,7 @@ int launch_tc_groups(const void* X, int ldx, const void* W, void* Y, int ldy, co
 // 16-byte boundaries, and no more row tiles than its table holds.
 extern "C" int vlrf_gemm_tcgen05_groups_takes(int rows, int G, int N, int K, int ldx, int x_gs, int ldy, int y_gs, int by_offsets) {
     if (rows < 1 || G < 1 || N < 1 || K < 8 || K % 8 != 0 || ldx % 8 != 0 || x_gs % 8 != 0 || y_gs % 8 != 0 || ldy % 8 != 0) return 0;
-    const long long row_tiles = by_offsets ? (rows + TC_BM - 1) / TC_BM + G : (long long)G * ((rows + TC_BM - 1) / TC_BM);
-    return row_tiles <= TC_GR_TAB ? 1 : 0;
+    return gr_row_tiles(rows, G, by_offsets != 0) <= TC_GR_TAB ? 1 : 0;
 }
 
 // offsets != null: rows offsets[g] … offsets[g+1]−1 of X [rows][K] times W[g]ᵀ into the same rows of Y [rows][N]
@@ -582,10 +623,18 @@ extern "C" int vlrf_gemm_tcgen05_groups(const void* X, int ldx, int x_gs, const 
     VLRF_REQUIRE(dev_err != nullptr && (out_dtype == VLRF_BF16 || out_dtype == VLRF_F32), "gemm_tcgen05_groups: bad arguments");
     VLRF_REQUIRE((reinterpret_cast<uintptr_t>(Y) & 15) == 0, "gemm_tcgen05_groups: Y must start on a 16-byte boundary");
     const TcGroups gr{offsets, G, x_gs, y_gs, rows};
-    if (N <= 64) {
-        return out_dtype == VLRF_BF16 ? launch_tc_groups<64, 4, __nv_bfloat16>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream)
-                                      : launch_tc_groups<64, 4, float>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream);
-    }
-    return out_dtype == VLRF_BF16 ? launch_tc_groups<128, 3, __nv_bfloat16>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream)
-                                  : launch_tc_groups<128, 3, float>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream);
+#define GROUPS(BNV, ST, SW) (out_dtype == VLRF_BF16 ? launch_tc_groups<BNV, ST, __nv_bfloat16, SW>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream) \
+                                                    : launch_tc_groups<BNV, ST, float, SW>(X, ldx, W, Y, ldy, gr, N, K, act, dev_err, stream))
+    const int each = gr_tile_rows(rows, G, offsets != nullptr);
+    if (each == 16) return GROUPS(16, 5, true);
+    if (each == 32) return GROUPS(32, 5, true);
+    if (each == 64) return GROUPS(64, 4, true);
+    if (N <= 64) return GROUPS(64, 4, false);
+    // the width by rounds and the bytes of a round, as for one matrix; half of a group's last tile is taken to be empty
+    const long long row_tiles = offsets ? (rows + TC_BM - 1) / TC_BM + G / 2 : gr_row_tiles(rows, G, false);
+    const int sms = sm_count_cached();
+    auto cost = [&](int bn) { return ((row_tiles * ((N + bn - 1) / bn) + sms - 1) / sms) * (bn + 128); };
+    if (N > 128 && cost(256) < cost(128)) return GROUPS(256, 4, false);
+    return GROUPS(128, 3, false);
+#undef GROUPS
 }
