@@ -61,11 +61,20 @@ __device__ __forceinline__ uint32_t w_pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// 2^x for x ≤ 0 or so, in one instruction (−inf gives 0; results below the normal range are flushed to 0)
+__device__ __forceinline__ float w_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // DEC: a tile of at most 16 rows (a decode step: one token, the R heads of the group).  The four warps then share the
 // rows and deal the keys of every tile among themselves, 16 each, and their sums are merged through shared memory.
 // NST: stages of key/value tiles (NST − 1 tiles are under way while one is multiplied).
+// Prompts: CTAs of up to 160 padded columns are held to registers of which an SM has enough for three of them, and long tiles come first (16 heads of 64
+// and 96 over 2 x 1,024 tokens, a window of 512: 58.7 us with two CTAs an SM, a mask on every tile and short tiles first, now 33.3 us).
 template <int DKP, int DVP, bool DEC, int NST, int MAPS>
-__global__ void __launch_bounds__(MAPS * WM_WARPS * 32)
+__global__ void __launch_bounds__(MAPS * WM_WARPS * 32, !DEC && MAPS == 1 ? (DKP + DVP <= 160 ? 3 : 2) : 1)
 attn_window_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv_bfloat16* __restrict__ Kc,
                        const __nv_bfloat16* __restrict__ Vc, const int* __restrict__ block_table, int max_blocks,
                        const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_pos0,
@@ -87,7 +96,7 @@ attn_window_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv_
     const int warp_all = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int map = MAPS == 1 ? 0 : warp_all / WM_WARPS, warp = MAPS == 1 ? warp_all : warp_all % WM_WARPS;
     const int g = lane >> 2, t = lane & 3;
-    const int qt = blockIdx.x / n_split, part = blockIdx.x % n_split, hk = blockIdx.y, seq = blockIdx.z;
+    const int qt = DEC ? blockIdx.x / n_split : gridDim.x / n_split - 1 - blockIdx.x / n_split, part = blockIdx.x % n_split, hk = blockIdx.y, seq = blockIdx.z;
     pdl_wait();
     pdl_launch_dependents();
     const int R = H / Hkv, TPT = WM_ROWS / R;       // query heads a key/value head serves; tokens of a tile
@@ -188,41 +197,58 @@ attn_window_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv_
                     w_mma16816(s[j], qf[ks + 1][0], qf[ks + 1][1], qf[ks + 1][2], qf[ks + 1][3], b2, b3);
                 }
             }
-            const bool need_mask = window > 0 || (k_base + WM_BK - 1 > q_first);
+            // (tiles that lie wholly inside what every row sees, most of a long window's, need no mask; each of the other terms is
+            // one branch for the whole tile)
+            const bool need_mask = k_base + WM_BK - 1 > q_first || (window > 0 && k_base <= q_last - window);
             float m_new[2] = {m_run[0], m_run[1]};
 #pragma unroll
             for (int j = 0; j < NT_S; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = e >> 1;
-                    float v = s[j][e] * sl2;
-                    if (softcap > 0.f)      // c · tanh(x / c) = c · (1 − 2 / (2^(2x log2e / c) + 1)), in units of log2 e
-                        v = cap2 * (1.f - __fdividef(2.f, exp2f(v * cap_in) + 1.f));
-                    const int key = k_base + wkey + j * 8 + 2 * t + (e & 1);
-                    v = fmaf(slope2[r], (float)(key - q_row[r]), v);
-                    if (need_mask) {
-                        if (key > q_row[r] || (window > 0 && key <= q_row[r] - window && key >= keep_first)) v = -INFINITY;
+                for (int e = 0; e < 4; ++e) s[j][e] *= sl2;
+            if (softcap > 0.f) {            // c · tanh(x / c) = c · (1 − 2 / (2^(2x log2e / c) + 1)), in units of log2 e
+#pragma unroll
+                for (int j = 0; j < NT_S; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[j][e] = cap2 * (1.f - __fdividef(2.f, exp2f(s[j][e] * cap_in) + 1.f));
+            }
+            if (slopes != nullptr) {
+#pragma unroll
+                for (int j = 0; j < NT_S; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s[j][e] = fmaf(slope2[e >> 1], (float)(k_base + wkey + j * 8 + 2 * t + (e & 1) - q_row[e >> 1]), s[j][e]);
+            }
+            if (need_mask) {
+#pragma unroll
+                for (int j = 0; j < NT_S; ++j)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int key = k_base + wkey + j * 8 + 2 * t + (e & 1), at = q_row[e >> 1];
+                        if (key > at || (window > 0 && key <= at - window && key >= keep_first)) s[j][e] = -INFINITY;
                     }
-                    s[j][e] = v;
-                    m_new[r] = fmaxf(m_new[r], v);
-                }
+            }
+#pragma unroll
+            for (int j = 0; j < NT_S; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) m_new[e >> 1] = fmaxf(m_new[e >> 1], s[j][e]);
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
                 m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], 1));
                 m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], 2));
             }
-            float corr[2], sum[2] = {0.f, 0.f};
+            float corr[2], sum[2] = {0.f, 0.f}, m_use[2];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) corr[r] = (m_run[r] == -INFINITY) ? 0.f : exp2f(m_run[r] - m_new[r]);
+            for (int r = 0; r < 2; ++r) {
+                corr[r] = (m_run[r] == -INFINITY) ? 0.f : w_exp2(m_run[r] - m_new[r]);
+                m_use[r] = (m_new[r] == -INFINITY) ? 0.f : m_new[r];              // (a row that sees nothing yet: every weight is 0)
+            }
+            uint32_t pk[NT_S][2];           // the weights as the output product takes them: rounded to bfloat16, two neighbours together
 #pragma unroll
             for (int j = 0; j < NT_S; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = e >> 1;
-                    // (the weights are rounded to bfloat16 for the output product; their sum is taken of the rounded values)
-                    const float p = (m_new[r] == -INFINITY) ? 0.f : __bfloat162float(__float2bfloat16_rn(exp2f(s[j][e] - m_new[r])));
-                    s[j][e] = p;
-                    sum[r] += p;
+                for (int r = 0; r < 2; ++r) {
+                    pk[j][r] = w_pack_bf16(w_exp2(s[j][2 * r] - m_use[r]), w_exp2(s[j][2 * r + 1] - m_use[r]));
+                    sum[r] += __uint_as_float(pk[j][r] << 16);                    // (their sum is taken of the rounded values)
+                    sum[r] += __uint_as_float(pk[j][r] & 0xffff0000u);
                 }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -235,8 +261,7 @@ attn_window_mma_kernel(const __nv_bfloat16* __restrict__ q, int ldq, const __nv_
             for (int j = 0; j < NT_O; ++j) { o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1]; }
 #pragma unroll
             for (int kk = 0; kk < KS_PV; ++kk) {
-                const uint32_t a0 = w_pack_bf16(s[2 * kk][0], s[2 * kk][1]), a1 = w_pack_bf16(s[2 * kk][2], s[2 * kk][3]);
-                const uint32_t a2 = w_pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]), a3 = w_pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+                const uint32_t a0 = pk[2 * kk][0], a1 = pk[2 * kk][1], a2 = pk[2 * kk + 1][0], a3 = pk[2 * kk + 1][1];
 #pragma unroll
                 for (int j = 0; j < NT_O; j += 2) {
                     // transposed loads: (keys 16kk…+7, columns 8j…), (keys +8…, same columns), then the same for columns 8(j+1)…
