@@ -424,3 +424,24 @@ def test_rotation_and_append_of_aligned_rows(H, G, dk, dv, rot, interleaved, map
             assert float((x - y).abs().max()) <= (1e-6 if dtype == torch.float32 else 2.0 ** -8) * max(1.0, float(y.abs().max()))
             assert torch.equal(x == 7.0, y == 7.0)
     assert (got[0][0][2] == 7.0).all() and (got[1][1] == 7.0).all() and (got[0][1] != 7.0).any()
+
+
+@pytest.mark.parametrize("splits", [2, 8, 9, 32, 33, 40])
+def test_parts_of_a_context_meet(monkeypatch, splits):
+    """A decode step's contexts cut into numbers of parts around the eight that the merge asks for together and the 32 that a warp holds, parts
+    without a visible key among them, against the whole softmax in float64 (weights and results are rounded to bfloat16)."""
+    from vlrf_b200.csrc import ops
+    monkeypatch.setattr(ops, "window_decode_splits", lambda *a, **k: splits)
+    g = torch.Generator().manual_seed(splits)
+    H, G, dk, dv = 8, 2, 32, 136 - 8
+    lens = [700, 65, 1]
+    T = sum(lens)
+    rd = lambda *shape: torch.randn(*shape, generator=g).bfloat16().double()   # noqa: E731
+    q, k, v = rd(T, H, dk), rd(T, G, dk), rd(T, G, dv)
+    positions, slot_of = [p for n in lens for p in range(n)], [i for i, n in enumerate(lens) for _ in range(n)]
+    want, start = [], 0
+    for n in lens:
+        want.append(plain.window_attention(q[start:start + n], k[start:start + n], v[start:start + n], 0.3, 0)[-1])
+        start += n
+    got, _ = run_attention(q.float(), k.float(), v.float(), positions, slot_of, lens, G, 0.3, 0, None, torch.bfloat16, 0.6, 1, None)
+    close(got, 0.6 * torch.stack(want), 2e-2, f"{splits} parts")

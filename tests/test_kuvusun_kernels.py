@@ -496,3 +496,11 @@ def test_products_per_group_by_the_rows_of_a_group(counts, N, K):
 @pytest.mark.parametrize("M,H,N,K", [(16, 16, 256, 64), (17, 3, 136, 72), (33, 2, 128, 256), (65, 4, 320, 64), (2, 700, 8, 8)])
 def test_products_per_head_of_few_rows(M, H, N, K):
     test_products_per_head_on_the_tensor_cores(M, H, N, K)
+
+
+@pytest.mark.parametrize("splits", [9, 32, 33, 40])
+def test_parts_of_a_latent_context_meet(splits, monkeypatch):
+    """Numbers of parts around the eight that the merge asks for together and the 32 that a warp holds."""
+    from vlrf_b200.csrc import ops
+    monkeypatch.setattr(ops, "latent_decode_splits", lambda *a, **k: splits)
+    test_tensor_core_attention_over_latent_rows(256, 32, 16, 1, monkeypatch)

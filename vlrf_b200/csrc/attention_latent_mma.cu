@@ -285,13 +285,15 @@ attn_latent_mma_kernel(const __nv_bfloat16* __restrict__ qp, int ld_q, const __n
     }
 }
 
-// the parts of every (token, head) into one: weights exp(m_s − max m) on the parts' unnormalised sums
+// The parts of every (token, head) into one: weights exp(m_s − max m) on the parts' unnormalised sums, in the order of the parts.  Lane s
+// of every warp reads part s's maximum and denominator, and a thread asks for its column of eight parts at a time, beside them: two round
+// trips in all, where three passes went part after part (a decode step of four such layers, 16 tokens of 16 heads, 394 -> 387 us).
 __global__ void __launch_bounds__(128)
 attn_latent_merge_kernel(const float* __restrict__ partials, const int* __restrict__ tok_slot, __nv_bfloat16* __restrict__ out,
                          int ld_out, int H, int C, int n_split, const float* __restrict__ sink, float out_scale) {
     pdl_wait();                 // chained launch: nothing is read before the kernels ahead have finished
     pdl_launch_dependents();
-    const int tok = blockIdx.x, h = blockIdx.y;
+    const int tok = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
     const int hgs = (H + 15) / 16, hg = h >> 4, r = h & 15;
     __nv_bfloat16* dst = out + (size_t)tok * ld_out + (size_t)h * C;
     if (tok_slot[tok] < 0) {
@@ -300,21 +302,32 @@ attn_latent_merge_kernel(const float* __restrict__ partials, const int* __restri
     }
     const float* base = partials + ((size_t)tok * hgs + hg) * n_split * 16 * (C + 2) + (size_t)r * (C + 2);
     const size_t stride = (size_t)16 * (C + 2);
-    float m = sink != nullptr ? sink[h] : -INFINITY;
-    for (int s = 0; s < n_split; ++s) m = fmaxf(m, base[s * stride + C]);
-    float denom = sink != nullptr ? expf(sink[h] - m) : 0.f;
-    for (int s = 0; s < n_split; ++s) {
-        const float ms = base[s * stride + C];
-        if (ms != -INFINITY) denom += expf(ms - m) * base[s * stride + C + 1];
-    }
+    auto maximum = [&](int s) { return s < n_split ? base[s * stride + C] : -INFINITY; };
+    const float ms = maximum(lane), ls = lane < n_split ? base[lane * stride + C + 1] : 0.f;
+    const float sk = sink != nullptr ? sink[h] : -INFINITY;
+    float m = fmaxf(sk, ms);
+    for (int s = lane + 32; s < n_split; s += 32) m = fmaxf(m, maximum(s));
+    m = warp_max(m);
+    auto weight = [&](float ms_of) { return ms_of != -INFINITY ? expf(ms_of - m) : 0.f; };
+    const float f = weight(ms);                                    // of part `lane`; those behind the 32nd are read again where they are used
+    float denom = sink != nullptr ? expf(sk - m) : 0.f;
+    for (int s = 0; s < n_split; ++s)
+        denom = s < 32 ? fmaf(__shfl_sync(0xffffffffu, f, s), __shfl_sync(0xffffffffu, ls, s), denom) : fmaf(weight(maximum(s)), base[s * stride + C + 1], denom);
     const float inv = denom > 0.f ? out_scale / denom : 0.f;
-    for (int c = threadIdx.x; c < C; c += 128) {
+    for (int c0 = 0; c0 < C; c0 += 128) {                          // (all lanes stay: they hold the parts' weights)
+        const int c = c0 + threadIdx.x;
         float v = 0.f;
-        for (int s = 0; s < n_split; ++s) {
-            const float ms = base[s * stride + C];
-            if (ms != -INFINITY) v += expf(ms - m) * base[s * stride + c];
+        for (int s0 = 0; s0 < n_split; s0 += 8) {
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = s0 + j < n_split && c < C ? base[(s0 + j) * stride + c] : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float first = __shfl_sync(0xffffffffu, f, (s0 + j) & 31), w = s0 < 32 ? first : weight(maximum(s0 + j));
+                if (s0 + j < n_split && w != 0.f) v = fmaf(w, x[j], v);      // (a part that saw no row left nothing to add)
+            }
         }
-        dst[c] = __float2bfloat16_rn(v * inv);
+        if (c < C) dst[c] = __float2bfloat16_rn(v * inv);
     }
 }
 
