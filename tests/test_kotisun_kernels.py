@@ -445,3 +445,42 @@ def test_parts_of_a_context_meet(monkeypatch, splits):
         start += n
     got, _ = run_attention(q.float(), k.float(), v.float(), positions, slot_of, lens, G, 0.3, 0, None, torch.bfloat16, 0.6, 1, None)
     close(got, 0.6 * torch.stack(want), 2e-2, f"{splits} parts")
+
+
+@pytest.mark.parametrize("Hs,P,N,G", [(4, 64, 64, 2), (3, 4, 16, 3), (2, 132, 34, 1), (32, 128, 128, 8), (2, 20, 512, 1)])
+def test_recurrence_of_one_token(Hs, P, N, G):
+    """The decode step's kernel from both copies of the state, a padding row, states of rows and columns beside its runs, against the
+    float64 step: a state is one product and one sum of float32 away, a result a sum of up to 512 of them over 256 threads."""
+    import types
+
+    from vlrf_b200.csrc import ops
+    g = torch.Generator().manual_seed(Hs * 1000 + P * 10 + N)
+    inner, channels, state_row = Hs * P, Hs * P + 2 * G * N, Hs * N * P + 8 + (-Hs * N * P) % 4
+    pos0, slots = [0, 3, 4, 7, 0, 128], [6, 0, 3, 5, -1, 2]
+    T = len(slots)
+    xbc, dt = torch.randn(T, channels, generator=g), torch.randn(T, Hs, generator=g) * 2.0
+    dt_bias, a_log, D = torch.randn(Hs, generator=g), torch.linspace(-6.0, 2.5, Hs), torch.randn(Hs, generator=g)
+    state = torch.full((8, 2, state_row), float("nan"))
+    for s, p in zip(slots, pos0):
+        if s >= 0:
+            state[s, p & 1, :Hs * N * P] = torch.randn(Hs * N * P, generator=g)
+    proj = dev(torch.cat([torch.randn(T, 3, generator=g), dt], 1))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)   # noqa: E731
+    ctx = types.SimpleNamespace(n_tokens=T, n_seqs=T, seq_slot=i32(slots), seq_start=i32(list(range(T + 1))), seq_pos0=i32(pos0), max_new=1,
+                                act_dtype=torch.bfloat16)
+    assert ops.ssd_step_takes(torch.bfloat16, ctx, Hs, G, N, P, channels, state_row)
+    assert not ops.ssd_step_takes(torch.float32, ctx, Hs, G, N, P, channels, state_row)
+    st, y = state.to(DEV), torch.full((T, inner), float("nan"), device=DEV)
+    ops.ssd_scan_step(dev(xbc), proj, 3, dev(dt_bias), dev(a_log), dev(D), st, ctx, y, Hs, G, N, P)
+    for t, (s, p) in enumerate(zip(slots, pos0)):
+        if s < 0:
+            assert torch.isnan(y[t]).all()
+            continue
+        x, B, C = xbc[t, :inner].double().reshape(Hs, P), xbc[t, inner:inner + G * N].double().reshape(G, N), xbc[t, inner + G * N:].double().reshape(G, N)
+        B, C = (b.repeat_interleave(Hs // G, 0) for b in (B, C))
+        step = plain.softplus(dt[t].double() + dt_bias.double())
+        S = state[s, p & 1, :Hs * N * P].double().reshape(Hs, N, P)
+        S = torch.exp(-torch.exp(a_log.double()) * step)[:, None, None] * S + (step[:, None] * B)[:, :, None] * x[:, None, :]
+        close(st[s, (p + 1) & 1, :Hs * N * P].reshape(Hs, N, P), S, 1e-6, f"state of slot {s}")
+        close(y[t].reshape(Hs, P), (S * C[:, :, None]).sum(1) + D.double()[:, None] * x, 3e-6, f"result of slot {s}")
+        assert torch.equal(st[s, p & 1].cpu().nan_to_num(7.0), state[s, p & 1].nan_to_num(7.0))

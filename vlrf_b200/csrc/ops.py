@@ -1253,10 +1253,36 @@ def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_
          ctx.max_new, n_heads, n_groups, n_state, p, _stream())
 
 
+def ssd_step_takes(dtype: torch.dtype, ctx, n_heads: int, n_groups: int, n_state: int, p: int, channels: int, state_row: int) -> bool:
+    """Whether a step's state-space recurrence runs on the decode step's kernel: one token a sequence, in the bfloat16 engine (the 32-bit
+    one keeps to one order of its sums for prompts and single tokens)."""
+    if dtype != torch.bfloat16 or ctx.max_new != 1:
+        return False
+    from . import library
+    return bool(library().vlrf_ssd_step_takes(n_heads, n_groups, n_state, p, channels, state_row))
+
+
+def ssd_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_heads: int, n_groups: int, n_state: int, p: int) -> None:
+    """`ssd_scan` of a decode step (see the kernel library's header)."""
+    _dev(xbc, "xbc", torch.float32); _rows(proj, "proj", torch.float32); _dev(state, "state", torch.float32); _dev(y, "y", torch.float32)
+    for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
+        _dev(t, name, torch.float32)
+        if t.numel() != n_heads:
+            raise KernelError(f"ssd_step: {name} has one number per head")
+    if y.shape[1] != n_heads * p or state.dim() != 3 or state.shape[1] != 2:
+        raise KernelError("ssd_step: sizes do not match")
+    call("vlrf_ssd_step", _ptr(xbc), xbc.shape[1], _ptr(proj), proj.stride(0), dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state),
+         state.shape[2], _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(y), ctx.n_seqs, n_heads, n_groups, n_state, p,
+         _stream())
+
+
 def ssd_scan_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_heads: int, n_groups: int, n_state: int, p: int) -> None:
     """The recurrence of a step with the kernel that suits it."""
     if ssd_chunks_takes(ctx.act_dtype, ctx, n_heads, n_groups, n_state, p, xbc.shape[1], state.shape[2]):
         ssd_chunks(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx, y, n_heads, n_groups, n_state, p)
+        return
+    if ssd_step_takes(ctx.act_dtype, ctx, n_heads, n_groups, n_state, p, xbc.shape[1], state.shape[2]):
+        ssd_step(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx, y, n_heads, n_groups, n_state, p)
         return
     ssd_scan(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, ctx.n_seqs, n_heads,
              n_groups, n_state, p, ctx.max_new)

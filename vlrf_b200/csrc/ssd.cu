@@ -21,6 +21,7 @@
 //                   C-weighted sums of the slices meet in shared memory once per batch;
 //                   serves prompts and single tokens alike, with the same arithmetic in the same order (long prompts of the
 //                   bfloat16 engine go to state_chunks.cu)
+//   ssd_step        one token a sequence, for the bfloat16 engine: the same state, sums over its rows in another order
 //   ssd_gate_norm   y · (z·sigmoid(z)), RMS norm in equal groups, weight, a factor; rounded to the activation dtype
 #include "common.cuh"
 
@@ -275,6 +276,70 @@ ssd_scan_kernel(const float* __restrict__ xbc, int channels, const float* __rest
         if (col && n0 + k < N) S_out[(size_t)(n0 + k) * P + p] = S[k];
 }
 
+// A decode step: one token a sequence.  A thread has a quad of columns and ROWS rows of a head's state, rows rg, rg + RG, … (RG = 256 / CQ, CQ
+// quads of columns a CTA), all asked for at once, beside the token's inputs.  What is left is to read and write the states; the kernel above
+// goes through shared memory and three barriers, a state's numbers one by one (a decode step of four such layers, 8 tokens of 32 heads of
+// 128 x 128, 407 -> 403 us).
+template <int ROWS>
+__global__ void __launch_bounds__(256)
+ssd_step_kernel(const float* __restrict__ xbc, int channels, const float* __restrict__ proj, int ld, int dt_off, const float* __restrict__ dt_bias,
+                const float* __restrict__ a_log, const float* __restrict__ Dv, float* __restrict__ state, int state_row,
+                const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_pos0, float* __restrict__ y,
+                int Hs, int G, int N, int P, int PB, int CQ) {
+    __shared__ float4 part_sm[256];
+    const int h = blockIdx.x / PB, pb = blockIdx.x - h * PB, s = blockIdx.y;
+    const float a = -expf(a_log[h]), dtb = dt_bias[h], dh = Dv[h];       // (weights: not from the kernel ahead)
+    pdl_wait();
+    pdl_launch_dependents();
+    const int slot = seq_slot[s], row = seq_start[s], n = seq_start[s + 1] - row, pos0 = seq_pos0[s];
+    if (slot < 0 || n != 1) return;
+    const int cq = threadIdx.x % CQ, rg = threadIdx.x / CQ, RG = 256 / CQ, p = (pb * CQ + cq) * 4;
+    const bool col = p < P;
+    const size_t at = (size_t)h * N * P + p;
+    const float* S_in = state + ((size_t)slot * 2 + (pos0 & 1)) * state_row + at;
+    float* S_out = state + ((size_t)slot * 2 + ((pos0 + 1) & 1)) * state_row + at;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 S[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) S[k] = col && rg + k * RG < N ? *reinterpret_cast<const float4*>(S_in + (size_t)(rg + k * RG) * P) : zero;
+    const float* in = xbc + (size_t)row * channels;
+    const float* bc = in + Hs * P + (h / (Hs / G)) * N;
+    const float4 x = col ? *reinterpret_cast<const float4*>(in + h * P + p) : zero;
+    float b[ROWS], c[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        const int r = rg + k * RG;
+        b[k] = r < N ? bc[r] : 0.f;
+        c[k] = r < N ? bc[G * N + r] : 0.f;
+    }
+    const float dt = softplus_f(proj[(size_t)row * ld + dt_off + h] + dtb), decay = expf(a * dt);
+    const float4 dx = make_float4(dt * x.x, dt * x.y, dt * x.z, dt * x.w);
+    float4 sum = zero;
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+        S[k].x = fmaf(decay, S[k].x, b[k] * dx.x); S[k].y = fmaf(decay, S[k].y, b[k] * dx.y);
+        S[k].z = fmaf(decay, S[k].z, b[k] * dx.z); S[k].w = fmaf(decay, S[k].w, b[k] * dx.w);
+        sum.x = fmaf(S[k].x, c[k], sum.x); sum.y = fmaf(S[k].y, c[k], sum.y);
+        sum.z = fmaf(S[k].z, c[k], sum.z); sum.w = fmaf(S[k].w, c[k], sum.w);
+        if (col && rg + k * RG < N) *reinterpret_cast<float4*>(S_out + (size_t)(rg + k * RG) * P) = S[k];
+    }
+    part_sm[threadIdx.x] = sum;
+    __syncthreads();
+    // a warp a column quad adds the row groups, each lane a run of them, then the lanes
+    for (int q = threadIdx.x >> 5; q < CQ; q += 8) {
+        const int lane = threadIdx.x & 31;
+        float4 t = zero;
+        for (int r = lane; r < RG; r += 32) { const float4 v = part_sm[r * CQ + q]; t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w; }
+        t.x = warp_sum(t.x); t.y = warp_sum(t.y); t.z = warp_sum(t.z); t.w = warp_sum(t.w);
+        const int pq = (pb * CQ + q) * 4;
+        if (lane == 0 && pq < P) {
+            const float4 own = *reinterpret_cast<const float4*>(in + h * P + pq);
+            *reinterpret_cast<float4*>(y + (size_t)row * Hs * P + h * P + pq) =
+                make_float4(fmaf(dh, own.x, t.x), fmaf(dh, own.y, t.y), fmaf(dh, own.z, t.z), fmaf(dh, own.w, t.w));
+        }
+    }
+}
+
 // (asked of the driver once per instantiation and size: more than 48 KB of shared memory is opt-in)
 template <int R, bool V> void scan_allow_smem(size_t smem) {
     static size_t allowed = 48 * 1024;
@@ -428,6 +493,40 @@ extern "C" int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, 
     else { if (vec) { GO(32, true); } else { GO(32, false); } }
 #undef GO
     return vlrf_check_launch("ssd_scan");
+}
+
+// Whether the decode step's kernel takes these sizes: quads of columns on 16 bytes, at most 512 rows.
+extern "C" int vlrf_ssd_step_takes(int H, int G, int N, int P, int channels, int state_row) {
+    return (H > 0 && G > 0 && H % G == 0 && N > 0 && N <= 512 && P > 0 && P % 4 == 0 && channels % 4 == 0 && state_row % 4 == 0 &&
+            channels == H * P + 2 * G * N) ? 1 : 0;
+}
+
+extern "C" int vlrf_ssd_step(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
+                             const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
+                             float* y, int n_seqs, int Hs, int G, int N, int P, cudaStream_t stream) {
+    VLRF_REQUIRE(vlrf_ssd_step_takes(Hs, G, N, P, channels, state_row), "ssd_step: a state of %d by %d or the rows' strides are not taken", N, P);
+    VLRF_REQUIRE(n_seqs >= 0 && n_seqs <= 65535 && dt_off >= 0 && dt_off + Hs <= ld && (size_t)Hs * N * P <= (size_t)state_row,
+                 "ssd_step: the rows do not hold what the sizes say");
+    VLRF_REQUIRE(((reinterpret_cast<uintptr_t>(xbc) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(y)) & 15) == 0,
+                 "ssd_step: misaligned rows");
+    if (n_seqs == 0) return VLRF_OK;
+    // columns a CTA: few enough that a thread has at most 16 rows, and that small steps still reach every SM
+    int sms = 148, devi = 0;
+    cudaGetDevice(&devi);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devi);
+    int CQ = 32;
+    while (CQ > 1 && ((N + 256 / CQ - 1) / (256 / CQ) > 16 || CQ >= 2 * (P / 4))) CQ /= 2;
+    while (CQ > 8 && (long long)Hs * ((P / 4 + CQ - 1) / CQ) * n_seqs < sms) CQ /= 2;
+    const int PB = (P / 4 + CQ - 1) / CQ, rows = (N + 256 / CQ - 1) / (256 / CQ);
+    const dim3 grid(Hs * PB, n_seqs);
+#define GO(R) launch_chained(ssd_step_kernel<R>, grid, dim3(256), (size_t)0, stream, xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, \
+                             seq_slot, seq_start, seq_pos0, y, Hs, G, N, P, PB, CQ)
+    if (rows <= 2) GO(2);
+    else if (rows <= 4) GO(4);
+    else if (rows <= 8) GO(8);
+    else GO(16);
+#undef GO
+    return vlrf_check_launch("ssd_step");
 }
 
 extern "C" int vlrf_ssd_gate_norm(const float* y, const float* proj, int ld, int z_off, const float* w, void* out, int out_dtype,

@@ -311,6 +311,11 @@ int vlrf_ssd_conv(const float* proj, int ld, int x_off, const float* w, const fl
 int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                   const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
                   float* y, int n_seqs, int max_new, int Hs, int G, int N, int P, cudaStream_t stream);
+// One token a sequence (decode steps): states of any number of rows up to 512, P a multiple of 4, rows on 16 bytes.
+int vlrf_ssd_step_takes(int H, int G, int N, int P, int channels, int state_row);
+int vlrf_ssd_step(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
+                  const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
+                  float* y, int n_seqs, int Hs, int G, int N, int P, cudaStream_t stream);
 // The same over prompts on the tensor cores, 64 tokens at a time (state_chunks.cu): every float32 operand in three bfloat16 parts.
 // scratch float32 (vlrf_ssd_chunks_scratch numbers, n_tokens the step's rows).  N 16, 32, 64 or 128, P a multiple of 4.
 int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, int state_row);
