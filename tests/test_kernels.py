@@ -639,6 +639,15 @@ def test_attention_prefill_tensor_cores(monkeypatch, kernel, H, Hkv, dh, seqs, w
         assert rel_err(mine, want[i]) < 1.5e-2, (i, p0, n)
 
 
+@pytest.mark.parametrize("kernel", ["tcgen05", "tcgen05_parts2"])
+@pytest.mark.parametrize("seqs", [[(0, 1013), (0, 517), (0, 31), (300, 1), (300, 1)], [(0, 128), (0, 129), (5, 127), (0, 1), (64, 256)],
+                                  [(3, 1)] * 31 + [(0, 260)], [(3, 1)] * 32 + [(0, 260)], [(0, 1), (0, 8100), (7, 9)], [(0, 8300), (0, 1)]])
+def test_attention_prefill_lists_the_tiles_that_exist(monkeypatch, kernel, seqs):
+    """Sequences of unequal lengths, whose tiles are listed instead of given a place each: around the edges of a tile, the 32 sequences and
+    the 64 tiles of the longest up to which they are listed."""
+    test_attention_prefill_tensor_cores(monkeypatch, kernel, 2, 1, 64, seqs, 0)
+
+
 def test_kv_append_writes_each_token_where_its_slot_says():
     from vlrf_b200.csrc import ops
     Hkv, dh, T = 3, 16, 70

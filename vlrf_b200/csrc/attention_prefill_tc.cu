@@ -75,7 +75,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                        int max_blocks, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                        const int* __restrict__ seq_pos0, __nv_bfloat16* __restrict__ out, int ld_out, int H, int Hkv,
                        float scale, int window, int n_parts, float* __restrict__ partials, int* __restrict__ counters,
-                       int* __restrict__ dev_err, long long* trace) {
+                       int n_tiles, int listed, int* __restrict__ dev_err, long long* trace) {
     extern __shared__ unsigned char ft_raw[];
     // (stations of the time stamps, kind 4: 0 the CTA begins, 1 the kernel ahead has finished, 6 the CTA is done)
     const int tcta = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
@@ -97,9 +97,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // z is the slowest index of the order in which CTAs are started: first parts before second parts, so that the
-    // CTAs without work (short tiles have fewer parts) come last, and within a part long tiles first
-    const int n_tiles = gridDim.z / n_parts;
-    const int part = blockIdx.z / n_tiles, qt = n_tiles - 1 - blockIdx.z % n_tiles, h = blockIdx.x, seq = blockIdx.y;
+    // CTAs without work (short tiles have fewer parts) come last, and within a part long tiles first.  n_tiles: of the longest sequence.
+    // listed: y counts the tiles that exist, the last tiles of all sequences first, where a place for every tile that the longest sequence
+    // has would leave most CTAs without work (a CTA that only sets itself up and leaves takes a place on an SM for some 3 us).
+    int part = blockIdx.z / n_tiles, qt = n_tiles - 1 - blockIdx.z % n_tiles, seq = blockIdx.y;
+    const int h = blockIdx.x;
 
     // set-up that reads nothing of the kernel ahead
     if (threadIdx.x == 0) {
@@ -122,6 +124,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     pdl_wait();
     if (threadIdx.x == 0) VLRF_TRACE(trace, 4, tcta, 1);
     pdl_launch_dependents();
+    if (listed > 0) {                                // (at most 32 sequences: a lane each, every warp for itself)
+        part = blockIdx.z;
+        const int mine = lane < listed && seq_slot[lane] >= 0 ? (seq_start[lane + 1] - seq_start[lane] + FT_BQ - 1) / FT_BQ : 0;
+        int left = blockIdx.y;
+        seq = -1;
+        for (qt = n_tiles - 1; qt >= 0; --qt) {
+            const unsigned has = __ballot_sync(0xffffffffu, mine > qt);
+            const int n = __popc(has);
+            if (left < n) {
+                seq = __ffs(__ballot_sync(0xffffffffu, mine > qt && __popc(has & ((1u << lane) - 1u)) == left)) - 1;
+                break;
+            }
+            left -= n;
+        }
+    }
+    const bool exists = seq >= 0;                    // (fewer tiles than places)
+    seq = max(seq, 0);
+    qt = max(qt, 0);
     const int row0 = seq_start[seq], row_end = seq_start[seq + 1], slot = seq_slot[seq], pos0 = seq_pos0[seq];
     const int n_new = row_end - row0;
     const int hk = h / (H / Hkv);
@@ -132,7 +152,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const int n_kb = kb_last - kb_first + 1;
     // the tile's key blocks are dealt to tile_parts CTAs; the others of its n_parts have nothing to do
     const int tile_parts = max(1, min(n_parts, (n_kb + FT_PART_BLOCKS - 1) / FT_PART_BLOCKS));
-    const bool active = qt * FT_BQ < n_new && slot >= 0 && part < tile_parts;     // uniform over the CTA
+    const bool active = exists && qt * FT_BQ < n_new && slot >= 0 && part < tile_parts;     // uniform over the CTA
     const int my_first = kb_first + part * n_kb / tile_parts;
     const int my_n = active ? kb_first + (part + 1) * n_kb / tile_parts - my_first : 0;
     const int cb_last = q_last / FT_CB;                              // last cache block that holds a visible key
@@ -450,10 +470,14 @@ extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const vo
     }
     const long long tiles = (max_new + FT_BQ - 1) / FT_BQ;
     VLRF_REQUIRE(tiles * n_parts <= 65535, "attn_prefill_tc: %lld tiles of %d parts are too many for one launch", tiles, n_parts);
-    dim3 grid(H, n_seqs, (unsigned)(tiles * n_parts));
+    // The tiles that exist are at most n_tokens / 128 + n_seqs: with sequences of unequal lengths far fewer than every sequence times the
+    // longest's (five prompts of 1,013 to 31 tokens and three single tokens, 25 heads: 22 of 64; 42.8 -> 31 us).
+    const long long places = (long long)n_tokens / FT_BQ + n_seqs;
+    const int listed = n_seqs > 1 && n_seqs <= 32 && tiles <= 64 && places < tiles * n_seqs ? n_seqs : 0;
+    dim3 grid(H, listed ? (unsigned)places : n_seqs, (unsigned)(listed ? n_parts : tiles * n_parts));
     cudaError_t e = launch_chained(attn_prefill_tc_kernel, grid, dim3(FT_THREADS), smem, stream, tq, tk, tv, q_off, block_table,
                                    max_blocks, seq_slot, seq_start, seq_pos0, (__nv_bfloat16*)out, ld_out, H, Hkv, scale,
-                                   window, n_parts, partials, counters, dev_err, vlrf_trace_buffer());
+                                   window, n_parts, partials, counters, (int)tiles, listed, dev_err, vlrf_trace_buffer());
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "attn_prefill_tc: %s", cudaGetErrorString(e));
     return vlrf_check_launch("attn_prefill_tc");
 }
