@@ -778,3 +778,33 @@ def test_penalties_and_ngram_block():
         assert (np.isfinite(got[i]) == fin).all()
         assert np.allclose(got[i][fin], want[fin], rtol=1e-6, atol=1e-6)
     assert np.array_equal(got[0], lg[0].numpy())      # nothing generated yet: untouched
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-6), (torch.bfloat16, 1e-2)])
+@pytest.mark.parametrize("dh,lens,window", [(64, [1, 7, 8, 9, 31, 32, 33, 64, 65, 130], 0), (64, [70, 129], 40), (16, [9, 40], 0), (48, [33], 0), (80, [66], 5), (256, [37], 0)])
+def test_general_attention_at_the_edges_of_its_runs(dh, lens, window, dtype, tol):
+    """Contexts around the 32 keys of a chunk and the eight values that are asked for together, head sizes with and without a kernel of their own;
+    the cache is NaN where nothing was written."""
+    from vlrf_b200.csrc import ops
+    H, Hkv, T = 4, 2, sum(lens)
+    qkv = randn(T, (H + 2 * Hkv) * dh, seed=dh).to(dtype)
+    n_max = max((n + 63) // 64 for n in lens)
+    table = torch.arange(len(lens) * n_max, dtype=torch.int32).flip(0).view(len(lens), n_max).contiguous()
+    kc = torch.full((len(lens) * n_max, Hkv, 64, dh), float("nan"), dtype=dtype, device=DEV)
+    vc = torch.full_like(kc, float("nan"))
+    slot = torch.tensor([i for i, n in enumerate(lens) for _ in range(n)], dtype=torch.int32, device=DEV)
+    pos = torch.tensor([p for n in lens for p in range(n)], dtype=torch.int32, device=DEV)
+    out, e = torch.full((T, H * dh), float("nan"), dtype=dtype, device=DEV), err_word()
+    x, td = qkv.to(DEV), table.to(DEV)
+    ops.kv_append(x, H * dh, (H + Hkv) * dh, kc, vc, td, slot, pos, T, Hkv, dh, e)
+    ops.attention_generic(x, 0, kc, vc, td, slot, pos, out, T, H, Hkv, dh, 0.2, window, e)
+    assert int(e.item()) == 0
+    at = 0
+    for n in lens:
+        rows = qkv[at:at + n].float()
+        q = rows[:, :H * dh].reshape(n, H, dh).permute(1, 0, 2)
+        k, v = (rows[:, o:o + Hkv * dh].reshape(n, Hkv, dh).permute(1, 0, 2) for o in (H * dh, (H + Hkv) * dh))
+        want = plain_attention(q, k, v, 0.2, window)
+        got = out[at:at + n].float().cpu().reshape(n, H, dh).permute(1, 0, 2)
+        assert torch.isfinite(got).all() and rel_err(got, want) < tol, (n, dh)
+        at += n

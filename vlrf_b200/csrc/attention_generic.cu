@@ -19,6 +19,8 @@ __global__ void kv_append_kernel(const ET* __restrict__ qkv, int ld, int k_off, 
                                  const int* __restrict__ block_table, int max_blocks,
                                  const int* __restrict__ tok_slot, const int* __restrict__ tok_pos,
                                  int Hkv, int dh, int BT, int* __restrict__ dev_err) {
+    pdl_wait();                 // chained launch: nothing is read before the kernels ahead have finished
+    pdl_launch_dependents();
     const int t = blockIdx.x;
     const int slot = tok_slot[t];
     if (slot < 0) return;  // padding row
@@ -39,38 +41,52 @@ __global__ void kv_append_kernel(const ET* __restrict__ qkv, int ld, int k_off, 
     }
 }
 
-template <typename ET> struct Vec16;
-template <> struct Vec16<float> {
-    static constexpr int N = 4;
-    static __device__ __forceinline__ void load(const float* p, float* out) {
-        const float4 v = *reinterpret_cast<const float4*>(p);
-        out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
-    }
+// Loads that stay where they are written: left to itself the compiler sinks them to their uses, one wait each, to save registers.
+__device__ __forceinline__ void load_now(const float* p, float (&v)[4]) {
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void load_now(const __nv_bfloat16* p, uint4& v) {
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+}
+__device__ __forceinline__ void load_now(const float* p, float& v) { asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); }
+__device__ __forceinline__ void load_now(const __nv_bfloat16* p, float& v) {
+    unsigned short u;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(u) : "l"(p));
+    v = __uint_as_float((uint32_t)u << 16);
+}
+template <typename ET> struct Piece;                       // 16 bytes as they arrive
+template <> struct Piece<float> {
+    float v[4];
+    __device__ __forceinline__ void load(const float* p) { load_now(p, v); }
+    __device__ __forceinline__ float at(int i) const { return v[i]; }
 };
-template <> struct Vec16<__nv_bfloat16> {
-    static constexpr int N = 8;
-    static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* out) {
-        const uint4 v = *reinterpret_cast<const uint4*>(p);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            out[2 * i] = __uint_as_float(w[i] << 16);
-            out[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-        }
+template <> struct Piece<__nv_bfloat16> {
+    uint4 v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { load_now(p, v); }
+    __device__ __forceinline__ float at(int i) const {
+        const uint32_t w = i < 2 ? v.x : i < 4 ? v.y : i < 6 ? v.z : v.w;
+        return __uint_as_float((i & 1) ? w & 0xffff0000u : w << 16);
     }
 };
 
 constexpr int ATT_WARPS = 4;
 constexpr int MAX_DH = 256;
 
-template <typename ET>
+// DH: the head size where it is known when compiling (0: the argument).  A key's row is asked for in runs of eight pieces of 16 bytes and the
+// values of eight keys together, ahead of the sums that take them one after another: with a wait for every piece and every key 240 tokens of 12
+// float32 heads of 64 took 67 us a layer, now 35 us.
+template <typename ET, int DH>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 attn_generic_kernel(const ET* __restrict__ qkv, int ld, int q_off, const ET* __restrict__ Kc,
                     const ET* __restrict__ Vc, const int* __restrict__ block_table, int max_blocks,
                     const int* __restrict__ tok_slot, const int* __restrict__ tok_pos,
-                    ET* __restrict__ out, int ld_out, int H, int Hkv, int dh, int BT, float scale,
+                    ET* __restrict__ out, int ld_out, int H, int Hkv, int dh_arg, int BT, float scale,
                     int window, int* __restrict__ dev_err) {
-    extern __shared__ float q_sm[];  // [ATT_WARPS][dh]
+    extern __shared__ __align__(16) float q_sm[];  // [ATT_WARPS][dh]
+    constexpr int ND = DH > 0 ? (DH + 31) / 32 : MAX_DH / 32, N = 16 / (int)sizeof(ET);
+    const int dh = DH > 0 ? DH : dh_arg;
+    pdl_wait();                 // chained launch: nothing is read before the kernels ahead have finished
+    pdl_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x;
     const int h = blockIdx.y * ATT_WARPS + warp;
@@ -83,9 +99,9 @@ attn_generic_kernel(const ET* __restrict__ qkv, int ld, int q_off, const ET* __r
     for (int i = lane; i < dh; i += 32) q[i] = ElemIO<ET>::load(qsrc + i) * scale;
     __syncwarp();
 
-    float acc[MAX_DH / 32];
+    float acc[ND];
 #pragma unroll
-    for (int i = 0; i < MAX_DH / 32; ++i) acc[i] = 0.f;
+    for (int i = 0; i < ND; ++i) acc[i] = 0.f;
     float m = -INFINITY, l = 0.f;
     const int first = (window > 0) ? max(0, pos - window + 1) : 0;
     const int* table = block_table + (size_t)slot * max_blocks;
@@ -101,11 +117,25 @@ attn_generic_kernel(const ET* __restrict__ qkv, int ld, int q_off, const ET* __r
         if (valid) {
             const ET* krow = Kc + base + (size_t)lane * dh;
             float dot = 0.f;
-            for (int c = 0; c < dh; c += Vec16<ET>::N) {
-                float kv[Vec16<ET>::N];
-                Vec16<ET>::load(krow + c, kv);
+            constexpr int RUN = 16 / N * 2;                     // pieces of 16 bytes that are asked for together (32 numbers)
+#pragma unroll 2
+            for (int c0 = 0; c0 < dh; c0 += RUN * N) {          // (head sizes are multiples of 16: the last run may be half)
+                Piece<ET> kv[RUN];
 #pragma unroll
-                for (int j = 0; j < Vec16<ET>::N; ++j) dot = fmaf(q[c + j], kv[j], dot);
+                for (int i = 0; i < RUN; ++i)
+                    if (c0 + i * N < dh) kv[i].load(krow + c0 + i * N);
+#pragma unroll
+                for (int i = 0; i < RUN; ++i)
+                    if (c0 + i * N < dh) {
+#pragma unroll
+                        for (int j = 0; j < N; j += 4) {
+                            const float4 qv = *reinterpret_cast<const float4*>(q + c0 + i * N + j);
+                            dot = fmaf(qv.x, kv[i].at(j), dot);
+                            dot = fmaf(qv.y, kv[i].at(j + 1), dot);
+                            dot = fmaf(qv.z, kv[i].at(j + 2), dot);
+                            dot = fmaf(qv.w, kv[i].at(j + 3), dot);
+                        }
+                    }
             }
             s = dot;
         }
@@ -114,17 +144,25 @@ attn_generic_kernel(const ET* __restrict__ qkv, int ld, int q_off, const ET* __r
         const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
         l = l * corr + warp_sum(p);
 #pragma unroll
-        for (int i = 0; i < MAX_DH / 32; ++i) acc[i] *= corr;
+        for (int i = 0; i < ND; ++i) acc[i] *= corr;
         const int n_here = min(32, pos - k0 + 1);
         const ET* vbase = Vc + base;
-        for (int j = 0; j < n_here; ++j) {
-            const float pj = __shfl_sync(0xffffffffu, p, j);
-            if (pj == 0.f) continue;  // uniform across the warp
-            const ET* vrow = vbase + (size_t)j * dh;
+        for (int j0 = 0; j0 < n_here; j0 += 8) {
+            float v[8][ND];
 #pragma unroll
-            for (int i = 0; i < MAX_DH / 32; ++i) {
-                const int c = i * 32 + lane;
-                if (c < dh) acc[i] = fmaf(pj, ElemIO<ET>::load(vrow + c), acc[i]);
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int i = 0; i < ND; ++i) {
+                    const int c = i * 32 + lane;
+                    v[j][i] = 0.f;
+                    if (j0 + j < n_here && c < dh) load_now(vbase + (size_t)(j0 + j) * dh + c, v[j][i]);
+                }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float pj = __shfl_sync(0xffffffffu, p, j0 + j);
+                if (pj == 0.f) continue;                        // uniform across the warp (keys behind the last weigh nothing)
+#pragma unroll
+                for (int i = 0; i < ND; ++i) acc[i] = fmaf(pj, v[j][i], acc[i]);
             }
         }
         m = m_new;
@@ -133,7 +171,7 @@ attn_generic_kernel(const ET* __restrict__ qkv, int ld, int q_off, const ET* __r
     const float inv = (l > 0.f) ? 1.f / l : 0.f;
     ET* dst = out + (size_t)t * ld_out + (size_t)h * dh;
 #pragma unroll
-    for (int i = 0; i < MAX_DH / 32; ++i) {
+    for (int i = 0; i < ND; ++i) {
         const int c = i * 32 + lane;
         if (c < dh) ElemIO<ET>::store(dst + c, acc[i] * inv);
     }
@@ -149,13 +187,11 @@ extern "C" int vlrf_kv_append(const void* qkv, int dtype, int ld, int k_off, int
     if (T == 0) return VLRF_OK;
     const int threads = (Hkv * dh >= 256) ? 256 : 128;
     if (dtype == VLRF_F32)
-        kv_append_kernel<float><<<T, threads, 0, stream>>>((const float*)qkv, ld, k_off, v_off, (float*)Kc,
-                                                          (float*)Vc, block_table, max_blocks, tok_slot,
-                                                          tok_pos, Hkv, dh, BT, dev_err);
+        launch_chained(kv_append_kernel<float>, dim3(T), dim3(threads), (size_t)0, stream, (const float*)qkv, ld, k_off, v_off, (float*)Kc,
+                       (float*)Vc, block_table, max_blocks, tok_slot, tok_pos, Hkv, dh, BT, dev_err);
     else if (dtype == VLRF_BF16)
-        kv_append_kernel<__nv_bfloat16><<<T, threads, 0, stream>>>(
-            (const __nv_bfloat16*)qkv, ld, k_off, v_off, (__nv_bfloat16*)Kc, (__nv_bfloat16*)Vc,
-            block_table, max_blocks, tok_slot, tok_pos, Hkv, dh, BT, dev_err);
+        launch_chained(kv_append_kernel<__nv_bfloat16>, dim3(T), dim3(threads), (size_t)0, stream, (const __nv_bfloat16*)qkv, ld, k_off, v_off,
+                       (__nv_bfloat16*)Kc, (__nv_bfloat16*)Vc, block_table, max_blocks, tok_slot, tok_pos, Hkv, dh, BT, dev_err);
     else
         return vlrf_fail(VLRF_ERR_INVALID_ARG, "kv_append: unknown dtype %d", dtype);
     return vlrf_check_launch("kv_append");
@@ -176,16 +212,12 @@ extern "C" int vlrf_attn_generic(const void* qkv, int dtype, int ld, int q_off, 
     if (T == 0) return VLRF_OK;
     dim3 grid(T, (H + ATT_WARPS - 1) / ATT_WARPS);
     const size_t smem = (size_t)ATT_WARPS * dh * sizeof(float);
-    if (dtype == VLRF_F32)
-        attn_generic_kernel<float><<<grid, ATT_WARPS * 32, smem, stream>>>(
-            (const float*)qkv, ld, q_off, (const float*)Kc, (const float*)Vc, block_table, max_blocks,
-            tok_slot, tok_pos, (float*)out, ld_out, H, Hkv, dh, BT, scale, window, dev_err);
-    else if (dtype == VLRF_BF16)
-        attn_generic_kernel<__nv_bfloat16><<<grid, ATT_WARPS * 32, smem, stream>>>(
-            (const __nv_bfloat16*)qkv, ld, q_off, (const __nv_bfloat16*)Kc, (const __nv_bfloat16*)Vc,
-            block_table, max_blocks, tok_slot, tok_pos, (__nv_bfloat16*)out, ld_out, H, Hkv, dh, BT, scale,
-            window, dev_err);
+#define GO(ET, DHV) launch_chained(attn_generic_kernel<ET, DHV>, grid, dim3(ATT_WARPS * 32), smem, stream, (const ET*)qkv, ld, q_off, (const ET*)Kc, (const ET*)Vc, \
+                                   block_table, max_blocks, tok_slot, tok_pos, (ET*)out, ld_out, H, Hkv, dh, BT, scale, window, dev_err)
+    if (dtype == VLRF_F32) { if (dh == 64) GO(float, 64); else GO(float, 0); }
+    else if (dtype == VLRF_BF16) { if (dh == 64) GO(__nv_bfloat16, 64); else GO(__nv_bfloat16, 0); }
     else
         return vlrf_fail(VLRF_ERR_INVALID_ARG, "attention: unknown dtype %d", dtype);
+#undef GO
     return vlrf_check_launch("attn_generic");
 }
