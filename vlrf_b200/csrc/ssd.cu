@@ -279,9 +279,9 @@ ssd_scan_kernel(const float* __restrict__ xbc, int channels, const float* __rest
 // A decode step: one token a sequence.  A thread has a quad of columns and ROWS rows of a head's state, rows rg, rg + RG, … (RG = 256 / CQ, CQ
 // quads of columns a CTA), all asked for at once, beside the token's inputs.  What is left is to read and write the states; the kernel above
 // goes through shared memory and three barriers, a state's numbers one by one (a decode step of four such layers, 8 tokens of 32 heads of
-// 128 x 128, 407 -> 403 us).
+// 128 x 128, 407 -> 403 us; held to the registers of two CTAs an SM instead of one, which it took by itself, 367 -> 351).
 template <int ROWS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, ROWS == 16 ? 2 : 4)
 ssd_step_kernel(const float* __restrict__ xbc, int channels, const float* __restrict__ proj, int ld, int dt_off, const float* __restrict__ dt_bias,
                 const float* __restrict__ a_log, const float* __restrict__ Dv, float* __restrict__ state, int state_row,
                 const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_pos0, float* __restrict__ y,
