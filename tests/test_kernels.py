@@ -808,3 +808,21 @@ def test_general_attention_at_the_edges_of_its_runs(dh, lens, window, dtype, tol
         got = out[at:at + n].float().cpu().reshape(n, H, dh).permute(1, 0, 2)
         assert torch.isfinite(got).all() and rel_err(got, want) < tol, (n, dh)
         at += n
+
+
+@pytest.mark.parametrize("M", [3, 4, 16, 17, 33, 64])
+@pytest.mark.parametrize("N,K", [(4096, 744), (4096, 752), (4095, 128), (4200, 8), (5632, 1024)])
+def test_wide_products_of_few_rows(M, N, K):
+    """Both sides of the line from which the operands' roles are exchanged (rows, columns, columns over depth), with bias, activation and residual."""
+    from vlrf_b200.csrc import ops
+    x, w = randn(M, K, seed=M, dtype=torch.bfloat16), (randn(N, K, seed=N) / math.sqrt(K)).bfloat16()
+    b, res = randn(N, seed=3), randn(M, N, seed=4)
+    assert ops._swapped_takes(M, N, K) == (M >= 4 and N >= 4096 and N >= 5.5 * K)
+    lin = x.double() @ w.double().T + b.double()
+    for dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-2)):
+        out = torch.full((M, N), float("nan"), dtype=dtype, device=DEV)
+        ops.linear(x.to(DEV), w.to(DEV), b.to(DEV), out)
+        assert rel_err(out.float().cpu(), lin) < tol
+    out = torch.full((M, N), float("nan"), device=DEV)
+    ops.linear(x.to(DEV), w.to(DEV), b.to(DEV), out, act="gelu_erf", residual=res.to(DEV))
+    assert rel_err(out.cpu(), torch.nn.functional.gelu(lin) + res.double()) < 1e-5

@@ -144,6 +144,12 @@ PREFILL_ATTENTION_PARTS = None       # a number here overrides attention_prefill
 SKINNY_MAX_ROWS = 64
 FUSED_NORM_MAX_ROWS = 16
 SWAPPED_MIN_COLUMNS = 16384
+#: … and from so many rows and columns on, products at least so many times as wide as they are deep.  A CTA of the exchanged kernel streams
+#: whole rows of W through a deep ring, with no sum to meet in; it needs tiles for most SMs, or short ones.  Whole decode steps, split-k against exchanged
+#: (us): 11,264 and 12,928 x 2,048 at 8 and 16 rows 380, 446 against 367, 414, but at one row 295 against 298; 7,296 x 1,024 at 4, 16 and 64 rows 202,
+#: 261, 359 against 197, 245, 336; 5,632 x 1,024 at 48 rows 364 against 347; four times as wide: 8,192 x 2,048 at 8 rows 576 against 581, 6,400 x 1,600
+#: at 32 rows 2,860 against 2,928.
+SWAPPED_WIDE_ROWS, SWAPPED_WIDE_COLUMNS, SWAPPED_WIDE_RATIO = 4, 4096, 5.5
 #: Few-row products whose weight matrix has at least this many bytes go to the split-k tcgen05 kernel (the
 #: second figure: with the LayerNorm fused in).  Measured on B200 inside whole decode steps, the split-k kernel
 #: wins at every size of GPT-2's: its CTAs leave room on an SM for the next kernel's to begin ahead, and it
@@ -273,11 +279,15 @@ def _kv_args(kv_scatter, N: int) -> list:
             kc.shape[2]]
 
 
+def _swapped_takes(M: int, N: int, K: int) -> bool:
+    return N >= SWAPPED_MIN_COLUMNS or (M >= SWAPPED_WIDE_ROWS and N >= SWAPPED_WIDE_COLUMNS and N >= SWAPPED_WIDE_RATIO * K)
+
+
 def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, stats=None) -> bool:
     bf16_out = out.dtype == torch.bfloat16
     if (x.dtype == torch.bfloat16 and M <= SKINNY_MAX_ROWS and K % 8 == 0 and USE_TCGEN05 and kv_scatter is None
-            and N >= SWAPPED_MIN_COLUMNS):
-        # few rows, very many columns (the head over the vocabulary): enough 128-row tiles of w to fill the GPU,
+            and _swapped_takes(M, N, K)):
+        # few rows, very many columns (the head over the vocabulary, wide input products): enough 128-row tiles of w to fill the GPU,
         # so w becomes the 128-row operand of the tcgen05 kernel and the rows of x its N
         call("vlrf_gemm_tcgen05", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), M, N, K, K, N,
              dtype_code(out.dtype), act, *_kv_args(None, N), _ptr(_dev_err()), _stream())
