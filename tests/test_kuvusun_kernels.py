@@ -504,3 +504,12 @@ def test_parts_of_a_latent_context_meet(splits, monkeypatch):
     from vlrf_b200.csrc import ops
     monkeypatch.setattr(ops, "latent_decode_splits", lambda *a, **k: splits)
     test_tensor_core_attention_over_latent_rows(256, 32, 16, 1, monkeypatch)
+
+
+@pytest.mark.parametrize("E", [1, 31, 32, 33, 64, 65, 512])
+def test_places_of_the_experts_rows(E):
+    from vlrf_b200.csrc import ops
+    counts = torch.randint(0, 9, (E,), generator=torch.Generator().manual_seed(E), dtype=torch.int32)
+    c, off = counts.cuda(), torch.full((E + 1,), -1, dtype=torch.int32, device="cuda")
+    ops.moe_plan(c, off, E)
+    assert off.tolist() == [0] + counts.cumsum(0).tolist() and int(c.abs().sum()) == 0
