@@ -471,7 +471,7 @@ extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const vo
     const long long tiles = (max_new + FT_BQ - 1) / FT_BQ;
     VLRF_REQUIRE(tiles * n_parts <= 65535, "attn_prefill_tc: %lld tiles of %d parts are too many for one launch", tiles, n_parts);
     // The tiles that exist are at most n_tokens / 128 + n_seqs: with sequences of unequal lengths far fewer than every sequence times the
-    // longest's (five prompts of 1,013 to 31 tokens and three single tokens, 25 heads: 22 of 64; 42.8 -> 31 us).
+    // longest's (five prompts of 1,013 to 31 tokens and three single tokens, 25 heads: 22 of 64; 42.8 -> 33.1 us).
     const long long places = (long long)n_tokens / FT_BQ + n_seqs;
     const int listed = n_seqs > 1 && n_seqs <= 32 && tiles <= 64 && places < tiles * n_seqs ? n_seqs : 0;
     dim3 grid(H, listed ? (unsigned)places : n_seqs, (unsigned)(listed ? n_parts : tiles * n_parts));

@@ -119,8 +119,8 @@ qkv_rope_append_kernel(const float* __restrict__ proj, int ld, int q_off, int k_
         // A warp per head, queries and keys alike: a lane holds up to four pairs of entries (the two of a rotation, or two
         // neighbours behind the rotated ones), the head's sum of squares is a sum over the warp, and norm, rotation and
         // store follow from the registers: every entry is read once and no warp waits for another.  The heads of a token are
-        // dealt to gridDim.y CTAs, a head a warp (one CTA a token walked 20 heads in five round trips: 7.0 us for 32 tokens inside
-        // a decode step, 20.7 us for 1,928 in a prompt step; now 3.4 and 10.2 us).
+        // dealt to gridDim.y CTAs where the step has few tokens (one CTA a token walks 20 heads in five round trips: 7.0 us for 32 tokens inside a
+        // decode step, under 3 us with a head a warp; 1,928 tokens of a prompt step fill the GPU as they are, 20.7 us against 26.5).
         const int hd2 = dk / 2;
         int blk = -1;
         if (write_cache) {
@@ -241,7 +241,7 @@ __device__ __forceinline__ void store_quad(__nv_bfloat16* p, const float4& v) {
 // entry i turns with entry i + rot/2, their four partners, works out their angles itself, and waits for nobody.  Its loads do not depend on one
 // another but for the cache's block.  The kernel above waits for slot, position, the angles of the whole token and then for a
 // few entries after the other: 7.6 us for 8 tokens of 18 heads of 128 inside a decode step, 13.6 us for 2,048 tokens of 16 + 4 heads of
-// 64; here 2.7 and 6.1 us.  blockIdx.y: 128 quads of the token.
+// 64; here 2.6 and 9.0 us.  blockIdx.y: 128 quads of the token.
 template <typename ET>
 __global__ void __launch_bounds__(128)
 qkv_rope_quads_kernel(const float* __restrict__ proj, int ld, int q_off, int k_off, int v_off, const float* __restrict__ freq,
@@ -473,7 +473,8 @@ extern "C" int vlrf_qkv_norm_rope_append(const float* proj, int ld, int q_off, i
         return vlrf_check_launch("qkv_rope_append");
     }
     const bool by_heads = norm == 1 && dk % 2 == 0 && dk <= 256;       // (the kernel's own rule for a warp a head)
-    const dim3 grid(T, by_heads ? (H + (write_cache ? Hkv : 0) + 3) / 4 : 1);
+    const int head_ctas = (H + (write_cache ? Hkv : 0) + 3) / 4, fill = 1184 / T;          // (eight CTAs an SM)
+    const dim3 grid(T, by_heads && fill > 1 ? (fill < head_ctas ? fill : head_ctas) : 1);
     if (dtype == VLRF_F32)
         launch_chained(qkv_rope_append_kernel<float>, grid, dim3(128), smem, stream, proj, ld, q_off, k_off, v_off, freq, rot,
                        (float*)q_out, ldq, (float*)Kc, (float*)Vc, block_table, max_blocks, tok_slot, tok_pos, H, Hkv, Hv, dk, dv, BT,

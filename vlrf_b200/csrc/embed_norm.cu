@@ -260,8 +260,8 @@ extern "C" int vlrf_layernorm(const float* x, const int* rows, const float* gamm
                  d, 48 * 1024 / 4 - 32);
     if (n_rows == 0) return VLRF_OK;
     // A warp a row wherever the row fits its registers, down to one row: one round trip and ten exchanges between lanes, where the
-    // block kernel has two barriers a sum and reads weight and bias behind them (1 row of 768 inside a decode step 8.0 -> 3.7 us, 4
-    // rows in float32 5.9 -> 2.8 us).  Longer rows, a warp reads three times: only where there are enough of them.
+    // block kernel has two barriers a sum and reads weight and bias behind them (1 row of 768 inside a decode step 8.0 -> 2.5 us, 4
+    // rows in float32 5.9 -> 2.3 us).  Longer rows, a warp reads three times: only where there are enough of them.
     const bool on16 = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) |
                         reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     if (d % 4 == 0 && on16 && (n_rows >= 8 || d <= 2048)) {

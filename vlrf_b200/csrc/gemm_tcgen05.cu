@@ -564,7 +564,7 @@ namespace {
 // Rows of a group's tile.  Few rows a group (a decode step's experts and heads): W is the 128-row operand and a tile has as many rows as
 // twice the average group fills (16, 32 or 64), so that a tile brings the weights and little else through the ring; with 128 rows of X beside
 // them, nearly all of other groups or none, it brought as many bytes again and filled half the ring with them (16 experts of 2,048 x 1,024 with 2 rows
-// each 24.1 -> 13.6 us inside a decode step, its down product 13.7 -> 8.3 us).  Heads' rows are known: the tile that takes them all.
+// each 24.1 -> 14.6 us inside a decode step, its down product 13.7 -> 10.6 us).  Heads' rows are known: the tile that takes them all.
 int gr_tile_rows(int rows, int G, bool by_offsets) {
     const long long fill = by_offsets ? (2ll * rows + G - 1) / G : rows;
     const int each = fill <= 16 ? 16 : fill <= 32 ? 32 : fill <= 64 ? 64 : TC_BM;
