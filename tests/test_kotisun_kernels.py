@@ -358,6 +358,58 @@ def test_recurrence_in_chunks(Hs, P, N, G):
         assert a <= max(1.5 * b, 2.0 ** -21), off
 
 
+@pytest.mark.parametrize("Hs,P,N,G", [(4, 64, 64, 2), (3, 132, 16, 1), (2, 128, 128, 2)])
+@pytest.mark.parametrize("where", ["x", "B", "C", "dt", "decay", "state", "large"])
+def test_recurrence_in_chunks_keeps_to_the_past(where, Hs, P, N, G):
+    """A NaN or an infinity at one token (or in the kept state, or a decay of nothing at all, or numbers whose products overflow) changes
+    no earlier token and gives what token by token gives, finite where that is finite and the same where it is not; the other sequence
+    of the step has nothing of it."""
+    import types
+
+    from vlrf_b200.csrc import ops
+    from vlrf_b200.parts.context import Workspace
+    g = torch.Generator().manual_seed(Hs * 1000 + P * 10 + N)
+    inner, channels, lens, pos0, slots = Hs * P, Hs * P + 2 * G * N, [150, 70], [4, 3], [1, 0]
+    T, state_row = sum(lens), Hs * N * P
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)   # noqa: E731
+    ctx = types.SimpleNamespace(n_tokens=T, n_seqs=2, seq_slot=i32(slots), seq_start=i32([0, 150, 220]), seq_pos0=i32(pos0), max_new=150,
+                                ws=Workspace(torch.device(DEV)), act_dtype=torch.bfloat16)
+    for token, value in ((77, float("nan")), (77, float("inf")), (149, float("-inf")), (0, float("inf"))):
+        xbc, dt = torch.randn(T, channels, generator=g), torch.randn(T, Hs, generator=g)
+        dt_bias, a_log, D = torch.randn(Hs, generator=g), torch.linspace(-6.0, 1.0, Hs), torch.randn(Hs, generator=g)
+        state = torch.randn(2, 2, state_row, generator=g)
+        if where == "x":
+            xbc[token, P + 2] = value                                      # head 1, column 2
+        elif where in "BC":
+            xbc[token, inner + (G * N if where == "C" else 0) + 3] = value
+        elif where == "dt":
+            dt[token, 1] = value
+        elif where == "decay":
+            a_log[1] = 95.0                                                # exp overflows: every token forgets all before it
+        elif where == "state":
+            state[slots[0], pos0[0] & 1, N * P + 5] = value                # head 1, column 5
+        else:
+            xbc[token, P + 2], xbc[token, inner + 3] = 3.39e38, 1e30
+        proj = dev(torch.cat([torch.randn(T, 3, generator=g), dt], 1))
+        got = []
+        for chunked in (False, True):
+            st, y = state.to(DEV), torch.full((T, inner), 7.0, device=DEV)
+            args = (dev(xbc), proj, 3, dev(dt_bias), dev(a_log), dev(D), st)
+            if chunked:
+                ops.ssd_chunks(*args, ctx, y, Hs, G, N, P)
+            else:
+                ops.ssd_scan(*args, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, 2, Hs, G, N, P, 150)
+            got.append((y.cpu(), st.cpu()))
+        for a, b in zip(*got):                                             # token by token, in chunks
+            odd = ~torch.isfinite(a)
+            assert torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a[odd & ~torch.isnan(a)], b[odd & ~torch.isnan(a)])
+            keep = ~odd & (a.abs() < 1e6)
+            assert float((a[keep] - b[keep]).abs().max() / a[keep].abs().max()) < 1e-5
+            assert torch.allclose(a[~odd], b[~odd], rtol=1e-3, atol=1e-4 * float(a[keep].abs().max()))
+        if where in ("x", "B", "C", "dt"):
+            assert torch.isfinite(got[1][0][:token]).all() and torch.isfinite(got[1][0][150:]).all()
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 5])
 def test_convolution_over_runs(taps):
     """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a

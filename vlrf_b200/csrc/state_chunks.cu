@@ -24,17 +24,26 @@
 // these are kept to 48 bits; no weight is above 1
 // before its gain.  The 32-bit engine keeps to the FMA kernels.
 //
+// Range.  A product of a zero weight and an infinity is not zero, and an infinity has no three parts: a token's infinity would reach the
+// tokens of its block that come before it.  So the writes look at every number that enters: where one of a head's in a tile of columns
+// (its rows, step sizes, decays, the state it starts from) is not finite or beyond RC_LIMIT, below which no product of this file
+// overflows, `wild` says so, the state is left as it was and the caller's token-by-token kernel does that head's columns again.
+//
 // Layouts: q, k, v float32 rows of any stride (multiples of 4 numbers, on 16 bytes); scratch per chunk and head K·V float32, laid
-// out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a float4 per chunk and head.
+// out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a float4 per chunk and head; wild an int per
+// chunk, head and tile of 64 columns.
 #include "common.cuh"
 #include "chunk_mma.cuh"
 
 namespace {
-constexpr int RC = 64;                 // tokens of a chunk
-constexpr int RT = 64;                 // columns of V that a CTA works on at a time (an item: a head and such a tile)
+constexpr int RC = STATE_CHUNK;        // tokens of a chunk
+constexpr int RT = STATE_TILE;         // columns of V that a CTA works on at a time (an item: a head and such a tile)
 constexpr int RX = RT + 8;             // … and their pitch in shared memory (16 bytes of padding keep ldmatrix off bank conflicts)
 constexpr int R_THREADS = 256;
 constexpr int R_ITEMS = 4;             // items a CTA works through with one set of q and k
+// Rows and gains: weights stay below 2^28, scores of 128 products below 2^63, what 64 tokens write or read below 2^125.  States: read below
+// 2^28 · 2^90 · 128.
+constexpr float RC_LIMIT = 268435456.f, RC_STATE_LIMIT = 1.2379400392853803e27f;      // 2^28, 2^90
 
 struct StateChunks {
     const float *q, *k, *v;
@@ -43,6 +52,7 @@ struct StateChunks {
     int ld_s0;
     float* scratch;
     float4* aux;                       // {F_L, –, –, –}
+    int* wild;
     float* state;
     int state_row;
     const int *seq_slot, *seq_start, *seq_pos0;
@@ -57,8 +67,9 @@ struct HeadScalars {
     float Lp[RC], Lo[RC], Ls[RC], gain[RC], before[4], after[4], block[4];
 };
 
-// A warp: the numbers of head h for the L tokens from `first` on (tokens 2·lane and 2·lane + 1 a lane).
-__device__ __forceinline__ void head_scalars(const StateChunks& A, int h, int first, int L, int lane, HeadScalars& out) {
+// A warp: the numbers of head h for the L tokens from `first` on (tokens 2·lane and 2·lane + 1 a lane).  Returns whether they are what the
+// products take.
+__device__ __forceinline__ bool head_scalars(const StateChunks& A, int h, int first, int L, int lane, HeadScalars& out) {
     const float a = -expf(A.a_log[h]), bias = A.dt_bias[h];
     float f[2], gain[2];
 #pragma unroll
@@ -98,6 +109,11 @@ __device__ __forceinline__ void head_scalars(const StateChunks& A, int h, int fi
         out.block[0] = t0; out.block[1] = t1; out.block[2] = t2; out.block[3] = t3;
         out.after[3] = 0.f; out.after[2] = t3; out.after[1] = t3 + t2; out.after[0] = t3 + t2 + t1;
     }
+    // (written so that a NaN fails; a sum of logarithms of one sign is finite only if each of them is)
+    return __all_sync(0xffffffffu, gain[0] < RC_LIMIT && gain[1] < RC_LIMIT) && t0 + t1 + t2 + t3 > -3e38f;
+}
+__device__ __forceinline__ bool tame(const float4& x, float limit) {
+    return fabsf(x.x) < limit && fabsf(x.y) < limit && fabsf(x.z) < limit && fabsf(x.w) < limit;
 }
 
 // Four numbers into the three planes of a tile, `plane` elements apart.
@@ -111,9 +127,9 @@ __device__ __forceinline__ void store_planes(__nv_bfloat16* at, int plane, const
 }
 __device__ __forceinline__ float4 quad_or_zero(const float* p, bool there) { return there ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f); }
 
-// The K numbers of the chunk's tokens (rows of stride ld) into planes [3][RC][K + 8].
+// The K numbers of the chunk's tokens (rows of stride ld) into planes [3][RC][K + 8].  Returns whether this thread's are what the products take.
 template <int K>
-__device__ __forceinline__ void load_rows(__nv_bfloat16* planes, const float* rows, int ld, int L, int tid) {
+__device__ __forceinline__ bool load_rows(__nv_bfloat16* planes, const float* rows, int ld, int L, int tid) {
     constexpr int QUADS = RC * K / 4, EACH = (QUADS + R_THREADS - 1) / R_THREADS;
     float4 x[EACH];
 #pragma unroll
@@ -126,6 +142,10 @@ __device__ __forceinline__ void load_rows(__nv_bfloat16* planes, const float* ro
         const int i = tid + e * R_THREADS, r = i / (K / 4), c = (i - r * (K / 4)) * 4;
         if (i < QUADS) store_planes(planes + r * (K + 8) + c, RC * (K + 8), x[e]);
     }
+    bool fine = true;
+#pragma unroll
+    for (int e = 0; e < EACH; ++e) fine = fine && tame(x[e], RC_LIMIT);
+    return fine;
 }
 
 template <int K> constexpr int writes_smem() { return (3 * RC * (K + 8) + 3 * RC * RX) * 2 + R_ITEMS * (int)sizeof(HeadScalars) + R_ITEMS * RC * 4; }
@@ -142,6 +162,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
     __nv_bfloat16* xs = ks + 3 * RC * KS;                                // [3][64][RX]
     HeadScalars* sc = reinterpret_cast<HeadScalars*>(xs + 3 * RC * RX);
     float* weight = reinterpret_cast<float*>(sc + R_ITEMS);              // [items][64]
+    __shared__ bool item_fine[R_ITEMS];
     const int s = blockIdx.z, c0 = blockIdx.x * RC;
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start;
     if (c0 >= n || A.seq_slot[s] < 0) return;
@@ -159,9 +180,17 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         }
     };
     ask(0);
+    // the queries enter here only to be looked at (the outputs load them again), a quad of a row a thread
+    bool rows_fine = true;
+#pragma unroll
+    for (int e = 0; e < RC * K / 4 / R_THREADS; ++e) {
+        const int i = tid + e * R_THREADS, r = i / (K / 4), c = (i - r * (K / 4)) * 4;
+        rows_fine = rows_fine && tame(quad_or_zero(A.q + (size_t)(first + r) * A.ldq + (size_t)g * K + c, r < L), RC_LIMIT);
+    }
     if (warp < items) {
         const int h = g * per_group + (i0 + warp) / v_tiles;
-        head_scalars(A, h, first, L, lane, sc[warp]);
+        const bool fine = head_scalars(A, h, first, L, lane, sc[warp]);
+        if (lane == 0) item_fine[warp] = fine;
         __syncwarp();
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
@@ -170,18 +199,28 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         }
         if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * A.H + h] = make_float4(sc[warp].before[3] + sc[warp].Lp[RC - 1], 0.f, 0.f, 0.f);
     }
-    load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid);
-    __syncthreads();
+    rows_fine = load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid) && rows_fine;
+    rows_fine = __syncthreads_and(rows_fine);
+    const float* from = A.state + ((size_t)A.seq_slot[s] * 2 + (A.seq_pos0[s] & 1)) * A.state_row;
+    const int chunks = (n + RC - 1) / RC;
     for (int item = 0; item < items; ++item) {
         const int h = g * per_group + (i0 + item) / v_tiles, v0 = (i0 + item) % v_tiles * RT;
+        bool fine = rows_fine && item_fine[item];
+        // the state that the sequence starts from: its chunks look at a share each
+        for (int i = blockIdx.x * R_THREADS + tid; i < K * RT / 4; i += chunks * R_THREADS) {
+            const int r = i / (RT / 4), c = v0 + i % (RT / 4) * 4;
+            fine = fine && tame(quad_or_zero(from + ((size_t)h * K + r) * A.V + c, c < A.V), RC_STATE_LIMIT);
+        }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = tid / 16 + 16 * e, c = tid % 16 * 4;
             const float w = weight[item * RC + r];
+            fine = fine && tame(x[e], RC_LIMIT);
             store_planes(xs + r * RX + c, RC * RX, make_float4(w * x[e].x, w * x[e].y, w * x[e].z, w * x[e].w));
         }
         if (item + 1 < items) ask(item + 1);
-        __syncthreads();
+        fine = __syncthreads_and(fine);
+        if (tid == 0) A.wild[(chunk * A.H + h) * v_tiles + v0 / RT] = fine ? 0 : 1;
         // 16 rows of the state by 32 columns at a time
         float* U = A.scratch + (chunk * A.H + h) * (size_t)K * A.V;
         for (int unit = warp; unit < K / 8; unit += R_THREADS / 32) {
@@ -219,7 +258,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
 
 // grid (quads of a sequence's states / 128, sequences)
 __global__ void __launch_bounds__(128)
-state_chunk_states_kernel(const StateChunks A, int per_head) {
+state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
     pdl_wait();
     pdl_launch_dependents();
     const int s = blockIdx.y, slot = A.seq_slot[s];
@@ -234,6 +273,8 @@ state_chunk_states_kernel(const StateChunks A, int per_head) {
     const size_t slot0 = (size_t)(start / RC + s);
     float* u = A.scratch + slot0 * all + i;
     const float4* aux = A.aux + slot0 * A.H + h;
+    const int* wild = A.wild + (slot0 * A.H + h) * v_tiles + (int)(i % A.V) / RT;
+    int any_wild = 0;
     constexpr int AHEAD = 8;                        // chunks asked for together
     for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
         float4 U[AHEAD];
@@ -242,6 +283,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head) {
         for (int j = 0; j < AHEAD; ++j) {
             U[j] = quad_or_zero(u + (size_t)(c0 + j) * all, c0 + j < chunks);
             F[j] = c0 + j < chunks ? aux[(size_t)(c0 + j) * A.H].x : 0.f;
+            any_wild |= c0 + j < chunks ? wild[(size_t)(c0 + j) * A.H * v_tiles] : 0;
         }
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j) {
@@ -252,7 +294,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head) {
             }
         }
     }
-    *reinterpret_cast<float4*>(to + i) = S;
+    if (!any_wild) *reinterpret_cast<float4*>(to + i) = S;      // (else it stays what token by token begins with: `to` may be `from`)
 }
 
 template <int K> constexpr int keys_or_state() { return 3 * (RC * (K + 8) > K * RX ? RC * (K + 8) : K * RX); }
@@ -435,7 +477,7 @@ template <int K> int launch_state_chunks(const StateChunks& A, int n_seqs, int m
     int st = vlrf_check_launch("state_chunks: writes");
     if (st != VLRF_OK) return st;
     const long long quads = (long long)A.H * K * A.V / 4;
-    launch_chained(state_chunk_states_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), (size_t)0, stream, A, K * A.V);
+    launch_chained(state_chunk_states_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), (size_t)0, stream, A, K * A.V, v_tiles);
     st = vlrf_check_launch("state_chunks: states");
     if (st != VLRF_OK) return st;
     launch_chained(state_chunk_outputs_kernel<K>, grid, dim3(R_THREADS), (size_t)outputs_smem<K>(), stream, A, v_tiles, parts);
@@ -450,8 +492,10 @@ extern "C" int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, i
             state_row % 4 == 0 && channels == H * P + 2 * G * N) ? 1 : 0;
 }
 
-// float32 scratch of a step of T tokens in n_seqs sequences
-extern "C" long long vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P) { return ((long long)T / RC + n_seqs) * H * ((long long)N * P + 4); }
+// float32 numbers of scratch of a step of T tokens in n_seqs sequences: a state, four numbers and the tiles' marks per chunk and head
+extern "C" long long vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P) {
+    return ((long long)T / RC + n_seqs) * H * ((long long)N * P + 4 + (P + RT - 1) / RT);
+}
 
 extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                                const float* D, float* scratch, float* state, int state_row, const int* seq_slot, const int* seq_start,
@@ -466,13 +510,16 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
     A.ldq = A.ldk = A.ldv = channels;
     A.s0 = proj + dt_off; A.ld_s0 = ld; A.dt_bias = dt_bias; A.a_log = a_log; A.skip = D;
     A.aux = reinterpret_cast<float4*>(scratch);
-    A.scratch = scratch + ((size_t)n_tokens / RC + n_seqs) * H * 4;
+    const size_t slots = ((size_t)n_tokens / RC + n_seqs) * H;          // (chunk, head)
+    A.scratch = scratch + slots * 4;
+    A.wild = reinterpret_cast<int*>(A.scratch + slots * (size_t)N * P);
     A.state = state; A.state_row = state_row; A.seq_slot = seq_slot; A.seq_start = seq_start; A.seq_pos0 = seq_pos0;
     A.y = y; A.ldy = H * P; A.H = H; A.G = G; A.V = P;
-    switch (N) {
-        case 16: return launch_state_chunks<16>(A, n_seqs, max_new, stream);
-        case 32: return launch_state_chunks<32>(A, n_seqs, max_new, stream);
-        case 64: return launch_state_chunks<64>(A, n_seqs, max_new, stream);
-        default: return launch_state_chunks<128>(A, n_seqs, max_new, stream);
-    }
+    const int st = N == 16   ? launch_state_chunks<16>(A, n_seqs, max_new, stream)
+                   : N == 32 ? launch_state_chunks<32>(A, n_seqs, max_new, stream)
+                   : N == 64 ? launch_state_chunks<64>(A, n_seqs, max_new, stream)
+                             : launch_state_chunks<128>(A, n_seqs, max_new, stream);
+    if (st != VLRF_OK) return st;
+    return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
+                                max_new, H, G, N, P, ScanRuns{1, 0, 1, A.wild}, stream);
 }

@@ -317,6 +317,7 @@ int vlrf_ssd_step(const float* xbc, int channels, const float* proj, int ld, int
                   const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
                   float* y, int n_seqs, int Hs, int G, int N, int P, cudaStream_t stream);
 // The same over prompts on the tensor cores, 64 tokens at a time (state_chunks.cu): every float32 operand in three bfloat16 parts.
+// Columns of heads whose numbers are not finite, or too large for products of parts, are done token by token behind it.
 // scratch float32 (vlrf_ssd_chunks_scratch numbers, n_tokens the step's rows).  N 16, 32, 64 or 128, P a multiple of 4.
 int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, int state_row);
 long long vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P);
