@@ -132,7 +132,7 @@ _SIGNATURES = {
     "vlrf_ssd_step": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p,
                       _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "vlrf_ssd_chunks_takes": [_c_int] * 6,
-    "vlrf_ssd_chunks_scratch": [_c_int] * 5,
+    "vlrf_ssd_chunks_scratch": [_c_int] * 5 + [_c_void_p],
     "vlrf_ssd_chunks": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "vlrf_ssd_gate_norm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -197,7 +197,6 @@ _SIGNATURES = {
     "vlrf_apply_penalties": [_c_void_p, _c_int, _c_int, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
                              _c_void_p, _c_void_p, _c_void_p, _c_void_p],
 }
-_LONG = {"vlrf_ssd_chunks_scratch"}        # entry points that return 64 bits
 
 
 def library() -> ctypes.CDLL:
@@ -221,7 +220,7 @@ def library() -> ctypes.CDLL:
             except AttributeError as exc:
                 raise KernelError(f"the kernel library lacks the symbol {name}") from exc
             fn.argtypes = argtypes
-            fn.restype = ctypes.c_longlong if name in _LONG else _c_int
+            fn.restype = _c_int
         _lib = lib
         return lib
 

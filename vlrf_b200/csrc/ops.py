@@ -1237,12 +1237,21 @@ def attention_window_step(q, k_cache, v_cache, block_table, out, ctx, n_heads: i
 SSD_CHUNKS, SSD_CHUNKS_MIN_RUN, SSD_CHUNKS_MAX_BYTES = True, 384, 8 << 30
 
 
+def _ssd_chunks_scratch(ctx, n_heads: int, n_state: int, p: int) -> int:
+    import ctypes
+
+    from . import call_host
+    n = ctypes.c_longlong(0)
+    call_host("vlrf_ssd_chunks_scratch", ctx.n_tokens, ctx.n_seqs, n_heads, n_state, p, ctypes.byref(n))
+    return n.value
+
+
 def ssd_chunks_takes(dtype: torch.dtype, ctx, n_heads: int, n_groups: int, n_state: int, p: int, channels: int, state_row: int) -> bool:
     """Whether a step's state-space recurrence runs in chunks: the bfloat16 engine's (the 32-bit one keeps to FMAs), prompts only."""
     if dtype != torch.bfloat16 or not SSD_CHUNKS or ctx.max_new < SSD_CHUNKS_MIN_RUN:
         return False
     from . import library
-    if 4 * library().vlrf_ssd_chunks_scratch(ctx.n_tokens, ctx.n_seqs, n_heads, n_state, p) > SSD_CHUNKS_MAX_BYTES:
+    if 4 * _ssd_chunks_scratch(ctx, n_heads, n_state, p) > SSD_CHUNKS_MAX_BYTES:
         return False
     return bool(library().vlrf_ssd_chunks_takes(n_heads, n_groups, n_state, p, channels, state_row))
 
@@ -1257,8 +1266,7 @@ def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_
             raise KernelError(f"ssd_chunks: {name} has one number per head")
     if y.shape[1] != n_heads * p or state.dim() != 3 or state.shape[1] != 2 or min(xbc.shape[0], proj.shape[0], y.shape[0]) < T:
         raise KernelError("ssd_chunks: sizes do not match")
-    from . import library
-    scratch = ctx.ws.get("ssd_chunks", 1, library().vlrf_ssd_chunks_scratch(T, ctx.n_seqs, n_heads, n_state, p), torch.float32)
+    scratch = ctx.ws.get("ssd_chunks", 1, _ssd_chunks_scratch(ctx, n_heads, n_state, p), torch.float32)
     call("vlrf_ssd_chunks", _ptr(xbc), xbc.shape[1], _ptr(proj), proj.stride(0), dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
          _ptr(scratch), _ptr(state), state.shape[2], _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(y), T, ctx.n_seqs,
          ctx.max_new, n_heads, n_groups, n_state, p, _stream())

@@ -493,8 +493,10 @@ extern "C" int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, i
 }
 
 // float32 numbers of scratch of a step of T tokens in n_seqs sequences: a state, four numbers and the tiles' marks per chunk and head
-extern "C" long long vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P) {
-    return ((long long)T / RC + n_seqs) * H * ((long long)N * P + 4 + (P + RT - 1) / RT);
+extern "C" int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P, long long* floats) {
+    VLRF_REQUIRE(T >= 0 && n_seqs >= 0 && H > 0 && N > 0 && P > 0 && floats != nullptr, "ssd_chunks_scratch: bad arguments");
+    *floats = ((long long)T / RC + n_seqs) * H * ((long long)N * P + 4 + (P + RT - 1) / RT);
+    return VLRF_OK;
 }
 
 extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,

@@ -320,7 +320,7 @@ int vlrf_ssd_step(const float* xbc, int channels, const float* proj, int ld, int
 // Columns of heads whose numbers are not finite, or too large for products of parts, are done token by token behind it.
 // scratch float32 (vlrf_ssd_chunks_scratch numbers, n_tokens the step's rows).  N 16, 32, 64 or 128, P a multiple of 4.
 int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, int state_row);
-long long vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P);
+int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P, long long* floats);
 int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                     const float* D, float* scratch, float* state, int state_row, const int* seq_slot, const int* seq_start,
                     const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int H, int G, int N, int P, cudaStream_t stream);
