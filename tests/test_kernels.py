@@ -648,6 +648,18 @@ def test_attention_prefill_lists_the_tiles_that_exist(monkeypatch, kernel, seqs)
     test_attention_prefill_tensor_cores(monkeypatch, kernel, 2, 1, 64, seqs, 0)
 
 
+@pytest.mark.parametrize("kernel", ["tcgen05", "tcgen05_parts2"])
+@pytest.mark.parametrize("H,Hkv,seqs,listed", [
+    (25, 5, [(0, 1013), (0, 517), (0, 31), (300, 1), (300, 1)], True), (40, 8, [(0, 128), (0, 129), (5, 127), (0, 1), (64, 256), (9, 2)], False),
+    (10, 2, [(3, 1)] * 31 + [(0, 260)], True), (10, 2, [(3, 1)] * 32 + [(0, 260)], False), (5, 1, [(0, 1), (0, 8100), (7, 9)], True),
+    (5, 1, [(0, 8300), (0, 1)], False)])
+def test_attention_prefill_where_the_tiles_fill_the_gpu(monkeypatch, kernel, H, Hkv, seqs, listed):
+    """Heads enough for the tiles that exist to be listed, at the same edges."""
+    from vlrf_b200.csrc import library
+    assert bool(library().vlrf_attn_prefill_tc_lists(sum(n for _, n in seqs), len(seqs), max(n for _, n in seqs), H, 1, 148)) == listed
+    test_attention_prefill_tensor_cores(monkeypatch, kernel, H, Hkv, 64, seqs, 0)
+
+
 def test_kv_append_writes_each_token_where_its_slot_says():
     from vlrf_b200.csrc import ops
     Hkv, dh, T = 3, 16, 70

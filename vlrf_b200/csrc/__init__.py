@@ -66,6 +66,7 @@ _SIGNATURES = {
     "vlrf_attn_prefill_tc_part_floats": [],
     "vlrf_attn_prefill_tc_max_parts": [],
     "vlrf_attn_prefill_tc_min_part_blocks": [],
+    "vlrf_attn_prefill_tc_lists": [_c_int] * 6,
     "vlrf_attn_prefill_tc_tile": [],
     "vlrf_attn_prefill_tc": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
                              _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,

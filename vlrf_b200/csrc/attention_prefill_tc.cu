@@ -124,9 +124,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     pdl_wait();
     if (threadIdx.x == 0) VLRF_TRACE(trace, 4, tcta, 1);
     pdl_launch_dependents();
+    int row0, row_end, slot, pos0;
+    bool exists = true;
     if (listed > 0) {                                // (at most 32 sequences: a lane each, every warp for itself)
         part = blockIdx.z;
-        const int mine = lane < listed && seq_slot[lane] >= 0 ? (seq_start[lane + 1] - seq_start[lane] + FT_BQ - 1) / FT_BQ : 0;
+        const bool there = lane < listed;
+        row0 = there ? seq_start[lane] : 0;
+        row_end = there ? seq_start[lane + 1] : 0;
+        slot = there ? seq_slot[lane] : -1;
+        pos0 = there ? seq_pos0[lane] : 0;
+        const int mine = slot >= 0 ? (row_end - row0 + FT_BQ - 1) / FT_BQ : 0;
         int left = blockIdx.y;
         seq = -1;
         for (qt = n_tiles - 1; qt >= 0; --qt) {
@@ -138,11 +145,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             }
             left -= n;
         }
+        exists = seq >= 0;                           // (fewer tiles than places)
+        seq = max(seq, 0);
+        qt = max(qt, 0);
+        row0 = __shfl_sync(0xffffffffu, row0, seq);
+        row_end = __shfl_sync(0xffffffffu, row_end, seq);
+        slot = __shfl_sync(0xffffffffu, slot, seq);
+        pos0 = __shfl_sync(0xffffffffu, pos0, seq);
+    } else {
+        row0 = seq_start[seq];
+        row_end = seq_start[seq + 1];
+        slot = seq_slot[seq];
+        pos0 = seq_pos0[seq];
     }
-    const bool exists = seq >= 0;                    // (fewer tiles than places)
-    seq = max(seq, 0);
-    qt = max(qt, 0);
-    const int row0 = seq_start[seq], row_end = seq_start[seq + 1], slot = seq_slot[seq], pos0 = seq_pos0[seq];
     const int n_new = row_end - row0;
     const int hk = h / (H / Hkv);
     const int q_first = pos0 + qt * FT_BQ;                           // absolute position of the tile's first query
@@ -440,6 +455,18 @@ extern "C" int vlrf_attn_prefill_tc_max_parts() { return FT_MAX_PARTS; }
 extern "C" int vlrf_attn_prefill_tc_min_part_blocks() { return FT_MIN_PART; }
 extern "C" int vlrf_attn_prefill_tc_tile() { return FT_BQ; }
 
+// Whether the tiles that exist are listed, instead of a place for each that the longest sequence has: where they alone take the two places of
+// every SM, and as many CTAs without work again would come and go between them (five prompts of 1,013 to 31 tokens and three single tokens,
+// 25 heads, 600 of 1,600 CTAs: 42.8 -> 33.1 us; that step of GPT-2 XL 9,610 -> 9,343).  With fewer tiles than places the kernels behind, which may
+// begin once the last CTA has, begin while SMs idle and crowd onto those: whole prompt steps of GPT-2 with 216 of 660 and of 864 CTAs listed 818 ->
+// 841 and 915 -> 946 us, GPT-2 medium 272 of 880 1,816 -> 1,878; with 300 of 560 (large) 3,950 -> 4,007, with 320 of 880 3,069 -> 3,000.
+extern "C" int vlrf_attn_prefill_tc_lists(int n_tokens, int n_seqs, int max_new, int H, int n_parts, int sms) {
+    if (n_seqs < 2 || n_seqs > 32 || max_new > 64 * FT_BQ) return 0;          // (a lane of a warp per sequence)
+    const long long all = (long long)((max_new + FT_BQ - 1) / FT_BQ) * n_seqs, exist = (long long)n_tokens / FT_BQ + n_seqs;
+    const long long each = (long long)H * n_parts, full = 2ll * sms;
+    return exist * each >= full && (all - exist) * each >= full ? 1 : 0;
+}
+
 // n_parts > 1 wants `partials` ([sequences × heads × tiles × n_parts] × part_floats) and `counters`
 // ([sequences × heads × tiles], zero; left zero).
 extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const void* Kc, const void* Vc, int n_blocks,
@@ -470,10 +497,8 @@ extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const vo
     }
     const long long tiles = (max_new + FT_BQ - 1) / FT_BQ;
     VLRF_REQUIRE(tiles * n_parts <= 65535, "attn_prefill_tc: %lld tiles of %d parts are too many for one launch", tiles, n_parts);
-    // The tiles that exist are at most n_tokens / 128 + n_seqs: with sequences of unequal lengths far fewer than every sequence times the
-    // longest's (five prompts of 1,013 to 31 tokens and three single tokens, 25 heads: 22 of 64; 42.8 -> 33.1 us).
-    const long long places = (long long)n_tokens / FT_BQ + n_seqs;
-    const int listed = n_seqs > 1 && n_seqs <= 32 && tiles <= 64 && places < tiles * n_seqs ? n_seqs : 0;
+    const long long places = (long long)n_tokens / FT_BQ + n_seqs;      // the tiles that exist are at most so many
+    const int listed = vlrf_attn_prefill_tc_lists(n_tokens, n_seqs, max_new, H, n_parts, vlrf_sm_count()) ? n_seqs : 0;
     dim3 grid(H, listed ? (unsigned)places : n_seqs, (unsigned)(listed ? n_parts : tiles * n_parts));
     cudaError_t e = launch_chained(attn_prefill_tc_kernel, grid, dim3(FT_THREADS), smem, stream, tq, tk, tv, q_off, block_table,
                                    max_blocks, seq_slot, seq_start, seq_pos0, (__nv_bfloat16*)out, ld_out, H, Hkv, scale,

@@ -18,6 +18,7 @@
 extern "C" const char* vlrf_last_error();
 int vlrf_fail(int code, const char* fmt, ...);
 int vlrf_check_launch(const char* what);
+int vlrf_sm_count();                             // asked of the driver once: the query is slow next to a launch
 
 #define VLRF_REQUIRE(cond, ...) \
     do { if (!(cond)) return vlrf_fail(VLRF_ERR_INVALID_ARG, __VA_ARGS__); } while (0)

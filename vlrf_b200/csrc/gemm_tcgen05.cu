@@ -26,17 +26,6 @@
 
 namespace {
 
-int sm_count_cached() {                          // asked once: the query is slow next to a launch
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0, v = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-        sms = v > 0 ? v : 148;
-    }
-    return sms;
-}
-
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;           // elements of K in one 128-byte swizzle atom: what one TMA load and one descriptor cover
 // Atoms of K in a stage of the ring.  One thread issues the MMAs, and a stage costs it about 550 cycles whatever
@@ -477,7 +466,7 @@ int launch_tc(const void* X, const void* W, const float* bias, const float* resi
         raised = true;
     }
     const long long tiles = SWAP ? (N + TC_BM - 1) / TC_BM : (long long)((N + BN - 1) / BN) * ((M + TC_BM - 1) / TC_BM);
-    const int sms = sm_count_cached();
+    const int sms = vlrf_sm_count();
     dim3 grid((unsigned)(tiles < sms ? tiles : sms));          // persistent: one CTA per SM at most
     cudaError_t e = launch_chained(kern, grid, dim3(TC_THREADS), smem, stream, tx, tw, bias, residual, (OT*)Y, M, N, K, ldy,
                                    act, kv, dev_err, vlrf_trace_buffer(), TcGroups{});
@@ -532,7 +521,7 @@ extern "C" int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias
     // follows when all SMs run (measured over the products of GPT-2 small to XL at 512 to 8,192 rows)
     int best_bn = 128;
     {
-        const int sms = sm_count_cached();
+        const int sms = vlrf_sm_count();
         long long best = -1;
         const int widths[7] = {256, 224, 192, 160, 128, 96, 64};
         for (int i = 0; i < 7; ++i) {
@@ -594,7 +583,7 @@ int launch_tc_groups(const void* X, int ldx, const void* W, void* Y, int ldy, co
     }
     const int w_tile = SWAP ? TC_BM : BN;
     const long long tiles = gr_row_tiles(gr.rows, gr.G, gr.offsets != nullptr) * ((N + w_tile - 1) / w_tile);
-    const int sms = sm_count_cached();
+    const int sms = vlrf_sm_count();
     dim3 grid((unsigned)(tiles < sms ? tiles : sms));
     cudaError_t e = launch_chained(kern, grid, dim3(TC_THREADS), smem, stream, SWAP ? tw : tx, SWAP ? tx : tw, (const float*)nullptr,
                                    (const float*)nullptr, (OT*)Y, gr.rows, N, K, ldy, act, TcKvScatter{}, dev_err, vlrf_trace_buffer(), gr);
@@ -632,7 +621,7 @@ extern "C" int vlrf_gemm_tcgen05_groups(const void* X, int ldx, int x_gs, const 
     if (N <= 64) return GROUPS(64, 4, false);
     // the width by rounds and the bytes of a round, as for one matrix; half of a group's last tile is taken to be empty
     const long long row_tiles = offsets ? (rows + TC_BM - 1) / TC_BM + G / 2 : gr_row_tiles(rows, G, false);
-    const int sms = sm_count_cached();
+    const int sms = vlrf_sm_count();
     auto cost = [&](int bn) { return ((row_tiles * ((N + bn - 1) / bn) + sms - 1) / sms) * (bn + 128); };
     if (N > 128 && cost(256) < cost(128)) return GROUPS(256, 4, false);
     return GROUPS(128, 3, false);

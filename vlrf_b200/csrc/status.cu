@@ -20,6 +20,17 @@ int vlrf_check_launch(const char* what) {
     return VLRF_OK;
 }
 
+int vlrf_sm_count() {
+    static int sms = 0;
+    if (sms == 0) {
+        int dev = 0, v = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        sms = v > 0 ? v : 148;
+    }
+    return sms;
+}
+
 extern "C" int vlrf_device_info(int* sm_count, int* cc_major, int* cc_minor, int* max_smem_optin) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);

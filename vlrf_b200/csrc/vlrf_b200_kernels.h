@@ -153,6 +153,7 @@ int vlrf_attn_prefill_tc_takes(int dh, int BT, int ld, int q_off, int ld_out);
 int vlrf_attn_prefill_tc_part_floats();
 int vlrf_attn_prefill_tc_max_parts();
 int vlrf_attn_prefill_tc_min_part_blocks();
+int vlrf_attn_prefill_tc_lists(int n_tokens, int n_seqs, int max_new, int H, int n_parts, int sms);
 int vlrf_attn_prefill_tc_tile();
 int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const void* Kc, const void* Vc, int n_blocks,
                          const int* block_table, int max_blocks, const int* seq_slot, const int* seq_start,
