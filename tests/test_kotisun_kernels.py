@@ -410,6 +410,64 @@ def test_recurrence_in_chunks_keeps_to_the_past(where, Hs, P, N, G):
             assert torch.isfinite(got[1][0][:token]).all() and torch.isfinite(got[1][0][150:]).all()
 
 
+def chunk_step(lens, pos0, slots, Hs, P, N, G, g, extra=0):
+    """The inputs of a step of these runs: (arguments of the recurrence, state, context)."""
+    import types
+
+    from vlrf_b200.parts.context import Workspace
+    T, channels = sum(lens), Hs * P + 2 * G * N
+    start = [0]
+    for n in lens:
+        start.append(start[-1] + n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)   # noqa: E731
+    ctx = types.SimpleNamespace(n_tokens=T, n_seqs=len(lens), seq_slot=i32(slots), seq_start=i32(start), seq_pos0=i32(pos0), max_new=max(lens),
+                                min_new=min(lens), ws=Workspace(torch.device(DEV)), act_dtype=torch.bfloat16)
+    xbc, proj = torch.randn(T, channels, generator=g), torch.randn(T, 3 + Hs, generator=g)
+    a_log = torch.linspace(-6.0, 1.0, Hs)
+    weights = [dev(torch.randn(Hs, generator=g)), dev(a_log), dev(torch.randn(Hs, generator=g))]
+    state = torch.randn(max(slots) + 1, 2, Hs * N * P + extra, generator=g)
+    return (dev(xbc), dev(proj), 3, *weights), state, ctx
+
+
+def test_chunks_in_passes_and_without_scratch(monkeypatch):
+    """Scratch for every head, for three of five groups and for one at a time gives the same bits; with no room for it at all the step goes
+    token by token."""
+    from vlrf_b200.csrc import ops
+    Hs, P, N, G = 10, 68, 32, 5
+    args, state, ctx = chunk_step([400, 1, 90], [0, 5, 2], [2, 0, 1], Hs, P, N, G, torch.Generator().manual_seed(1))
+    slots, marks = ctx.n_tokens // 64 + 3, Hs * 2
+
+    def run(entry):
+        st, y = state.to(DEV), torch.full((ctx.n_tokens, Hs * P), float("nan"), device=DEV)
+        entry(*args, st, ctx, y, Hs, G, N, P)
+        return y.cpu(), st.cpu()
+    want = run(ops.ssd_chunks)
+    whole = ctx.ws.get("ssd_chunks", 1, 1, torch.float32).untyped_storage().nbytes()
+    assert whole == 4 * slots * (Hs * (N * P + 4) + marks)
+    for groups in (3, 1):
+        monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * groups * (N * P + 4) + marks) + 3)
+        ctx.ws = type(ctx.ws)(torch.device(DEV))
+        for a, b in zip(run(ops.ssd_chunks), want):
+            assert torch.equal(a, b)
+        assert ctx.ws.get("ssd_chunks", 1, 1, torch.float32).untyped_storage().nbytes() <= ops.SSD_CHUNKS_MAX_BYTES
+    monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * (N * P + 4) + marks) - 4)
+    assert not ops.ssd_chunks_takes(torch.bfloat16, ctx, Hs, G, N, P, args[0].shape[1], state.shape[2])
+    monkeypatch.undo()
+    real = torch.empty
+
+    def full(*a, **k):
+        if a and isinstance(a[0], int) and a[0] > 100000:
+            raise torch.OutOfMemoryError("no room")
+        return real(*a, **k)
+    ctx.ws = type(ctx.ws)(torch.device(DEV))
+    monkeypatch.setattr(torch, "empty", full)
+    got = run(ops.ssd_scan_step)
+    monkeypatch.undo()
+    for a, b in zip(got, want):
+        close(a, b, 1e-5, "token by token")
+    assert not torch.equal(got[0], want[0])
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 5])
 def test_convolution_over_runs(taps):
     """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a

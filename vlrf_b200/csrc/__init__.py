@@ -133,8 +133,8 @@ _SIGNATURES = {
     "vlrf_ssd_step": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p,
                       _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "vlrf_ssd_chunks_takes": [_c_int] * 6,
-    "vlrf_ssd_chunks_scratch": [_c_int] * 5 + [_c_void_p],
-    "vlrf_ssd_chunks": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
+    "vlrf_ssd_chunks_scratch": [_c_int] * 6 + [ctypes.c_longlong, _c_void_p],
+    "vlrf_ssd_chunks": [_c_void_p, _c_int, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, ctypes.c_longlong, _c_void_p, _c_int,
                         _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "vlrf_ssd_gate_norm": [_c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                            _c_float, _c_float, _c_void_p],

@@ -1230,34 +1230,35 @@ def attention_window_step(q, k_cache, v_cache, block_table, out, ctx, n_heads: i
                      second_map=second_map)
 
 
-#: Where a step's state-space recurrence runs in chunks: runs of at least so many new tokens, and at most so much scratch.  Token by token
+#: Where a step's state-space recurrence runs in chunks: runs of at least so many new tokens, in at most so much scratch.  Token by token
 #: takes as long as the longest run, in chunks hardly longer for a long one than for a short one: for 32 heads of 64 x 64, 256, 512, 1,024
 #: and 2 x 1,024 tokens 37, 70, 137, 137 against 47, 48, 52, 67 us, eight runs of 160 61 against 67 us; for 128 x 128 51, 98, 191, 343
-#: against 64, 76, 128, 289 us.
-SSD_CHUNKS, SSD_CHUNKS_MIN_RUN, SSD_CHUNKS_MAX_BYTES = True, 384, 8 << 30
+#: against 64, 76, 128, 289 us.  The scratch holds 7,800 tokens of 32 heads of 128 x 128 whole; more, or larger ones, take several passes.
+SSD_CHUNKS_MIN_RUN, SSD_CHUNKS_MAX_BYTES = 384, 256 << 20
 
 
-def _ssd_chunks_scratch(ctx, n_heads: int, n_state: int, p: int) -> int:
+def _ssd_chunks_scratch(ctx, n_heads: int, n_groups: int, n_state: int, p: int) -> int:
+    """float32 numbers of scratch for the step (0: it does not fit what it may have)."""
     import ctypes
 
     from . import call_host
     n = ctypes.c_longlong(0)
-    call_host("vlrf_ssd_chunks_scratch", ctx.n_tokens, ctx.n_seqs, n_heads, n_state, p, ctypes.byref(n))
+    call_host("vlrf_ssd_chunks_scratch", ctx.n_tokens, ctx.n_seqs, n_heads, n_groups, n_state, p, SSD_CHUNKS_MAX_BYTES // 4, ctypes.byref(n))
     return n.value
 
 
 def ssd_chunks_takes(dtype: torch.dtype, ctx, n_heads: int, n_groups: int, n_state: int, p: int, channels: int, state_row: int) -> bool:
     """Whether a step's state-space recurrence runs in chunks: the bfloat16 engine's (the 32-bit one keeps to FMAs), prompts only."""
-    if dtype != torch.bfloat16 or not SSD_CHUNKS or ctx.max_new < SSD_CHUNKS_MIN_RUN:
+    if dtype != torch.bfloat16 or ctx.max_new < SSD_CHUNKS_MIN_RUN:
         return False
     from . import library
-    if 4 * _ssd_chunks_scratch(ctx, n_heads, n_state, p) > SSD_CHUNKS_MAX_BYTES:
-        return False
-    return bool(library().vlrf_ssd_chunks_takes(n_heads, n_groups, n_state, p, channels, state_row))
+    return bool(library().vlrf_ssd_chunks_takes(n_heads, n_groups, n_state, p, channels, state_row)) \
+        and _ssd_chunks_scratch(ctx, n_heads, n_groups, n_state, p) > 0
 
 
 def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_heads: int, n_groups: int, n_state: int, p: int) -> None:
-    """`ssd_scan` of a prompt step in chunks (see the kernel library's header)."""
+    """`ssd_scan` of a prompt step in chunks (see the kernel library's header).  Raises torch.OutOfMemoryError, having launched nothing,
+    where its scratch cannot be had."""
     T = ctx.n_tokens
     _dev(xbc, "xbc", torch.float32); _rows(proj, "proj", torch.float32); _dev(state, "state", torch.float32); _dev(y, "y", torch.float32)
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
@@ -1266,9 +1267,10 @@ def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_
             raise KernelError(f"ssd_chunks: {name} has one number per head")
     if y.shape[1] != n_heads * p or state.dim() != 3 or state.shape[1] != 2 or min(xbc.shape[0], proj.shape[0], y.shape[0]) < T:
         raise KernelError("ssd_chunks: sizes do not match")
-    scratch = ctx.ws.get("ssd_chunks", 1, _ssd_chunks_scratch(ctx, n_heads, n_state, p), torch.float32)
+    n = _ssd_chunks_scratch(ctx, n_heads, n_groups, n_state, p)
+    scratch = ctx.ws.get("ssd_chunks", 1, n, torch.float32, exact=True)
     call("vlrf_ssd_chunks", _ptr(xbc), xbc.shape[1], _ptr(proj), proj.stride(0), dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-         _ptr(scratch), _ptr(state), state.shape[2], _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(y), T, ctx.n_seqs,
+         _ptr(scratch), n, _ptr(state), state.shape[2], _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(y), T, ctx.n_seqs,
          ctx.max_new, n_heads, n_groups, n_state, p, _stream())
 
 
@@ -1298,8 +1300,11 @@ def ssd_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_he
 def ssd_scan_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_heads: int, n_groups: int, n_state: int, p: int) -> None:
     """The recurrence of a step with the kernel that suits it."""
     if ssd_chunks_takes(ctx.act_dtype, ctx, n_heads, n_groups, n_state, p, xbc.shape[1], state.shape[2]):
-        ssd_chunks(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx, y, n_heads, n_groups, n_state, p)
-        return
+        try:
+            ssd_chunks(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx, y, n_heads, n_groups, n_state, p)
+            return
+        except torch.OutOfMemoryError:
+            pass                               # token by token needs no scratch
     if ssd_step_takes(ctx.act_dtype, ctx, n_heads, n_groups, n_state, p, xbc.shape[1], state.shape[2]):
         ssd_step(xbc, proj, dt_off, dt_bias, a_log, d_skip, state, ctx, y, n_heads, n_groups, n_state, p)
         return

@@ -31,7 +31,8 @@
 //
 // Layouts: q, k, v float32 rows of any stride (multiples of 4 numbers, on 16 bytes); scratch per chunk and head K·V float32, laid
 // out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a float4 per chunk and head; wild an int per
-// chunk, head and tile of 64 columns.
+// chunk, head and tile of 64 columns.  Heads are independent: where the scratch that a caller has does not hold every head's states, the three
+// kernels run over a range of groups at a time (a pass), one range after another in the same scratch.
 #include "common.cuh"
 #include "chunk_mma.cuh"
 
@@ -58,6 +59,9 @@ struct StateChunks {
     const int *seq_slot, *seq_start, *seq_pos0;
     float* y;
     int ldy, H, G, V;
+    int g0, groups;                    // the groups of this pass; scratch and aux hold their heads only
+    __host__ __device__ int per_group() const { return H / G; }
+    __host__ __device__ int heads() const { return groups * per_group(); }
 };
 
 // What a head's tokens of a chunk weigh.  Lp + Lo: the log decays of a token's block of 16 up to and with it, in two floats, for the
@@ -167,8 +171,8 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start;
     if (c0 >= n || A.seq_slot[s] < 0) return;
     const int L = min(RC, n - c0), first = start + c0;
-    const int g = blockIdx.y / parts, per_group = A.H / A.G, i0 = (blockIdx.y - g * parts) * R_ITEMS, items = min(R_ITEMS, per_group * v_tiles - i0);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int part = blockIdx.y % parts, g = A.g0 + blockIdx.y / parts, per_group = A.per_group(), i0 = part * R_ITEMS, items = min(R_ITEMS, per_group * v_tiles - i0);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, heads = A.heads(), h_first = A.g0 * per_group;
     const size_t chunk = (size_t)(start / RC + s + blockIdx.x);
     float4 x[4];                                                         // the next item's values, a quarter of a token's tile a thread
     auto ask = [&](int item) {
@@ -197,7 +201,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
             const int t = lane + 32 * e;
             weight[warp * RC + t] = expf(sc[warp].Ls[t] + sc[warp].after[t >> 4]) * sc[warp].gain[t];
         }
-        if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * A.H + h] = make_float4(sc[warp].before[3] + sc[warp].Lp[RC - 1], 0.f, 0.f, 0.f);
+        if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * heads + h - h_first] = make_float4(sc[warp].before[3] + sc[warp].Lp[RC - 1], 0.f, 0.f, 0.f);
     }
     rows_fine = load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid) && rows_fine;
     rows_fine = __syncthreads_and(rows_fine);
@@ -222,7 +226,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         fine = __syncthreads_and(fine);
         if (tid == 0) A.wild[(chunk * A.H + h) * v_tiles + v0 / RT] = fine ? 0 : 1;
         // 16 rows of the state by 32 columns at a time
-        float* U = A.scratch + (chunk * A.H + h) * (size_t)K * A.V;
+        float* U = A.scratch + (chunk * heads + h - h_first) * (size_t)K * A.V;
         for (int unit = warp; unit < K / 8; unit += R_THREADS / 32) {
             const int r0 = (unit >> 1) * 16, cc = (unit & 1) * 32;
             float acc[4][4];
@@ -264,16 +268,17 @@ state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
     const int s = blockIdx.y, slot = A.seq_slot[s];
     if (slot < 0) return;
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start, pos0 = A.seq_pos0[s];
-    const size_t all = (size_t)per_head * A.H, i = 4 * ((size_t)blockIdx.x * 128 + threadIdx.x);
+    const int heads = A.heads(), h_first = A.g0 * A.per_group();
+    const size_t all = (size_t)per_head * heads, i = 4 * ((size_t)blockIdx.x * 128 + threadIdx.x);
     if (i >= all || n <= 0) return;
-    const float* from = A.state + ((size_t)slot * 2 + (pos0 & 1)) * A.state_row;
-    float* to = A.state + ((size_t)slot * 2 + ((pos0 + n) & 1)) * A.state_row;
-    const int chunks = (n + RC - 1) / RC, h = (int)(i / per_head);
+    const float* from = A.state + ((size_t)slot * 2 + (pos0 & 1)) * A.state_row + (size_t)h_first * per_head;
+    float* to = A.state + ((size_t)slot * 2 + ((pos0 + n) & 1)) * A.state_row + (size_t)h_first * per_head;
+    const int chunks = (n + RC - 1) / RC, hl = (int)(i / per_head);
     float4 S = *reinterpret_cast<const float4*>(from + i);
     const size_t slot0 = (size_t)(start / RC + s);
     float* u = A.scratch + slot0 * all + i;
-    const float4* aux = A.aux + slot0 * A.H + h;
-    const int* wild = A.wild + (slot0 * A.H + h) * v_tiles + (int)(i % A.V) / RT;
+    const float4* aux = A.aux + slot0 * heads + hl;
+    const int* wild = A.wild + (slot0 * A.H + h_first + hl) * v_tiles + (int)(i % A.V) / RT;
     int any_wild = 0;
     constexpr int AHEAD = 8;                        // chunks asked for together
     for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
@@ -282,7 +287,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j) {
             U[j] = quad_or_zero(u + (size_t)(c0 + j) * all, c0 + j < chunks);
-            F[j] = c0 + j < chunks ? aux[(size_t)(c0 + j) * A.H].x : 0.f;
+            F[j] = c0 + j < chunks ? aux[(size_t)(c0 + j) * heads].x : 0.f;
             any_wild |= c0 + j < chunks ? wild[(size_t)(c0 + j) * A.H * v_tiles] : 0;
         }
 #pragma unroll
@@ -321,8 +326,9 @@ state_chunk_outputs_kernel(const StateChunks A, int v_tiles, int parts) {
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start;
     if (c0 >= n || A.seq_slot[s] < 0) return;
     const int L = min(RC, n - c0), first = start + c0;
-    const int grp = blockIdx.y / parts, per_group = A.H / A.G, i0 = (blockIdx.y - grp * parts) * R_ITEMS,
+    const int part = blockIdx.y % parts, grp = A.g0 + blockIdx.y / parts, per_group = A.per_group(), i0 = part * R_ITEMS,
               items = min(R_ITEMS, per_group * v_tiles - i0);
+    const int heads = A.heads(), h_first = A.g0 * per_group;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int rb = warp >> 1, cc = (warp & 1) * 32, row0 = rb * 16;
     const size_t chunk = (size_t)(start / RC + s + blockIdx.x);
@@ -335,7 +341,7 @@ state_chunk_outputs_kernel(const StateChunks A, int v_tiles, int parts) {
             const int r = tid / 16 + 16 * e, c = tid % 16 * 4;
             x[e] = quad_or_zero(A.v + (size_t)(first + r) * A.ldv + (size_t)h * A.V + v0 + c, r < L && v0 + c < A.V);
         }
-        const float* from = A.scratch + (chunk * A.H + h) * (size_t)K * A.V + v0;
+        const float* from = A.scratch + (chunk * heads + h - h_first) * (size_t)K * A.V + v0;
 #pragma unroll
         for (int e = 0; e < SE; ++e) {
             const int i = tid + e * R_THREADS, r = i / 16, c = i % 16 * 4;
@@ -471,12 +477,12 @@ template <int K> int launch_state_chunks(const StateChunks& A, int n_seqs, int m
         raised = true;
     }
     const int chunks = (max_new + RC - 1) / RC, v_tiles = (A.V + RT - 1) / RT, parts = (A.H / A.G * v_tiles + R_ITEMS - 1) / R_ITEMS;
-    VLRF_REQUIRE((long long)A.G * parts <= 65535, "state_chunks: too many heads");
-    const dim3 grid(chunks, A.G * parts, n_seqs);
+    VLRF_REQUIRE((long long)A.groups * parts <= 65535, "state_chunks: too many heads");
+    const dim3 grid(chunks, A.groups * parts, n_seqs);
     launch_chained(state_chunk_writes_kernel<K>, grid, dim3(R_THREADS), (size_t)writes_smem<K>(), stream, A, v_tiles, parts);
     int st = vlrf_check_launch("state_chunks: writes");
     if (st != VLRF_OK) return st;
-    const long long quads = (long long)A.H * K * A.V / 4;
+    const long long quads = (long long)A.heads() * K * A.V / 4;
     launch_chained(state_chunk_states_kernel, dim3((unsigned)((quads + 127) / 128), n_seqs), dim3(128), (size_t)0, stream, A, K * A.V, v_tiles);
     st = vlrf_check_launch("state_chunks: states");
     if (st != VLRF_OK) return st;
@@ -492,15 +498,27 @@ extern "C" int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, i
             state_row % 4 == 0 && channels == H * P + 2 * G * N) ? 1 : 0;
 }
 
-// float32 numbers of scratch of a step of T tokens in n_seqs sequences: a state, four numbers and the tiles' marks per chunk and head
-extern "C" int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int N, int P, long long* floats) {
-    VLRF_REQUIRE(T >= 0 && n_seqs >= 0 && H > 0 && N > 0 && P > 0 && floats != nullptr, "ssd_chunks_scratch: bad arguments");
-    *floats = ((long long)T / RC + n_seqs) * H * ((long long)N * P + 4 + (P + RT - 1) / RT);
+// How the groups of a step of T tokens in n_seqs sequences share scratch of at most `limit` numbers: how many a pass takes (0: not even
+// one fits), as evenly as passes allow.  Per chunk: a state and four numbers for every head of a pass, and the marks of all heads' tiles.
+static int chunk_groups(int T, int n_seqs, int H, int G, int N, int P, long long limit, long long* floats) {
+    const long long slots = (long long)T / RC + n_seqs, marks = slots * H * ((P + RT - 1) / RT), group = slots * (H / G) * ((long long)N * P + 4);
+    long long most = limit < marks ? 0 : (limit - marks) / group;
+    if (most > G) most = G;
+    if (most < 1) { *floats = 0; return 0; }
+    const int passes = (int)((G + most - 1) / most), groups = (G + passes - 1) / passes;
+    *floats = groups * group + marks;
+    return groups;
+}
+
+// float32 numbers of scratch that a step of T tokens in n_seqs sequences takes where it may have `limit`; 0: it cannot run in so little
+extern "C" int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int G, int N, int P, long long limit, long long* floats) {
+    VLRF_REQUIRE(T >= 0 && n_seqs > 0 && H > 0 && G > 0 && H % G == 0 && N > 0 && P > 0 && floats != nullptr, "ssd_chunks_scratch: bad arguments");
+    chunk_groups(T, n_seqs, H, G, N, P, limit, floats);
     return VLRF_OK;
 }
 
 extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
-                               const float* D, float* scratch, float* state, int state_row, const int* seq_slot, const int* seq_start,
+                               const float* D, float* scratch, long long scratch_floats, float* state, int state_row, const int* seq_slot, const int* seq_start,
                                const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int H, int G, int N, int P, cudaStream_t stream) {
     VLRF_REQUIRE(vlrf_ssd_chunks_takes(H, G, N, P, channels, state_row), "ssd_chunks: a state of %d by %d or the rows' strides are not taken", N, P);
     VLRF_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && n_seqs <= 65535 && max_new >= 0 && scratch != nullptr && dt_off + H <= ld, "ssd_chunks: bad arguments");
@@ -511,17 +529,23 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
     A.v = xbc; A.k = xbc + (size_t)H * P; A.q = A.k + (size_t)G * N;
     A.ldq = A.ldk = A.ldv = channels;
     A.s0 = proj + dt_off; A.ld_s0 = ld; A.dt_bias = dt_bias; A.a_log = a_log; A.skip = D;
-    A.aux = reinterpret_cast<float4*>(scratch);
-    const size_t slots = ((size_t)n_tokens / RC + n_seqs) * H;          // (chunk, head)
-    A.scratch = scratch + slots * 4;
-    A.wild = reinterpret_cast<int*>(A.scratch + slots * (size_t)N * P);
     A.state = state; A.state_row = state_row; A.seq_slot = seq_slot; A.seq_start = seq_start; A.seq_pos0 = seq_pos0;
     A.y = y; A.ldy = H * P; A.H = H; A.G = G; A.V = P;
-    const int st = N == 16   ? launch_state_chunks<16>(A, n_seqs, max_new, stream)
-                   : N == 32 ? launch_state_chunks<32>(A, n_seqs, max_new, stream)
-                   : N == 64 ? launch_state_chunks<64>(A, n_seqs, max_new, stream)
-                             : launch_state_chunks<128>(A, n_seqs, max_new, stream);
-    if (st != VLRF_OK) return st;
+    long long floats = 0;
+    const int groups = chunk_groups(n_tokens, n_seqs, H, G, N, P, scratch_floats, &floats);
+    VLRF_REQUIRE(groups > 0, "ssd_chunks: %lld numbers of scratch do not hold a group's chunks", scratch_floats);
+    const size_t slots = ((size_t)n_tokens / RC + n_seqs) * groups * (H / G);          // (chunk, head of a pass)
+    A.aux = reinterpret_cast<float4*>(scratch);
+    A.scratch = scratch + slots * 4;
+    A.wild = reinterpret_cast<int*>(A.scratch + slots * (size_t)N * P);
+    for (A.g0 = 0; A.g0 < G; A.g0 += groups) {
+        A.groups = G - A.g0 < groups ? G - A.g0 : groups;
+        const int st = N == 16   ? launch_state_chunks<16>(A, n_seqs, max_new, stream)
+                       : N == 32 ? launch_state_chunks<32>(A, n_seqs, max_new, stream)
+                       : N == 64 ? launch_state_chunks<64>(A, n_seqs, max_new, stream)
+                                 : launch_state_chunks<128>(A, n_seqs, max_new, stream);
+        if (st != VLRF_OK) return st;
+    }
     return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
                                 max_new, H, G, N, P, ScanRuns{1, 0, 1, A.wild}, stream);
 }

@@ -36,7 +36,9 @@ class Workspace:
         #: whose last write also made the next block's read says so here; forgotten by the model at every step's start
         self.normed_ready = None
 
-    def get(self, name: str, rows: int, cols: int, dtype: torch.dtype) -> torch.Tensor:
+    def get(self, name: str, rows: int, cols: int, dtype: torch.dtype, exact: bool = False) -> torch.Tensor:
+        """`exact`: a buffer that grows takes what is asked for instead of twice what it had (for large ones), and gives back
+        what it had first."""
         key = (name, rows, cols, dtype)
         view = self._views.get(key)
         if view is not None:
@@ -47,8 +49,13 @@ class Workspace:
             if self.frozen:
                 raise RuntimeError(f"workspace '{name}' would have to grow while a captured step uses it")
             cap = max(n, 1)
-            if buf is not None and buf.dtype == dtype:
+            if buf is not None and buf.dtype == dtype and not exact:
                 cap = max(cap, 2 * buf.numel())
+            if exact:
+                self.generation += 1             # (the old buffer goes even if there is no room for the new one)
+                self._views.clear()
+                self._bufs.pop(name, None)
+                buf = None
             buf = torch.empty(cap, dtype=dtype, device=self.device)
             self._bufs[name] = buf
             self.generation += 1
