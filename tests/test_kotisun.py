@@ -197,3 +197,47 @@ def test_trace_replay_of_a_batch_of_unequal_requests(kot_dirs, truth, tmp_path):
             fed[k] += 1
         live = [k for k in live if fed[k] < len(reqs[k])]
     rp.close()
+
+
+def test_long_prompts_and_what_joins_them(kot_dirs, monkeypatch):
+    """bfloat16: prompts above the length from which the recurrence runs in chunks, alone and in a step with a shorter one and single tokens,
+    then token by token; the second and third time the prompt step is captured and replayed."""
+    from vlrf_b200.csrc import ops
+    from vlrf_b200.engine.step import StepEntry
+    cfg, w = plain.read_model_dir(kot_dirs["kot_sharp"])
+    lens = [ops.SSD_CHUNKS_MIN_RUN + 120 + 6, ops.SSD_CHUNKS_MIN_RUN + 6, 90 + 6, 40, 21]
+    reqs = [random_ids(cfg["vocab"], n, 400 + i) for i, n in enumerate(lens)]
+    want = [plain.logits_all_positions(cfg, w, ids) for ids in reqs]
+    ran, real = [], {n: getattr(ops, n) for n in ("ssd_chunks", "ssd_scan", "ssd_step")}
+    for n in real:
+        monkeypatch.setattr(ops, n, lambda *a, n=n, **k: (ran.append(n), real[n](*a, **k)))
+    eng = make_engine(kot_dirs, "kot_sharp", "bfloat16", 2048)
+    compare(drive_whole(eng, reqs[:1]), want[:1], "bfloat16", "a long prompt", "kot_sharp")
+    assert set(ran) == {"ssd_chunks"}
+    graphs = 0
+    for _ in range(3):
+        ran.clear()
+        slots = [eng.start_sequence() for _ in reqs]
+        got = [[] for _ in reqs]
+        fed = [0] * len(reqs)
+
+        def step(news):
+            entries = [StepEntry(slots[i], reqs[i][fed[i]:fed[i] + n], list(range(n))) for i, n in news]
+            logits, at = eng.step(entries).float().cpu(), 0
+            for i, n in news:
+                got[i].append(logits[at:at + n].clone())
+                fed[i] += n
+                at += n
+        step([(3, 39), (4, 20)])
+        step([(3, 1), (0, lens[0] - 6), (2, 90), (4, 1), (1, lens[1] - 6)])
+        if ran:
+            assert {"ssd_chunks", "ssd_step"} <= set(ran)
+        for _ in range(6):
+            step([(0, 1), (1, 1), (2, 1)])
+        compare([torch.cat(g) for g in got], want, "bfloat16", "long prompts and what joins them", "kot_sharp")
+        for s in slots:
+            eng.end_sequence(s)
+        graphs = max(graphs, len(eng._graphs))
+    assert graphs > 0 and "ssd_chunks" not in ran                     # (the last time the prompt steps were replayed)
+    eng.check_device_errors()
+    eng.cache.check()

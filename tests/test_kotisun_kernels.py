@@ -468,6 +468,75 @@ def test_chunks_in_passes_and_without_scratch(monkeypatch):
     assert not torch.equal(got[0], want[0])
 
 
+def test_a_sequence_does_not_see_what_shares_its_step():
+    """Single tokens, runs below and at the chunks' least length, and long ones: each has, bit for bit, the results and the state that it has
+    in a step of its own, whatever the longest run of the step is."""
+    from vlrf_b200.csrc import ops
+    Hs, P, N, G = 4, 64, 64, 2
+    least = ops.SSD_CHUNKS_MIN_RUN
+    lens, pos0, slots = [1, least - 1, least, 2, 1, 700, 65], [9, 0, 2, 3, 0, 7, 128], [3, 0, 6, 2, 5, 1, 4]
+    args, state, ctx = chunk_step(lens, pos0, slots, Hs, P, N, G, torch.Generator().manual_seed(3))
+    xbc, proj = args[:2]
+
+    def run(some):
+        rows = torch.cat([torch.arange(sum(lens[:i]), sum(lens[:i + 1])) for i in some]).to(DEV)
+        _, _, c = chunk_step([lens[i] for i in some], [pos0[i] for i in some], [slots[i] for i in some], Hs, P, N, G, torch.Generator())
+        st, y = state.to(DEV), torch.full((len(rows), Hs * P), float("nan"), device=DEV)
+        ops.ssd_scan_step(xbc[rows], proj[rows], *args[2:], st, c, y, Hs, G, N, P)
+        return y.cpu(), st.cpu()
+    own = [run([i]) for i in range(len(lens))]
+    for some in (range(7), [0, 1, 3, 4, 6], [5, 4], [0, 4], [3, 0], [6, 5, 2, 1]):
+        y, st = run(list(some))
+        assert torch.isfinite(y).all()
+        at = 0
+        for i in some:
+            assert torch.equal(y[at:at + lens[i]], own[i][0]), (list(some), i)
+            assert torch.equal(st[slots[i]], own[i][1][slots[i]]), (list(some), i)
+            at += lens[i]
+
+
+def test_long_runs_in_chunks():
+    """Runs at the length from which the library takes chunks, and at the edges of the eight chunks that a state's thread asks for together,
+    beside single tokens, from zero and from kept states, through the rule that chooses the kernels; a kept state shows in the last token
+    (decays down to e^-0.002 a token).  As far from the float64 recurrence as token by token is, or within 2^-21 of the largest result."""
+    from vlrf_b200.csrc import ops
+    Hs, P, N, G = 4, 64, 64, 2
+    lens, pos0, slots = [383, 1, 384, 512, 513, 1, 1100], [0, 5, 0, 2, 7, 0, 64], [0, 1, 2, 3, 4, 5, 6]
+    args, state, ctx = chunk_step(lens, pos0, slots, Hs, P, N, G, torch.Generator().manual_seed(4))
+    for i, p in enumerate(pos0):
+        if p == 0:
+            state[slots[i], 0] = 0.0
+    xbc, proj = args[0].cpu().double(), args[1].cpu().double()
+    dt_bias, a_log, D = (t.cpu().double() for t in args[3:])
+    a_log = a_log.float()                                              # (as the kernel has it)
+    want, ends, at, inner = [], [], 0, Hs * P
+    for n, p, s in zip(lens, pos0, slots):
+        x, B, C = xbc[at:at + n, :inner].reshape(n, Hs, P), xbc[at:at + n, inner:inner + G * N], xbc[at:at + n, inner + G * N:]
+        B, C = (t.reshape(n, G, N).repeat_interleave(Hs // G, 1) for t in (B, C))
+        step = plain.softplus(proj[at:at + n, 3:] + dt_bias)
+        S, y = state[s, p & 1].double().reshape(Hs, N, P).clone(), torch.empty(n, Hs, P, dtype=torch.float64)
+        for t in range(n):
+            S = torch.exp(-torch.exp(a_log.double()) * step[t])[:, None, None] * S + (step[t][:, None] * B[t])[:, :, None] * x[t][:, None, :]
+            y[t] = (S * C[t][:, :, None]).sum(1) + D[:, None] * x[t]
+        want.append(y.reshape(n, inner)); ends.append(S); at += n
+    off = {}
+    for chunked in (False, True):
+        st, y = state.to(DEV), torch.full((at, inner), float("nan"), device=DEV)
+        if chunked:
+            assert ops.ssd_chunks_takes(torch.bfloat16, ctx, Hs, G, N, P, args[0].shape[1], state.shape[2])
+            ops.ssd_scan_step(*args, st, ctx, y, Hs, G, N, P)
+        else:
+            ops.ssd_scan(*args, st, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, ctx.n_seqs, Hs, G, N, P, ctx.max_new)
+        y, st, i, off[chunked] = y.cpu().double(), st.cpu(), 0, []
+        for n, p, s, w, e in zip(lens, pos0, slots, want, ends):
+            got = y[i:i + n]
+            off[chunked].append(float((got - w).norm() / w.norm()))
+            assert float((got[-1] - w[-1]).abs().max() / w.abs().max()) < 1e-5, (n, "last token")
+            close(st[s, (p + n) & 1].reshape(Hs, N, P), e, 1e-5, f"state of slot {s}")
+            i += n
+    assert all(a <= max(1.5 * b, 2.0 ** -21) for a, b in zip(off[True], off[False])), off
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 5])
 def test_convolution_over_runs(taps):
     """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a

@@ -505,10 +505,10 @@ int vlrf_launch_ssd_scan(const float* xbc, int channels, const float* proj, int 
 
 extern "C" int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias,
                              const float* a_log, const float* D, float* state, int state_row, const int* seq_slot,
-                             const int* seq_start, const int* seq_pos0, float* y, int n_seqs, int max_new, int Hs, int G, int N, int P,
+                             const int* seq_start, const int* seq_pos0, float* y, int n_seqs, int max_new, int least, int Hs, int G, int N, int P,
                              cudaStream_t stream) {
     return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
-                                max_new, Hs, G, N, P, ScanRuns{0, 0x7fffffff, 0x7fffffff, nullptr}, stream);
+                                max_new, Hs, G, N, P, ScanRuns{least, 0x7fffffff, 0x7fffffff, nullptr}, stream);
 }
 
 // Whether the decode step's kernel takes these sizes: quads of columns on 16 bytes, at most 512 rows.

@@ -59,6 +59,7 @@ struct StateChunks {
     const int *seq_slot, *seq_start, *seq_pos0;
     float* y;
     int ldy, H, G, V;
+    int least;                         // tokens of the runs that are taken here
     int g0, groups;                    // the groups of this pass; scratch and aux hold their heads only
     __host__ __device__ int per_group() const { return H / G; }
     __host__ __device__ int heads() const { return groups * per_group(); }
@@ -169,7 +170,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
     __shared__ bool item_fine[R_ITEMS];
     const int s = blockIdx.z, c0 = blockIdx.x * RC;
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start;
-    if (c0 >= n || A.seq_slot[s] < 0) return;
+    if (c0 >= n || n < A.least || A.seq_slot[s] < 0) return;
     const int L = min(RC, n - c0), first = start + c0;
     const int part = blockIdx.y % parts, g = A.g0 + blockIdx.y / parts, per_group = A.per_group(), i0 = part * R_ITEMS, items = min(R_ITEMS, per_group * v_tiles - i0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, heads = A.heads(), h_first = A.g0 * per_group;
@@ -270,7 +271,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start, pos0 = A.seq_pos0[s];
     const int heads = A.heads(), h_first = A.g0 * A.per_group();
     const size_t all = (size_t)per_head * heads, i = 4 * ((size_t)blockIdx.x * 128 + threadIdx.x);
-    if (i >= all || n <= 0) return;
+    if (i >= all || n < A.least) return;
     const float* from = A.state + ((size_t)slot * 2 + (pos0 & 1)) * A.state_row + (size_t)h_first * per_head;
     float* to = A.state + ((size_t)slot * 2 + ((pos0 + n) & 1)) * A.state_row + (size_t)h_first * per_head;
     const int chunks = (n + RC - 1) / RC, hl = (int)(i / per_head);
@@ -324,7 +325,7 @@ state_chunk_outputs_kernel(const StateChunks A, int v_tiles, int parts) {
     float* col_all = reinterpret_cast<float*>(sc + R_ITEMS);             // [warps][64]
     const int s = blockIdx.z, c0 = blockIdx.x * RC;
     const int start = A.seq_start[s], n = A.seq_start[s + 1] - start;
-    if (c0 >= n || A.seq_slot[s] < 0) return;
+    if (c0 >= n || n < A.least || A.seq_slot[s] < 0) return;
     const int L = min(RC, n - c0), first = start + c0;
     const int part = blockIdx.y % parts, grp = A.g0 + blockIdx.y / parts, per_group = A.per_group(), i0 = part * R_ITEMS,
               items = min(R_ITEMS, per_group * v_tiles - i0);
@@ -519,9 +520,11 @@ extern "C" int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int G, int N, i
 
 extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                                const float* D, float* scratch, long long scratch_floats, float* state, int state_row, const int* seq_slot, const int* seq_start,
-                               const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int H, int G, int N, int P, cudaStream_t stream) {
+                               const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int chunked, int scanned, int H, int G, int N,
+                               int P, cudaStream_t stream) {
     VLRF_REQUIRE(vlrf_ssd_chunks_takes(H, G, N, P, channels, state_row), "ssd_chunks: a state of %d by %d or the rows' strides are not taken", N, P);
-    VLRF_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && n_seqs <= 65535 && max_new >= 0 && scratch != nullptr && dt_off + H <= ld, "ssd_chunks: bad arguments");
+    VLRF_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && n_seqs <= 65535 && max_new >= 0 && scratch != nullptr && dt_off + H <= ld && chunked >= 1 && scanned >= 1,
+                 "ssd_chunks: bad arguments");
     VLRF_REQUIRE((size_t)H * N * P <= (size_t)state_row, "ssd_chunks: the state row does not hold the states");
     VLRF_REQUIRE(sc_on16(xbc) && sc_on16(scratch) && sc_on16(state) && sc_on16(y), "ssd_chunks: misaligned rows");
     if (n_seqs == 0 || max_new == 0) return VLRF_OK;
@@ -530,6 +533,7 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
     A.ldq = A.ldk = A.ldv = channels;
     A.s0 = proj + dt_off; A.ld_s0 = ld; A.dt_bias = dt_bias; A.a_log = a_log; A.skip = D;
     A.state = state; A.state_row = state_row; A.seq_slot = seq_slot; A.seq_start = seq_start; A.seq_pos0 = seq_pos0;
+    A.least = chunked;
     A.y = y; A.ldy = H * P; A.H = H; A.G = G; A.V = P;
     long long floats = 0;
     const int groups = chunk_groups(n_tokens, n_seqs, H, G, N, P, scratch_floats, &floats);
@@ -547,5 +551,5 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
         if (st != VLRF_OK) return st;
     }
     return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
-                                max_new, H, G, N, P, ScanRuns{1, 0, 1, A.wild}, stream);
+                                max_new, H, G, N, P, ScanRuns{scanned, chunked - 1, chunked, A.wild}, stream);
 }

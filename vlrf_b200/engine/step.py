@@ -55,7 +55,7 @@ class Engine:
         # Steps of a shape seen before are replayed from a captured CUDA graph: the step's integer tables
         # live at fixed device addresses, so only their contents change from step to step.
         self.capture_repeated_steps = True
-        self._graphs: dict = {}        # (tokens, sequences, longest run, wanted rows) -> (graph, logits)
+        self._graphs: dict = {}        # (tokens, sequences, longest and shortest run, wanted rows, from the start) -> (graph, logits)
         self._seen: dict = {}
         self._graph_generation = -1
         from ..csrc import ops
@@ -174,10 +174,10 @@ class Engine:
             seq_start=views[4], seq_pos0=views[5], max_new=max(p["lens"]),
             max_context=max(a + b for a, b in zip(p["pos0"], p["lens"])), logit_rows=views[6],
             n_logit_rows=n_want, act_dtype=self.model.act_dtype, dev_err=self.dev_err, ws=self.ws,
-            host_seq_slots=[e.slot for e in entries], host_seq_lens=p["lens"], host_seq_pos0=p["pos0"])
+            host_seq_slots=[e.slot for e in entries], host_seq_lens=p["lens"], host_seq_pos0=p["pos0"], min_new=min(p["lens"]))
         # (a captured step is replayed for steps of the same sizes; whether every sequence begins at its first token
-        # belongs to them, since parts may launch other kernels for such a step)
-        logits = self._forward(ctx, (T, B, ctx.max_new, n_want, not any(p["pos0"])))
+        # belongs to them, since parts may launch other kernels for such a step, as do the longest and the shortest run)
+        logits = self._forward(ctx, (T, B, ctx.max_new, ctx.min_new, n_want, not any(p["pos0"])))
         for e in entries:
             self.cache.advance(e.slot, len(e.tokens))
         self.steps_run += 1

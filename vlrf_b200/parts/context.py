@@ -118,5 +118,7 @@ class StepContext:
     host_seq_slots: list = dataclasses.field(default_factory=list)
     host_seq_lens: list = dataclasses.field(default_factory=list)
     host_seq_pos0: list = dataclasses.field(default_factory=list)
+    #: shortest run of new tokens of one sequence, where it is known (1 says nothing)
+    min_new: int = 1
     #: the block that the model runs after the one it is calling (None behind the last): a block may prepare its input
     next_block: object = None
