@@ -3,18 +3,6 @@
 #pragma once
 #include "common.cuh"
 
-// Tokens of a chunk and columns of a state's tile (state_chunks.cu).
-constexpr int STATE_CHUNK = 64, STATE_TILE = 64;
-// Which sequences the token-by-token recurrence of ssd.cu serves: runs of `least` to `most` tokens, and of runs of at least `chunked` tokens the
-// columns that the chunks left to it (wild: see state_chunks.cu; may be null).
-struct ScanRuns {
-    int least, most, chunked;
-    const int* wild;
-};
-int vlrf_launch_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
-                         const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
-                         float* y, int n_seqs, int max_new, int Hs, int G, int N, int P, ScanRuns runs, cudaStream_t stream);
-
 __device__ __forceinline__ uint32_t fc_sm(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // 16 bytes, or zeros where there is nothing
 __device__ __forceinline__ void fc_cp16(void* dst, const void* src, bool there) {

@@ -1139,8 +1139,8 @@ def ssd_conv(proj, x_off: int, weight, bias, state, conv_off: int, seq_slot, seq
 
 
 def ssd_scan(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, seq_slot, seq_start, seq_pos0, y, n_seqs: int, n_heads: int,
-             n_groups: int, n_state: int, p: int, max_new: int = 16, least: int = 0) -> None:
-    """The recurrence over the new tokens of every sequence that brings at least `least`, from and into the state rows; y float32
+             n_groups: int, n_state: int, p: int, max_new: int = 16, least: int = 0, most: int = 2 ** 31 - 1) -> None:
+    """The recurrence over the new tokens of every sequence that brings `least` to `most`, from and into the state rows; y float32
     [T, heads·p]."""
     _dev(xbc, "xbc", torch.float32); _rows(proj, "proj", torch.float32); _dev(state, "state", torch.float32); _dev(y, "y", torch.float32)
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
@@ -1150,8 +1150,8 @@ def ssd_scan(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, seq_slot, se
     if y.shape[1] != n_heads * p or state.dim() != 3 or state.shape[1] != 2:
         raise KernelError("ssd_scan: sizes do not match")
     call("vlrf_ssd_scan", _ptr(xbc), xbc.shape[1], _ptr(proj), proj.stride(0), dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
-         _ptr(state), state.shape[2], _ptr(seq_slot), _ptr(seq_start), _ptr(seq_pos0), _ptr(y), n_seqs, int(max_new), int(least), n_heads,
-         n_groups, n_state, p, _stream())
+         _ptr(state), state.shape[2], _ptr(seq_slot), _ptr(seq_start), _ptr(seq_pos0), _ptr(y), n_seqs, int(max_new), int(least),
+         int(most), n_heads, n_groups, n_state, p, _stream())
 
 
 def ssd_gate_norm(y, proj, z_off: int, weight, groups: int, eps: float, factor: float, out, n_rows: int) -> None:
@@ -1258,9 +1258,9 @@ def ssd_chunks_takes(dtype: torch.dtype, ctx, n_heads: int, n_groups: int, n_sta
 
 
 def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_heads: int, n_groups: int, n_state: int, p: int,
-               chunked: int = 1, scanned: int = 1) -> None:
-    """`ssd_scan` of a prompt step: runs of at least `chunked` tokens in chunks, those of `scanned` to `chunked` − 1 token by token, shorter ones
-    left out (see the kernel library's header).  Raises torch.OutOfMemoryError, having launched nothing, where its scratch cannot be had."""
+               chunked: int = 1) -> None:
+    """`ssd_scan` of a prompt step's runs of at least `chunked` tokens in chunks (see the kernel library's header).  Raises
+    torch.OutOfMemoryError, having launched nothing, where its scratch cannot be had."""
     T = ctx.n_tokens
     _dev(xbc, "xbc", torch.float32); _rows(proj, "proj", torch.float32); _dev(state, "state", torch.float32); _dev(y, "y", torch.float32)
     for name, t in (("dt_bias", dt_bias), ("a_log", a_log), ("d_skip", d_skip)):
@@ -1273,7 +1273,7 @@ def ssd_chunks(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y, n_
     scratch = ctx.ws.get("ssd_chunks", 1, n, torch.float32, exact=True)
     call("vlrf_ssd_chunks", _ptr(xbc), xbc.shape[1], _ptr(proj), proj.stride(0), dt_off, _ptr(dt_bias), _ptr(a_log), _ptr(d_skip),
          _ptr(scratch), n, _ptr(state), state.shape[2], _ptr(ctx.seq_slot), _ptr(ctx.seq_start), _ptr(ctx.seq_pos0), _ptr(y), T, ctx.n_seqs,
-         ctx.max_new, chunked, scanned, n_heads, n_groups, n_state, p, _stream())
+         ctx.max_new, chunked, n_heads, n_groups, n_state, p, _stream())
 
 
 def _ssd_step_sizes(dtype: torch.dtype, n_heads: int, n_groups: int, n_state: int, p: int, channels: int, state_row: int) -> bool:
@@ -1309,16 +1309,17 @@ def ssd_scan_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y,
     args, sizes = (xbc, proj, dt_off, dt_bias, a_log, d_skip, state), (n_heads, n_groups, n_state, p)
     takes = sizes + (xbc.shape[1], state.shape[2])
     ones = _ssd_step_sizes(ctx.act_dtype, *takes)                      # single tokens have a kernel of their own
-    if not (ones and ctx.max_new == 1):
-        chunks = ssd_chunks_takes(ctx.act_dtype, ctx, *takes)
-        if chunks:
-            try:
-                ssd_chunks(*args, ctx, y, *sizes, chunked=SSD_CHUNKS_MIN_RUN, scanned=2 if ones else 1)
-            except torch.OutOfMemoryError:
-                chunks = False                                         # token by token needs no scratch
-        if not chunks:
-            ssd_scan(*args, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, ctx.n_seqs, *sizes, ctx.max_new, 2 if ones else 0)
-    if ones and getattr(ctx, "min_new", 1) == 1 and (ctx.max_new == 1 or ctx.n_seqs > 1):
+    shortest = ctx.max_new if ctx.n_seqs == 1 else getattr(ctx, "min_new", 1)
+    left = ctx.max_new                                                 # runs up to here are not in chunks
+    if ssd_chunks_takes(ctx.act_dtype, ctx, *takes):
+        try:
+            ssd_chunks(*args, ctx, y, *sizes, SSD_CHUNKS_MIN_RUN)
+            left = SSD_CHUNKS_MIN_RUN - 1
+        except torch.OutOfMemoryError:
+            pass                                                       # token by token needs no scratch
+    if left > (1 if ones else 0) and shortest <= left:
+        ssd_scan(*args, ctx.seq_slot, ctx.seq_start, ctx.seq_pos0, y, ctx.n_seqs, *sizes, min(left, ctx.max_new), 2 if ones else 0, left)
+    if ones and shortest == 1:
         ssd_step(*args, ctx, y, *sizes)
 
 

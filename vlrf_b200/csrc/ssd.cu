@@ -24,7 +24,6 @@
 //   ssd_step        one token a sequence, for the bfloat16 engine: the same state, sums over its rows in another order
 //   ssd_gate_norm   y · (z·sigmoid(z)), RMS norm in equal groups, weight, a factor; rounded to the activation dtype
 #include "common.cuh"
-#include "chunk_mma.cuh"
 
 namespace {
 constexpr int CONV_RUN = 16;
@@ -138,7 +137,7 @@ __global__ void __launch_bounds__(512)
 ssd_scan_kernel(const float* __restrict__ xbc, int channels, const float* __restrict__ proj, int ld, int dt_off,
                 const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ Dv,
                 float* __restrict__ state, int state_row, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
-                const int* __restrict__ seq_pos0, float* __restrict__ y, int Hs, int G, int N, int P, int PB, int SC_BATCH, const ScanRuns runs) {
+                const int* __restrict__ seq_pos0, float* __restrict__ y, int Hs, int G, int N, int P, int PB, int SC_BATCH, int least, int most) {
     pdl_wait();
     pdl_launch_dependents();
     // shared memory: the C-weighted sums of the slices [2][SC_BATCH][slices][32], then per stage the batch's inputs:
@@ -149,14 +148,7 @@ ssd_scan_kernel(const float* __restrict__ xbc, int channels, const float* __rest
     const int slot = seq_slot[s];
     if (slot < 0) return;
     const int start = seq_start[s], n = seq_start[s + 1] - start, pos0 = seq_pos0[s];
-    if (n < runs.least || n > runs.most) {
-        if (n < runs.chunked || runs.wild == nullptr) return;
-        const int chunks = (n + STATE_CHUNK - 1) / STATE_CHUNK, tiles = (P + STATE_TILE - 1) / STATE_TILE;
-        const int* w = runs.wild + ((size_t)(start / STATE_CHUNK + s) * Hs + h) * tiles + pb * 32 / STATE_TILE;
-        int any = 0;
-        for (int c = threadIdx.x; c < chunks; c += blockDim.x) any |= w[(size_t)c * Hs * tiles];
-        if (!__syncthreads_or(any)) return;
-    }
+    if (n < least || n > most) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, slices = blockDim.x >> 5;
     const int NP = (N + 3) & ~3, stage_floats = SC_BATCH * (32 + 2 * NP);
     float* part_sm = sc_sm;
@@ -471,9 +463,10 @@ extern "C" int vlrf_ssd_conv(const float* proj, int ld, int x_off, const float* 
     return VLRF_OK;
 }
 
-int vlrf_launch_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
-                         const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
-                         float* y, int n_seqs, int max_new, int Hs, int G, int N, int P, ScanRuns runs, cudaStream_t stream) {
+extern "C" int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias,
+                             const float* a_log, const float* D, float* state, int state_row, const int* seq_slot,
+                             const int* seq_start, const int* seq_pos0, float* y, int n_seqs, int max_new, int least, int most, int Hs, int G,
+                             int N, int P, cudaStream_t stream) {
     VLRF_REQUIRE(n_seqs >= 0 && Hs > 0 && G > 0 && N > 0 && P > 0, "ssd_scan: bad sizes");
     VLRF_REQUIRE(Hs % G == 0, "ssd_scan: %d heads cannot share %d groups", Hs, G);
     VLRF_REQUIRE(N <= 512, "ssd_scan: a state of %d rows is above 512", N);
@@ -494,21 +487,13 @@ int vlrf_launch_ssd_scan(const float* xbc, int channels, const float* proj, int 
     const int batch = max_new < 1 ? 1 : max_new < SC_MAX_BATCH ? max_new : SC_MAX_BATCH;
     const size_t smem = (size_t)(2 * batch * slices * 32 + 2 * batch * (32 + 2 * ((N + 3) & ~3))) * sizeof(float);
 #define GO(R, V) scan_allow_smem<R, V>(smem); launch_chained(ssd_scan_kernel<R, V>, grid, block, smem, stream, xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, \
-                                state_row, seq_slot, seq_start, seq_pos0, y, Hs, G, N, P, PB, batch, runs)
+                                state_row, seq_slot, seq_start, seq_pos0, y, Hs, G, N, P, PB, batch, least, most)
     if (NR == 4) { if (vec) { GO(4, true); } else { GO(4, false); } }
     else if (NR == 8) { if (vec) { GO(8, true); } else { GO(8, false); } }
     else if (NR == 16) { if (vec) { GO(16, true); } else { GO(16, false); } }
     else { if (vec) { GO(32, true); } else { GO(32, false); } }
 #undef GO
     return vlrf_check_launch("ssd_scan");
-}
-
-extern "C" int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias,
-                             const float* a_log, const float* D, float* state, int state_row, const int* seq_slot,
-                             const int* seq_start, const int* seq_pos0, float* y, int n_seqs, int max_new, int least, int Hs, int G, int N, int P,
-                             cudaStream_t stream) {
-    return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
-                                max_new, Hs, G, N, P, ScanRuns{least, 0x7fffffff, 0x7fffffff, nullptr}, stream);
 }
 
 // Whether the decode step's kernel takes these sizes: quads of columns on 16 bytes, at most 512 rows.

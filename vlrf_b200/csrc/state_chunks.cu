@@ -27,7 +27,7 @@
 // Range.  A product of a zero weight and an infinity is not zero, and an infinity has no three parts: a token's infinity would reach the
 // tokens of its block that come before it.  So the writes look at every number that enters: where one of a head's in a tile of columns
 // (its rows, step sizes, decays, the state it starts from) is not finite or beyond RC_LIMIT, below which no product of this file
-// overflows, `wild` says so, the state is left as it was and the caller's token-by-token kernel does that head's columns again.
+// overflows, `wild` says so, the states leave that tile as it was, and a fourth kernel does it again, token by token.
 //
 // Layouts: q, k, v float32 rows of any stride (multiples of 4 numbers, on 16 bytes); scratch per chunk and head K·V float32, laid
 // out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a float4 per chunk and head; wild an int per
@@ -37,8 +37,8 @@
 #include "chunk_mma.cuh"
 
 namespace {
-constexpr int RC = STATE_CHUNK;        // tokens of a chunk
-constexpr int RT = STATE_TILE;         // columns of V that a CTA works on at a time (an item: a head and such a tile)
+constexpr int RC = 64;                 // tokens of a chunk
+constexpr int RT = 64;                 // columns of V that a CTA works on at a time (an item: a head and such a tile)
 constexpr int RX = RT + 8;             // … and their pitch in shared memory (16 bytes of padding keep ldmatrix off bank conflicts)
 constexpr int R_THREADS = 256;
 constexpr int R_ITEMS = 4;             // items a CTA works through with one set of q and k
@@ -118,7 +118,7 @@ __device__ __forceinline__ bool head_scalars(const StateChunks& A, int h, int fi
     return __all_sync(0xffffffffu, gain[0] < RC_LIMIT && gain[1] < RC_LIMIT) && t0 + t1 + t2 + t3 > -3e38f;
 }
 __device__ __forceinline__ bool tame(const float4& x, float limit) {
-    return fabsf(x.x) < limit && fabsf(x.y) < limit && fabsf(x.z) < limit && fabsf(x.w) < limit;
+    return (fabsf(x.x) < limit) & (fabsf(x.y) < limit) & (fabsf(x.z) < limit) & (fabsf(x.w) < limit);
 }
 
 // Four numbers into the three planes of a tile, `plane` elements apart.
@@ -149,7 +149,7 @@ __device__ __forceinline__ bool load_rows(__nv_bfloat16* planes, const float* ro
     }
     bool fine = true;
 #pragma unroll
-    for (int e = 0; e < EACH; ++e) fine = fine && tame(x[e], RC_LIMIT);
+    for (int e = 0; e < EACH; ++e) fine &= tame(x[e], RC_LIMIT);
     return fine;
 }
 
@@ -185,12 +185,12 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         }
     };
     ask(0);
-    // the queries enter here only to be looked at (the outputs load them again), a quad of a row a thread
+    // the queries enter here only to be looked at (the outputs load them again); no `&&`, which would ask for one behind the other
     bool rows_fine = true;
 #pragma unroll
     for (int e = 0; e < RC * K / 4 / R_THREADS; ++e) {
         const int i = tid + e * R_THREADS, r = i / (K / 4), c = (i - r * (K / 4)) * 4;
-        rows_fine = rows_fine && tame(quad_or_zero(A.q + (size_t)(first + r) * A.ldq + (size_t)g * K + c, r < L), RC_LIMIT);
+        rows_fine &= tame(quad_or_zero(A.q + (size_t)(first + r) * A.ldq + (size_t)g * K + c, r < L), RC_LIMIT);
     }
     if (warp < items) {
         const int h = g * per_group + (i0 + warp) / v_tiles;
@@ -204,7 +204,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         }
         if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * heads + h - h_first] = make_float4(sc[warp].before[3] + sc[warp].Lp[RC - 1], 0.f, 0.f, 0.f);
     }
-    rows_fine = load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid) && rows_fine;
+    rows_fine &= load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid);
     rows_fine = __syncthreads_and(rows_fine);
     const float* from = A.state + ((size_t)A.seq_slot[s] * 2 + (A.seq_pos0[s] & 1)) * A.state_row;
     const int chunks = (n + RC - 1) / RC;
@@ -214,13 +214,13 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
         // the state that the sequence starts from: its chunks look at a share each
         for (int i = blockIdx.x * R_THREADS + tid; i < K * RT / 4; i += chunks * R_THREADS) {
             const int r = i / (RT / 4), c = v0 + i % (RT / 4) * 4;
-            fine = fine && tame(quad_or_zero(from + ((size_t)h * K + r) * A.V + c, c < A.V), RC_STATE_LIMIT);
+            fine &= tame(quad_or_zero(from + ((size_t)h * K + r) * A.V + c, c < A.V), RC_STATE_LIMIT);
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int r = tid / 16 + 16 * e, c = tid % 16 * 4;
             const float w = weight[item * RC + r];
-            fine = fine && tame(x[e], RC_LIMIT);
+            fine &= tame(x[e], RC_LIMIT);
             store_planes(xs + r * RX + c, RC * RX, make_float4(w * x[e].x, w * x[e].y, w * x[e].z, w * x[e].w));
         }
         if (item + 1 < items) ask(item + 1);
@@ -469,6 +469,68 @@ state_chunk_outputs_kernel(const StateChunks A, int v_tiles, int parts) {
     }
 }
 
+// The tiles that the chunks could not do, token by token: a CTA looks at R_REDO of a sequence's, a warp each, and does those in turn; thread (row group,
+// column).  Nothing to do, as nearly always, costs a launch of few CTAs (the same inside the outputs made these slower: 1,164 against 1,184 us for a
+// prompt step of two runs of 1,024 over four layers of 32 heads of 64 x 64).
+constexpr int R_REDO = 8;
+template <int K>
+__global__ void __launch_bounds__(R_THREADS)
+state_chunk_redo_kernel(const StateChunks A, int v_tiles) {
+    constexpr int ROWS = K / 4;
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float sums[2 * 4 * RT];              // the row groups' sums of a token, [2][4][RT]
+    __shared__ bool todo[R_REDO];
+    const int s = blockIdx.y, start = A.seq_start[s], n = A.seq_start[s + 1] - start;
+    if (n < A.least || A.seq_slot[s] < 0) return;
+    const int tid = threadIdx.x, col = tid % RT, rg = tid / RT, item0 = A.g0 * A.per_group() * v_tiles + blockIdx.x * R_REDO,
+              item_end = (A.g0 + A.groups) * A.per_group() * v_tiles;
+    {
+        const int item = item0 + (tid >> 5);
+        int any = 0;
+        if (item < item_end)
+            for (int c = tid & 31; c < (n + RC - 1) / RC; c += 32) any |= A.wild[(size_t)(start / RC + s + c) * A.H * v_tiles + item];
+        any = __any_sync(0xffffffffu, any);
+        if ((tid & 31) == 0) todo[tid >> 5] = any != 0;
+        if (!__syncthreads_or(any)) return;
+    }
+    const int pos0 = A.seq_pos0[s];
+    for (int i = 0; i < R_REDO; ++i) {
+        if (!todo[i]) continue;
+        const int h = (item0 + i) / v_tiles, v0 = (item0 + i) % v_tiles * RT;
+        const int v = v0 + col, g = h / A.per_group();
+        const bool there = v < A.V;
+        const size_t at = ((size_t)h * K + rg * ROWS) * A.V + v, slot = (size_t)A.seq_slot[s] * 2;
+        const float* from = A.state + (slot + (pos0 & 1)) * A.state_row + at;
+        float* to = A.state + (slot + ((pos0 + n) & 1)) * A.state_row + at;
+        float S[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) S[r] = there ? from[(size_t)r * A.V] : 0.f;
+        const float a = -expf(A.a_log[h]), bias = A.dt_bias[h], skip = A.skip[h];
+        for (int t = 0; t < n; ++t) {
+            const size_t row = (size_t)start + t;
+            const float dt = softplus_f(A.s0[row * A.ld_s0 + h] + bias), decay = expf(a * dt);
+            const float x = there ? A.v[row * A.ldv + (size_t)h * A.V + v] : 0.f, dx = dt * x;
+            const float* k = A.k + row * A.ldk + g * K + rg * ROWS;
+            const float* q = A.q + row * A.ldq + g * K + rg * ROWS;
+            float part = 0.f;
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                S[r] = fmaf(decay, S[r], k[r] * dx);
+                part = fmaf(S[r], q[r], part);
+            }
+            float* mine = sums + (t & 1) * 4 * RT;
+            mine[rg * RT + col] = part;
+            __syncthreads();                            // (the other copy is written before anyone can come back to this one)
+            if (rg == 0 && there) A.y[row * A.ldy + (size_t)h * A.V + v] = fmaf(skip, x, ((mine[col] + mine[RT + col]) + mine[2 * RT + col]) + mine[3 * RT + col]);
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+            if (there) to[(size_t)r * A.V] = S[r];
+        __syncthreads();                            // the sums' buffers are free again
+    }
+}
+
 template <int K> int launch_state_chunks(const StateChunks& A, int n_seqs, int max_new, cudaStream_t stream) {
     static bool raised = false;
     if (!raised) {
@@ -488,7 +550,10 @@ template <int K> int launch_state_chunks(const StateChunks& A, int n_seqs, int m
     st = vlrf_check_launch("state_chunks: states");
     if (st != VLRF_OK) return st;
     launch_chained(state_chunk_outputs_kernel<K>, grid, dim3(R_THREADS), (size_t)outputs_smem<K>(), stream, A, v_tiles, parts);
-    return vlrf_check_launch("state_chunks: outputs");
+    st = vlrf_check_launch("state_chunks: outputs");
+    if (st != VLRF_OK) return st;
+    launch_chained(state_chunk_redo_kernel<K>, dim3((A.heads() * v_tiles + R_REDO - 1) / R_REDO, n_seqs), dim3(R_THREADS), (size_t)0, stream, A, v_tiles);
+    return vlrf_check_launch("state_chunks: redo");
 }
 bool sc_on16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 }  // namespace
@@ -520,10 +585,10 @@ extern "C" int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int G, int N, i
 
 extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                                const float* D, float* scratch, long long scratch_floats, float* state, int state_row, const int* seq_slot, const int* seq_start,
-                               const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int chunked, int scanned, int H, int G, int N,
-                               int P, cudaStream_t stream) {
+                               const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int chunked, int H, int G, int N, int P,
+                               cudaStream_t stream) {
     VLRF_REQUIRE(vlrf_ssd_chunks_takes(H, G, N, P, channels, state_row), "ssd_chunks: a state of %d by %d or the rows' strides are not taken", N, P);
-    VLRF_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && n_seqs <= 65535 && max_new >= 0 && scratch != nullptr && dt_off + H <= ld && chunked >= 1 && scanned >= 1,
+    VLRF_REQUIRE(n_tokens >= 0 && n_seqs >= 0 && n_seqs <= 65535 && max_new >= 0 && scratch != nullptr && dt_off + H <= ld && chunked >= 1,
                  "ssd_chunks: bad arguments");
     VLRF_REQUIRE((size_t)H * N * P <= (size_t)state_row, "ssd_chunks: the state row does not hold the states");
     VLRF_REQUIRE(sc_on16(xbc) && sc_on16(scratch) && sc_on16(state) && sc_on16(y), "ssd_chunks: misaligned rows");
@@ -550,6 +615,5 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
                                  : launch_state_chunks<128>(A, n_seqs, max_new, stream);
         if (st != VLRF_OK) return st;
     }
-    return vlrf_launch_ssd_scan(xbc, channels, proj, ld, dt_off, dt_bias, a_log, D, state, state_row, seq_slot, seq_start, seq_pos0, y, n_seqs,
-                                max_new, H, G, N, P, ScanRuns{scanned, chunked - 1, chunked, A.wild}, stream);
+    return VLRF_OK;
 }

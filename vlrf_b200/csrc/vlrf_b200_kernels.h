@@ -311,21 +311,21 @@ int vlrf_ssd_conv(const float* proj, int ld, int x_off, const float* w, const fl
 // sequence (it sizes the batches in which the inputs are staged; 1 for a decode step).
 int vlrf_ssd_scan(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                   const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
-                  float* y, int n_seqs, int max_new, int least, int Hs, int G, int N, int P, cudaStream_t stream);
+                  float* y, int n_seqs, int max_new, int least, int most, int Hs, int G, int N, int P, cudaStream_t stream);
 // One token a sequence (decode steps): states of any number of rows up to 512, P a multiple of 4, rows on 16 bytes.
 int vlrf_ssd_step_takes(int H, int G, int N, int P, int channels, int state_row);
 int vlrf_ssd_step(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                   const float* D, float* state, int state_row, const int* seq_slot, const int* seq_start, const int* seq_pos0,
                   float* y, int n_seqs, int Hs, int G, int N, int P, cudaStream_t stream);
 // The same over prompts on the tensor cores, 64 tokens at a time (state_chunks.cu): every float32 operand in three bfloat16 parts.
-// Runs of at least `chunked` tokens; those of `scanned` to `chunked` − 1 are done token by token in the same call, shorter ones not at all.
-// Columns of heads whose numbers are not finite, or too large for products of parts, are done token by token behind it.
+// Runs of at least `chunked` tokens only.  Columns of heads whose numbers are not finite, or too large for products of parts, are done token
+// by token.
 // scratch float32 (vlrf_ssd_chunks_scratch numbers for the step's rows, in less of them the more the caller limits it).  N 16, 32, 64 or 128, P a multiple of 4.
 int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, int state_row);
 int vlrf_ssd_chunks_scratch(int T, int n_seqs, int H, int G, int N, int P, long long limit, long long* floats);
 int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj, int ld, int dt_off, const float* dt_bias, const float* a_log,
                     const float* D, float* scratch, long long scratch_floats, float* state, int state_row, const int* seq_slot,
-                    const int* seq_start, const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int chunked, int scanned,
+                    const int* seq_start, const int* seq_pos0, float* y, int n_tokens, int n_seqs, int max_new, int chunked,
                     int H, int G, int N, int P, cudaStream_t stream);
 // out[r] = factor · groupnorm(y[r] · silu(proj[r][z_off …])) · w: RMS norm in `groups` equal parts; out of out_dtype
 // with row stride ld_out.
