@@ -1,5 +1,11 @@
 """Rules that choose between kernels, on the host: no GPU is needed to ask them."""
+import shutil
+import subprocess
+from pathlib import Path
+
 import pytest
+
+SRC = Path(__file__).resolve().parent.parent / "vlrf_b200" / "csrc"
 
 
 @pytest.mark.parametrize("H,lens,parts,listed", [
@@ -12,3 +18,32 @@ import pytest
 def test_prompt_tiles_are_listed_only_where_they_fill_the_gpu(H, lens, parts, listed):
     from vlrf_b200.csrc import library
     assert bool(library().vlrf_attn_prefill_tc_lists(sum(lens), len(lens), max(lens), H, parts, 148)) == listed
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
+def test_a_kernel_is_prepared_once_on_every_device(tmp_path):
+    """Shared memory beyond 48 KB is granted per device: the second device of a process asks too, a failed grant is asked for again, and
+    the kernels of the float32 product and of the chunked recurrence ask this way."""
+    (tmp_path / "t.cpp").write_text('''
+#include "device_marks.h"
+#include <cassert>
+int main() {
+    static DeviceMarks marks, other;
+    int asked[70] = {0}, answer = 0;
+    auto ask = [&](DeviceMarks& m, int device) { return m.once(device, [&] { ++asked[device]; return answer; }); };
+    assert(ask(marks, 0) == 0 && ask(marks, 0) == 0 && asked[0] == 1);
+    assert(ask(marks, 1) == 0 && asked[1] == 1 && ask(marks, 0) == 0 && ask(marks, 1) == 0 && asked[0] == 1 && asked[1] == 1);
+    answer = 7;
+    assert(ask(marks, 63) == 7 && ask(marks, 63) == 7 && asked[63] == 2);
+    answer = 0;
+    assert(ask(marks, 63) == 0 && ask(marks, 63) == 0 && asked[63] == 3);
+    assert(ask(marks, 64) == 0 && ask(marks, 64) == 0 && asked[64] == 2);
+    assert(ask(other, 0) == 0 && asked[0] == 2);
+    return 0;
+}
+''')
+    subprocess.run(["g++", "-std=c++17", "-I", str(SRC), str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    subprocess.run([str(tmp_path / "t")], check=True)
+    for name in ("gemm_simt.cu", "state_chunks.cu"):
+        text = (SRC / name).read_text()
+        assert "static bool" not in text and "cudaFuncSetAttribute" not in text and "allow_shared_memory(" in text

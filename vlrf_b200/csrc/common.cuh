@@ -14,6 +14,7 @@
 // activations, the bits of the device-side error word that kernels set instead of faulting, and the prototype of
 // every exported function: the definitions in the .cu files are checked against them by the compiler.
 #include "vlrf_b200_kernels.h"
+#include "device_marks.h"
 
 extern "C" const char* vlrf_last_error();
 int vlrf_fail(int code, const char* fmt, ...);
@@ -130,6 +131,15 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t own_addr, uint32_t r
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(own_addr), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
     return v;
+}
+
+// `bytes` of dynamic shared memory for a kernel on the current device; marks: of that kernel
+template <typename Kernel> cudaError_t allow_shared_memory(DeviceMarks& marks, Kernel kernel, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)marks.once(device, [&] { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 template <typename T> struct ElemIO;

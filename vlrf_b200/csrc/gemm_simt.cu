@@ -296,12 +296,9 @@ int launch_f32_rows(const float* X, const float* W, const float* bias, const flo
     constexpr size_t smem = (size_t)STAGES * rows_stage_floats<R, C>() * 4;
     static_assert(smem <= 227 * 1024 && STAGES * rows_stage_floats<R, C>() >= PARTS * R * C, "shared memory");
     auto kern = gemm_f32_rows_kernel<R, C, STAGES, VEC>;
-    static bool raised = false;
-    if (!raised && smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
+    static DeviceMarks marks;
+    const cudaError_t e = allow_shared_memory(marks, kern, smem);
+    if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     launch_chained(kern, dim3((N + C - 1) / C), dim3(C * PARTS), smem, stream, X, W, bias, residual, Y, M, N, K, ldx, ldy, act);
     return vlrf_check_launch("gemm_f32_rows");
 }
@@ -327,12 +324,9 @@ int launch_f32(const float* X, const float* W, const float* bias, const float* r
     if (M <= 8) return launch_f32_rows_for<8, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
     if (M <= 16) return launch_f32_rows_for<16, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
     auto kern = gemm_f32_tile_kernel<VEC>;
-    static bool raised = false;
-    if (!raised) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
-        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %d bytes of shared memory: %s", TILE_SMEM, cudaGetErrorString(e));
-        raised = true;
-    }
+    static DeviceMarks marks;
+    const cudaError_t e = allow_shared_memory(marks, kern, TILE_SMEM);
+    if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %d bytes of shared memory: %s", TILE_SMEM, cudaGetErrorString(e));
     const dim3 grid((unsigned)((N + TILE - 1) / TILE * PARTS), (unsigned)((M + TILE - 1) / TILE));
     launch_chained_cluster(kern, grid, dim3(TILE_THREADS), TILE_SMEM, dim3(PARTS), stream, X, W, bias, residual, Y, M, N, K, ldx, ldy, act);
     return vlrf_check_launch("gemm_f32_tile");

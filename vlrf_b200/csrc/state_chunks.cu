@@ -532,13 +532,10 @@ state_chunk_redo_kernel(const StateChunks A, int v_tiles) {
 }
 
 template <int K> int launch_state_chunks(const StateChunks& A, int n_seqs, int max_new, cudaStream_t stream) {
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(state_chunk_writes_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, writes_smem<K>());
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(state_chunk_outputs_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, outputs_smem<K>());
-        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "state_chunks: %d bytes of shared memory: %s", outputs_smem<K>(), cudaGetErrorString(e));
-        raised = true;
-    }
+    static DeviceMarks writes_marks, outputs_marks;
+    cudaError_t e = allow_shared_memory(writes_marks, state_chunk_writes_kernel<K>, writes_smem<K>());
+    if (e == cudaSuccess) e = allow_shared_memory(outputs_marks, state_chunk_outputs_kernel<K>, outputs_smem<K>());
+    if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "state_chunks: %d bytes of shared memory: %s", outputs_smem<K>(), cudaGetErrorString(e));
     const int chunks = (max_new + RC - 1) / RC, v_tiles = (A.V + RT - 1) / RT, parts = (A.H / A.G * v_tiles + R_ITEMS - 1) / R_ITEMS;
     VLRF_REQUIRE((long long)A.groups * parts <= 65535, "state_chunks: too many heads");
     const dim3 grid(chunks, A.groups * parts, n_seqs);
