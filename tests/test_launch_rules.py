@@ -20,6 +20,20 @@ def test_prompt_tiles_are_listed_only_where_they_fill_the_gpu(H, lens, parts, li
     assert bool(library().vlrf_attn_prefill_tc_lists(sum(lens), len(lens), max(lens), H, parts, 148)) == listed
 
 
+@pytest.mark.parametrize("M,N,K,then,exchanged", [
+    # alone: wide products from four rows on, a vocabulary always
+    (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),
+    # the next product reads the result: measured slower up to 16 rows
+    (4, 11264, 2048, "product", False), (16, 12288, 2048, "product", False), (24, 12288, 2048, "product", True), (64, 5632, 1024, "product", True),
+    # a gate and the next product read it
+    (4, 4224, 768, "gate", False), (8, 7040, 1280, "gate", False), (9, 9600, 1600, "gate", False), (8, 11264, 2048, "gate", True),
+    (12, 5632, 1024, "gate", True), (14, 12288, 1024, "gate", False), (10, 14336, 2048, "gate", False), (16, 11264, 2048, "gate", True),
+    (17, 14336, 2048, "gate", True)])
+def test_wide_products_of_few_rows_by_what_reads_them(M, N, K, then, exchanged):
+    from vlrf_b200.csrc import ops
+    assert ops._swapped_takes(M, N, K, then) == exchanged
+
+
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs a C++ compiler")
 def test_a_kernel_is_prepared_once_on_every_device(tmp_path):
     """Shared memory beyond 48 KB is granted per device: the second device of a process asks too, a failed grant is asked for again, and

@@ -99,12 +99,13 @@ def layernorm(x, gamma, beta, eps: float, out, rows=None) -> None:
 
 
 def linear(x, w, bias, out, *, act=None, residual=None, rows: int | None = None, kv_scatter=None,
-           stats: "RowStats | None" = None) -> bool:
+           stats: "RowStats | None" = None, gated: bool = False) -> bool:
     """out = act(x · wᵀ + bias) (+ residual).  x [M,K], w [N,K] (same dtype), bias/residual float32,
     out [M,N] float32 or bfloat16.  act: "gelu_tanh", "gelu_erf", "relu2"; "silu" where `linear_takes_silu` says so.  `rows` limits M to the first rows of x/out/residual.  `kv_scatter`
     (see linear_layernorm) asks the kernel to write K/V columns into a cache as well; the return value
     says whether it did (only the tensor-core kernels can).  `stats`: where the statistics of float32 result rows
-    are left when the kernel that takes the shape computes them (and where stale ones of `out` are forgotten)."""
+    are left when the kernel that takes the shape computes them (and where stale ones of `out` are forgotten).  `gated`: what reads
+    the result is a gate and the next product (it may decide which kernel runs, not what comes out)."""
     _dev(x, "x"); _dev(w, "w", x.dtype); _dev(out, "out")
     M = x.shape[0] if rows is None else rows
     K = x.shape[1]
@@ -126,8 +127,8 @@ def linear(x, w, bias, out, *, act=None, residual=None, rows: int | None = None,
     if act == "silu":
         if not linear_takes_silu(x.dtype, M, N, K):
             raise KernelError(f"linear: no product of {M} x {N} x {K} in {x.dtype} takes x·sigmoid(x) in its epilogue")
-        return _linear_dispatch(x, w, bias, out, GATE[act], residual, M, N, K, kv_scatter, stats)
-    return _linear_dispatch(x, w, bias, out, ACT[act], residual, M, N, K, kv_scatter, stats)
+        return _linear_dispatch(x, w, bias, out, GATE[act], residual, M, N, K, kv_scatter, stats, gated)
+    return _linear_dispatch(x, w, bias, out, ACT[act], residual, M, N, K, kv_scatter, stats, gated)
 
 
 def linear_takes_silu(dtype: torch.dtype, M: int, N: int, K: int) -> bool:
@@ -149,7 +150,17 @@ SWAPPED_MIN_COLUMNS = 16384
 #: (us): 11,264 and 12,928 x 2,048 at 8 and 16 rows 380, 446 against 367, 414, but at one row 295 against 298; 7,296 x 1,024 at 4, 16 and 64 rows 202,
 #: 261, 359 against 197, 245, 336; 5,632 x 1,024 at 48 rows 364 against 347; four times as wide: 8,192 x 2,048 at 8 rows 576 against 581, 6,400 x 1,600
 #: at 32 rows 2,860 against 2,928.
+#: The line at 5.5 is where both have been measured inside steps; alone in front of a small kernel the exchanged kernel loses 2 to 12 % at up to 8 rows
+#: between 4 and 5.5 times (80 tiles of w and more: 0 to 11 % ahead) and wins 5 to 30 % from 16 rows on.
 SWAPPED_WIDE_ROWS, SWAPPED_WIDE_COLUMNS, SWAPPED_WIDE_RATIO = 4, 4096, 5.5
+#: What follows matters as much.  A bfloat16 result goes to the next product, whose CTAs fetch weights beside split-k's but not beside
+#: the exchanged kernel's: the pair takes (split-k against exchanged, 5.5 and 6 times as wide) 0.81 to 1.0 of the time at 4 to 8 rows, 0.84 to 1.2 at 16,
+#: 1.0 to 1.19 from 24 rows on.
+SWAPPED_PRODUCT_ROWS = 24
+#: In front of a gate and the next product, the whole group: below 10 rows 0.94 to 1.0 with 33 to 76 tiles of w, 1.0 to 1.1 from 80 on; at 10 to 16
+#: rows 1.0 to 1.2, but 0.88 to 0.95 from 12,288 columns on (12,288 and 13,312 x 1,024 and 2,048, 14,336 x 2,048; the time jumps by 5 us there, why
+#: is not known); above 16 rows 1.05 to 1.3.
+SWAPPED_GATE_COLUMNS = (10240, 12288)
 #: Few-row products whose weight matrix has at least this many bytes go to the split-k tcgen05 kernel (the
 #: second figure: with the LayerNorm fused in).  Measured on B200 inside whole decode steps, the split-k kernel
 #: wins at every size of GPT-2's: its CTAs leave room on an SM for the next kernel's to begin ahead, and it
@@ -279,14 +290,24 @@ def _kv_args(kv_scatter, N: int) -> list:
             kc.shape[2]]
 
 
-def _swapped_takes(M: int, N: int, K: int) -> bool:
-    return N >= SWAPPED_MIN_COLUMNS or (M >= SWAPPED_WIDE_ROWS and N >= SWAPPED_WIDE_COLUMNS and N >= SWAPPED_WIDE_RATIO * K)
+def _swapped_takes(M: int, N: int, K: int, then: str = "kernels") -> bool:
+    """Whether a product of few rows exchanges the operands' roles; `then`: what reads its result, "kernels" of their own, a "gate" and the
+    next product, or the next "product" itself (a bfloat16 result)."""
+    if N >= SWAPPED_MIN_COLUMNS:
+        return True
+    if M < SWAPPED_WIDE_ROWS or N < SWAPPED_WIDE_COLUMNS or N < SWAPPED_WIDE_RATIO * K:
+        return False
+    if then == "product":
+        return M >= SWAPPED_PRODUCT_ROWS
+    if then == "gate":
+        return N >= SWAPPED_GATE_COLUMNS[0] if M < 10 else M > 16 or N < SWAPPED_GATE_COLUMNS[1]
+    return True
 
 
-def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, stats=None) -> bool:
+def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, stats=None, gated=False) -> bool:
     bf16_out = out.dtype == torch.bfloat16
     if (x.dtype == torch.bfloat16 and M <= SKINNY_MAX_ROWS and K % 8 == 0 and USE_TCGEN05 and kv_scatter is None
-            and _swapped_takes(M, N, K)):
+            and _swapped_takes(M, N, K, "gate" if gated else "product" if bf16_out else "kernels")):
         # few rows, very many columns (the head over the vocabulary, wide input products): enough 128-row tiles of w to fill the GPU,
         # so w becomes the 128-row operand of the tcgen05 kernel and the rows of x its N
         call("vlrf_gemm_tcgen05", _ptr(x), _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), M, N, K, K, N,

@@ -89,7 +89,7 @@ class GatedMLP:
     def forward(self, h, x: torch.Tensor, ctx: StepContext, norm=None, accumulate: bool = True) -> None:
         T, ff = ctx.n_tokens, self.inner
         gu = ctx.ws.get("ffn_gate_up", T, 2 * ff, torch.float32)
-        ops.linear(h, self.in_weight, None, gu)
+        ops.linear(h, self.in_weight, None, gu, gated=True)
         u = ctx.ws.get("ffn_inner", T, ff, ctx.act_dtype)
         self.core(gu, u, ctx)
         ops.linear(u, self.out_weight, None, x, residual=x if accumulate else None)

@@ -159,7 +159,7 @@ class RoutedExperts:
         T, (w_gu, _, ffs) = ctx.n_tokens, self.shared
         if self.leading_rows(T) == self.n_logits:
             su = ctx.ws.get("moe_shared_gate_up", T, 2 * ffs, ctx.act_dtype)
-            ops.linear(h, w_gu, None, su)
+            ops.linear(h, w_gu, None, su, gated=True)
             ops.gate_mul(su[:, :ffs], su[:, ffs:], merged, "silu", T, ffs)
         else:
             at = self.n_logits
