@@ -537,6 +537,38 @@ def test_long_runs_in_chunks():
     assert all(a <= max(1.5 * b, 2.0 ** -21) for a, b in zip(off[True], off[False])), off
 
 
+def test_tokens_one_by_one_with_nothing_between():
+    """The one-token kernel launched again and again, each launch reading the state that the one just ahead of it writes (it may begin while
+    that one still runs), against the float64 recurrence."""
+    from vlrf_b200.csrc import ops
+    Hs, P, N, G, T = 4, 64, 64, 2, 40
+    inner = Hs * P
+    args, state, ctx = chunk_step([1, 1, 1], [0, 3, 4], [2, 0, 1], Hs, P, N, G, torch.Generator().manual_seed(8))
+    g = torch.Generator().manual_seed(9)
+    xbc, proj = torch.randn(T, 3, inner + 2 * G * N, generator=g), torch.randn(T, 3, 3 + Hs, generator=g)
+    xd, pd, y = dev(xbc), dev(proj), torch.empty(T, 3, inner, device=DEV)
+    pos = torch.tensor([[0, 3, 4]] * T, dtype=torch.int32) + torch.arange(T, dtype=torch.int32)[:, None]
+    pos = pos.to(DEV)
+    import types
+    steps = [types.SimpleNamespace(**{**vars(ctx), "seq_pos0": pos[t]}) for t in range(T)]
+    for _ in range(3):                                                 # (and again: what a run left must not show)
+        st = state.to(DEV)
+        torch.cuda.synchronize()
+        for t in range(T):
+            ops.ssd_step(xd[t], pd[t], *args[2:], st, steps[t], y[t], Hs, G, N, P)
+        dt_bias, a_log, D = (t.cpu().double() for t in args[3:])
+        for i, (slot, p0) in enumerate(((2, 0), (0, 3), (1, 4))):
+            S, want = state[slot, p0 & 1].double().reshape(Hs, N, P), []
+            for t in range(T):
+                x, B, C = xbc[t, i, :inner].double().reshape(Hs, P), xbc[t, i, inner:inner + G * N].double(), xbc[t, i, inner + G * N:].double()
+                B, C = (v.reshape(G, N).repeat_interleave(Hs // G, 0) for v in (B, C))
+                step = plain.softplus(proj[t, i, 3:].double() + dt_bias)
+                S = torch.exp(-torch.exp(a_log) * step)[:, None, None] * S + (step[:, None] * B)[:, :, None] * x[:, None, :]
+                want.append(((S * C[:, :, None]).sum(1) + D[:, None] * x).reshape(inner))
+            close(y[:, i], torch.stack(want), 1e-5, f"sequence {i}")
+            close(st[slot, (p0 + T) & 1].reshape(Hs, N, P), S, 1e-5, f"state {i}")
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 5])
 def test_convolution_over_runs(taps):
     """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a

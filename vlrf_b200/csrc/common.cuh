@@ -33,7 +33,12 @@ int vlrf_sm_count();                             // asked of the driver once: th
 // kernel begins, at least one kernel that is not a product lies complete between it and whatever wrote the
 // positions, the block tables and the cache of earlier positions (the sampling kernel of the step before,
 // host copies, the step before's projections): decode attention may fetch those before its wait, but
-// nothing that the kernels just ahead write (activations, the new position's key and value).
+// nothing that the kernels just ahead write (activations, the new position's key and value).  "Just ahead" is
+// the launch before in whatever order a caller makes them: a kernel that is launched twice in a row has itself
+// ahead, so one that updates a state in place of its own (the one-token recurrences) reads that state behind its
+// wait, although inside a step other kernels lie between.  (Checked on the device: words read ahead of the wait against
+// the same words behind it.  Written by a kernel or a copy two launches back, or more: none of 170 million
+// reads differs, plain, read-only or at L2, with and without idle SMs.  Written by the launch just ahead: they do.)
 // `vlrf_set_chained_launch(0)` turns the launch attribute off (the calls then do nothing).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
