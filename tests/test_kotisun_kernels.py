@@ -569,6 +569,29 @@ def test_tokens_one_by_one_with_nothing_between():
             close(st[slot, (p0 + T) & 1].reshape(Hs, N, P), S, 1e-5, f"state {i}")
 
 
+@pytest.mark.parametrize("which", ["xbc", "state", "y"])
+def test_recurrence_of_rows_beside_16_bytes(which):
+    """Rows, states or results that do not begin on 16 bytes are taken, as token by token takes them, in decode and in prompt steps."""
+    from vlrf_b200.csrc import ops
+    Hs, P, N, G = 4, 64, 64, 2
+    for lens in ([1, 1], [400, 1, 30]):
+        args, state, ctx = chunk_step(lens, [0, 3, 4][:len(lens)], [2, 0, 1][:len(lens)], Hs, P, N, G, torch.Generator().manual_seed(5))
+
+        def beside(t, name):
+            if name != which:
+                return t.to(DEV)
+            flat = torch.empty(t.numel() + 1, device=DEV)[1:]
+            return flat.copy_(t.flatten()).view(t.shape)
+        results = []
+        for shifted in (False, True):
+            place = beside if shifted else lambda t, name: t.to(DEV)
+            st, y = place(state, "state"), place(torch.zeros(ctx.n_tokens, Hs * P), "y")
+            ops.ssd_scan_step(place(args[0], "xbc"), *args[1:], st, ctx, y, Hs, G, N, P)
+            results.append((y.cpu(), st.cpu()))
+        for a, b in zip(*results):
+            close(b, a, 1e-5, which)
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 5])
 def test_convolution_over_runs(taps):
     """Runs at the edges of a thread's 16 tokens, from zero and from kept inputs, with the number of taps known when compiling and not; a

@@ -1329,10 +1329,11 @@ def ssd_scan_step(xbc, proj, dt_off: int, dt_bias, a_log, d_skip, state, ctx, y,
     SSD_CHUNKS_MIN_RUN, or more; what shares the step does not change a sequence's arithmetic."""
     args, sizes = (xbc, proj, dt_off, dt_bias, a_log, d_skip, state), (n_heads, n_groups, n_state, p)
     takes = sizes + (xbc.shape[1], state.shape[2])
-    ones = _ssd_step_sizes(ctx.act_dtype, *takes)                      # single tokens have a kernel of their own
+    on16 = all(t.data_ptr() % 16 == 0 for t in (xbc, state, y))        # (what both kernels beside the token-by-token one ask for)
+    ones = on16 and _ssd_step_sizes(ctx.act_dtype, *takes)             # single tokens have a kernel of their own
     shortest = ctx.max_new if ctx.n_seqs == 1 else getattr(ctx, "min_new", 1)
     left = ctx.max_new                                                 # runs up to here are not in chunks
-    if ssd_chunks_takes(ctx.act_dtype, ctx, *takes):
+    if on16 and ssd_chunks_takes(ctx.act_dtype, ctx, *takes):
         try:
             ssd_chunks(*args, ctx, y, *sizes, SSD_CHUNKS_MIN_RUN)
             left = SSD_CHUNKS_MIN_RUN - 1
