@@ -105,7 +105,9 @@ VLRF_B200_API void vlrf_b200_default_sampling(VlrfB200Sampling* out_params);
  * another; prompt_lens[i]: tokens of prompt i (0: start from the model's bos token).  params: n_params = 1 (the same
  * for all) or n_prompts.  out_ids: n_prompts rows of out_cap ids each, receiving the NEW tokens of each prompt;
  * out_lens[i]: how many; out_reasons[i] (may be NULL): VLRF_B200_FINISH_*.  Requests beyond the cache's slots wait and
- * take the rows of those that ended.  A request's tokens do not depend on the others. */
+ * take the rows of those that ended.  A request's tokens do not depend on what the others are; in bfloat16 its logits may
+ * differ by rounding with how many share a step (products of few and of many rows run on different kernels), and with
+ * them a choice between tokens that are equally likely to that precision. */
 VLRF_B200_API VlrfB200Status vlrf_b200_generate_ids(VlrfB200Model model, const int32_t* prompt_ids,
                                                     const int32_t* prompt_lens, int32_t n_prompts,
                                                     const VlrfB200Sampling* params, int32_t n_params, int32_t* out_ids,

@@ -3,7 +3,7 @@
 `Engine.step(entries)` takes for each sequence its next tokens and the places among them whose logits
 are wanted.  All tokens of all sequences run as one flat batch (prompts of unequal lengths in one step,
 or one token each); each token carries its sequence's slot and its position, so no padding exists and
-what else is in the batch changes no result.  Only the given tokens are computed: everything earlier
+what else is in the batch changes no result beyond the rounding of the kernels that a step's size chooses.  Only the given tokens are computed: everything earlier
 comes from the cache that previous steps left.  The reference has one sequence and a `forward(ids,
 use_cache)` that returns the last row (include/model/transformer.hpp:335-424).
 """
