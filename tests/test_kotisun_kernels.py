@@ -443,14 +443,14 @@ def test_chunks_in_passes_and_without_scratch(monkeypatch):
         return y.cpu(), st.cpu()
     want = run(ops.ssd_chunks)
     whole = ctx.ws.get("ssd_chunks", 1, 1, torch.float32).untyped_storage().nbytes()
-    assert whole == 4 * slots * (Hs * (N * P + 4) + marks)
+    assert whole == 4 * slots * (Hs * (N * P + 1) + marks)
     for groups in (3, 1):
-        monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * groups * (N * P + 4) + marks) + 3)
+        monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * groups * (N * P + 1) + marks) + 3)
         ctx.ws = type(ctx.ws)(torch.device(DEV))
         for a, b in zip(run(ops.ssd_chunks), want):
             assert torch.equal(a, b)
         assert ctx.ws.get("ssd_chunks", 1, 1, torch.float32).untyped_storage().nbytes() <= ops.SSD_CHUNKS_MAX_BYTES
-    monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * (N * P + 4) + marks) - 4)
+    monkeypatch.setattr(ops, "SSD_CHUNKS_MAX_BYTES", 4 * slots * (2 * (N * P + 1) + marks) - 4)
     assert not ops.ssd_chunks_takes(torch.bfloat16, ctx, Hs, G, N, P, args[0].shape[1], state.shape[2])
     monkeypatch.undo()
     real = torch.empty

@@ -30,7 +30,7 @@
 // overflows, `wild` says so, the states leave that tile as it was, and a fourth kernel does it again, token by token.
 //
 // Layouts: q, k, v float32 rows of any stride (multiples of 4 numbers, on 16 bytes); scratch per chunk and head K·V float32, laid
-// out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a float4 per chunk and head; wild an int per
+// out as the state is, the chunks of sequence s beginning at seq_start[s] / 64 + s; aux a number per chunk and head; wild an int per
 // chunk, head and tile of 64 columns.  Heads are independent: where the scratch that a caller has does not hold every head's states, the three
 // kernels run over a range of groups at a time (a pass), one range after another in the same scratch.
 #include "common.cuh"
@@ -52,7 +52,7 @@ struct StateChunks {
     const float *s0, *dt_bias, *a_log, *skip;
     int ld_s0;
     float* scratch;
-    float4* aux;                       // {F_L, –, –, –}
+    float* aux;                        // F_L
     int* wild;
     float* state;
     int state_row;
@@ -202,7 +202,7 @@ state_chunk_writes_kernel(const StateChunks A, int v_tiles, int parts) {
             const int t = lane + 32 * e;
             weight[warp * RC + t] = expf(sc[warp].Ls[t] + sc[warp].after[t >> 4]) * sc[warp].gain[t];
         }
-        if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * heads + h - h_first] = make_float4(sc[warp].before[3] + sc[warp].Lp[RC - 1], 0.f, 0.f, 0.f);
+        if (lane == 0 && (i0 + warp) % v_tiles == 0) A.aux[chunk * heads + h - h_first] = sc[warp].before[3] + sc[warp].Lp[RC - 1];
     }
     rows_fine &= load_rows<K>(ks, A.k + (size_t)first * A.ldk + (size_t)g * K, A.ldk, L, tid);
     rows_fine = __syncthreads_and(rows_fine);
@@ -278,7 +278,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
     float4 S = *reinterpret_cast<const float4*>(from + i);
     const size_t slot0 = (size_t)(start / RC + s);
     float* u = A.scratch + slot0 * all + i;
-    const float4* aux = A.aux + slot0 * heads + hl;
+    const float* aux = A.aux + slot0 * heads + hl;
     const int* wild = A.wild + (slot0 * A.H + h_first + hl) * v_tiles + (int)(i % A.V) / RT;
     int any_wild = 0;
     constexpr int AHEAD = 8;                        // chunks asked for together
@@ -288,7 +288,7 @@ state_chunk_states_kernel(const StateChunks A, int per_head, int v_tiles) {
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j) {
             U[j] = quad_or_zero(u + (size_t)(c0 + j) * all, c0 + j < chunks);
-            F[j] = c0 + j < chunks ? aux[(size_t)(c0 + j) * heads].x : 0.f;
+            F[j] = c0 + j < chunks ? aux[(size_t)(c0 + j) * heads] : 0.f;
             any_wild |= c0 + j < chunks ? wild[(size_t)(c0 + j) * A.H * v_tiles] : 0;
         }
 #pragma unroll
@@ -562,9 +562,9 @@ extern "C" int vlrf_ssd_chunks_takes(int H, int G, int N, int P, int channels, i
 }
 
 // How the groups of a step of T tokens in n_seqs sequences share scratch of at most `limit` numbers: how many a pass takes (0: not even
-// one fits), as evenly as passes allow.  Per chunk: a state and four numbers for every head of a pass, and the marks of all heads' tiles.
+// one fits), as evenly as passes allow.  Per chunk: a state and a number for every head of a pass, and the marks of all heads' tiles.
 static int chunk_groups(int T, int n_seqs, int H, int G, int N, int P, long long limit, long long* floats) {
-    const long long slots = (long long)T / RC + n_seqs, marks = slots * H * ((P + RT - 1) / RT), group = slots * (H / G) * ((long long)N * P + 4);
+    const long long slots = (long long)T / RC + n_seqs, marks = slots * H * ((P + RT - 1) / RT), group = slots * (H / G) * ((long long)N * P + 1);
     long long most = limit < marks ? 0 : (limit - marks) / group;
     if (most > G) most = G;
     if (most < 1) { *floats = 0; return 0; }
@@ -601,9 +601,9 @@ extern "C" int vlrf_ssd_chunks(const float* xbc, int channels, const float* proj
     const int groups = chunk_groups(n_tokens, n_seqs, H, G, N, P, scratch_floats, &floats);
     VLRF_REQUIRE(groups > 0, "ssd_chunks: %lld numbers of scratch do not hold a group's chunks", scratch_floats);
     const size_t slots = ((size_t)n_tokens / RC + n_seqs) * groups * (H / G);          // (chunk, head of a pass)
-    A.aux = reinterpret_cast<float4*>(scratch);
-    A.scratch = scratch + slots * 4;
-    A.wild = reinterpret_cast<int*>(A.scratch + slots * (size_t)N * P);
+    A.scratch = scratch;
+    A.aux = scratch + slots * (size_t)N * P;
+    A.wild = reinterpret_cast<int*>(A.aux + slots);
     for (A.g0 = 0; A.g0 < G; A.g0 += groups) {
         A.groups = G - A.g0 < groups ? G - A.g0 : groups;
         const int st = N == 16   ? launch_state_chunks<16>(A, n_seqs, max_new, stream)
