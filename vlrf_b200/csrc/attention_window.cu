@@ -473,7 +473,7 @@ extern "C" int vlrf_qkv_norm_rope_append(const float* proj, int ld, int q_off, i
         return vlrf_check_launch("qkv_rope_append");
     }
     const bool by_heads = norm == 1 && dk % 2 == 0 && dk <= 256;       // (the kernel's own rule for a warp a head)
-    const int head_ctas = (H + (write_cache ? Hkv : 0) + 3) / 4, fill = 1184 / T;          // (eight CTAs an SM)
+    const int head_ctas = (H + (write_cache ? Hkv : 0) + 3) / 4, fill = 8 * vlrf_sm_count() / T;          // (eight CTAs an SM)
     const dim3 grid(T, by_heads && fill > 1 ? (fill < head_ctas ? fill : head_ctas) : 1);
     if (dtype == VLRF_F32)
         launch_chained(qkv_rope_append_kernel<float>, grid, dim3(128), smem, stream, proj, ld, q_off, k_off, v_off, freq, rot,

@@ -303,14 +303,15 @@ int launch_f32_rows(const float* X, const float* W, const float* bias, const flo
     return vlrf_check_launch("gemm_f32_rows");
 }
 
-// Columns a CTA: as few as leave every SM a CTA (4 below 8 x 148 columns), 32 where even those make two waves (a head over
+// Columns a CTA: as few as leave every SM a CTA (4 where 8 would not), 32 where even those make two waves (a head over
 // a vocabulary), so that x is read from L2 less often.
 template <int R, bool VEC>
 int launch_f32_rows_for(const float* X, const float* W, const float* bias, const float* residual, float* Y, int M, int N, int K, int ldx, int ldy,
                         int act, cudaStream_t stream) {
     constexpr int S = R <= 8 ? 5 : 4;
-    if (N < 8 * 148) return launch_f32_rows<R, 4, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
-    if (N < 2 * 32 * 148) return launch_f32_rows<R, 8, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    const int sms = vlrf_sm_count();
+    if (N < 8 * sms) return launch_f32_rows<R, 4, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
+    if (N < 2 * 32 * sms) return launch_f32_rows<R, 8, S, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
     return launch_f32_rows<R, 32, 2, VEC>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, stream);
 }
 

@@ -428,7 +428,7 @@ int gate_norm_quads(const float* y, const float* proj, int ld, int z_off, const 
     const int gs = d / groups;
     const uintptr_t all = (uintptr_t)y | (uintptr_t)proj | (uintptr_t)w | (uintptr_t)out;
     if (gs % 128 != 0 || all % 16 != 0 || ld % 4 != 0 || z_off % 4 != 0 || ld_out % 4 != 0) return 0;
-    const int nv = n_rows > 2 * 148 && d % 512 == 0 ? 4 : 1;
+    const int nv = n_rows > 2 * vlrf_sm_count() && d % 512 == 0 ? 4 : 1;
     if (d / (4 * nv) <= 1024) return nv;
     return d % 512 == 0 && d / 16 <= 1024 ? 4 : 0;
 }
@@ -512,9 +512,7 @@ extern "C" int vlrf_ssd_step(const float* xbc, int channels, const float* proj, 
                  "ssd_step: misaligned rows");
     if (n_seqs == 0) return VLRF_OK;
     // columns a CTA: few enough that a thread has at most 16 rows, and that small steps still reach every SM
-    int sms = 148, devi = 0;
-    cudaGetDevice(&devi);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, devi);
+    const int sms = vlrf_sm_count();
     int CQ = 32;
     while (CQ > 1 && ((N + 256 / CQ - 1) / (256 / CQ) > 16 || CQ >= 2 * (P / 4))) CQ /= 2;
     while (CQ > 8 && (long long)Hs * ((P / 4 + CQ - 1) / CQ) * n_seqs < sms) CQ /= 2;
