@@ -20,6 +20,15 @@ def test_prompt_tiles_are_listed_only_where_they_fill_the_gpu(H, lens, parts, li
     assert bool(library().vlrf_attn_prefill_tc_lists(sum(lens), len(lens), max(lens), H, parts, 148)) == listed
 
 
+@pytest.mark.parametrize("rows,G,N,width", [
+    (2000, 16, 1024, 128), (1000, 16, 2048, 128), (4096, 16, 1024, 128), (4096, 16, 2048, 256), (5000, 8, 64, 64), (5000, 8, 128, 128)])
+def test_wide_tiles_of_experts_only_where_full_tiles_gain_too(rows, G, N, width):
+    """2,000 rows over 16 experts are 16 full row tiles of 128, one round of narrow tiles; counted with a half-empty tile a group they
+    looked like two."""
+    from vlrf_b200.csrc import library
+    assert library().vlrf_gemm_tcgen05_groups_width(rows, G, N, 1, 148) == width
+
+
 @pytest.mark.parametrize("M,N,K,then,exchanged", [
     # alone: wide products from four rows on, a vocabulary always
     (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),

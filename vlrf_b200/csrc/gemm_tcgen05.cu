@@ -553,7 +553,9 @@ namespace {
 // Rows of a group's tile.  Few rows a group (a decode step's experts and heads): W is the 128-row operand and a tile has as many rows as
 // twice the average group fills (16, 32 or 64), so that a tile brings the weights and little else through the ring; with 128 rows of X beside
 // them, nearly all of other groups or none, it brought as many bytes again and filled half the ring with them (16 experts of 2,048 x 1,024 with 2 rows
-// each 24.1 -> 14.6 us inside a decode step, its down product 13.7 -> 10.6 us).  Heads' rows are known: the tile that takes them all.
+// each 24.1 -> 14.6 us inside a decode step, its down product 13.7 -> 10.6 us).  Routers that spread rows unevenly (shares 1, 1/2, 1/3, …) gain less (64 to
+// 500 rows of 16 or 32 experts 1.0 to 1.3 times as fast as with 128 rows of X, even shares 1.1 to 1.3); what loses is a step whose rows all go to one or two of
+// 32 experts of 2,816 x 2,048 (128 to 500 rows 16.5 to 18.6 -> 20.7 to 29.1 us).  Heads' rows are known: the tile that takes them all.
 int gr_tile_rows(int rows, int G, bool by_offsets) {
     const long long fill = by_offsets ? (2ll * rows + G - 1) / G : rows;
     const int each = fill <= 16 ? 16 : fill <= 32 ? 32 : fill <= 64 ? 64 : TC_BM;
@@ -599,6 +601,18 @@ extern "C" int vlrf_gemm_tcgen05_groups_takes(int rows, int G, int N, int K, int
     return gr_row_tiles(rows, G, by_offsets != 0) <= TC_GR_TAB ? 1 : 0;
 }
 
+// Columns of W a tile where it has 128 rows of X: by rounds and the bytes of a round, as for one matrix.  How rows sorted by expert spread is not known
+// here: 256 only where it is the cheaper both if half of a group's last tile is empty and if all tiles are full (16 experts of 1,024 x 1,024 with 125 rows
+// each are one round of 128-wide tiles, 16.7 us, and were 64 tiles of 256, 19.2 us; 2,048 wide with 256 rows each 36.7 -> 33.9 us with 256).
+extern "C" int vlrf_gemm_tcgen05_groups_width(int rows, int G, int N, int by_offsets, int sms) {
+    if (N <= 64) return 64;
+    if (N <= 128) return 128;
+    auto cost = [&](long long row_tiles, int bn) { return ((row_tiles * ((N + bn - 1) / bn) + sms - 1) / sms) * (bn + 128); };
+    const long long full = (rows + TC_BM - 1) / TC_BM, spread = by_offsets ? full + G / 2 : gr_row_tiles(rows, G, false);
+    const bool wide = cost(spread, 256) < cost(spread, 128) && (!by_offsets || cost(full, 256) < cost(full, 128));
+    return wide ? 256 : 128;
+}
+
 // offsets != null: rows offsets[g] … offsets[g+1]−1 of X [rows][K] times W[g]ᵀ into the same rows of Y [rows][N]
 // (x_gs = y_gs = 0).  offsets == null: every group (head) multiplies all rows, reading X at column g·x_gs and writing Y at
 // column g·y_gs.  W [G][N][K]; X and W bfloat16, Y bfloat16 or float32; an activation (VLRF_ACT_NONE, _GELU_TANH, _GELU_ERF or _RELU2) on
@@ -618,12 +632,10 @@ extern "C" int vlrf_gemm_tcgen05_groups(const void* X, int ldx, int x_gs, const 
     if (each == 16) return GROUPS(16, 5, true);
     if (each == 32) return GROUPS(32, 5, true);
     if (each == 64) return GROUPS(64, 4, true);
-    if (N <= 64) return GROUPS(64, 4, false);
-    // the width by rounds and the bytes of a round, as for one matrix; half of a group's last tile is taken to be empty
-    const long long row_tiles = offsets ? (rows + TC_BM - 1) / TC_BM + G / 2 : gr_row_tiles(rows, G, false);
-    const int sms = vlrf_sm_count();
-    auto cost = [&](int bn) { return ((row_tiles * ((N + bn - 1) / bn) + sms - 1) / sms) * (bn + 128); };
-    if (N > 128 && cost(256) < cost(128)) return GROUPS(256, 4, false);
-    return GROUPS(128, 3, false);
+    switch (vlrf_gemm_tcgen05_groups_width(rows, G, N, offsets != nullptr, vlrf_sm_count())) {
+        case 64: return GROUPS(64, 4, false);
+        case 256: return GROUPS(256, 4, false);
+        default: return GROUPS(128, 3, false);
+    }
 #undef GROUPS
 }

@@ -94,6 +94,7 @@ int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias, const flo
 // x_gs = y_gs = 0).  offsets == null: every group multiplies all rows, reading X at column g·x_gs and writing Y at
 // column g·y_gs (heads).  W [G][N][K]; an activation on the result (VLRF_ACT_NONE, _GELU_TANH, _GELU_ERF, _RELU2); no bias,
 // residual or scatter.
+int vlrf_gemm_tcgen05_groups_width(int rows, int G, int N, int by_offsets, int sms);
 int vlrf_gemm_tcgen05_groups_takes(int rows, int G, int N, int K, int ldx, int x_gs, int ldy, int y_gs, int by_offsets);
 int vlrf_gemm_tcgen05_groups(const void* X, int ldx, int x_gs, const void* W, void* Y, int ldy, int y_gs, const int* offsets,
                              int G, int rows, int N, int K, int out_dtype, int act, int* dev_err, cudaStream_t stream);
