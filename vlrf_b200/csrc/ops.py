@@ -1255,7 +1255,7 @@ def attention_window_step(q, k_cache, v_cache, block_table, out, ctx, n_heads: i
 #: Where a step's state-space recurrence runs in chunks: runs of at least so many new tokens, in at most so much scratch.  Token by token
 #: takes as long as the longest run, in chunks hardly longer for a long one than for a short one: for 32 heads of 64 x 64, 256, 512, 1,024
 #: and 2 x 1,024 tokens 37, 70, 137, 137 against 47, 48, 52, 67 us, eight runs of 160 61 against 67 us; for 128 x 128 51, 98, 191, 343
-#: against 64, 76, 128, 289 us.  The scratch holds 7,800 tokens of 32 heads of 128 x 128 whole; more, or larger ones, take several passes.
+#: against 64, 76, 128, 283 us.  The scratch holds 7,800 tokens of 32 heads of 128 x 128 whole; more, or larger ones, take several passes.
 SSD_CHUNKS_MIN_RUN, SSD_CHUNKS_MAX_BYTES = 384, 256 << 20
 
 

@@ -14,9 +14,10 @@
 //
 // Token by token (ssd.cu) a prompt of 1,024 tokens is 1,024 dependent steps of about 330 cycles, in as many CTAs as there are heads
 // and column blocks, whatever idles beside them.  In chunks the dependent steps are 16, and the arithmetic is products: 2 x 1,024 tokens, 32 heads of
-// 64 x 64 in 4 groups, 137 -> 67 us (writes 18, states 9, outputs 40), 32 heads of 128 x 128 in 8 groups 343 -> 289 us.  The outputs reach
-// 120 TFLOP/s of the 550 that `mma.sync` has: with 8 or 16 warps an SM a scheduler issues in 0.28 of its cycles, and a warp waits in turn for fixed
-// latencies, memory, barriers, instructions and the tensor pipe, none of them above a fifth; two chains of products beside each other changed nothing.  Its error against 64 bits is 0.9e-7 where token by token's is 1.2e-7.
+// 64 x 64 in 4 groups, 137 -> 69 us, 32 heads of 128 x 128 in 8 groups 343 -> 283 us.  The outputs keep the tensor pipe busy for 25 % of
+// their cycles (23 % at 128 x 128): with 8 or 16 warps an SM a scheduler issues in 0.27 (0.19) of its cycles, and a warp waits in turn for memory, fixed
+// latencies, instructions, barriers and the tensor pipe, none of them much above a fifth; two chains of products beside each other changed nothing.
+// Its error against 64 bits is 0.9e-7 where token by token's is 1.2e-7.
 //
 // Precision.  Everything that was float32 enters the products whole: each operand as the sum of three bfloat16 numbers (24 bits) and
 // each product as the six partial ones that reach 2^-24 of it (fc_mma3), summed in float32.  Exponents are sums of
