@@ -340,7 +340,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // The weights do not depend on the kernel ahead: the first stages' tiles of W are requested at once, and
     // the norm's weights for this part's columns are copied to shared memory.
     const int first = n_kb < stages ? n_kb : stages;
-    if (warp == 4 && lane == 0) {
+    if (warp == 4 && elect_one()) {
         for (int i = 0; i < first; ++i) {
             tbar_expect_tx(&full[i], a_bytes + (LN ? 0 : B_BYTES));
             tma_load_2d(a_tiles + (size_t)i * a_bytes, &tmap_w, (kb0 + i) * SP_BK, n0, &full[i]);
@@ -367,7 +367,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     float pre_res[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, pre_bias[2] = {0.f, 0.f};
 
     if (warp == 4) {
-        if (lane == 0) {
+        if (elect_one()) {
             if (!LN)
                 for (int i = 0; i < first; ++i)
                     tma_load_2d(b_tiles + (size_t)i * B_BYTES, &tmap_x, (kb0 + i) * SP_BK, 0, &full[i]);
@@ -380,22 +380,25 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
     } else if (warp == 5) {
-        if (!SYNC && lane == 0) {
+        if (!SYNC) {
             constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
+            const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
             bool ok = true;
             if (LN && !tbar_wait_or_abort(x_ready, 0, s_abort)) { atomicExch(s_abort, 1); ok = false; }
             for (int i = 0; i < n_kb && ok; ++i) {
                 const int s = i % stages;
                 if (!tbar_wait_or_abort(&full[s], (uint32_t)((i / stages) & 1), s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t da = umma_desc_k128(a_tiles + (size_t)s * a_bytes);
-                const uint64_t db = umma_desc_k128(b_tiles + (size_t)(LN ? i : s) * B_BYTES);
+                if (elect_one()) {
+                    const uint64_t da = da0 + (uint64_t)(s * (a_bytes >> 4)), db = db0 + (uint64_t)((LN ? i : s) * (B_BYTES >> 4));
 #pragma unroll
-                for (int k = 0; k < SP_BK / 16; ++k)
-                    umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&empty[s]);
+                    for (int k = 0; k < SP_BK / 16; ++k)
+                        umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(&empty[s]);
+                    if (i + 1 == n_kb) umma_commit(acc_full);
+                }
+                __syncwarp();
             }
-            if (ok) umma_commit(acc_full);
         }
     } else {
         if (LN) {

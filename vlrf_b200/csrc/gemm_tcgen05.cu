@@ -5,7 +5,7 @@
 //   warp 8  producer: for every 64-wide k block it waits until the ring stage is free, announces the
 //           bytes on the stage's "full" mbarrier and issues two tiled TMA loads (128 rows of X, BN rows of
 //           W; 128-byte swizzle; rows and columns outside the matrices read as zeros);
-//   warp 9  one elected thread issues the MMAs: four `tcgen05.mma.cta_group::1.kind::f16` of shape
+//   warp 9  waits as a whole and issues the MMAs by one elected lane (tcgen05.cuh): four `tcgen05.mma.cta_group::1.kind::f16` of shape
 //           128 × BN × 16 per k block, operands straight from shared memory through matrix descriptors,
 //           accumulator in tensor memory (two accumulators alternate, so a tile's epilogue overlaps the
 //           next tile's MMAs); `tcgen05.commit` frees the stage when those MMAs have read it, and after the
@@ -28,10 +28,9 @@ namespace {
 
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;           // elements of K in one 128-byte swizzle atom: what one TMA load and one descriptor cover
-// Atoms of K in a stage of the ring.  One thread issues the MMAs, and a stage costs it about 550 cycles whatever
-// the tile's width: some 63 for each of an atom's four MMAs, the rest for the wait, the commit and the loop.  The
-// tensor pipe needs 4 x 186 cycles for an atom of a 256-wide tile but only 4 x 70 of a 96-wide one, so narrow
-// tiles take two atoms a stage and pay the fixed part half as often.
+// Atoms of K in a stage of the ring.  One lane issues the MMAs, and a stage costs it a fixed time whatever the tile's
+// width (the wait, the commit, the loop).  The tensor pipe needs 4 x 186 cycles for an atom of a 256-wide tile but only
+// 4 x 70 of a 96-wide one, so narrow tiles take two atoms a stage and pay the fixed part half as often.
 __host__ __device__ constexpr int tc_atoms(int bn) { return bn <= 128 ? 2 : 1; }
 constexpr int TC_THREADS = 320;      // warps 0-7: epilogue (two per 32 accumulator lanes), 8: producer, 9: MMA issue
 
@@ -137,7 +136,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         __syncthreads();
     }
     const int early = (int)blockIdx.x < n_tiles ? min(STAGES, n_kb) : 0;
-    if (warp == 8 && lane == 0 && early > 0) {
+    if (warp == 8 && early > 0 && elect_one()) {
         int a_row, b_row, xk0;
         place(blockIdx.x, a_row, b_row, xk0);
         for (int kb = 0; kb < early; ++kb) {
@@ -175,7 +174,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
     }
 
     if (warp == 8) {
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t kc = 0;                       // k-blocks requested so far, over all tiles
             for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x) {
                 int a_row, b_row, xk0;
@@ -202,21 +201,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             }
         }
     } else if (warp == 9) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
-            uint32_t kc = 0, tc = 0;
-            for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x, ++tc) {
-                const uint32_t b = tc & 1, use = tc >> 1;
-                if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
+        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
+        const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
+        uint32_t kc = 0, tc = 0;
+        for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x, ++tc) {
+            const uint32_t b = tc & 1, use = tc >> 1;
+            if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tmem_d = tmem_base + b * ACC_STRIDE;
+            bool ok = true;
+            for (int kb = 0; kb < n_kb; ++kb, ++kc) {
+                const uint32_t s = kc % STAGES;
+                if (!tbar_wait_or_abort(&full[s], (kc / STAGES) & 1, s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t tmem_d = tmem_base + b * ACC_STRIDE;
-                bool ok = true;
-                for (int kb = 0; kb < n_kb; ++kb, ++kc) {
-                    const int s = kc % STAGES;
-                    if (!tbar_wait_or_abort(&full[s], (kc / STAGES) & 1, s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t da = umma_desc_k128(a_tiles + (size_t)s * A_BYTES);
-                    const uint64_t db = umma_desc_k128(b_tiles + (size_t)s * B_BYTES);
+                if (elect_one()) {
+                    const uint64_t da = da0 + (uint64_t)(s * (A_BYTES >> 4)), db = db0 + (uint64_t)(s * (B_BYTES >> 4));
 #pragma unroll
                     for (int a = 0; a < KA; ++a) {
 #pragma unroll
@@ -225,10 +224,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                                       (kb > 0 || a > 0 || k > 0) ? 1u : 0u);
                     }
                     umma_commit(&empty[s]);                   // the stage is free once these MMAs have read it
+                    if (kb + 1 == n_kb) umma_commit(&acc_full[b]);    // arrives when every MMA issued so far is complete
                 }
-                if (!ok) break;
-                umma_commit(&acc_full[b]);                    // arrives when every MMA issued so far is complete
+                __syncwarp();
             }
+            if (!ok) break;
         }
     } else {
         // epilogue: warps q and q+4 share accumulator lanes 32q … 32q+31 and take half of the columns each
