@@ -405,6 +405,42 @@ def test_float32_products_of_few_and_of_many_rows_form_one_sum(N, K):
     assert torch.equal(some, full[:5])
 
 
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8])
+@pytest.mark.parametrize("N,K,scatter", [(768, 768, False), (2304, 768, True), (1183, 4, False), (1184, 132, True), (9, 260, False), (200, 1024, True)])
+def test_float32_product_with_a_norm_ahead(M, N, K, scatter):
+    """The same bits as the norm, the product and the append by kernels of their own; a token without a slot is left out, one whose block is
+    not mapped is reported, rows and columns beyond the result are untouched."""
+    from vlrf_b200.csrc import ops
+    x, w, b = randn(M, K, seed=111).to(DEV), randn(N, K, seed=112).to(DEV), randn(N, seed=113).to(DEV)
+    gamma, beta = (1 + 0.1 * randn(K, seed=114)).to(DEV), randn(K, seed=115).to(DEV)
+    assert ops.can_fuse_layernorm(M, K, torch.float32, x, gamma, beta, w) and not ops.can_fuse_layernorm(9, K, torch.float32)
+    assert not ops.can_fuse_layernorm(M, K, torch.float32, torch.empty(5, device=DEV)[1:])
+    want, got = torch.empty(M, N, device=DEV), torch.full((M + 1, N), float("nan"), device=DEV)
+    h = torch.empty(M, K, device=DEV)
+    ops.layernorm(x, gamma, beta, 1e-5, h)
+    ops.linear(h, w, b, want, act="gelu_tanh")
+    if not scatter:
+        ops.linear_layernorm(x, gamma, beta, 1e-5, w, b, got, act="gelu_tanh", rows=M)
+    else:
+        Hkv, dh = 2, 16
+        k_off, v_off = N - 2 * Hkv * dh - 8, N - Hkv * dh - 4
+        table = torch.tensor([[3, 1], [5, -1]], dtype=torch.int32, device=DEV)
+        slot = torch.tensor([0, 1, -1, 0, 1, 0, 1, 0][:M], dtype=torch.int32, device=DEV)
+        pos = torch.tensor([63, 9, 0, 64, 70, 1, 10, 100][:M], dtype=torch.int32, device=DEV)
+        caches = [torch.full((6, Hkv, 64, dh), float("nan"), device=DEV) for _ in range(4)]
+        ops.kv_append(want, k_off, v_off, caches[0], caches[1], table, slot, pos, M, Hkv, dh, ops._dev_err())
+        reported = ops.device_errors()
+        assert (reported != 0) == (M >= 5)
+        ops.linear_layernorm(x, gamma, beta, 1e-5, w, b, got, act="gelu_tanh", rows=M,
+                             kv_scatter=(caches[2], caches[3], table, slot, pos, k_off, v_off, Hkv, dh))
+        assert ops.device_errors() == reported
+        for one, other in ((0, 2), (1, 3)):
+            assert torch.equal(caches[one].view(torch.int32), caches[other].view(torch.int32))
+    assert torch.equal(got[:M], want)
+    assert torch.isnan(got[M]).all()
+    assert ops.device_errors() == 0
+
+
 # ------------------------------------------------------------------------------------------------
 def paged(k, v, n_blocks, order_seed, dtype):
     """Put [H, C, dh] keys and values of one sequence into a pool with scattered blocks; unused pool

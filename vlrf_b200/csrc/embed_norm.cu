@@ -8,6 +8,7 @@
 //             shared memory, statistics in float32, biased variance
 //             (reference: include/model/ops.hpp:443-476)
 #include "common.cuh"
+#include "layernorm_row.cuh"
 
 template <typename WT>
 __global__ void embed_pos_kernel(const WT* __restrict__ wte, const WT* __restrict__ wpe,
@@ -210,39 +211,19 @@ __global__ void __launch_bounds__(256) layernorm_warp_small_kernel(const float* 
     pdl_wait();
     pdl_launch_dependents();
     if (r >= n_rows) return;
-    const float* src = x + (size_t)(rows ? rows[r] : r) * d;
     float4 v[NV];
-    float s = 0.f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const int i = j * 32 + lane;
-        v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < nv)      // an explicit load: the values stay in registers for all three passes
-            asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v[j].x), "=f"(v[j].y), "=f"(v[j].z), "=f"(v[j].w) : "l"(src + 4 * i));
-        s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
-    }
-    const float mean = warp_sum(s) / (float)d;
-    float q = 0.f;
-#pragma unroll
-    for (int j = 0; j < NV; ++j)
-        if (j * 32 + lane < nv) {
-            const float a = v[j].x - mean, b = v[j].y - mean, c = v[j].z - mean, e = v[j].w - mean;
-            q += (a * a + b * b) + (c * c + e * e);
-        }
-    const float inv = 1.f / sqrtf(warp_sum(q) / (float)d + eps);
+    float mean, inv;
+    layernorm_row<NV>(x + (size_t)(rows ? rows[r] : r) * d, nv, d, eps, lane, v, mean, inv);
     OT* dst = out + (size_t)r * d;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
         const int i = j * 32 + lane;
         if (i < nv) {
-            const float4 gm = s_gamma[i], bt = s_beta[i];
-            const float y0 = (v[j].x - mean) * inv * gm.x + bt.x, y1 = (v[j].y - mean) * inv * gm.y + bt.y;
-            const float y2 = (v[j].z - mean) * inv * gm.z + bt.z, y3 = (v[j].w - mean) * inv * gm.w + bt.w;
+            const float4 y = layernorm_apply(v[j], mean, inv, s_gamma[i], s_beta[i]);
             if (sizeof(OT) == 4) {
-                reinterpret_cast<float4*>(dst)[i] = make_float4(y0, y1, y2, y3);
+                reinterpret_cast<float4*>(dst)[i] = y;
             } else {
-                __nv_bfloat162 lo = __floats2bfloat162_rn(y0, y1), hi = __floats2bfloat162_rn(y2, y3);
+                __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
                 uint2 pk;
                 pk.x = *reinterpret_cast<uint32_t*>(&lo);
                 pk.y = *reinterpret_cast<uint32_t*>(&hi);

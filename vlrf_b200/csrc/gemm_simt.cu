@@ -11,10 +11,12 @@
 // one order.  In float32 that order is: K in PARTS = 8 runs of equal length (`part_length`), each a chain of FMAs in the
 // order of k, the eight sums added in their order.  The parts are what a few rows are spread over the GPU by (a chain of
 // all K terms in one thread took 104 us a product at 4 rows, whatever its size):
+//   up to 8 rows     gemm_f32_norm_kernel: the next, with a LayerNorm ahead and a cache write behind
 //   up to 16 rows    gemm_f32_rows_kernel: a thread per (column, part); bound by streaming W once
 //   more rows        gemm_f32_tile_kernel: 64 x 64 tiles, the eight parts of a tile one CTA each of a cluster; bound by FMAs
 // bfloat16 operands take gemm_simt_kernel (shapes outside the tensor-core kernels' rules: rare and small).
 #include "common.cuh"
+#include "layernorm_row.cuh"
 
 namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, THREADS = 256;
@@ -192,6 +194,117 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, c
     }
 }
 
+// Up to R rows with a LayerNorm ahead and, for a q/k/v projection, the write of its k and v columns into one layer's paged cache behind:
+// the norm's kernel and the append's are launches of their own otherwise, 2.5 us each inside a decode step for rows that every CTA here
+// has read and normed in 1.  The sums are those of gemm_f32_rows_kernel, the norm is that of embed_norm.cu (a warp a row, the row in
+// registers), so the same bits come out.  The whole rows lie in shared memory, each part's run 16 bytes further than its place
+// asks for, which keeps a warp's reads of several parts on banks of their own.
+struct F32Scatter {
+    float* Kc; float* Vc;                                  // [block][kv_head][BT][dh]; Kc == nullptr: none
+    const int* block_table; const int* tok_slot; const int* tok_pos;
+    int max_blocks, k_off, v_off, width, dh, Hkv, BT;      // width = Hkv·dh
+};
+constexpr int NORM_MAX_K = 1024, NORM_NV = NORM_MAX_K / 128;
+template <int R, int C, int STAGES> __host__ __device__ constexpr size_t norm_smem(int K) {
+    return ((size_t)STAGES * PARTS * C * KPITCH + (size_t)R * (K + 4 * PARTS)) * 4;
+}
+
+template <int R, int C, int STAGES>
+__global__ void __launch_bounds__(C * PARTS)
+gemm_f32_norm_kernel(const float* __restrict__ X, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
+                     const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ Y, int M, int N, int K, int act,
+                     F32Scatter kv, int* __restrict__ dev_err) {
+    extern __shared__ __align__(16) float ring[];
+    __shared__ int s_blk[R], s_row[R];                     // where each row's token lies in the cache
+    constexpr int STAGE = PARTS * C * KPITCH, THREADS_R = C * PARTS, PIECES = KB / 4;
+    pdl_launch_dependents();
+    const int tid = threadIdx.x, c = tid % C, p = tid / C, n0 = blockIdx.x * C, warp = tid >> 5, lane = tid & 31;
+    const int len = part_length(K), n_chunks = (min(len, K) + KB - 1) / KB, pitch = K + 4 * PARTS, nv = K >> 2;
+    float* rows = ring + STAGES * STAGE;                   // [R][K + 4·PARTS]
+    auto load_w = [&](int chunk) {
+        float* at = ring + (chunk % STAGES) * STAGE;
+        for (int i = tid; i < PARTS * C * PIECES; i += THREADS_R) {
+            const int piece = i % PIECES, cc = i / PIECES % C, pp = i / (PIECES * C);
+            stage_piece<true>(at + (pp * C + cc) * KPITCH, W, K, n0 + cc, N, pp * len + chunk * KB, min(K, (pp + 1) * len), piece);
+        }
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < n_chunks) load_w(s);
+        cp_async_commit();
+    }
+    float4 gm[NORM_NV], bt[NORM_NV];
+#pragma unroll
+    for (int j = 0; j < NORM_NV; ++j) {
+        const int i = j * 32 + lane;
+        gm[j] = i < nv ? reinterpret_cast<const float4*>(gamma)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        bt[j] = i < nv ? reinterpret_cast<const float4*>(beta)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+    if (kv.Kc != nullptr && tid < R) {
+        int blk = -1, row = 0;
+        const int slot = tid < M ? kv.tok_slot[tid] : -1;
+        if (slot >= 0) {
+            const int pos = kv.tok_pos[tid], bi = pos / kv.BT;
+            blk = pos >= 0 && bi < kv.max_blocks ? kv.block_table[(size_t)slot * kv.max_blocks + bi] : -1;
+            row = pos % kv.BT;
+            if (blk < 0 && blockIdx.x == 0) atomicOr(dev_err, VLRF_DEVERR_NO_BLOCK);
+        }
+        s_blk[tid] = blk;
+        s_row[tid] = row;
+    }
+    for (int r = warp; r < R; r += THREADS_R / 32) {
+        float4 v[NORM_NV];
+        float mean, inv;
+        layernorm_row<NORM_NV>(X + (size_t)min(r, M - 1) * K, nv, K, eps, lane, v, mean, inv);
+#pragma unroll
+        for (int j = 0; j < NORM_NV; ++j) {
+            const int i = j * 32 + lane;
+            if (i < nv) *reinterpret_cast<float4*>(rows + (size_t)r * pitch + 4 * i + 4 * (4 * i / len)) = layernorm_apply(v[j], mean, inv, gm[j], bt[j]);
+        }
+    }
+    float acc[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                                   // the stage (and the rows) are here, and the stage before it has been read by everyone
+        if (chunk + STAGES - 1 < n_chunks) load_w(chunk + STAGES - 1);
+        cp_async_commit();
+        const float4* w4 = (const float4*)(ring + (chunk % STAGES) * STAGE + (p * C + c) * KPITCH);
+        const int k0 = p * len + chunk * KB, k1 = min(K, (p + 1) * len);
+        const float* x0 = rows + k0 + 4 * p;
+#pragma unroll
+        for (int k = 0; k < KB / 4; ++k) {
+            if (k0 + 4 * k >= k1) break;                   // (the weights behind the part's end are zeros, the rows there another part's)
+            const float4 w = w4[k];
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r] = fma4(*reinterpret_cast<const float4*>(x0 + (size_t)r * pitch + 4 * k), w, acc[r]);
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    float* sums = ring;                                    // [part][row][column]
+#pragma unroll
+    for (int r = 0; r < R; ++r) sums[(p * R + r) * C + c] = acc[r];
+    __syncthreads();
+    for (int i = tid; i < R * C; i += THREADS_R) {
+        const int r = i / C, n = n0 + i % C;
+        if (r >= M || n >= N) continue;
+        float v = sums[i];
+#pragma unroll
+        for (int pp = 1; pp < PARTS; ++pp) v += sums[pp * R * C + i];
+        if (bias) v += bias[n];
+        v = apply_act_rt(v, act);
+        Y[(size_t)r * N + n] = v;
+        if (kv.Kc != nullptr && n >= kv.k_off && s_blk[r] >= 0) {
+            const bool is_v = n >= kv.v_off;
+            const int col = n - (is_v ? kv.v_off : kv.k_off);
+            if (col < kv.width) (is_v ? kv.Vc : kv.Kc)[(((size_t)s_blk[r] * kv.Hkv + col / kv.dh) * kv.BT + s_row[r]) * kv.dh + col % kv.dh] = v;
+        }
+    }
+}
+
 // Many rows.  The PARTS CTAs of a cluster multiply one 64 x 64 tile, each over its part of K (128 threads, 8 x 4 elements a
 // thread read four k at a time: 12 shared-memory wavefronts for 128 FMA instructions of a warp, so the FMAs bound it); then
 // each adds the eight sums of 8 of the tile's rows out of its neighbours' shared memory, in the order of the parts.  N x K at 64, 240
@@ -303,6 +416,26 @@ int launch_f32_rows(const float* X, const float* W, const float* bias, const flo
     return vlrf_check_launch("gemm_f32_rows");
 }
 
+template <int R, int C>
+int launch_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y, int M, int N, int K,
+                    int act, const F32Scatter& kv, int* dev_err, cudaStream_t stream) {
+    constexpr int STAGES = 4;
+    static_assert((size_t)STAGES * C * KPITCH >= (size_t)R * C, "the sums take the ring's place");
+    const size_t smem = norm_smem<R, C, STAGES>(K);
+    auto kern = gemm_f32_norm_kernel<R, C, STAGES>;
+    static DeviceMarks marks;
+    const cudaError_t e = allow_shared_memory(marks, kern, norm_smem<R, C, STAGES>(NORM_MAX_K));
+    if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+    launch_chained(kern, dim3((N + C - 1) / C), dim3(C * PARTS), smem, stream, X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err);
+    return vlrf_check_launch("gemm_f32_norm");
+}
+template <int R>
+int launch_f32_norm_for(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y, int M, int N,
+                        int K, int act, const F32Scatter& kv, int* dev_err, cudaStream_t stream) {
+    if (N < 8 * vlrf_sm_count()) return launch_f32_norm<R, 4>(X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err, stream);
+    return launch_f32_norm<R, 8>(X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err, stream);
+}
+
 // Columns a CTA: as few as leave every SM a CTA (4 where 8 would not), 32 where even those make two waves (a head over
 // a vocabulary), so that x is read from L2 less often.
 template <int R, bool VEC>
@@ -356,4 +489,27 @@ extern "C" int vlrf_gemm_simt(const void* X, const void* W, const float* bias, c
     else return vlrf_fail(VLRF_ERR_INVALID_ARG, "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
 #undef LAUNCH
     return vlrf_check_launch("gemm_simt");
+}
+
+// Whether the product with a LayerNorm ahead takes these rows: up to 8 (beyond, a norm of its own costs less than every CTA's), as many
+// columns as the norm keeps in registers.
+extern "C" int vlrf_gemm_f32_norm_takes(int M, int K) { return M >= 1 && M <= 8 && K >= 4 && K % 4 == 0 && K <= NORM_MAX_K ? 1 : 0; }
+
+// Y = act(LayerNorm(X) · Wᵀ + bias) in float32, X [M][K], Y [M][N]; Kc != null: columns k_off … and v_off … also into the cache.
+extern "C" int vlrf_gemm_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y,
+                                  int M, int N, int K, int act, float* Kc, float* Vc, const int* block_table, int max_blocks,
+                                  const int* tok_slot, const int* tok_pos, int k_off, int v_off, int Hkv, int dh, int BT, int* dev_err,
+                                  cudaStream_t stream) {
+    VLRF_REQUIRE(vlrf_gemm_f32_norm_takes(M, K) && N > 0, "gemm_f32_norm: %d rows of %d columns are not taken", M, K);
+    VLRF_REQUIRE((((uintptr_t)X | (uintptr_t)W | (uintptr_t)gamma | (uintptr_t)beta) & 15) == 0, "gemm_f32_norm: rows must begin on 16 bytes");
+    VLRF_REQUIRE(act >= 0 && act <= VLRF_ACT_LAST_FUSED && dev_err != nullptr, "gemm_f32_norm: bad arguments");
+    F32Scatter kv{};
+    if (Kc != nullptr) {
+        VLRF_REQUIRE(Vc && block_table && tok_slot && tok_pos && Hkv > 0 && dh > 0 && BT > 0 && max_blocks > 0 && k_off >= 0 && v_off >= k_off + Hkv * dh,
+                     "gemm_f32_norm: incomplete cache scatter arguments");
+        kv = F32Scatter{Kc, Vc, block_table, tok_slot, tok_pos, max_blocks, k_off, v_off, Hkv * dh, dh, Hkv, BT};
+    }
+    if (M == 1) return launch_f32_norm_for<1>(X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err, stream);
+    if (M <= 4) return launch_f32_norm_for<4>(X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err, stream);
+    return launch_f32_norm_for<8>(X, gamma, beta, eps, W, bias, Y, M, N, K, act, kv, dev_err, stream);
 }

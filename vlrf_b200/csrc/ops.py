@@ -277,11 +277,11 @@ def sm_count() -> int:
     return _SM_COUNT
 
 
-def _kv_args(kv_scatter, N: int) -> list:
+def _kv_args(kv_scatter, N: int, dtype: torch.dtype = torch.bfloat16) -> list:
     if kv_scatter is None:
         return [0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0]
     kc, vc, table, tok_slot, tok_pos, k_off, v_off, hkv, dh = kv_scatter
-    _dev(kc, "k_cache", torch.bfloat16); _dev(vc, "v_cache", torch.bfloat16)
+    _dev(kc, "k_cache", dtype); _dev(vc, "v_cache", dtype)
     _dev(table, "block_table", torch.int32); _dev(tok_slot, "tok_slot", torch.int32)
     _dev(tok_pos, "tok_pos", torch.int32)
     if kc.shape[1] != hkv or kc.shape[3] != dh or max(k_off, v_off) + hkv * dh > N:
@@ -341,9 +341,13 @@ def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, s
     return False
 
 
-def can_fuse_layernorm(n_rows: int, width: int, w_dtype: torch.dtype) -> bool:
-    """Whether `linear_layernorm` takes this many rows of this width."""
+def can_fuse_layernorm(n_rows: int, width: int, w_dtype: torch.dtype, *tensors) -> bool:
+    """Whether `linear_layernorm` takes this many rows of this width; `tensors`: the rows, the norm's weight and bias and the
+    product's weights, which in float32 must begin on 16 bytes."""
     # with more rows, every CTA repeating the norm costs more than a norm kernel of its own
+    if w_dtype == torch.float32:
+        from . import library
+        return all(t.data_ptr() % 16 == 0 for t in tensors) and bool(library().vlrf_gemm_f32_norm_takes(n_rows, width))
     if w_dtype != torch.bfloat16 or n_rows > FUSED_NORM_MAX_ROWS or n_rows < 1 or width % 32 != 0:
         return False
     from . import library
@@ -353,10 +357,12 @@ def can_fuse_layernorm(n_rows: int, width: int, w_dtype: torch.dtype) -> bool:
 def linear_layernorm(x, gamma, beta, eps: float, w, bias, out, *, act=None, rows: int | None = None,
                      kv_scatter=None, stats: "RowStats | None" = None) -> None:
     """out = act(LayerNorm(x) · wᵀ + bias) for few rows, the norm fused into the product's prologue.
-    x float32 [M,K]; w bfloat16 [N,K]; out bfloat16 or float32.  `kv_scatter` = (k_cache, v_cache,
+    x float32 [M,K]; w bfloat16 [N,K]; out bfloat16 or float32 (or w and out float32).  `kv_scatter` = (k_cache, v_cache,
     block_table, tok_slot, tok_pos, k_off, v_off, n_kv_heads, head_dim) also writes those columns of the
     result into one layer's paged cache."""
-    _dev(x, "x", torch.float32); _dev(w, "w", torch.bfloat16); _dev(out, "out")
+    _dev(x, "x", torch.float32); _dev(w, "w"); _dev(out, "out")
+    if w.dtype not in (torch.bfloat16, torch.float32) or (w.dtype == torch.float32 and out.dtype != torch.float32):
+        raise KernelError("linear_layernorm: bfloat16 weights, or float32 weights and a float32 result")
     _dev(gamma, "gamma", torch.float32); _dev(beta, "beta", torch.float32)
     M = x.shape[0] if rows is None else rows
     K, N = x.shape[1], w.shape[0]
@@ -364,7 +370,13 @@ def linear_layernorm(x, gamma, beta, eps: float, w, bias, out, *, act=None, rows
         raise KernelError("linear_layernorm: sizes do not match")
     if bias is not None:
         _dev(bias, "bias", torch.float32)
-    kv = _kv_args(kv_scatter, N)
+    kv = _kv_args(kv_scatter, N, w.dtype)
+    if w.dtype == torch.float32:
+        if stats is not None:
+            stats.written(out)
+        call("vlrf_gemm_f32_norm", _ptr(x), _ptr(gamma), _ptr(beta), float(eps), _ptr(w), _ptr(bias), _ptr(out), M, N, K, ACT[act], *kv,
+             _ptr(_dev_err()), _stream())
+        return
     known = stats.describing(x, M, K) if stats is not None else None
     if stats is not None:
         stats.written(out)

@@ -82,6 +82,13 @@ int vlrf_layernorm(const float* x, const int* rows, const float* gamma, const fl
 int vlrf_gemm_simt(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K,
                    int ldx, int ldy, int in_dtype, int out_dtype, int act, cudaStream_t stream);
 
+// act(LayerNorm(X) · Wᵀ + bias) in float32 for up to 8 rows, the norm in the product's prologue; Kc != null: columns k_off … and v_off … of
+// the result also into one layer's paged cache.  The bits of vlrf_layernorm, vlrf_gemm_simt and vlrf_kv_append one after the other.
+int vlrf_gemm_f32_norm_takes(int M, int K);
+int vlrf_gemm_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y, int M,
+                       int N, int K, int act, float* Kc, float* Vc, const int* block_table, int max_blocks, const int* tok_slot,
+                       const int* tok_pos, int k_off, int v_off, int Hkv, int dh, int BT, int* dev_err, cudaStream_t stream);
+
 // Many rows, bfloat16 X and W, on the tcgen05 tensor cores (TMA ring, accumulators in tensor memory); with few rows
 // and very many columns the operands' roles are exchanged.  K a multiple of 8.
 int vlrf_gemm_tcgen05_takes(int M, int N, int K, int ldx);

@@ -46,7 +46,8 @@ class DenseMLP:
     def forward(self, h, x: torch.Tensor, ctx: StepContext, norm=None, accumulate: bool = True) -> None:
         T = ctx.n_tokens
         u = ctx.ws.get("ffn_inner", T, self.inner, ctx.act_dtype)
-        if h is None and getattr(norm, "fusable_as", None) == "layernorm" and ops.can_fuse_layernorm(T, x.shape[1], self.w_in.dtype):
+        if h is None and getattr(norm, "fusable_as", None) == "layernorm" \
+                and ops.can_fuse_layernorm(T, x.shape[1], self.w_in.dtype, x, norm.weight, norm.bias, self.w_in):
             ops.linear_layernorm(x, norm.weight, norm.bias, norm.eps, self.w_in, self.b_in, u, act=self.activation,
                                  stats=ctx.ws.row_stats)
         else:

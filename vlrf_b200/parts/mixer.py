@@ -74,7 +74,8 @@ class CausalSelfAttention:
         T = ctx.n_tokens
         qkv = ctx.ws.get("attn_qkv", T, self.qkv_width, ctx.act_dtype)
         appended = False
-        if h is None and getattr(norm, "fusable_as", None) == "layernorm" and ops.can_fuse_layernorm(T, x.shape[1], self.w_qkv.dtype):
+        if h is None and getattr(norm, "fusable_as", None) == "layernorm" \
+                and ops.can_fuse_layernorm(T, x.shape[1], self.w_qkv.dtype, x, norm.weight, norm.bias, self.w_qkv):
             # few rows: norm, projection and the cache write in one kernel
             scatter = None
             if writes_cache:
