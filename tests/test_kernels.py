@@ -347,6 +347,60 @@ def test_tcgen05_tile_widths(width):
         lib.vlrf_gemm_tcgen05_force_width(0)
 
 
+@pytest.mark.parametrize("rows", [32, 64, 96, 128, 160, 192, 224, 256])
+def test_products_by_pairs_of_sms(rows):
+    """Tiles of every number of rows, asked for by name (the choice by size would pick one): whole tiles and the rows left behind them,
+    columns of which the second CTA of a pair has none, tails in K; float32 with the residual in place, bfloat16 with an activation (rows of
+    odd length and rows that begin between two numbers of a pair among them), and the cache scatter with heads of 8, 16 and 64 columns; more tiles
+    than pairs of SMs, so that the accumulators alternate."""
+    from vlrf_b200.csrc import call, ops
+
+    def product(x, w, bias, out, residual=None, act=None, kv_scatter=None):
+        M, K = x.shape
+        N = w.shape[0]
+        call("vlrf_gemm_pair", x.data_ptr(), w.data_ptr(), bias.data_ptr(), 0 if residual is None else residual.data_ptr(), out.data_ptr(), M, N, K,
+             K, N, ops.dtype_code(out.dtype), ops.ACT[act], rows, *ops._kv_args(kv_scatter, N), ops._dev_err().data_ptr(),
+             torch.cuda.current_stream().cuda_stream)
+
+    for M, N, K in ((300, 1000, 200), (rows, 256, 64), (rows - 1, 130, 72), (rows + 1, 131, 8), (1, 8, 136), (1200, 6000, 136)):
+        x, w = randn(M, K, seed=90, dtype=torch.bfloat16), randn(N, K, seed=91, dtype=torch.bfloat16, scale=0.3)
+        bias, res = randn(N, seed=92), randn(M, N, seed=93)
+        want = x.double() @ w.double().T + bias.double()
+        acc = torch.full((M + 1, N), float("nan"), device=DEV)
+        acc[:M] = res.to(DEV)
+        product(x.to(DEV), w.to(DEV), bias.to(DEV), acc, residual=acc)
+        assert rel_err(acc[:M].cpu(), want + res.double()) < f32_sum_tol(K)
+        assert torch.isnan(acc[M]).all()
+        for first in (0, 1):
+            room = torch.full((M * N + 2,), float("nan"), dtype=torch.bfloat16, device=DEV)
+            out = room[first:first + M * N].view(M, N)
+            product(x.to(DEV), w.to(DEV), bias.to(DEV), out, act="gelu_tanh")
+            assert rel_err(out.float().cpu(), plain.gelu_tanh(want)) < 5e-3
+            assert torch.isnan(room[first + M * N:]).all() and torch.isnan(room[:first]).all()
+    K = 200
+    for H, Hkv, dh in ((6, 3, 8), (4, 2, 16), (3, 3, 64)):
+        Nq = (H + 2 * Hkv) * dh
+        T = 150
+        wq, bq = randn(Nq, K, seed=94, dtype=torch.bfloat16, scale=0.2), randn(Nq, seed=95)
+        table = torch.tensor([[3, 1, 4], [5, 0, -1]], dtype=torch.int32)
+        slot = torch.tensor([0] * 100 + [-1] * 10 + [1] * 40, dtype=torch.int32)
+        pos = torch.tensor(list(range(60, 160)) + [0] * 10 + list(range(30, 70)), dtype=torch.int32)
+        kc = torch.full((6, Hkv, 64, dh), float("nan"), dtype=torch.bfloat16, device=DEV)
+        vc = torch.full_like(kc, float("nan"))
+        o = torch.empty(T, Nq, dtype=torch.bfloat16, device=DEV)
+        product(randn(T, K, seed=96, dtype=torch.bfloat16).to(DEV), wq.to(DEV), bq.to(DEV), o,
+                kv_scatter=(kc, vc, table.to(DEV), slot.to(DEV), pos.to(DEV), H * dh, (H + Hkv) * dh, Hkv, dh))
+        oc = o.cpu()
+        for m in range(T):
+            if slot[m] < 0:
+                continue
+            blk = int(table[slot[m], pos[m] // 64])
+            assert torch.equal(kc[blk, :, pos[m] % 64].cpu().reshape(-1), oc[m, H * dh:(H + Hkv) * dh])
+            assert torch.equal(vc[blk, :, pos[m] % 64].cpu().reshape(-1), oc[m, (H + Hkv) * dh:])
+        assert (~torch.isnan(kc.float())).sum().item() == 140 * Hkv * dh     # nothing else was touched
+    assert ops.device_errors() == 0
+
+
 def test_split_k_rows_do_not_depend_on_the_batch(split_k_always):
     import os
     if os.environ.get("VLRF_B200_SPLITK_MMA"):

@@ -29,6 +29,15 @@ def test_wide_tiles_of_experts_only_where_full_tiles_gain_too(rows, G, N, width)
     assert library().vlrf_gemm_tcgen05_groups_width(rows, G, N, 1, 148) == width
 
 
+@pytest.mark.parametrize("M,N,rows", [
+    (2048, 768, 96), (2048, 2304, 256), (2048, 3072, 192), (2050, 1600, 224), (2050, 4800, 192), (2050, 6400, 192), (1928, 11264, 256),
+    (1500, 1280, 128), (700, 3072, 128), (512, 768, 64), (65, 256, 64)])
+def test_rows_of_a_tile_of_a_pair(M, N, rows):
+    """The rows with which each of these was fastest (or within 5 %)."""
+    from vlrf_b200.csrc import library
+    assert library().vlrf_gemm_pair_rows(M, N, 148) == rows
+
+
 @pytest.mark.parametrize("M,N,K,then,exchanged", [
     # alone: wide products from four rows on, a vocabulary always
     (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),

@@ -58,6 +58,10 @@ _SIGNATURES = {
     "vlrf_gemm_tcgen05": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                           _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
                           _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
+    "vlrf_gemm_pair_rows": [_c_int] * 3,
+    "vlrf_gemm_pair": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
+                       _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
+                       _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "vlrf_gemm_tcgen05_groups_width": [_c_int] * 5,
     "vlrf_gemm_tcgen05_groups_takes": [_c_int] * 9,
     "vlrf_gemm_tcgen05_groups": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_int, _c_int,

@@ -1,5 +1,6 @@
 // Y[M,N] = act(X[M,K] · W[N,K]^T + bias) (+ residual) on the 5th-generation tensor cores (tcgen05), for
-// the many-row products of a prompt step.  bfloat16 operands, float32 accumulation in tensor memory.
+// the many-row products of a prompt step that gemm_pair.cu does not take (vlrf_gemm_tcgen05 chooses), for few rows and very many columns,
+// and for a matrix per group.  bfloat16 operands, float32 accumulation in tensor memory.
 //
 // A persistent CTA computes 128 × BN tiles of Y, one after another.  Its ten warps have fixed jobs:
 //   warp 8  producer: for every 64-wide k block it waits until the ring stage is free, announces the
@@ -515,6 +516,17 @@ extern "C" int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias
         if (M <= 32) return SWAPPED(32);
         return SWAPPED(64);
 #undef SWAPPED
+    }
+    // By pairs of SMs (gemm_pair.cu): float32 results, which its whole-line stores finish sooner at every size; bfloat16 results where K is long and
+    // tiles are wide, so that half the bytes of an operand a stage count for more than 2-byte columns to store.  One CTA a tile against
+    // pairs, float32 with a residual: 512 x 768 x 768 5.8 -> 5.1 us, 2,048 x 768 x 768 7.3 -> 7.0, 2,050 x 1,600 x 1,600 17.0 -> 14.8, 2,050 x 1,600 x 6,400 43.3 ->
+    // 40.6, 1,928 x 4,096 x 2,048 37.4 -> 31.5, 4,096 cubed 125 -> 111 (2,048 x 768 x 3,072 13.0 -> 13.4); bfloat16: 1,928 x 11,264 x 2,048 74.0 -> 67.9, 4,096
+    // cubed 104 -> 97, 2,050 x 1,600 x 6,400 37.0 -> 37.3, but 2,048 x 2,304 x 768 9.2 -> 10.2, 2,048 x 768 x 3,072 11.1 -> 12.8.
+    if (g_forced_width == 0) {
+        const int rows = vlrf_gemm_pair_rows(M, N, vlrf_sm_count());
+        if (out_dtype == VLRF_F32 || (K >= 2048 && rows >= 192))
+            return vlrf_gemm_pair(X, W, bias, residual, Y, M, N, K, ldx, ldy, out_dtype, act, rows, Kc, Vc, block_table, max_blocks, tok_slot,
+                                  tok_pos, k_off, v_off, Hkv, dh, BT, dev_err, stream);
     }
     // tile width: the fewest rounds of the persistent CTAs, each weighted by the bytes a tile's stage pulls through
     // L2 (128 rows of one operand and the tile's width of the other): that, not the MMAs, is what a round's time

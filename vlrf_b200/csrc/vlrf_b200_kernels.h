@@ -96,6 +96,13 @@ int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias, const flo
                       int ldx, int ldy, int out_dtype, int act, void* Kc, void* Vc, const int* block_table,
                       int max_blocks, const int* tok_slot, const int* tok_pos, int k_off, int v_off, int Hkv, int dh,
                       int BT, int* dev_err, cudaStream_t stream);
+// The same product by pairs of SMs (`cta_group::2`), tiles of 256 columns by bn rows (a multiple of 32 up to 256); vlrf_gemm_tcgen05 chooses it by
+// size, with the rows that vlrf_gemm_pair_rows gives.
+int vlrf_gemm_pair_rows(int M, int N, int sms);
+int vlrf_gemm_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
+                   int ldy, int out_dtype, int act, int bn, void* Kc, void* Vc, const int* block_table, int max_blocks,
+                   const int* tok_slot, const int* tok_pos, int k_off, int v_off, int Hkv, int dh, int BT, int* dev_err,
+                   cudaStream_t stream);
 // The same kernel with a weight matrix per group.  offsets != null (device, G + 1 entries): rows offsets[g] …
 // offsets[g+1]−1 of X [rows][K] times W[g]ᵀ into the same rows of Y [rows][N] (experts over rows sorted by expert;
 // x_gs = y_gs = 0).  offsets == null: every group multiplies all rows, reading X at column g·x_gs and writing Y at
