@@ -750,6 +750,53 @@ def test_attention_prefill_where_the_tiles_fill_the_gpu(monkeypatch, kernel, H, 
     test_attention_prefill_tensor_cores(monkeypatch, kernel, H, Hkv, 64, seqs, 0)
 
 
+@pytest.mark.parametrize("climb", [0.0, 0.1, 8.0, 30.0, -8.0])
+@pytest.mark.parametrize("n_parts", [1, 2])
+def test_attention_prefill_where_the_maximum_climbs(climb, n_parts):
+    """Scores that rise by `climb` powers of two from one block of 128 keys to the next (1, 1.5 and 2 times that for every third row): the tcgen05
+    kernel scales what it has summed where a row's maximum grows, the two halves of a block's keys agreeing on it.  P and the
+    result are rounded to bfloat16, 2^-9 each."""
+    from vlrf_b200.csrc import ops
+    H, dh, n, scale = 2, 64, 700, 0.125
+    q, k, v = (0.3 * randn(H, n, dh, seed=s) for s in (101, 102, 103))
+    q[:, :, 0] = (1.0 + torch.arange(n).float() % 3 / 2) * 8.0
+    k[:, :, 0] = climb * 0.6931 / scale / 8.0 * (torch.arange(n) // 128).float()
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    qkv = torch.cat([t.permute(1, 0, 2).reshape(n, H * dh) for t in (q, k, v)], dim=1).contiguous()
+    kp, vp, perm = paged(k, v, 14, 5, torch.bfloat16)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    out, e = torch.empty(n, H * dh, dtype=torch.bfloat16, device=DEV), err_word()
+    floats, counts = ops.attention_prefill_scratch(1, n, H, n_parts)
+    ops.attention_prefill(qkv.to(DEV), 0, kp.to(DEV), vp.to(DEV), i32([perm.tolist()]), i32([0]), i32([0, n]), i32([0]), out, n, 1, n, H, H, dh,
+                          scale, 0, e, n_parts, torch.empty(floats, device=DEV), torch.zeros(counts, dtype=torch.int32, device=DEV))
+    assert int(e.item()) == 0
+    got = out.float().cpu().reshape(n, H, dh).permute(1, 0, 2)
+    want = plain_attention(q.float(), k.float(), v.float(), scale)
+    for rows in (slice(0, n), slice(0, 128), slice(128, 140), slice(600, 700)):
+        assert rel_err(got[:, rows], want[:, rows]) < 1.5e-2
+
+
+def test_attention_prefill_reads_no_value_that_it_did_not_load():
+    """A tile whose last query lies in the first half of a block of 128 keys loads that half only, although the sequence goes on: what the other half
+    of the buffer holds (here NaN, left by the launch before) meets probabilities of zero and must not be read."""
+    from vlrf_b200.csrc import ops
+    H, dh, n, pos0 = 20, 64, 513, 37
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    q, k, v = (randn(H, pos0 + n, dh, seed=s).to(torch.bfloat16) for s in (121, 122, 123))
+    kp, vp, perm = paged(k, v, 12, 6, torch.bfloat16)
+    qkv = torch.zeros(n, 3 * H * dh, dtype=torch.bfloat16)
+    qkv[:, :H * dh] = q[:, pos0:].permute(1, 0, 2).reshape(n, H * dh)
+    nan = torch.full_like(kp, float("nan")).to(DEV)
+    out, e = torch.empty(n, H * dh, dtype=torch.bfloat16, device=DEV), err_word()
+    args = (i32([perm.tolist()]), i32([0]), i32([0, n]), i32([pos0]), out, n, 1, n, H, H, dh, 0.125, 0, e)
+    for _ in range(3):
+        ops.attention_prefill(qkv.to(DEV), 0, nan, nan, *args)
+        ops.attention_prefill(qkv.to(DEV), 0, kp.to(DEV), vp.to(DEV), *args)
+        assert int(e.item()) == 0
+        got = out.float().cpu().reshape(n, H, dh).permute(1, 0, 2)
+        assert rel_err(got, plain_attention(q[:, pos0:].float(), k.float(), v.float(), 0.125)) < 1.5e-2
+
+
 def test_kv_append_writes_each_token_where_its_slot_says():
     from vlrf_b200.csrc import ops
     Hkv, dh, T = 3, 16, 70

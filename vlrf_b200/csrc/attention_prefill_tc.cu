@@ -3,28 +3,32 @@
 //
 // A CTA takes 128 consecutive new tokens of one sequence and one head, and walks the sequence's keys in
 // blocks of 128 (two cache blocks) up to the diagonal (reference include/model/attention.hpp:233; visibility
-// k ≤ past + q :253-260; scale :373-374; softmax :265-307).  Its six warps have fixed jobs:
-//   warp 4  producer: the query tile once, then key and value tiles in turn through a ring of three
+// k ≤ past + q :253-260; scale :373-374; softmax :265-307).  Its ten warps have fixed jobs:
+//   warp 8  producer: the query tile once, then key and value tiles in turn through a ring of four
 //           shared-memory slots (tiled TMA loads, 128-byte swizzle, one load per 64-token cache block);
-//   warp 5  one elected thread issues the MMAs: S = Q·Kᵀ (128 × 128, four k steps) into tensor memory, and,
-//           once the probabilities are in shared memory, O_j = P·V (128 × 64, eight k steps; V is read as it
-//           lies in the cache, head dimension contiguous, through an MN-major descriptor);
-//   warps 0-3  softmax: a thread owns one query row, which is one lane of tensor memory, so the row's
-//           maximum and sum need no exchange between threads.  It reads S twice with `tcgen05.ld` (maximum,
-//           then exponentials), masks the blocks on the diagonal and at the window's edge, writes P as
-//           bfloat16 into shared memory in the layout the MMA expects, and keeps the running maximum, the
-//           sum and the 64 outputs of its row in registers: O_j of each block is read back from tensor
-//           memory and added after rescaling, so tensor memory is never rescaled in place.
+//   warp 9  issues the MMAs: S = Q·Kᵀ (128 × 128, four k steps) into tensor memory, and, once the
+//           probabilities are there too, O += P·V (128 × 64, eight k steps; P is the operand in tensor memory, V is
+//           read as it lies in the cache, head dimension contiguous, through an MN-major descriptor);
+//   warps 0-7  softmax: a query row is one lane of tensor memory, and two threads, of warps q and q + 4, have a half of a block's
+//           keys each; they exchange the row's maximum through shared memory.  A thread takes its 64 scores of a block into
+//           registers at once, which frees S for the next block's scores, and writes P as bfloat16 into tensor memory.  Blocks on
+//           the diagonal and at the window's edge are masked, and a warp leaves out chunks of 32 keys that lie behind all of its
+//           rows.  O stays in tensor memory until the CTA's last block; where a row's maximum grew, its O is read back, scaled and
+//           written again once P is on its way.  (Scaling only where the maximum has grown by much would save that mostly, but
+//           then the largest P is not 1, which bfloat16 holds exactly, and peaked rows lose: 1.42e-3 -> 1.54e-3 off 64 bits.)
+// A thread a row (its 128 scores read twice, P through shared memory, O added up in registers) took 20.1 us for 2 x 1,024 tokens of 12 heads,
+// 30.6 for 4 x 1,024 of 16; sixteen softmax warps an SM instead of eight keep the exponentials' unit and the issue slots busier.
 // A CTA's blocks are a chain (scores, softmax, output product, one after the other), so a step with few
 // tiles is bound by its longest tile, not by the SMs' throughput.  The keys of a long tile can therefore be
 // dealt to up to `n_parts` CTAs: each leaves its rows' maximum, sum and outputs in global scratch, and the
 // one that finishes last (a counter per tile says which) merges all of them in a fixed order, so the result
 // does not depend on which CTA that is.  Long tiles come first in the grid.
-// Two CTAs fit an SM (96 KiB of shared memory, 256 columns of tensor memory each): while one waits for its
+// Two CTAs fit an SM (82 KiB of shared memory, 256 columns of tensor memory each): while one waits for its
 // MMAs the other computes exponentials.  Rows of the last cache block behind the sequence's end hold
 // whatever was there before; their scores are masked by assignment and their rows of V are cleared before
 // the MMA reads them (0 · NaN would not be 0).  Every wait is bounded; a CTA that gives up sets the device
 // error word, waits (bounded) for its copies in flight, frees its tensor memory and leaves.
+#include <type_traits>
 #include "common.cuh"
 #include "tma.cuh"
 #include "tcgen05.cuh"
@@ -32,10 +36,10 @@
 namespace {
 
 constexpr int FT_BQ = 128, FT_BK = 128, FT_DH = 64, FT_CB = 64;   // queries / keys per block, head size, tokens per cache block
-constexpr int FT_THREADS = 192;
+constexpr int FT_THREADS = 320;
 constexpr int FT_TILE = FT_BK * FT_DH * 2;                         // bytes of a K or V tile (and of the Q tile)
-constexpr int FT_SLOTS = 3;
-constexpr int FT_TMEM_COLS = 256;                                  // S: columns 0-127, O_j: 128-191
+constexpr int FT_SLOTS = 4;
+constexpr int FT_TMEM_COLS = 256;                                  // S: columns 0-127, O: 128-191, P (two bfloat16 a column): 192-255
 constexpr int FT_MIN_PART = 2;                                     // key blocks a part holds at least (what the host plans with)
 constexpr int FT_PART_BLOCKS = 3;                                  // key blocks a part holds at most, while the tile has parts left
 constexpr int FT_MAX_PARTS = 8;
@@ -65,10 +69,32 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
-// (With 168 registers a thread an SM's four schedulers hold two CTAs of six warps only if their warps fall
-// three to a scheduler, so a CTA that ends is often replaced only when its neighbour has ended too; a limit
-// of 128 registers, under which any placement fits, was measured: every block became 5 % slower, which cost
-// more than the waiting, since CTAs that share an SM are of similar length in the order below.)
+// D += A · B with A (bfloat16, two of a row's elements a column) in tensor memory
+__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};\n"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, int q_off, const int* __restrict__ block_table,
@@ -82,13 +108,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     if (threadIdx.x == 0) VLRF_TRACE(trace, 4, tcta, 0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* q_tile = smem;                                    // [128][128 B]
-    unsigned char* kv_tiles = smem + FT_TILE;                        // [3][128][128 B]: K_0, V_0, K_1, V_1, … in turn
-    unsigned char* p_tile = kv_tiles + FT_SLOTS * FT_TILE;           // [2][128][128 B]: keys 0-63, 64-127 of the block
-    uint64_t* q_full = reinterpret_cast<uint64_t*>(p_tile + 2 * FT_TILE);
-    uint64_t* full = q_full + 1;                                     // [3]
-    uint64_t* empty = full + FT_SLOTS;                               // [3]
+    unsigned char* kv_tiles = smem + FT_TILE;                        // [FT_SLOTS][128][128 B]: K_0, V_0, K_1, V_1, … in turn
+    float* s_part = reinterpret_cast<float*>(kv_tiles + FT_SLOTS * FT_TILE);      // [2][2][128]: the halves' maxima of a block (by its parity); sums at the end
+    uint64_t* q_full = reinterpret_cast<uint64_t*>(s_part + 4 * FT_BQ);
+    uint64_t* full = q_full + 1;                                     // [FT_SLOTS]
+    uint64_t* empty = full + FT_SLOTS;                               // [FT_SLOTS]
     uint64_t* s_full = empty + FT_SLOTS;
-    uint64_t* p_full = s_full + 1;
+    uint64_t* s_read = s_full + 1;                                   // the scores are in registers: S may be written again
+    uint64_t* p_full = s_read + 1;
     uint64_t* o_full = p_full + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
@@ -108,14 +135,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         tbar_init(q_full, 1);
         for (int i = 0; i < FT_SLOTS; ++i) { tbar_init(&full[i], 1); tbar_init(&empty[i], 1); }
         tbar_init(s_full, 1);
-        tbar_init(p_full, 4);
+        tbar_init(s_read, 8);
+        tbar_init(p_full, 8);
         tbar_init(o_full, 1);
         *s_abort = 0;
         *s_never = 0;
         *s_last = 1;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 4) {
+    if (warp == 8) {
         if (lane == 0) { tma_prefetch_descriptor(&tmap_q); tma_prefetch_descriptor(&tmap_k); tma_prefetch_descriptor(&tmap_v); }
         __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tsm(tmem_slot)), "r"((uint32_t)FT_TMEM_COLS) : "memory");
@@ -177,10 +205,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + 128;
+    const uint32_t tmem_s = *tmem_slot, tmem_o = tmem_s + 128, tmem_p = tmem_s + 192;
 
-    if (warp == 4) {
-        if (lane == 0 && my_n > 0) {
+    if (warp == 8) {
+        if (my_n > 0 && elect_one()) {
             tbar_expect_tx(q_full, FT_TILE);
             tma_load_2d(q_tile, &tmap_q, q_off + h * FT_DH, row0 + qt * FT_BQ, q_full);
             int n_issued = 0;                         // tiles requested: 2j is K of block j, 2j+1 its V
@@ -210,183 +238,224 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                     tbar_wait_or_abort(&full[t % FT_SLOTS], (uint32_t)((t / FT_SLOTS) & 1), s_never);
             }
         }
-    } else if (warp == 5) {
-        if (lane == 0 && my_n > 0) {
+    } else if (warp == 9) {
+        if (my_n > 0) {                              // (the whole warp waits, one lane issues: tcgen05.cuh)
             constexpr uint32_t idesc_s = umma_idesc_bf16(FT_BQ, FT_BK);
             constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(FT_BQ, FT_DH);
             bool ok = tbar_wait_or_abort(q_full, 0, s_abort);
-            const uint64_t dq = umma_desc_k128(q_tile);
+            const uint64_t dq = umma_desc_k128(q_tile), dk0 = umma_desc_k128(kv_tiles), dv0 = umma_desc_mn128(kv_tiles);
             // S_j = Q · K_jᵀ into tensor memory, four k steps
             auto issue_s = [&](int j) -> bool {
-                const int tk = 2 * j;
-                if (!tbar_wait_or_abort(&full[tk % FT_SLOTS], (uint32_t)((tk / FT_SLOTS) & 1), s_abort)) return false;
+                const uint32_t tk = 2u * j, sl = tk % FT_SLOTS;
+                if (!tbar_wait_or_abort(&full[sl], (tk / FT_SLOTS) & 1u, s_abort)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dk = umma_desc_k128(kv_tiles + (size_t)(tk % FT_SLOTS) * FT_TILE);
+                if (elect_one()) {
+                    const uint64_t dk = dk0 + (uint64_t)(sl * (FT_TILE >> 4));
 #pragma unroll
-                for (int k = 0; k < FT_DH / 16; ++k) umma_bf16(tmem_s, dq + 2 * k, dk + 2 * k, idesc_s, k > 0 ? 1u : 0u);
-                umma_commit(&empty[tk % FT_SLOTS]);
-                umma_commit(s_full);
+                    for (int k = 0; k < FT_DH / 16; ++k) umma_bf16(tmem_s, dq + 2 * k, dk + 2 * k, idesc_s, k > 0 ? 1u : 0u);
+                    umma_commit(s_full);
+                    umma_commit(&empty[sl]);
+                }
+                __syncwarp();
                 return true;
             };
             ok = ok && issue_s(0);
             for (int j = 0; j < my_n && ok; ++j) {
-                // the softmax warps have read S_j and written P_j.  S_{j+1} goes first, so that they can start on
-                // it while O_j = P_j · V_j is still being computed (they want O_j only after their first pass).
+                // S_{j+1} as soon as the softmax warps hold S_j in registers, O += P_j · V_j once they have written P_j
+                if (j + 1 < my_n && !(tbar_wait_or_abort(s_read, (uint32_t)(j & 1), s_abort) && issue_s(j + 1))) { ok = false; break; }
+                const uint32_t tv = 2u * j + 1, sl = tv % FT_SLOTS;
+                if (!tbar_wait_or_abort(&full[sl], (tv / FT_SLOTS) & 1u, s_abort)) { ok = false; break; }
                 if (!tbar_wait_or_abort(p_full, (uint32_t)(j & 1), s_abort)) { ok = false; break; }
-                if (j + 1 < my_n && !issue_s(j + 1)) { ok = false; break; }
-                const int tv = 2 * j + 1;
-                if (!tbar_wait_or_abort(&full[tv % FT_SLOTS], (uint32_t)((tv / FT_SLOTS) & 1), s_abort)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint64_t dv = umma_desc_mn128(kv_tiles + (size_t)(tv % FT_SLOTS) * FT_TILE);
+                if (elect_one()) {
+                    const uint64_t dv = dv0 + (uint64_t)(sl * (FT_TILE >> 4));
 #pragma unroll
-                for (int k = 0; k < FT_BK / 16; ++k) {
-                    // 16 keys a step: P's piece lies 32 bytes further in its 64-key half, V's 16 rows further
-                    const uint64_t dp = umma_desc_k128(p_tile + (size_t)(k >> 2) * FT_TILE) + 2 * (k & 3);
-                    umma_bf16(tmem_o, dp, dv + (uint64_t)(k * 16 * 128 >> 4), idesc_o, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < FT_BK / 16; ++k)      // 16 keys a step: 8 columns of P, 16 rows of V
+                        umma_bf16_ta(tmem_o, tmem_p + 8u * k, dv + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(o_full);
+                    umma_commit(&empty[sl]);
                 }
-                umma_commit(&empty[tv % FT_SLOTS]);
-                umma_commit(o_full);
+                __syncwarp();
             }
             if (!ok) atomicExch(s_abort, 1);
         }
     } else if (active) {
-        // ---- softmax warps: thread = query row = lane of tensor memory ----
-        const int r = warp * 32 + lane;
+        // ---- softmax warps: a lane of tensor memory is a query row; warps q and q + 4 have a half of a block's keys each
+        const int q = warp & 3, half = warp >> 2, r = q * 32 + lane;
         const int q_pos = q_first + r;
-        const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;
+        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
         const float sl2 = scale * 1.4426950408889634f;               // scores in units of log2(e)
         const unsigned win_eff = window > 0 ? (unsigned)window : 0x7fffffffu;   // key visible: 0 ≤ q_pos − key < win_eff
-        float o_acc[FT_DH];
-#pragma unroll
-        for (int d = 0; d < FT_DH; ++d) o_acc[d] = 0.f;
-        float m_run = -INFINITY, l_run = 0.f, corr = 0.f;            // corr: what block j's maximum did to the sums before it
+        float m_run = -INFINITY, l_run = 0.f;                        // the row's maximum; the sum of this half
         bool ok = true;
-        // O of the block before is complete (and P's buffer free): o_acc holds the blocks before that one
-        // relative to the maximum before it; rescale and add
-        auto add_o = [&]() {
-#pragma unroll
-            for (int c = 0; c < FT_DH; c += 32) {
-                uint32_t ov[32];
-                tmem_ld32(tmem_o + lane_addr + (uint32_t)c, ov);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o_acc[c + i] = fmaf(o_acc[c + i], corr, __uint_as_float(ov[i]));
+        // one block; MASKED: some key of it is hidden from some row
+        auto block = [&](int j, auto masked_c) {
+            constexpr bool MASKED = decltype(masked_c)::value;
+            const int k0 = (my_first + j) * FT_BK + half * 64;        // the half's first key
+            // chunks of 32 keys of which a row of this warp sees any (those behind lie above the diagonal)
+            const int q_top = q_first + q * 32 + 31;
+            const int n_live = MASKED ? (q_top < k0 ? 0 : min(2, ((q_top - k0) >> 5) + 1)) : 2;
+            // (a warp that has given up goes on meeting its neighbour, who may not have)
+            if (!ok || !tbar_wait_or_abort(s_full, (uint32_t)(j & 1), s_abort)) {
+                ok = false;
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+                return;
             }
-        };
-        for (int j = 0; j < my_n; ++j) {
-            const int k_base = (my_first + j) * FT_BK;
-            const bool need_mask = window > 0 || (k_base + FT_BK - 1 > q_first);     // uniform over the CTA
-            if (!ok || !tbar_wait_or_abort(s_full, (uint32_t)(j & 1), s_abort)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // pass 1: the row's maximum over this block (of the raw scores: the scale is positive)
+            // the row's maximum over this block (of the raw scores: the scale is positive).  Blocks without a mask keep the scores in
+            // registers; a mask's blocks, one in a tile's row of them, read a chunk at a time, twice.
+            const uint32_t s_at = tmem_s + lane_addr + (uint32_t)(half * 64);
+            uint32_t sv[2][32];
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll 1
-            for (int c = 0; c < FT_BK; c += 32) {
-                uint32_t sv[32];
-                tmem_ld32(tmem_s + lane_addr + (uint32_t)c, sv);
+            if (!MASKED) {
+                tmem_ld32(s_at, sv[0]);
+                tmem_ld32(s_at + 32u, sv[1]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (need_mask) {
-                    const int d0 = q_pos - (k_base + c);              // q_pos − key for i = 0
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tbar_arrive(s_read);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const float v = ((unsigned)(d0 - i) < win_eff) ? __uint_as_float(sv[i]) : -INFINITY;
-                        mx[i & 3] = fmaxf(mx[i & 3], v);
-                    }
-                } else {
+                for (int c = 0; c < 2; ++c)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sv[i]));
-                }
-            }
-            const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2);
-            const float m_use = (m_new == -INFINITY) ? 0.f : m_new;   // a row that sees nothing yet: every p is 0
-            const float corr_new = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - m_new);
-            if (j > 0) {
-                if (!tbar_wait_or_abort(o_full, (uint32_t)((j - 1) & 1), s_abort)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                add_o();
-            }
-            corr = corr_new;
-            // pass 2: exponentials, their sum, P as bfloat16 into shared memory
-            float sm4[4] = {0.f, 0.f, 0.f, 0.f};
+                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sv[c][i]));
+            } else {
 #pragma unroll 1
-            for (int c = 0; c < FT_BK; c += 32) {
-                uint32_t sv[32];
-                tmem_ld32(tmem_s + lane_addr + (uint32_t)c, sv);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float p[32];
-                if (need_mask) {
-                    const int d0 = q_pos - (k_base + c);
+                for (int c = 0; c < n_live; ++c) {
+                    tmem_ld32(s_at + (uint32_t)(c * 32), sv[0]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    const int d0 = q_pos - (k0 + c * 32);             // q_pos − key for i = 0
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const float e = fast_exp2(fmaf(__uint_as_float(sv[i]), sl2, -m_use));
-                        p[i] = ((unsigned)(d0 - i) < win_eff) ? e : 0.f;
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) p[i] = fast_exp2(fmaf(__uint_as_float(sv[i]), sl2, -m_use));
-                }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) sm4[i & 3] += p[i];
-                unsigned char* prow = p_tile + (size_t)(c >> 6) * FT_TILE + r * 128;
-#pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8) {
-                    uint4 pk;
-                    pk.x = pack2(p[g8 * 8 + 0], p[g8 * 8 + 1]); pk.y = pack2(p[g8 * 8 + 2], p[g8 * 8 + 3]);
-                    pk.z = pack2(p[g8 * 8 + 4], p[g8 * 8 + 5]); pk.w = pack2(p[g8 * 8 + 6], p[g8 * 8 + 7]);
-                    const int piece = ((c & 63) >> 3) + g8;
-                    *reinterpret_cast<uint4*>(prow + ((piece ^ (r & 7)) << 4)) = pk;
+                    for (int i = 0; i < 32; ++i) mx[i & 3] = fmaxf(mx[i & 3], (unsigned)(d0 - i) < win_eff ? __uint_as_float(sv[0][i]) : -INFINITY);
                 }
             }
-            l_run = fmaf(l_run, corr, (sm4[0] + sm4[1]) + (sm4[2] + sm4[3]));
+            const float m_half = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            s_part[((j & 1) * 2 + half) * FT_BQ + r] = m_half;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+            const float m_new = fmaxf(m_run, fmaxf(m_half, s_part[((j & 1) * 2 + (half ^ 1)) * FT_BQ + r]) * sl2);
+            const float corr = m_run == -INFINITY ? 1.f : fast_exp2(m_run - m_new);      // (from −inf on the row's sums are 0 so far)
+            l_run *= corr;
             m_run = m_new;
-            // rows of V behind the sequence's last token hold whatever was there before: clear them
-            const int valid = pos0 + n_new - k_base;                  // keys of this block that exist
-            if (valid < FT_BK) {
-                const int tv = 2 * j + 1;
-                if (!tbar_wait_or_abort(&full[tv % FT_SLOTS], (uint32_t)((tv / FT_SLOTS) & 1), s_abort)) { ok = false; break; }
-                unsigned char* vt = kv_tiles + (size_t)(tv % FT_SLOTS) * FT_TILE;
-                const int first_row = max(valid, 0);
-                for (int idx = r; idx < (FT_BK - first_row) * 8; idx += 128)
-                    *reinterpret_cast<uint4*>(vt + (first_row + (idx >> 3)) * 128 + ((idx & 7) << 4)) = make_uint4(0, 0, 0, 0);
+            const float m_use = (m_run == -INFINITY) ? 0.f : m_run;   // a row that sees nothing yet: every p is 0
+            if (j > 0) {                                              // O holds the blocks before, and P may be written again
+                if (!tbar_wait_or_abort(o_full, (uint32_t)((j - 1) & 1), s_abort)) { ok = false; return; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
+            // exponentials, their sum, P as bfloat16 into tensor memory
+            float sm4[4] = {0.f, 0.f, 0.f, 0.f};
+            auto chunk = [&](int c, const uint32_t (&x)[32]) {
+                uint32_t pk[16];
+                const int d0 = q_pos - (k0 + c * 32);
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) {
+                    float p0 = fast_exp2(fmaf(__uint_as_float(x[i]), sl2, -m_use)), p1 = fast_exp2(fmaf(__uint_as_float(x[i + 1]), sl2, -m_use));
+                    if (MASKED) {
+                        p0 = (unsigned)(d0 - i) < win_eff ? p0 : 0.f;
+                        p1 = (unsigned)(d0 - i - 1) < win_eff ? p1 : 0.f;
+                    }
+                    sm4[i & 3] += p0;
+                    sm4[(i + 1) & 3] += p1;
+                    pk[i >> 1] = pack2(p0, p1);
+                }
+                tmem_st16(tmem_p + lane_addr + (uint32_t)(half * 32 + c * 16), pk);
+            };
+            if (!MASKED) {
+                chunk(0, sv[0]);
+                chunk(1, sv[1]);
+            } else {
+#pragma unroll 1
+                for (int c = 0; c < 2; ++c) {
+                    if (c < n_live) {
+                        tmem_ld32(s_at + (uint32_t)(c * 32), sv[0]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        chunk(c, sv[0]);
+                    } else {
+                        uint32_t none[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) none[i] = 0u;
+                        tmem_st16(tmem_p + lane_addr + (uint32_t)(half * 32 + c * 16), none);
+                    }
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tbar_arrive(s_read);
+            }
+            l_run += (sm4[0] + sm4[1]) + (sm4[2] + sm4[3]);
+            if (j > 0 && __any_sync(0xffffffffu, corr != 1.f)) {      // a row's maximum grew: its O (a half of the columns here) follows
+                uint32_t ov[32];
+                tmem_ld32(tmem_o + lane_addr + (uint32_t)half * 32u, ov);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+                tmem_st32(tmem_o + lane_addr + (uint32_t)half * 32u, ov);
+            }
+            // rows of V that this CTA did not load, or that lie behind the sequence's last token, hold whatever was there before: clear them
+            const int there = min(pos0 + n_new - (my_first + j) * FT_BK, ((my_first + j) * 2 + 1 <= cb_last ? 2 : 1) * FT_CB);
+            if (there < FT_BK) {
+                const int tv = 2 * j + 1;
+                if (!tbar_wait_or_abort(&full[tv % FT_SLOTS], (uint32_t)((tv / FT_SLOTS) & 1), s_abort)) { ok = false; return; }
+                unsigned char* vt = kv_tiles + (size_t)(tv % FT_SLOTS) * FT_TILE;
+                const int first_row = max(there, 0);
+                for (int idx = warp * 32 + lane; idx < (FT_BK - first_row) * 8; idx += 256)
+                    *reinterpret_cast<uint4*>(vt + (first_row + (idx >> 3)) * 128 + ((idx & 7) << 4)) = make_uint4(0, 0, 0, 0);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the MMA reads them
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // P (and V's cleared rows) are read by the MMA
             __syncwarp();
             if (lane == 0) tbar_arrive(p_full);
+        };
+        for (int j = 0; j < my_n; ++j) {
+            if (window > 0 || (my_first + j) * FT_BK + FT_BK - 1 > q_first) block(j, std::true_type{});      // (uniform over the CTA)
+            else block(j, std::false_type{});
         }
+        // the row's result of this half's columns, and the sum of both halves of the keys
+        constexpr int HD = FT_DH / 2;
+        float o_acc[HD];
+#pragma unroll
+        for (int d = 0; d < HD; ++d) o_acc[d] = 0.f;
         if (my_n > 0) {
             if (ok && tbar_wait_or_abort(o_full, (uint32_t)((my_n - 1) & 1), s_abort)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                add_o();
+                uint32_t ov[HD];
+                tmem_ld32(tmem_o + lane_addr + (uint32_t)(half * HD), ov);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < HD; ++i) o_acc[i] = __uint_as_float(ov[i]);
             } else {
                 ok = false;
                 atomicExch(s_abort, 1);
             }
         }
+        asm volatile("bar.sync 5, 256;" ::: "memory");               // (also behind the last block's maxima)
+        s_part[half * FT_BQ + r] = l_run;
+        asm volatile("bar.sync 5, 256;" ::: "memory");
+        l_run = s_part[r] + s_part[FT_BQ + r];
         bool writes_out = true;
         if (tile_parts > 1) {
             // leave this part's result in scratch ([d][row], so that a warp writes whole lines), then see
             // whether the tile's other parts are all there
             float* mine = partials + ((size_t)tile_id * n_parts + part) * FT_PART_FLOATS;
 #pragma unroll
-            for (int d = 0; d < FT_DH; ++d) mine[d * FT_BQ + r] = o_acc[d];
-            mine[FT_DH * FT_BQ + r] = m_run;
-            mine[FT_DH * FT_BQ + FT_BQ + r] = l_run;
+            for (int d = 0; d < HD; ++d) mine[(half * HD + d) * FT_BQ + r] = o_acc[d];
+            if (half == 0) {
+                mine[FT_DH * FT_BQ + r] = m_run;
+                mine[FT_DH * FT_BQ + FT_BQ + r] = l_run;
+            }
             __threadfence();
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (r == 0) {
+            asm volatile("bar.sync 5, 256;" ::: "memory");
+            if (threadIdx.x == 0) {
                 const int before = atomicAdd(&counters[tile_id], 1);
                 *s_last = (before == tile_parts - 1) ? 1 : 0;
                 if (before == tile_parts - 1) counters[tile_id] = 0;          // left as it was found
             }
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            asm volatile("bar.sync 5, 256;" ::: "memory");
             writes_out = *s_last != 0;
             if (writes_out) {
                 __threadfence();
                 // every part in turn, this CTA's own included: the sum does not depend on who came last
                 m_run = -INFINITY; l_run = 0.f;
 #pragma unroll
-                for (int d = 0; d < FT_DH; ++d) o_acc[d] = 0.f;
+                for (int d = 0; d < HD; ++d) o_acc[d] = 0.f;
                 for (int p = 0; p < tile_parts; ++p) {
                     const float* theirs = partials + ((size_t)tile_id * n_parts + p) * FT_PART_FLOATS;
                     const float m_p = __ldcg(theirs + FT_DH * FT_BQ + r), l_p = __ldcg(theirs + FT_DH * FT_BQ + FT_BQ + r);
@@ -396,36 +465,40 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                     l_run = fmaf(l_run, a, l_p * b);
                     m_run = m_new;
 #pragma unroll
-                    for (int d0 = 0; d0 < FT_DH; d0 += 16) {
+                    for (int d0 = 0; d0 < HD; d0 += 16) {
                         float v[16];
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = __ldcg(theirs + (d0 + i) * FT_BQ + r);
+                        for (int i = 0; i < 16; ++i) v[i] = __ldcg(theirs + (half * HD + d0 + i) * FT_BQ + r);
 #pragma unroll
                         for (int i = 0; i < 16; ++i) o_acc[d0 + i] = fmaf(o_acc[d0 + i], a, v[i] * b);
                     }
                 }
             }
         }
-        if (writes_out && ok) {
-            // the row as bfloat16 into shared memory (P's tile: no MMA reads it any more), then each warp
-            // writes its 32 rows four at a time, so that a store instruction fills whole lines
+        if (writes_out) {
+            // the row as bfloat16 into shared memory (Q's tile: no MMA reads it any more), then each warp
+            // writes 16 rows four at a time, so that a store instruction fills whole lines
             const float inv = (l_run > 0.f) ? 1.f / l_run : 0.f;
-            unsigned char* stage = p_tile;                            // [128][128 B], 16-byte pieces swizzled by row
+            unsigned char* stage = q_tile;                            // [128][128 B], 16-byte pieces swizzled by row
+            if (ok) {
 #pragma unroll
-            for (int d = 0; d < FT_DH; d += 8) {
-                uint4 pk;
-                pk.x = pack2(o_acc[d] * inv, o_acc[d + 1] * inv); pk.y = pack2(o_acc[d + 2] * inv, o_acc[d + 3] * inv);
-                pk.z = pack2(o_acc[d + 4] * inv, o_acc[d + 5] * inv); pk.w = pack2(o_acc[d + 6] * inv, o_acc[d + 7] * inv);
-                *reinterpret_cast<uint4*>(stage + r * 128 + ((((d >> 3)) ^ (r & 7)) << 4)) = pk;
+                for (int d = 0; d < HD; d += 8) {
+                    uint4 pk;
+                    pk.x = pack2(o_acc[d] * inv, o_acc[d + 1] * inv); pk.y = pack2(o_acc[d + 2] * inv, o_acc[d + 3] * inv);
+                    pk.z = pack2(o_acc[d + 4] * inv, o_acc[d + 5] * inv); pk.w = pack2(o_acc[d + 6] * inv, o_acc[d + 7] * inv);
+                    *reinterpret_cast<uint4*>(stage + r * 128 + (((half * HD + d) >> 3 ^ (r & 7)) << 4)) = pk;
+                }
             }
-            __syncwarp();
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+            if (ok) {
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int rr = warp * 32 + it * 4 + (lane >> 3), piece = lane & 7;
-                const int q_local = qt * FT_BQ + rr;
-                if (q_local < n_new) {
-                    const uint4 pk = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((piece ^ (rr & 7)) << 4));
-                    *reinterpret_cast<uint4*>(out + (size_t)(row0 + q_local) * ld_out + (size_t)h * FT_DH + piece * 8) = pk;
+                for (int it = 0; it < 4; ++it) {
+                    const int rr = q * 32 + half * 16 + it * 4 + (lane >> 3), piece = lane & 7;
+                    const int q_local = qt * FT_BQ + rr;
+                    if (q_local < n_new) {
+                        const uint4 pk = *reinterpret_cast<const uint4*>(stage + rr * 128 + ((piece ^ (rr & 7)) << 4));
+                        *reinterpret_cast<uint4*>(out + (size_t)(row0 + q_local) * ld_out + (size_t)h * FT_DH + piece * 8) = pk;
+                    }
                 }
             }
         }
@@ -434,7 +507,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (warp == 4) {
+    if (warp == 8) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"((uint32_t)FT_TMEM_COLS) : "memory");
     }
     if (threadIdx.x == 0) VLRF_TRACE(trace, 4, tcta, 6);
@@ -488,7 +561,7 @@ extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const vo
     if (st != VLRF_OK) return st;
     st = vlrf_make_tmap_bf16(Vc, kv_rows, dh, dh, FT_CB, 64, &tv);
     if (st != VLRF_OK) return st;
-    const size_t smem = 1024 + (size_t)(1 + FT_SLOTS + 2) * FT_TILE + 16 * 8;
+    const size_t smem = 1024 + (size_t)(1 + FT_SLOTS) * FT_TILE + 4 * FT_BQ * 4 + 24 * 8;
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
