@@ -39,6 +39,7 @@
 // Launched "chained": weights are requested before the kernel ahead has finished, activations only after.
 // Every wait on an mbarrier is bounded; a CTA that gives up sets the device error word, sends nothing (its
 // receivers then give up too, after their own bounded wait) and frees its tensor memory.
+#include <type_traits>
 #include "common.cuh"
 #include <cstdlib>
 #include <cstring>
@@ -517,19 +518,23 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             float acc[RP];
 #pragma unroll
             for (int e = 0; e < RP; ++e) acc[e] = 0.f;
+#pragma unroll 1
+            for (int s0 = 0; s0 < splits; s0 += 4) {                // always in the order of the parts, four asked for at a time
+                float v[4][RP];
 #pragma unroll
-            for (int s = 0; s < SP_MAX_SPLITS; ++s) {               // always in the order of the parts
-                if (s < splits) {
+                for (int i = 0; i < 4; ++i) {
+                    const float* from = mine + (size_t)min(s0 + i, splits - 1) * n_j * 128 * RP;
                     if (RP == 4) {
-                        const float4 v = *reinterpret_cast<const float4*>(mine + (size_t)s * n_j * 128 * RP);
-                        acc[0] += v.x; acc[RP / 4] += v.y; acc[RP / 2] += v.z; acc[RP - 1] += v.w;
-                    } else {
-                        acc[0] += mine[(size_t)s * n_j * 128 * RP];
-                    }
+                        const float4 x = *reinterpret_cast<const float4*>(from);
+                        v[i][0] = x.x; v[i][RP / 4] = x.y; v[i][RP / 2] = x.z; v[i][RP - 1] = x.w;
+                    } else v[i][0] = *from;
                 }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) acc[e] = s0 + i < splits ? acc[e] + v[i][e] : acc[e];
             }
             const float bv = j < 2 ? (j == 0 ? pre_bias[0] : pre_bias[1]) : ((bias && n < N) ? bias[n] : 0.f);
-            const int n_seg = min(32, N - seg0);
             // where this column lies in the cache, if it is a key's or a value's (the same for every row of the piece)
             __nv_bfloat16* kv_col = nullptr;
             if (n < N && kv.Kc != nullptr && n >= kv.k_off) {
@@ -540,30 +545,69 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                     kv_col = reinterpret_cast<__nv_bfloat16*>(is_v ? kv.Vc : kv.Kc) + (size_t)hh * kv.BT * kv.dh + cc;
                 }
             }
+            // Pieces whose rows and columns all exist go without a branch a row, and the activation is resolved once a piece: a single warp a
+            // scheduler finishes them, at the latency of every instruction (17 to 64 rows 3,600 to 6,200 cycles of a product before).
+            const bool whole = seg0 + 32 <= N && m0 + RP <= M;
+            float y[RP];
+            if (j < 2) {
 #pragma unroll
-            for (int e = 0; e < RP; ++e) {
-                const int m = m0 + e;
-                if (m >= M) break;                                  // (uniform over the warp)
-                float res = 0.f;
-                if (j < 2) res = j == 0 ? pre_res[0][e] : pre_res[1][e];
-                else if (residual && n < N) res = residual[(size_t)m * ldy + n];
-                const float y = apply_act_out<OT>(acc[e] + bv, act) + res;
-                if (n < N) ElemIO<OT>::store(Y + (size_t)m * ldy + n, y);
-                if (stats_out != nullptr && seg0 < N) {
-                    // what a LayerNorm of these rows will need: this segment's sum and squared deviation from its
-                    // own mean (of the values as stored; statistics are kept of float32 rows only)
-                    const float yv = n < N ? y : 0.f;
-                    const float sum = warp_sum(yv);
-                    const float d = n < N ? yv - sum / (float)n_seg : 0.f;
-                    const float m2 = warp_sum(d * d);
-                    if (lane == 0) {
-                        float* so = stats_out + ((size_t)m * ((N + 31) >> 5) + (seg0 >> 5)) * 2;
-                        so[0] = sum; so[1] = m2;
+                for (int e = 0; e < RP; ++e) y[e] = j == 0 ? pre_res[0][e] : pre_res[1][e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < RP; ++e) y[e] = residual && n < N && m0 + e < M ? residual[(size_t)(m0 + e) * ldy + n] : 0.f;
+            }
+            auto finish = [&](auto act_c) {
+                constexpr int ACT = decltype(act_c)::value;
+#pragma unroll
+                for (int e = 0; e < RP; ++e) y[e] = apply_act_const<OT, ACT>(acc[e] + bv) + y[e];
+            };
+            if (act == VLRF_ACT_NONE) finish(std::integral_constant<int, VLRF_ACT_NONE>{});
+            else if (act == VLRF_ACT_GELU_TANH) finish(std::integral_constant<int, VLRF_ACT_GELU_TANH>{});
+            else if (act == VLRF_ACT_RELU2) finish(std::integral_constant<int, VLRF_ACT_RELU2>{});
+            else finish(std::integral_constant<int, VLRF_ACT_GELU_ERF>{});
+            auto write = [&](auto whole_c) {
+                constexpr bool WHOLE = decltype(whole_c)::value;
+#pragma unroll
+                for (int e = 0; e < RP; ++e)
+                    if (WHOLE || (m0 + e < M && n < N)) ElemIO<OT>::store(Y + (size_t)(m0 + e) * ldy + n, y[e]);
+                if (kv_col != nullptr) {
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) {
+                        if (!WHOLE && m0 + e >= M) break;
+                        const int blk = s_kv_blk[m0 + e];
+                        if (blk >= 0) kv_col[((size_t)blk * kv.Hkv * kv.BT + s_kv_row[m0 + e]) * kv.dh] = __float2bfloat16_rn(y[e]);
                     }
                 }
-                if (kv_col != nullptr) {
-                    const int blk = s_kv_blk[m];
-                    if (blk >= 0) kv_col[((size_t)blk * kv.Hkv * kv.BT + s_kv_row[m]) * kv.dh] = __float2bfloat16_rn(y);
+            };
+            if (whole) write(std::true_type{});
+            else write(std::false_type{});
+            if (stats_out != nullptr && seg0 < N) {
+                // what a LayerNorm of these rows will need: this segment's sum and squared deviation from its
+                // own mean (of the values as stored; statistics are kept of float32 rows only)
+                const int n_seg = min(32, N - seg0);
+                float sum[RP], m2[RP];
+#pragma unroll
+                for (int e = 0; e < RP; ++e) sum[e] = n < N ? y[e] : 0.f;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
+#pragma unroll
+                for (int e = 0; e < RP; ++e) {
+                    const float d = n < N ? y[e] - sum[e] / (float)n_seg : 0.f;
+                    m2[e] = d * d;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int e = 0; e < RP; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
+                if (lane == 0) {
+#pragma unroll
+                    for (int e = 0; e < RP; ++e)
+                        if (m0 + e < M) {
+                            float* so = stats_out + ((size_t)(m0 + e) * ((N + 31) >> 5) + (seg0 >> 5)) * 2;
+                            so[0] = sum[e]; so[1] = m2[e];
+                        }
                 }
             }
         }
