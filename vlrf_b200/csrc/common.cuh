@@ -215,6 +215,15 @@ __device__ __forceinline__ void ld_global_32B(const void* p, float (&v)[8]) {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]),
                  "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
 }
+// a store that a lane may leave out, as a predicate on the instruction: rows that end within an unrolled run of stores otherwise become a
+// branch each, some 140 cycles of a warp that finishes a tile alone
+__device__ __forceinline__ void store_if(bool there, float* p, float v) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\n@p st.global.f32 [%0], %1;\n}\n" ::"l"(p), "f"(v), "r"((int)there) : "memory");
+}
+__device__ __forceinline__ void store_if(bool there, __nv_bfloat16* p, float v) {
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %2, 0;\n@p st.global.b16 [%0], %1;\n}\n" ::"l"(p), "h"(*reinterpret_cast<const unsigned short*>(&b)), "r"((int)there) : "memory");
+}
 // the same with the activation known at compile time (a run-time `act` per element costs issue slots: the
 // branches become predicates, and the paths not taken are still issued)
 template <typename OT, int ACT> __device__ __forceinline__ float apply_act_const(float x) {

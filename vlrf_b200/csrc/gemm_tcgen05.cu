@@ -275,18 +275,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                               "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                             : "r"(tmem_d + (uint32_t)c0));
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        if (n < N) {
+                        {
                             auto rows = [&](auto act_c) {                 // the activation as a compile-time constant
                                 constexpr int ACT = decltype(act_c)::value;
+                                float x[16];
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) {
-                                    const int m = r0 + c0 + j;
-                                    if (m < m_lim) {
-                                        float x = apply_act_const<OT, ACT>(__uint_as_float(r[j]) + bv);
-                                        if (residual) x += residual[(size_t)m * ldy + n];
-                                        ElemIO<OT>::store(Yt + (size_t)m * ldy + n, x);
-                                    }
+                                for (int j = 0; j < 16; ++j) x[j] = apply_act_const<OT, ACT>(__uint_as_float(r[j]) + bv);
+                                if (residual) {
+#pragma unroll
+                                    for (int j = 0; j < 16; ++j)
+                                        if (n < N && r0 + c0 + j < m_lim) x[j] += residual[(size_t)(r0 + c0 + j) * ldy + n];
                                 }
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) store_if(n < N && r0 + c0 + j < m_lim, Yt + (size_t)(r0 + c0 + j) * ldy + n, x[j]);
                             };
                             if (act == VLRF_ACT_NONE) rows(std::integral_constant<int, VLRF_ACT_NONE>{});
                             else if (act == VLRF_ACT_GELU_TANH) rows(std::integral_constant<int, VLRF_ACT_GELU_TANH>{});
