@@ -211,15 +211,16 @@ __global__ void __launch_bounds__(256) layernorm_warp_small_kernel(const float* 
     pdl_wait();
     pdl_launch_dependents();
     if (r >= n_rows) return;
-    float4 v[NV];
-    float mean, inv;
-    layernorm_row<NV>(x + (size_t)(rows ? rows[r] : r) * d, nv, d, eps, lane, v, mean, inv);
+    float4 v[1][NV];
+    float mean[1], inv[1];
+    const float* const src[1] = {x + (size_t)(rows ? rows[r] : r) * d};
+    layernorm_rows<NV, 1>(src, nv, d, eps, lane, v, mean, inv);
     OT* dst = out + (size_t)r * d;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
         const int i = j * 32 + lane;
         if (i < nv) {
-            const float4 y = layernorm_apply(v[j], mean, inv, s_gamma[i], s_beta[i]);
+            const float4 y = layernorm_apply(v[0][j], mean[0], inv[0], s_gamma[i], s_beta[i]);
             if (sizeof(OT) == 4) {
                 reinterpret_cast<float4*>(dst)[i] = y;
             } else {

@@ -206,7 +206,7 @@ struct F32Scatter {
 };
 constexpr int NORM_MAX_K = 1024, NORM_NV = NORM_MAX_K / 128;
 template <int R, int C, int STAGES> __host__ __device__ constexpr size_t norm_smem(int K) {
-    return ((size_t)STAGES * PARTS * C * KPITCH + (size_t)R * (K + 4 * PARTS)) * 4;
+    return ((size_t)STAGES * PARTS * C * KPITCH + (size_t)R * (K + 4 * PARTS) + 2 * (size_t)K) * 4;
 }
 
 template <int R, int C, int STAGES>
@@ -233,13 +233,13 @@ gemm_f32_norm_kernel(const float* __restrict__ X, const float* __restrict__ gamm
         if (s < n_chunks) load_w(s);
         cp_async_commit();
     }
-    float4 gm[NORM_NV], bt[NORM_NV];
-#pragma unroll
-    for (int j = 0; j < NORM_NV; ++j) {
-        const int i = j * 32 + lane;
-        gm[j] = i < nv ? reinterpret_cast<const float4*>(gamma)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        bt[j] = i < nv ? reinterpret_cast<const float4*>(beta)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4* const gm = reinterpret_cast<float4*>(rows + R * pitch);      // the norm's weight and bias
+    float4* const bt = gm + nv;
+    for (int i = tid; i < nv; i += THREADS_R) {
+        gm[i] = reinterpret_cast<const float4*>(gamma)[i];
+        bt[i] = reinterpret_cast<const float4*>(beta)[i];
     }
+    __syncthreads();
     pdl_wait();
     if (kv.Kc != nullptr && tid < R) {
         int blk = -1, row = 0;
@@ -253,14 +253,23 @@ gemm_f32_norm_kernel(const float* __restrict__ X, const float* __restrict__ gamm
         s_blk[tid] = blk;
         s_row[tid] = row;
     }
-    for (int r = warp; r < R; r += THREADS_R / 32) {
-        float4 v[NORM_NV];
-        float mean, inv;
-        layernorm_row<NORM_NV>(X + (size_t)min(r, M - 1) * K, nv, K, eps, lane, v, mean, inv);
+    constexpr int WARPS = THREADS_R / 32, RW = R / WARPS >= 2 ? 2 : 1;   // two of a warp's rows at a time
+    for (int r = warp * RW; r < R; r += WARPS * RW) {
+        float4 v[RW][NORM_NV];
+        float mean[RW], inv[RW];
+        const float* src[RW];
+#pragma unroll
+        for (int e = 0; e < RW; ++e) src[e] = X + (size_t)min(r + e, M - 1) * K;
+        layernorm_rows<NORM_NV, RW>(src, nv, K, eps, lane, v, mean, inv);
 #pragma unroll
         for (int j = 0; j < NORM_NV; ++j) {
             const int i = j * 32 + lane;
-            if (i < nv) *reinterpret_cast<float4*>(rows + (size_t)r * pitch + 4 * i + 4 * (4 * i / len)) = layernorm_apply(v[j], mean, inv, gm[j], bt[j]);
+            if (i < nv) {
+                const float4 g4 = gm[i], b4 = bt[i];
+                const int at = 4 * i + 4 * (4 * i / len);
+#pragma unroll
+                for (int e = 0; e < RW; ++e) *reinterpret_cast<float4*>(rows + (size_t)(r + e) * pitch + at) = layernorm_apply(v[e][j], mean[e], inv[e], g4, b4);
+            }
         }
     }
     float acc[R];
