@@ -20,18 +20,6 @@ def test_prompt_tiles_are_listed_only_where_they_fill_the_gpu(H, lens, parts, li
     assert bool(library().vlrf_attn_prefill_tc_lists(sum(lens), len(lens), max(lens), H, parts, 148)) == listed
 
 
-@pytest.mark.parametrize("n_seqs,longest,H,parts", [
-    (1, 1024, 2, 2), (1, 2048, 2, 4), (1, 700, 4, 2), (1, 500, 12, 1), (1, 1024, 12, 1), (2, 1024, 12, 1), (1, 2048, 12, 2), (1, 8192, 12, 1),
-    (1, 1024, 25, 1), (1, 2048, 25, 1), (6, 100, 12, 1)])
-def test_long_chains_of_prompt_attention_are_cut_only_where_sms_idle(monkeypatch, n_seqs, longest, H, parts):
-    """The parts with which each of these was fastest, or within a tenth."""
-    import torch
-    from vlrf_b200.csrc import ops
-    monkeypatch.setattr(ops, "_SM_COUNT", 148)
-    monkeypatch.setattr(ops, "PREFILL_ATTENTION_PARTS", None)
-    assert ops.attention_prefill_parts(torch.bfloat16, n_seqs, longest, H, 64, 64, 3 * H * 64, 0) == parts
-
-
 @pytest.mark.parametrize("rows,G,N,width", [
     (2000, 16, 1024, 128), (1000, 16, 2048, 128), (4096, 16, 1024, 128), (4096, 16, 2048, 256), (5000, 8, 64, 64), (5000, 8, 128, 128)])
 def test_wide_tiles_of_experts_only_where_full_tiles_gain_too(rows, G, N, width):

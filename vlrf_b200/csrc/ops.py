@@ -543,9 +543,9 @@ def attention_prefill_parts(dtype: torch.dtype, n_seqs: int, max_new: int, n_hea
     more want scratch, see there).  A tile's key blocks are a chain, so a step with few tiles is bound by its
     longest one (`tiles` blocks, for sequences that start at 0), not by the SMs: all blocks together, spread
     over the two CTAs that an SM holds, come to `even` blocks each, and parts pay when the chain is the longer
-    of the two by more than a part's own cost, and sooner where half of the SMs have no tile at all.  Time with one part and with
-    the number chosen (us): 2 heads of 1,024 tokens 13.0, 11.9 (2), of 2,048 22.3, 12.8 (4); 12 heads of 1,024 13.6 (2 parts: 14.9),
-    twice 1,024 16.0 (17.7), 2,048 27.4, 22.8 (2), 8,192 157 (177); 25 heads of 2,048 33.2 (41.2)."""
+    of the two.  (In whole steps: launched again and again alone, a launch begins beside the end of the one ahead, which
+    hides what the longest chain costs: twice 1,024 tokens of 12 heads alone 17.7 us with two parts and 16.0 with one, a step
+    of GPT-2 with them 881 and 900.)"""
     from . import library
     lib = library()
     if not PREFILL_ATTENTION_TCGEN05 or dtype != torch.bfloat16 \
@@ -553,8 +553,7 @@ def attention_prefill_parts(dtype: torch.dtype, n_seqs: int, max_new: int, n_hea
         return 1
     tiles = -(-max_new // lib.vlrf_attn_prefill_tc_tile())
     even = tiles * (tiles + 1) / 2 * n_heads * n_seqs / (2 * sm_count())
-    least = lib.vlrf_attn_prefill_tc_min_part_blocks() * (1 if 2 * tiles * n_heads * n_seqs <= sm_count() else 2)
-    parts = int(tiles / (1.8 * max(even, least)) + 0.5)                                       # 1.8: a part's own cost
+    parts = int(tiles / (1.3 * max(even, lib.vlrf_attn_prefill_tc_min_part_blocks())) + 0.5)   # 1.3: a part's own cost
     if PREFILL_ATTENTION_PARTS is not None:
         parts = PREFILL_ATTENTION_PARTS
     return max(1, min(parts, lib.vlrf_attn_prefill_tc_max_parts()))
