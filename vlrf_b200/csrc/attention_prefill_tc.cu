@@ -17,7 +17,7 @@
 //           written again once P is on its way.  (Scaling only where the maximum has grown by much would save that mostly, but
 //           then the largest P is not 1, which bfloat16 holds exactly, and peaked rows lose: 1.42e-3 -> 1.54e-3 off 64 bits.)
 // A thread a row (its 128 scores read twice, P through shared memory, O added up in registers) took 20.1 us for 2 x 1,024 tokens of 12 heads,
-// 30.6 for 4 x 1,024 of 16; sixteen softmax warps an SM instead of eight keep the exponentials' unit and the issue slots busier.
+// 30.6 for 4 x 1,024 of 16, now 17.7 and 23.1; sixteen softmax warps an SM instead of eight keep the exponentials' unit and the issue slots busier.
 // A CTA's blocks are a chain (scores, softmax, output product, one after the other), so a step with few
 // tiles is bound by its longest tile, not by the SMs' throughput.  The keys of a long tile can therefore be
 // dealt to up to `n_parts` CTAs: each leaves its rows' maximum, sum and outputs in global scratch, and the
