@@ -797,6 +797,39 @@ def test_attention_prefill_reads_no_value_that_it_did_not_load():
         assert rel_err(got, plain_attention(q[:, pos0:].float(), k.float(), v.float(), 0.125)) < 1.5e-2
 
 
+@pytest.mark.parametrize("n_parts", [1, 2])
+def test_attention_prefill_reports_a_block_that_is_not_mapped(n_parts):
+    """The tiles that need the block are called off while their other warps wait; the launch ends, the other sequence's rows are right, and so is
+    all of the next launch."""
+    from vlrf_b200.csrc import ops
+    H, dh, n = 6, 64, 900
+    q, k, v = ([randn(H, n, dh, seed=10 * s + i).to(torch.bfloat16) for i in range(2)] for s in (141, 142, 143))
+    qkv = torch.zeros(2 * n, 3 * H * dh, dtype=torch.bfloat16)
+    qkv[:, :H * dh] = torch.cat(q, dim=1).permute(1, 0, 2).reshape(2 * n, H * dh)
+    caches = [paged(k[i], v[i], 15, 7 + i, torch.bfloat16) for i in range(2)]
+    kp, vp = (torch.cat([c[j] for c in caches]).to(DEV) for j in (0, 1))
+    table = torch.tensor([caches[0][2].tolist(), [15 + b for b in caches[1][2].tolist()]], dtype=torch.int32)
+    lost = table.clone()
+    lost[0, 5] = -1
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    floats, counts = ops.attention_prefill_scratch(2, n, H, n_parts)
+    partials, counters = torch.empty(floats, device=DEV), torch.zeros(counts, dtype=torch.int32, device=DEV)
+    out, e = torch.empty(2 * n, H * dh, dtype=torch.bfloat16, device=DEV), err_word()
+    want = [plain_attention(q[i].float(), k[i].float(), v[i].float(), 0.125) for i in range(2)]
+    for _ in range(5):
+        for t, right in ((lost, [1]), (table, [0, 1])):
+            ops.attention_prefill(qkv.to(DEV), 0, kp, vp, t.to(DEV), i32([0, 1]), i32([0, n, 2 * n]), i32([0, 0]), out, 2 * n, 2, n, H, H, dh, 0.125, 0,
+                                  e, n_parts, partials, counters)
+            word = int(e.item())
+            assert (word & 4 != 0) == (t is lost) and (word == 0) == (t is table)       # VLRF_DEVERR_NO_BLOCK
+            e.zero_()
+            got = out.float().cpu().reshape(2, n, H, dh).permute(0, 2, 1, 3)
+            for i in right:
+                assert rel_err(got[i], want[i]) < 1.5e-2
+            assert rel_err(got[0][:, :256], want[0][:, :256]) < 1.5e-2                   # (tiles ahead of the block)
+            assert int(counters.abs().sum()) == 0
+
+
 def test_kv_append_writes_each_token_where_its_slot_says():
     from vlrf_b200.csrc import ops
     Hkv, dh, T = 3, 16, 70

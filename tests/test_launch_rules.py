@@ -79,3 +79,27 @@ int main() {
     for name in ("gemm_simt.cu", "state_chunks.cu"):
         text = (SRC / name).read_text()
         assert "static bool" not in text and "cudaFuncSetAttribute" not in text and "allow_shared_memory(" in text
+
+
+@pytest.mark.parametrize("name", ["attention_prefill_tc.cu", "gemm_pair.cu", "gemm_splitk.cu", "gemm_tcgen05.cu"])
+def test_warps_that_go_on_together_wait_with_one_answer(name):
+    """`elect.sync`, `tcgen05.ld` and shuffles want all 32 lanes of a warp, so a wait ahead of them gives one answer to all of them; a wait of a lane's
+    own, and a look at the flag that calls a CTA's work off, stand only where one lane acts."""
+    import re
+    text = re.sub(r"//[^\n]*", "", (SRC / name).read_text())
+    scopes, statement = [], ""                       # the text ahead of each open brace; the text since the last brace or semicolon
+    for piece in re.split(r"([{};])", text):
+        if piece == "{":
+            scopes.append(statement)
+            statement = ""
+        elif piece == "}":
+            scopes.pop()
+            statement = ""
+        elif piece == ";":
+            statement = ""
+        else:
+            statement += piece
+            if re.search(r"tbar_wait_or_abort\(|\*\(volatile int\*\)&?s_abort", statement):
+                alone = any(re.search(r"elect_one\(\)|\b(lane|threadIdx\.x) == 0", s) for s in scopes + [statement])
+                assert alone, f"{name}: {' '.join(statement.split())}"
+    assert not scopes and "tbar_wait_warp(" in text

@@ -178,7 +178,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             }
         }
     } else if (warp == 9) {
-        if (rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
             uint32_t s = 0, phase = 0, tc = 0;
             bool ok = true;
@@ -189,25 +189,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 for (int kb = 0; kb < n_kb; ++kb) {
                     if (!tbar_wait_or_abort(&full[s], phase, &s_abort)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    if (elect_one()) {
-                        uint64_t da = da0 + (uint64_t)(s * (a_stage >> 4)), db = db0 + (uint64_t)(s * (b_stage >> 4));
+                    uint64_t da = da0 + (uint64_t)(s * (a_stage >> 4)), db = db0 + (uint64_t)(s * (b_stage >> 4));
 #pragma unroll
-                        for (int k = 0; k < PR_BK / 16; ++k)      // 16 elements = 32 bytes = 2 descriptor units along K
-                            pr_mma(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        if (ka == 2) {
-                            da += PR_A_BYTES >> 4;
-                            db += b_bytes >> 4;
+                    for (int k = 0; k < PR_BK / 16; ++k)          // 16 elements = 32 bytes = 2 descriptor units along K
+                        pr_mma(tmem_d, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    if (ka == 2) {
+                        da += PR_A_BYTES >> 4;
+                        db += b_bytes >> 4;
 #pragma unroll
-                            for (int k = 0; k < PR_BK / 16; ++k) pr_mma(tmem_d, da + 2 * k, db + 2 * k, idesc, 1u);
-                        }
-                        pr_commit(&empty[s]);
-                        if (kb + 1 == n_kb) pr_commit(&acc_full[b]);
+                        for (int k = 0; k < PR_BK / 16; ++k) pr_mma(tmem_d, da + 2 * k, db + 2 * k, idesc, 1u);
                     }
-                    __syncwarp();
+                    pr_commit(&empty[s]);
+                    if (kb + 1 == n_kb) pr_commit(&acc_full[b]);
                     if (++s == (uint32_t)stages) { s = 0; phase ^= 1; }
                 }
             }
-            if (!ok && lane == 0) call_off();
+            if (!ok) call_off();
         }
     } else {
         // epilogue: warps q and q+4 share accumulator lanes 32q … 32q+31, 32 columns of Y, and take half of the rows each
@@ -250,7 +247,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     to = reinterpret_cast<__nv_bfloat16*>(is_v ? kv.Vc : kv.Kc) + (size_t)(col / kv.dh) * kv.BT * kv.dh + col % kv.dh;
             }
             const bool scatters = __any_sync(0xffffffffu, to != nullptr);
-            if (*(volatile int*)&s_abort || !tbar_wait_or_abort(&acc_full[b], (tc >> 1) & 1, &s_abort)) { if (lane == 0) call_off(); break; }
+            if (!tbar_wait_warp(&acc_full[b], (tc >> 1) & 1, &s_abort)) { if (lane == 0) call_off(); break; }
             if (threadIdx.x == 0) { if (tc == 0) VLRF_TRACE(trace, 3, (int)blockIdx.x, 2); VLRF_TRACE(trace, 3, (int)blockIdx.x, 3); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + b * acc_stride + ((uint32_t)(q * 32) << 16);

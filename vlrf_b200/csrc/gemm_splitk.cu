@@ -169,7 +169,7 @@ __device__ __forceinline__ bool sp_sync_product(int row0, int lane, int M, int n
     const int b_row = (lane & 7) + ((lane >> 4) << 3);
     for (int i = 0; i < n_kb; ++i) {
         const int s = i % stages;
-        if (!tbar_wait_or_abort(&full[s], (uint32_t)((i / stages) & 1), s_abort)) return false;
+        if (!tbar_wait_warp(&full[s], (uint32_t)((i / stages) & 1), s_abort)) return false;
         const uint32_t a_base = tsm(a_tiles + (size_t)s * a_bytes), b_base = tsm(b_tiles + (size_t)(LN ? i : s) * b_bytes);
         uint32_t a[SP_BK / 16][MT][4], b[SP_BK / 16][4];
 #pragma unroll
@@ -381,7 +381,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
     } else if (warp == 5) {
-        if (!SYNC) {
+        if (!SYNC && elect_one()) {
             constexpr uint32_t idesc = umma_idesc_bf16(128, BN);
             const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
             bool ok = true;
@@ -390,15 +390,12 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 const int s = i % stages;
                 if (!tbar_wait_or_abort(&full[s], (uint32_t)((i / stages) & 1), s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (elect_one()) {
-                    const uint64_t da = da0 + (uint64_t)(s * (a_bytes >> 4)), db = db0 + (uint64_t)((LN ? i : s) * (B_BYTES >> 4));
+                const uint64_t da = da0 + (uint64_t)(s * (a_bytes >> 4)), db = db0 + (uint64_t)((LN ? i : s) * (B_BYTES >> 4));
 #pragma unroll
-                    for (int k = 0; k < SP_BK / 16; ++k)
-                        umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(&empty[s]);
-                    if (i + 1 == n_kb) umma_commit(acc_full);
-                }
-                __syncwarp();
+                for (int k = 0; k < SP_BK / 16; ++k)
+                    umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                umma_commit(&empty[s]);
+                if (i + 1 == n_kb) umma_commit(acc_full);
             }
         }
     } else {
@@ -420,7 +417,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 // of the W tile (an `mma.sync` is slow here, so the more warps share them the better)
                 asm volatile("bar.sync 3, 256;" ::: "memory");
                 if (threadIdx.x == 0) VLRF_TRACE(trace, 1, tcta, 2);
-                if (lw * 16 < bm && !*(volatile int*)s_abort) {
+                if (lw * 16 < bm) {
                     bool ok;
                     if (M > 8) ok = sp_sync_product<2, 1, LN>(lw * 16, lane, M, n_kb, stages, a_tiles, a_bytes, b_tiles, B_BYTES, full, empty,
                                                               s_abort, recv, recv_bar, s_piece, segs, split, n_j);
@@ -454,7 +451,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
         if (SYNC && !LN && warp < 4) {
-            if (warp * 32 < bm && !*(volatile int*)s_abort) {
+            if (warp * 32 < bm) {
                 bool ok;
                 if (M > 8) ok = sp_sync_product<2, 2, LN>(warp * 32, lane, M, n_kb, stages, a_tiles, a_bytes, b_tiles, B_BYTES, full, empty, s_abort,
                                                           recv, recv_bar, s_piece, segs, split, n_j);
@@ -465,7 +462,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
         if (!SYNC && warp < 4) {
-            const bool have = !*(volatile int*)s_abort && tbar_wait_or_abort(acc_full, 0, s_abort);
+            const bool have = tbar_wait_warp(acc_full, 0, s_abort);
             if (threadIdx.x == 0) VLRF_TRACE(trace, 1, tcta, 3);
             if (!have) atomicExch(s_abort, 1);
             float r[BN];
@@ -508,9 +505,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
     __syncwarp();
     if (!SYNC && threadIdx.x == 0) VLRF_TRACE(trace, 1, tcta, 4);
-    if (warp < 4 && !*(volatile int*)s_abort && !tbar_wait_or_abort(recv_bar, 0, s_abort)) atomicExch(s_abort, 1);
+    const bool here = warp < 4 && tbar_wait_warp(recv_bar, 0, s_abort);
+    if (warp < 4 && !here) atomicExch(s_abort, 1);
     if (threadIdx.x == 0) VLRF_TRACE(trace, 1, tcta, 5);
-    if (warp < 4 && !*(volatile int*)s_abort) {
+    if (here) {
         int j = 0;
         for (int u = gw; u < units; u += ustride, ++j) {
             const int m0 = (u / segs) * RP, seg0 = n0 + (u % segs) * 32, n = seg0 + lane;

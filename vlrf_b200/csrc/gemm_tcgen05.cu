@@ -6,7 +6,7 @@
 //   warp 8  producer: for every 64-wide k block it waits until the ring stage is free, announces the
 //           bytes on the stage's "full" mbarrier and issues two tiled TMA loads (128 rows of X, BN rows of
 //           W; 128-byte swizzle; rows and columns outside the matrices read as zeros);
-//   warp 9  waits as a whole and issues the MMAs by one elected lane (tcgen05.cuh): four `tcgen05.mma.cta_group::1.kind::f16` of shape
+//   warp 9  one elected lane issues the MMAs (tcgen05.cuh): four `tcgen05.mma.cta_group::1.kind::f16` of shape
 //           128 × BN × 16 per k block, operands straight from shared memory through matrix descriptors,
 //           accumulator in tensor memory (two accumulators alternate, so a tile's epilogue overlaps the
 //           next tile's MMAs); `tcgen05.commit` frees the stage when those MMAs have read it, and after the
@@ -202,20 +202,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
             }
         }
     } else if (warp == 9) {
-        constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
-        const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
-        uint32_t kc = 0, tc = 0;
-        for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x, ++tc) {
-            const uint32_t b = tc & 1, use = tc >> 1;
-            if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t tmem_d = tmem_base + b * ACC_STRIDE;
-            bool ok = true;
-            for (int kb = 0; kb < n_kb; ++kb, ++kc) {
-                const uint32_t s = kc % STAGES;
-                if (!tbar_wait_or_abort(&full[s], (kc / STAGES) & 1, s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
+        if (elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(TC_BM, BN);
+            const uint64_t da0 = umma_desc_k128(a_tiles), db0 = umma_desc_k128(b_tiles);
+            uint32_t kc = 0, tc = 0;
+            for (int tile = blockIdx.x; tile < n_tiles && !*(volatile int*)s_abort; tile += gridDim.x, ++tc) {
+                const uint32_t b = tc & 1, use = tc >> 1;
+                if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (elect_one()) {
+                const uint32_t tmem_d = tmem_base + b * ACC_STRIDE;
+                bool ok = true;
+                for (int kb = 0; kb < n_kb; ++kb, ++kc) {
+                    const uint32_t s = kc % STAGES;
+                    if (!tbar_wait_or_abort(&full[s], (kc / STAGES) & 1, s_abort)) { atomicExch(s_abort, 1); ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t da = da0 + (uint64_t)(s * (A_BYTES >> 4)), db = db0 + (uint64_t)(s * (B_BYTES >> 4));
 #pragma unroll
                     for (int a = 0; a < KA; ++a) {
@@ -227,9 +227,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     umma_commit(&empty[s]);                   // the stage is free once these MMAs have read it
                     if (kb + 1 == n_kb) umma_commit(&acc_full[b]);    // arrives when every MMA issued so far is complete
                 }
-                __syncwarp();
+                if (!ok) break;
             }
-            if (!ok) break;
         }
     } else {
         // epilogue: warps q and q+4 share accumulator lanes 32q … 32q+31 and take half of the columns each
@@ -255,7 +254,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
                     if (kv_blk < 0) atomicOr(dev_err, VLRF_DEVERR_NO_BLOCK);
                 }
             }
-            if (*(volatile int*)s_abort || !tbar_wait_or_abort(&acc_full[b], (tc >> 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
+            if (!tbar_wait_warp(&acc_full[b], (tc >> 1) & 1, s_abort)) { atomicExch(s_abort, 1); break; }
             if (threadIdx.x == 0) { if (tc == 0) VLRF_TRACE(trace, 3, (int)blockIdx.x, 2); VLRF_TRACE(trace, 3, (int)blockIdx.x, 3); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + b * ACC_STRIDE + ((uint32_t)(q * 32) << 16);

@@ -25,9 +25,10 @@ __device__ __forceinline__ bool tbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(ok) : "r"(tsm(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-// True in one lane of a converged warp.  The warps that issue MMAs and tiled loads wait on their barriers as whole warps and
-// elect the lane that issues: descriptors and coordinates then are a warp's, not a lane's, and need not be moved to
-// where these instructions read them for every issue, as they were behind `lane == 0`.  Products of prompt steps (a whole
+// True in one lane of a converged warp.  The lane that issues MMAs or tiled loads is elected: descriptors and coordinates then are a
+// warp's, not a lane's, and need not be moved to where these instructions read them for every issue, as they were behind
+// `lane == 0`.  It is elected once and goes its way alone, its waits included (with a warp that waits as a whole, and elects for every
+// stage, steps of 2,048 prompt tokens of GPT-2 take 880 us instead of 875).  Products of prompt steps (a whole
 // launch, weights from memory, float32 results): 512 x 768 x 768 5.8 -> 5.2 us, 2,048 x 768 x 768 7.0 -> 6.6, 2,048 x 768 x 3,072 14.9 -> 13.4,
 // 2,050 x 1,600 x 6,400 40.1 -> 39.1, 4,096 cubed 113.7 -> 111.8.
 __device__ __forceinline__ bool elect_one() {
@@ -81,6 +82,16 @@ __device__ __forceinline__ bool tbar_wait_or_abort(uint64_t* bar, uint32_t parit
     for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
         if (tbar_try_wait(bar, parity)) return true;
         if ((i & 255u) == 255u && *abort_flag) return false;
+    }
+    return false;
+}
+// The same for a warp that goes on together (to read tensor memory, to shuffle): one answer for all of its lanes.  Lanes that poll each for itself
+// may part where the flag, or the last poll, ends the waits of some when those of the others have just succeeded, and then meet the next
+// instruction of the whole warp alone, which waits for ever.
+__device__ __forceinline__ bool tbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
+        if (__all_sync(0xffffffffu, tbar_try_wait(bar, parity))) return true;
+        if ((i & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
     }
     return false;
 }
