@@ -401,6 +401,35 @@ def test_products_by_pairs_of_sms(rows):
     assert ops.device_errors() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 1000, 200), (1200, 6000, 136), (512, 768, 3072), (100, 130, 5000)])
+def test_a_pair_of_sms_that_gives_up_leaves_nothing_behind(M, N, K):
+    """Waits that give up after so many polls, whichever role's they are: the launch ends, says so, and has written nothing beside its result;
+    the next product is right.  (With no polls at all the MMAs are given up while every load of the ring is under way.)"""
+    from vlrf_b200.csrc import call, library, ops
+    lib = library()
+    x, w, bias = randn(M, K, seed=130, dtype=torch.bfloat16).to(DEV), randn(N, K, seed=131, dtype=torch.bfloat16, scale=0.3).to(DEV), randn(N, seed=132).to(DEV)
+    want = (x.double() @ w.double().T + bias.double()).cpu()
+    for dtype, rows in ((torch.float32, 256), (torch.float32, 96), (torch.bfloat16, 192), (torch.bfloat16, 64)):
+        def product(out):
+            call("vlrf_gemm_pair", x.data_ptr(), w.data_ptr(), bias.data_ptr(), 0, out.data_ptr(), M, N, K, K, N, ops.dtype_code(dtype), 0, rows,
+                 *ops._kv_args(None, N), ops._dev_err().data_ptr(), torch.cuda.current_stream().cuda_stream)
+        for polls in (0, 1, 3, 20, 300, 3000):
+            room = torch.full((M + 1, N), float("nan"), dtype=dtype, device=DEV)
+            try:
+                lib.vlrf_gemm_pair_wait_polls(polls)
+                for _ in range(3):
+                    product(room)
+            finally:
+                lib.vlrf_gemm_pair_wait_polls(-1)
+            word = ops.device_errors()
+            assert word == 8 or (word == 0 and polls > 0)       # VLRF_DEVERR_WAIT_TIMEOUT
+            assert torch.isnan(room[M]).all()
+            out = torch.empty(M, N, dtype=dtype, device=DEV)
+            product(out)
+            assert rel_err(out.float().cpu(), want) < (f32_sum_tol(K) if dtype == torch.float32 else 5e-3)
+            assert ops.device_errors() == 0
+
+
 def test_split_k_rows_do_not_depend_on_the_batch(split_k_always):
     import os
     if os.environ.get("VLRF_B200_SPLITK_MMA"):

@@ -17,9 +17,10 @@
 //   acc_empty[b]  in CTA 0: the 16 epilogue warps of both have read it
 // CTAs are persistent: a pair takes the tiles (pair number), + number of pairs, …; the rows that are left behind whole tiles
 // make tiles of their own, as wide as they need, which come last.  Two accumulators alternate, so a tile's
-// epilogue overlaps the next tile's MMAs.  Every wait is bounded; a wait that gives up calls off the work of both CTAs and sets
-// a bit of the device error word; the loads in flight are waited for, both CTAs meet at the end on every path, and only
-// then is tensor memory given back.
+// epilogue overlaps the next tile's MMAs.  Every wait is bounded; a wait that gives up, whichever role's, calls off the work of both CTAs and
+// sets a bit of the device error word.  Both CTAs meet at the end on every path; where the work was called off, what either has
+// requested and the MMAs issued are waited for then (bounded too), since they write, read and signal the shared memory of
+// both, and both meet once more.  Only then is tensor memory given back.
 //
 // The product is the reference's linear(x, W) = x · Wᵀ (include/model/compute.hpp:64-68), its epilogues those of
 // include/model/feedforward.hpp:54-76 and include/model/transformer_block.hpp:153,158, its scatter include/model/kv_cache.hpp:215-251.
@@ -67,6 +68,10 @@ __device__ __forceinline__ void pr_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(tsm(bar)), "h"((uint16_t)3) : "memory");
 }
+// takes bytes off what a barrier of this CTA still expects
+__device__ __forceinline__ void pr_take_off(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(tsm(bar)), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void pr_arrive_at(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
@@ -75,11 +80,11 @@ template <typename OT>
 __global__ void __launch_bounds__(PR_THREADS)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ CUtensorMap tmap_rest, const float* __restrict__ bias, const float* residual, OT* Y, int M,
-                 int N, int K, int ldy, int act, int bn, int stages, int ka, PrKvScatter kv, int* __restrict__ dev_err, long long* trace) {
+                 int N, int K, int ldy, int act, int bn, int stages, int ka, uint32_t polls, PrKvScatter kv, int* __restrict__ dev_err, long long* trace) {
     extern __shared__ unsigned char pr_raw[];
-    __shared__ uint64_t bars[2 * PR_MAX_STAGES + 4];
+    __shared__ uint64_t bars[2 * PR_MAX_STAGES + 5];
     __shared__ uint32_t tmem_slot;
-    __shared__ int s_abort, s_never;
+    __shared__ int s_abort, s_never, s_issued;                       // s_issued: stages that this CTA has requested, over all tiles
     if (threadIdx.x == 0) VLRF_TRACE(trace, 3, (int)blockIdx.x, 0);
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(pr_raw) + 1023) & ~(uintptr_t)1023);
     const uint32_t b_bytes = (uint32_t)bn * PR_BK;                   // half of a whole tile's rows, 128 bytes each
@@ -90,6 +95,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     uint64_t* empty = bars + PR_MAX_STAGES;
     uint64_t* acc_full = bars + 2 * PR_MAX_STAGES;
     uint64_t* acc_empty = acc_full + 2;
+    uint64_t* drained = acc_empty + 2;                               // in both: no MMA is under way (only where the work was called off)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -107,8 +113,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) { tbar_init(&full[s], 1); tbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) { tbar_init(&acc_full[b], 1); tbar_init(&acc_empty[b], 16); }
+        tbar_init(drained, 1);
         s_abort = 0;
         s_never = 0;
+        s_issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -158,7 +166,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 const CUtensorMap* map_x = tile < whole ? &tmap_x : &tmap_rest;
                 for (int kb = 0; kb < n_kb; ++kb) {
                     if (n_issued >= early) {
-                        if (use >= 1 && !tbar_wait_or_abort(&empty[s], (use - 1) & 1, &s_abort)) { ok = false; break; }
+                        if (use >= 1 && !tbar_wait_or_abort(&empty[s], (use - 1) & 1, &s_abort, polls)) { ok = false; break; }
                         if (rank == 0) tbar_expect_tx(&full[s], 2u * ka * (PR_A_BYTES + rows * PR_BK));
                         for (int a = 0; a < ka; ++a)
                             pr_load(tsm(a_tiles + (size_t)s * a_stage + a * PR_A_BYTES), &tmap_w, (kb * ka + a) * PR_BK, w_row, full0 + 8u * s);
@@ -169,13 +177,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     if (++s == stages) { s = 0; ++use; }
                 }
             }
-            if (!ok) {
-                call_off();
-                // the copies already requested land in this pair's shared memory: wait for them before leaving
-                if (rank == 0)
-                    for (int t = max(0, n_issued - stages); t < n_issued; ++t)
-                        tbar_wait_or_abort(&full[t % stages], (uint32_t)((t / stages) & 1), &s_never);
-            }
+            s_issued = n_issued;
+            if (!ok) call_off();
         }
     } else if (warp == 9) {
         if (rank == 0 && elect_one()) {
@@ -184,10 +187,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             bool ok = true;
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
                 const uint32_t b = tc & 1, use = tc >> 1;
-                if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, &s_abort)) { ok = false; break; }
+                if (use >= 1 && !tbar_wait_or_abort(&acc_empty[b], (use - 1) & 1, &s_abort, polls)) { ok = false; break; }
                 const uint32_t tmem_d = tmem_base + b * acc_stride, idesc = umma_idesc_bf16(2 * PR_BM, tile < whole ? bn : rest);
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!tbar_wait_or_abort(&full[s], phase, &s_abort)) { ok = false; break; }
+                    if (!tbar_wait_or_abort(&full[s], phase, &s_abort, polls)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     uint64_t da = da0 + (uint64_t)(s * (a_stage >> 4)), db = db0 + (uint64_t)(s * (b_stage >> 4));
 #pragma unroll
@@ -247,7 +250,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     to = reinterpret_cast<__nv_bfloat16*>(is_v ? kv.Vc : kv.Kc) + (size_t)(col / kv.dh) * kv.BT * kv.dh + col % kv.dh;
             }
             const bool scatters = __any_sync(0xffffffffu, to != nullptr);
-            if (!tbar_wait_warp(&acc_full[b], (tc >> 1) & 1, &s_abort)) { if (lane == 0) call_off(); break; }
+            if (!tbar_wait_warp(&acc_full[b], (tc >> 1) & 1, &s_abort, polls)) { if (lane == 0) call_off(); break; }
             if (threadIdx.x == 0) { if (tc == 0) VLRF_TRACE(trace, 3, (int)blockIdx.x, 2); VLRF_TRACE(trace, 3, (int)blockIdx.x, 3); }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t tmem_d = tmem_base + b * acc_stride + ((uint32_t)(q * 32) << 16);
@@ -326,10 +329,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync_all();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (s_abort) {                                 // (the same in both CTAs: who calls off tells the other before they meet)
+        if (warp == 9) {
+            if (rank == 0 && elect_one()) pr_commit(drained);        // arrives in both CTAs behind the MMAs issued so far
+            __syncwarp();
+            tbar_wait_warp(drained, 0, &s_never);
+        } else if (warp == 8 && rank == 0 && elect_one()) {
+            // The last use of each stage by either CTA.  CTA 0 announces the bytes of both, so a use that only it has requested lacks
+            // the other's half, and one that only CTA 1 has requested is not announced yet.
+            int theirs;
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(theirs) : "r"(pr_map(tsm(&s_issued), 1)) : "memory");
+            const int mine = s_issued, most = max(mine, theirs);
+            for (int t = max(0, most - stages); t < most; ++t) {
+                int w_tile, row, rows;
+                place(pair + t / n_kb * n_pairs, w_tile, row, rows);
+                const uint32_t half = ka * (PR_A_BYTES + rows * PR_BK);
+                if (t >= mine) tbar_expect_tx(&full[t % stages], half);
+                else if (t >= theirs) pr_take_off(&full[t % stages], half);
+                tbar_wait_or_abort(&full[t % stages], (uint32_t)((t / stages) & 1), &s_never);
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();
+    }
     if (warp == 9)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     if (threadIdx.x == 0 && s_abort) atomicOr(dev_err, VLRF_DEVERR_WAIT_TIMEOUT);
 }
+
+thread_local int g_polls = -1;
 
 template <typename OT>
 int launch_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
@@ -354,7 +382,7 @@ int launch_pair(const void* X, const void* W, const float* bias, const float* re
     const int pairs = vlrf_sm_count() / 2;
     dim3 grid(2u * (unsigned)(tiles < pairs ? tiles : pairs));
     e = launch_chained_cluster(kern, grid, dim3(PR_THREADS), smem, dim3(2), stream, tw, tx, tr, bias, residual, (OT*)Y, M, N, K, ldy,
-                               act, bn, stages, ka, kv, dev_err, vlrf_trace_buffer());
+                               act, bn, stages, ka, g_polls < 0 ? TC_WAIT_LIMIT : (uint32_t)g_polls, kv, dev_err, vlrf_trace_buffer());
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm_pair: %s", cudaGetErrorString(e));
     return vlrf_check_launch("gemm_pair");
 }
@@ -382,6 +410,10 @@ extern "C" int vlrf_gemm_pair_rows(int M, int N, int sms) {
     }
     return rows;
 }
+
+// How often a wait of the calling thread's next launches polls its barrier before it gives up (negative: as ever), but for those that follow on
+// giving up.  For tests of a pair whose work is called off.
+extern "C" int vlrf_gemm_pair_wait_polls(int polls) { g_polls = polls; return VLRF_OK; }
 
 // bn: rows of a tile (a multiple of 32 up to 256)
 extern "C" int vlrf_gemm_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K,

@@ -78,8 +78,8 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 }
 
 // a wait that also gives up when another role of the CTA has already given up
-__device__ __forceinline__ bool tbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool tbar_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t polls = TC_WAIT_LIMIT) {
+    for (uint32_t i = 0; i < polls; ++i) {
         if (tbar_try_wait(bar, parity)) return true;
         if ((i & 255u) == 255u && *abort_flag) return false;
     }
@@ -88,8 +88,8 @@ __device__ __forceinline__ bool tbar_wait_or_abort(uint64_t* bar, uint32_t parit
 // The same for a warp that goes on together (to read tensor memory, to shuffle): one answer for all of its lanes.  Lanes that poll each for itself
 // may part where the flag, or the last poll, ends the waits of some when those of the others have just succeeded, and then meet the next
 // instruction of the whole warp alone, which waits for ever.
-__device__ __forceinline__ bool tbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
+__device__ __forceinline__ bool tbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint32_t polls = TC_WAIT_LIMIT) {
+    for (uint32_t i = 0; i < polls; ++i) {
         if (__all_sync(0xffffffffu, tbar_try_wait(bar, parity))) return true;
         if ((i & 255u) == 255u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
     }
