@@ -76,12 +76,39 @@ __device__ __forceinline__ void pr_arrive_at(uint32_t cluster_bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 
-template <typename OT>
+// What a pair whose work was called off waits for (bounded): the MMAs issued, and the last use of each stage by either CTA.  A function of its own, which
+// keeps the kernel's registers as they are without it (inlined, steps of 2,048 prompt tokens of GPT-2 took 885 us instead of 881).
+__device__ __noinline__ void pr_drain(int warp, uint32_t rank, int pair, int n_pairs, int n_kb, int whole, int bn, int rest, int ka, int stages,
+                                      uint64_t* full, uint64_t* drained, int* s_issued, int* s_never) {
+    if (warp == 9) {
+        if (rank == 0 && elect_one()) pr_commit(drained);           // arrives in both CTAs behind the MMAs issued so far
+        __syncwarp();
+        tbar_wait_warp(drained, 0, s_never);
+    } else if (warp == 8 && rank == 0 && elect_one()) {
+        // CTA 0 announces the bytes of both, so a use that only it has requested lacks the other's half, and one that only CTA 1 has
+        // requested is not announced yet
+        int theirs;
+        asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(theirs) : "r"(pr_map(tsm(s_issued), 1)) : "memory");
+        const int mine = *s_issued, most = max(mine, theirs);
+        for (int t = max(0, most - stages); t < most; ++t) {
+            const uint32_t half = ka * (PR_A_BYTES + (pair + t / n_kb * n_pairs < whole ? bn : rest) * PR_BK);
+            if (t >= mine) tbar_expect_tx(&full[t % stages], half);
+            else if (t >= theirs) pr_take_off(&full[t % stages], half);
+            tbar_wait_or_abort(&full[t % stages], (uint32_t)((t / stages) & 1), s_never);
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();
+}
+
+// LIMITED: waits give up after `limit` polls (tests of a pair whose work is called off; the limit as an argument costs the MMAs' lane a per cent)
+template <typename OT, bool LIMITED>
 __global__ void __launch_bounds__(PR_THREADS)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ CUtensorMap tmap_rest, const float* __restrict__ bias, const float* residual, OT* Y, int M,
-                 int N, int K, int ldy, int act, int bn, int stages, int ka, uint32_t polls, PrKvScatter kv, int* __restrict__ dev_err, long long* trace) {
+                 int N, int K, int ldy, int act, int bn, int stages, int ka, uint32_t limit, PrKvScatter kv, int* __restrict__ dev_err, long long* trace) {
     extern __shared__ unsigned char pr_raw[];
+    const uint32_t polls = LIMITED ? limit : TC_WAIT_LIMIT;
     __shared__ uint64_t bars[2 * PR_MAX_STAGES + 5];
     __shared__ uint32_t tmem_slot;
     __shared__ int s_abort, s_never, s_issued;                       // s_issued: stages that this CTA has requested, over all tiles
@@ -329,29 +356,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     cluster_sync_all();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (s_abort) {                                 // (the same in both CTAs: who calls off tells the other before they meet)
-        if (warp == 9) {
-            if (rank == 0 && elect_one()) pr_commit(drained);        // arrives in both CTAs behind the MMAs issued so far
-            __syncwarp();
-            tbar_wait_warp(drained, 0, &s_never);
-        } else if (warp == 8 && rank == 0 && elect_one()) {
-            // The last use of each stage by either CTA.  CTA 0 announces the bytes of both, so a use that only it has requested lacks
-            // the other's half, and one that only CTA 1 has requested is not announced yet.
-            int theirs;
-            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(theirs) : "r"(pr_map(tsm(&s_issued), 1)) : "memory");
-            const int mine = s_issued, most = max(mine, theirs);
-            for (int t = max(0, most - stages); t < most; ++t) {
-                int w_tile, row, rows;
-                place(pair + t / n_kb * n_pairs, w_tile, row, rows);
-                const uint32_t half = ka * (PR_A_BYTES + rows * PR_BK);
-                if (t >= mine) tbar_expect_tx(&full[t % stages], half);
-                else if (t >= theirs) pr_take_off(&full[t % stages], half);
-                tbar_wait_or_abort(&full[t % stages], (uint32_t)((t / stages) & 1), &s_never);
-            }
-        }
-        __syncwarp();
-        cluster_sync_all();
-    }
+    if (s_abort)                                   // (the same in both CTAs: who calls off tells the other before they meet)
+        pr_drain(warp, rank, pair, n_pairs, n_kb, whole, bn, rest, ka, stages, full, drained, &s_issued, &s_never);
     if (warp == 9)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     if (threadIdx.x == 0 && s_abort) atomicOr(dev_err, VLRF_DEVERR_WAIT_TIMEOUT);
@@ -359,8 +365,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
 thread_local int g_polls = -1;
 
-template <typename OT>
-int launch_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
+template <typename OT, bool LIMITED>
+int launch_pair_as(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
                 int ldy, int act, int bn, const PrKvScatter& kv, int* dev_err, cudaStream_t stream) {
     CUtensorMap tw, tx, tr;
     int st = vlrf_make_tmap_bf16(W, N, K, K, PR_BM, PR_BK, &tw);
@@ -375,16 +381,22 @@ int launch_pair(const void* X, const void* W, const float* bias, const float* re
     const int stages = PR_SMEM / stage < PR_MAX_STAGES ? PR_SMEM / stage : PR_MAX_STAGES;
     const size_t smem = 1024 + (size_t)stages * stage;
     static DeviceMarks marks;
-    auto kern = gemm_pair_kernel<OT>;
+    auto kern = gemm_pair_kernel<OT, LIMITED>;
     cudaError_t e = allow_shared_memory(marks, kern, 1024 + PR_SMEM);
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm_pair: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const long long tiles = (long long)((M + bn - 1) / bn) * ((N + 2 * PR_BM - 1) / (2 * PR_BM));
     const int pairs = vlrf_sm_count() / 2;
     dim3 grid(2u * (unsigned)(tiles < pairs ? tiles : pairs));
     e = launch_chained_cluster(kern, grid, dim3(PR_THREADS), smem, dim3(2), stream, tw, tx, tr, bias, residual, (OT*)Y, M, N, K, ldy,
-                               act, bn, stages, ka, g_polls < 0 ? TC_WAIT_LIMIT : (uint32_t)g_polls, kv, dev_err, vlrf_trace_buffer());
+                               act, bn, stages, ka, (uint32_t)g_polls, kv, dev_err, vlrf_trace_buffer());
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "gemm_pair: %s", cudaGetErrorString(e));
     return vlrf_check_launch("gemm_pair");
+}
+template <typename OT>
+int launch_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
+                int ldy, int act, int bn, const PrKvScatter& kv, int* dev_err, cudaStream_t stream) {
+    return g_polls < 0 ? launch_pair_as<OT, false>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, bn, kv, dev_err, stream)
+                       : launch_pair_as<OT, true>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, bn, kv, dev_err, stream);
 }
 }  // namespace
 
