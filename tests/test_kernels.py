@@ -859,6 +859,46 @@ def test_attention_prefill_reports_a_block_that_is_not_mapped(n_parts):
             assert int(counters.abs().sum()) == 0
 
 
+@pytest.mark.parametrize("n_parts", [1, 3])
+@pytest.mark.parametrize("window", [0, 200])
+def test_attention_prefill_that_gives_up_leaves_nothing_behind(n_parts, window):
+    """Waits that give up after so many polls, whichever role's they are: the launch ends, says so, leaves its counters at zero, and the next is right.
+    (With no polls at all a CTA leaves while its queries, and all keys and values that its ring holds, are under way.)"""
+    from vlrf_b200.csrc import library, ops
+    H, dh, n = 7, 64, 1100
+    q, k, v = (randn(H, n, dh, seed=s).to(torch.bfloat16) for s in (151, 152, 153))
+    qkv = torch.zeros(n, 3 * H * dh, dtype=torch.bfloat16)
+    qkv[:, :H * dh] = q.permute(1, 0, 2).reshape(n, H * dh)
+    qkv = qkv.to(DEV)
+    kp, vp, perm = paged(k, v, 20, 9, torch.bfloat16)
+    kp, vp = kp.to(DEV), vp.to(DEV)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    floats, counts = ops.attention_prefill_scratch(1, n, H, n_parts)
+    partials, counters = torch.empty(floats, device=DEV), torch.zeros(counts, dtype=torch.int32, device=DEV)
+    e, args = err_word(), (i32([perm.tolist()]), i32([0]), i32([0, n]), i32([0]))
+    want = plain_attention(q.float(), k.float(), v.float(), 0.125, window)
+
+    def attend(out):
+        ops.attention_prefill(qkv, 0, kp, vp, *args, out, n, 1, n, H, H, dh, 0.125, window, e, n_parts, partials, counters)
+
+    for polls in (0, 1, 3, 20, 300, 3000):
+        room = torch.full((n, H * dh), float("nan"), dtype=torch.bfloat16, device=DEV)
+        try:
+            library().vlrf_attn_prefill_tc_wait_polls(polls)
+            for _ in range(3):
+                attend(room)
+        finally:
+            library().vlrf_attn_prefill_tc_wait_polls(-1)
+        word = int(e.item())
+        assert word == 8 or (word == 0 and polls > 0)             # VLRF_DEVERR_WAIT_TIMEOUT
+        assert int(counters.abs().sum()) == 0
+        e.zero_()
+        out = torch.empty(n, H * dh, dtype=torch.bfloat16, device=DEV)
+        attend(out)
+        assert rel_err(out.float().cpu().reshape(n, H, dh).permute(1, 0, 2), want) < 1.5e-2
+        assert int(e.item()) == 0
+
+
 def test_kv_append_writes_each_token_where_its_slot_says():
     from vlrf_b200.csrc import ops
     Hkv, dh, T = 3, 16, 70

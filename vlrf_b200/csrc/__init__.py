@@ -78,6 +78,7 @@ _SIGNATURES = {
     "vlrf_attn_prefill_tc_min_part_blocks": [],
     "vlrf_attn_prefill_tc_lists": [_c_int] * 6,
     "vlrf_attn_prefill_tc_tile": [],
+    "vlrf_attn_prefill_tc_wait_polls": [_c_int],
     "vlrf_attn_prefill_tc": [_c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_int, _c_void_p, _c_void_p,
                              _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float,
                              _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p],

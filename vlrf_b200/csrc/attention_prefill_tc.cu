@@ -95,13 +95,31 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
 }
 
+// What a CTA whose work was called off, whichever role gave up, waits for (bounded): the copies requested, which land in its shared memory, and the
+// MMAs issued, which read it.
+__device__ __noinline__ void ft_drain(int warp, uint64_t* q_full, uint64_t* full, uint64_t* drained, int n_issued, int* s_never) {
+    if (warp == 9) {
+        if (elect_one()) umma_commit(drained);
+        __syncwarp();
+        tbar_wait_warp(drained, 0, s_never);
+    } else if (warp == 8 && elect_one()) {
+        tbar_wait_or_abort(q_full, 0, s_never);
+        for (int t = max(0, n_issued - FT_SLOTS); t < n_issued; ++t)
+            tbar_wait_or_abort(&full[t % FT_SLOTS], (uint32_t)((t / FT_SLOTS) & 1), s_never);
+    }
+    __syncthreads();
+}
+
+// LIMITED: waits give up after `limit` polls (tests of a CTA whose work is called off)
+template <bool LIMITED>
 __global__ void __launch_bounds__(FT_THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, int q_off, const int* __restrict__ block_table,
                        int max_blocks, const int* __restrict__ seq_slot, const int* __restrict__ seq_start,
                        const int* __restrict__ seq_pos0, __nv_bfloat16* __restrict__ out, int ld_out, int H, int Hkv,
                        float scale, int window, int n_parts, float* __restrict__ partials, int* __restrict__ counters,
-                       int n_tiles, int listed, int* __restrict__ dev_err, long long* trace) {
+                       int n_tiles, int listed, uint32_t limit, int* __restrict__ dev_err, long long* trace) {
+    const uint32_t polls = LIMITED ? limit : TC_WAIT_LIMIT;
     extern __shared__ unsigned char ft_raw[];
     // (stations of the time stamps, kind 4: 0 the CTA begins, 1 the kernel ahead has finished, 6 the CTA is done)
     const int tcta = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
@@ -117,10 +135,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     uint64_t* s_read = s_full + 1;                                   // the scores are in registers: S may be written again
     uint64_t* p_full = s_read + 1;
     uint64_t* o_full = p_full + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 1);
+    uint64_t* drained = o_full + 1;                                  // no MMA is under way (only where the work was called off)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
     int* s_abort = reinterpret_cast<int*>(tmem_slot + 1);
     int* s_never = s_abort + 1;                                      // stays 0: for waits that nothing calls off
     int* s_last = s_never + 1;                                       // whether this CTA merges its tile's parts
+    int* s_issued = s_last + 1;                                      // tiles requested: 2j is K of block j, 2j+1 its V
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // z is the slowest index of the order in which CTAs are started: first parts before second parts, so that the
@@ -138,6 +158,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         tbar_init(s_read, 8);
         tbar_init(p_full, 8);
         tbar_init(o_full, 1);
+        tbar_init(drained, 1);
         *s_abort = 0;
         *s_never = 0;
         *s_last = 1;
@@ -211,11 +232,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         if (my_n > 0 && elect_one()) {
             tbar_expect_tx(q_full, FT_TILE);
             tma_load_2d(q_tile, &tmap_q, q_off + h * FT_DH, row0 + qt * FT_BQ, q_full);
-            int n_issued = 0;                         // tiles requested: 2j is K of block j, 2j+1 its V
+            int n_issued = 0;
             bool ok = true;
             for (int t = 0; t < 2 * my_n && ok; ++t) {
                 const int sl = t % FT_SLOTS, use = t / FT_SLOTS;
-                if (use >= 1 && !tbar_wait_or_abort(&empty[sl], (uint32_t)((use - 1) & 1), s_abort)) { ok = false; break; }
+                if (use >= 1 && !tbar_wait_or_abort(&empty[sl], (uint32_t)((use - 1) & 1), s_abort, polls)) { ok = false; break; }
                 const int cb0 = (my_first + (t >> 1)) * 2;            // the block's two cache blocks
                 const int n_cb = (cb0 + 1 <= cb_last) ? 2 : 1;
                 int blk[2];
@@ -230,24 +251,19 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                                 (blk[i] * Hkv + hk) * FT_CB, &full[sl]);
                 ++n_issued;
             }
-            if (!ok) {
-                atomicExch(s_abort, 1);
-                // the copies already requested land in this CTA's shared memory: wait for them before leaving
-                tbar_wait_or_abort(q_full, 0, s_never);
-                for (int t = max(0, n_issued - FT_SLOTS); t < n_issued; ++t)
-                    tbar_wait_or_abort(&full[t % FT_SLOTS], (uint32_t)((t / FT_SLOTS) & 1), s_never);
-            }
+            *s_issued = n_issued;
+            if (!ok) atomicExch(s_abort, 1);
         }
     } else if (warp == 9) {
         if (my_n > 0) {                              // (the whole warp waits, with one answer, and elects a lane for every issue: 1 % less time here than a lane alone)
             constexpr uint32_t idesc_s = umma_idesc_bf16(FT_BQ, FT_BK);
             constexpr uint32_t idesc_o = umma_idesc_bf16_bmn(FT_BQ, FT_DH);
-            bool ok = tbar_wait_warp(q_full, 0, s_abort);
+            bool ok = tbar_wait_warp(q_full, 0, s_abort, polls);
             const uint64_t dq = umma_desc_k128(q_tile), dk0 = umma_desc_k128(kv_tiles), dv0 = umma_desc_mn128(kv_tiles);
             // S_j = Q · K_jᵀ into tensor memory, four k steps
             auto issue_s = [&](int j) -> bool {
                 const uint32_t tk = 2u * j, sl = tk % FT_SLOTS;
-                if (!tbar_wait_warp(&full[sl], (tk / FT_SLOTS) & 1u, s_abort)) return false;
+                if (!tbar_wait_warp(&full[sl], (tk / FT_SLOTS) & 1u, s_abort, polls)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
                     const uint64_t dk = dk0 + (uint64_t)(sl * (FT_TILE >> 4));
@@ -262,10 +278,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             ok = ok && issue_s(0);
             for (int j = 0; j < my_n && ok; ++j) {
                 // S_{j+1} as soon as the softmax warps hold S_j in registers, O += P_j · V_j once they have written P_j
-                if (j + 1 < my_n && !(tbar_wait_warp(s_read, (uint32_t)(j & 1), s_abort) && issue_s(j + 1))) { ok = false; break; }
+                if (j + 1 < my_n && !(tbar_wait_warp(s_read, (uint32_t)(j & 1), s_abort, polls) && issue_s(j + 1))) { ok = false; break; }
                 const uint32_t tv = 2u * j + 1, sl = tv % FT_SLOTS;
-                if (!tbar_wait_warp(&full[sl], (tv / FT_SLOTS) & 1u, s_abort)) { ok = false; break; }
-                if (!tbar_wait_warp(p_full, (uint32_t)(j & 1), s_abort)) { ok = false; break; }
+                if (!tbar_wait_warp(&full[sl], (tv / FT_SLOTS) & 1u, s_abort, polls)) { ok = false; break; }
+                if (!tbar_wait_warp(p_full, (uint32_t)(j & 1), s_abort, polls)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
                     const uint64_t dv = dv0 + (uint64_t)(sl * (FT_TILE >> 4));
@@ -296,7 +312,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             const int q_top = q_first + q * 32 + 31;
             const int n_live = MASKED ? (q_top < k0 ? 0 : min(2, ((q_top - k0) >> 5) + 1)) : 2;
             // (a warp that has given up goes on meeting its neighbour, who may not have)
-            if (!ok || !tbar_wait_warp(s_full, (uint32_t)(j & 1), s_abort)) {
+            if (!ok || !tbar_wait_warp(s_full, (uint32_t)(j & 1), s_abort, polls)) {
                 ok = false;
                 asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
                 return;
@@ -337,7 +353,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             m_run = m_new;
             const float m_use = (m_run == -INFINITY) ? 0.f : m_run;   // a row that sees nothing yet: every p is 0
             if (j > 0) {                                              // O holds the blocks before, and P may be written again
-                if (!tbar_wait_warp(o_full, (uint32_t)((j - 1) & 1), s_abort)) { ok = false; return; }
+                if (!tbar_wait_warp(o_full, (uint32_t)((j - 1) & 1), s_abort, polls)) { ok = false; return; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             // exponentials, their sum, P as bfloat16 into tensor memory
@@ -392,7 +408,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             const int there = min(pos0 + n_new - (my_first + j) * FT_BK, ((my_first + j) * 2 + 1 <= cb_last ? 2 : 1) * FT_CB);
             if (there < FT_BK) {
                 const int tv = 2 * j + 1;
-                if (!tbar_wait_warp(&full[tv % FT_SLOTS], (uint32_t)((tv / FT_SLOTS) & 1), s_abort)) { ok = false; return; }
+                if (!tbar_wait_warp(&full[tv % FT_SLOTS], (uint32_t)((tv / FT_SLOTS) & 1), s_abort, polls)) { ok = false; return; }
                 unsigned char* vt = kv_tiles + (size_t)(tv % FT_SLOTS) * FT_TILE;
                 const int first_row = max(there, 0);
                 for (int idx = warp * 32 + lane; idx < (FT_BK - first_row) * 8; idx += 256)
@@ -414,7 +430,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 #pragma unroll
         for (int d = 0; d < HD; ++d) o_acc[d] = 0.f;
         if (my_n > 0) {
-            if (ok && tbar_wait_warp(o_full, (uint32_t)((my_n - 1) & 1), s_abort)) {
+            if (ok && tbar_wait_warp(o_full, (uint32_t)((my_n - 1) & 1), s_abort, polls)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t ov[HD];
                 tmem_ld32(tmem_o + lane_addr + (uint32_t)(half * HD), ov);
@@ -507,12 +523,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (*s_abort) ft_drain(warp, q_full, full, drained, *s_issued, s_never);
     if (warp == 8) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"((uint32_t)FT_TMEM_COLS) : "memory");
     }
     if (threadIdx.x == 0) VLRF_TRACE(trace, 4, tcta, 6);
     if (threadIdx.x == 0 && *s_abort) atomicOr(dev_err, VLRF_DEVERR_WAIT_TIMEOUT);
 }
+thread_local int g_polls = -1;
 }  // namespace
 
 // Whether the tcgen05 prompt attention takes these sizes (bfloat16 only): head size 64, cache blocks of 64
@@ -540,6 +558,10 @@ extern "C" int vlrf_attn_prefill_tc_lists(int n_tokens, int n_seqs, int max_new,
     return exist * each >= full && (all - exist) * each >= full ? 1 : 0;
 }
 
+// How often a wait of the calling thread's next launches polls its barrier before it gives up (negative: as ever), but for those that follow on
+// giving up.  For tests of a CTA whose work is called off.
+extern "C" int vlrf_attn_prefill_tc_wait_polls(int polls) { g_polls = polls; return VLRF_OK; }
+
 // n_parts > 1 wants `partials` ([sequences × heads × tiles × n_parts] × part_floats) and `counters`
 // ([sequences × heads × tiles], zero; left zero).
 extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const void* Kc, const void* Vc, int n_blocks,
@@ -562,20 +584,18 @@ extern "C" int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const vo
     st = vlrf_make_tmap_bf16(Vc, kv_rows, dh, dh, FT_CB, 64, &tv);
     if (st != VLRF_OK) return st;
     const size_t smem = 1024 + (size_t)(1 + FT_SLOTS) * FT_TILE + 4 * FT_BQ * 4 + 24 * 8;
-    static bool raised = false;
-    if (!raised) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "attn_prefill_tc: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
-        raised = true;
-    }
+    static DeviceMarks marks[2];
+    auto kern = g_polls < 0 ? attn_prefill_tc_kernel<false> : attn_prefill_tc_kernel<true>;
+    cudaError_t e = allow_shared_memory(marks[g_polls < 0 ? 0 : 1], kern, smem);
+    if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "attn_prefill_tc: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
     const long long tiles = (max_new + FT_BQ - 1) / FT_BQ;
     VLRF_REQUIRE(tiles * n_parts <= 65535, "attn_prefill_tc: %lld tiles of %d parts are too many for one launch", tiles, n_parts);
     const long long places = (long long)n_tokens / FT_BQ + n_seqs;      // the tiles that exist are at most so many
     const int listed = vlrf_attn_prefill_tc_lists(n_tokens, n_seqs, max_new, H, n_parts, vlrf_sm_count()) ? n_seqs : 0;
     dim3 grid(H, listed ? (unsigned)places : n_seqs, (unsigned)(listed ? n_parts : tiles * n_parts));
-    cudaError_t e = launch_chained(attn_prefill_tc_kernel, grid, dim3(FT_THREADS), smem, stream, tq, tk, tv, q_off, block_table,
-                                   max_blocks, seq_slot, seq_start, seq_pos0, (__nv_bfloat16*)out, ld_out, H, Hkv, scale,
-                                   window, n_parts, partials, counters, (int)tiles, listed, dev_err, vlrf_trace_buffer());
+    e = launch_chained(kern, grid, dim3(FT_THREADS), smem, stream, tq, tk, tv, q_off, block_table, max_blocks, seq_slot, seq_start, seq_pos0,
+                       (__nv_bfloat16*)out, ld_out, H, Hkv, scale, window, n_parts, partials, counters, (int)tiles, listed, (uint32_t)g_polls,
+                       dev_err, vlrf_trace_buffer());
     if (e != cudaSuccess) return vlrf_fail(VLRF_ERR_CUDA, "attn_prefill_tc: %s", cudaGetErrorString(e));
     return vlrf_check_launch("attn_prefill_tc");
 }

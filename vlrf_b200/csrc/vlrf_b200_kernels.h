@@ -172,6 +172,8 @@ int vlrf_attn_prefill_tc_max_parts();
 int vlrf_attn_prefill_tc_min_part_blocks();
 int vlrf_attn_prefill_tc_lists(int n_tokens, int n_seqs, int max_new, int H, int n_parts, int sms);
 int vlrf_attn_prefill_tc_tile();
+// How often a wait of the calling thread's next launches polls before it gives up (negative: as ever); for tests.
+int vlrf_attn_prefill_tc_wait_polls(int polls);
 int vlrf_attn_prefill_tc(const void* qkv, int ld, int q_off, const void* Kc, const void* Vc, int n_blocks,
                          const int* block_table, int max_blocks, const int* seq_slot, const int* seq_start,
                          const int* seq_pos0, void* out, int ld_out, int n_tokens, int n_seqs, int max_new, int H,
