@@ -38,6 +38,35 @@ def test_rows_of_a_tile_of_a_pair(M, N, rows):
     assert library().vlrf_gemm_pair_rows(M, N, 148) == rows
 
 
+def test_rows_of_a_tile_of_a_pair_cost_the_same_to_find_on_any_gpu():
+    """Every many-row product asks.  The pair that has most to do is always the first, so nothing is gone through pair by pair: the same rows as where it
+    is, and no more time for 268 million pairs than for 74."""
+    import random
+    import time
+    from vlrf_b200.csrc import library
+
+    def by_pair(M, N, sms):
+        pairs, tiles_w, best = max(1, sms // 2), -(-N // 256), None
+        for bn in range(256, 63, -32):
+            whole, left = M // bn * tiles_w, (M % bn + 31) // 32 * 32
+            tiles = whole + (tiles_w if left else 0)
+            most = 0
+            for p in range(pairs):
+                mine, of_all = whole // pairs + (p < whole % pairs), tiles // pairs + (p < tiles % pairs)
+                most = max(most, mine * (bn + 96) + (of_all - mine) * (left + 96))
+            if best is None or most < best[0]:
+                best = (most, bn)
+        return best[1]
+
+    r = random.Random(5)
+    for _ in range(3000):
+        M, N, sms = int(2 ** r.uniform(6, 15)), int(2 ** r.uniform(3, 16)), r.choice([148, 148, 132, 8, 3, 1])
+        assert library().vlrf_gemm_pair_rows(M, N, sms) == by_pair(M, N, sms), (M, N, sms)
+    t0 = time.perf_counter()
+    library().vlrf_gemm_pair_rows(2048, 2304, 2 ** 29)
+    assert time.perf_counter() - t0 < 0.1
+
+
 @pytest.mark.parametrize("M,N,K,then,exchanged", [
     # alone: wide products from four rows on, a vocabulary always
     (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),

@@ -411,13 +411,10 @@ extern "C" int vlrf_gemm_pair_rows(int M, int N, int sms) {
     int rows = 64;
     for (int bn = 256; bn >= 64; bn -= 32) {
         const long long whole = M / bn * tiles_w, left = (M % bn + 31) & ~31;
-        // whole tiles first, tile t to pair t mod pairs; then a tile of the rows that are left for each of W's
-        long long most = 0;
-        for (int p = 0; p < pairs; ++p) {
-            const long long mine = whole / pairs + (p < whole % pairs ? 1 : 0), all = whole + (left ? tiles_w : 0);
-            const long long tiles = all / pairs + (p < all % pairs ? 1 : 0), cost = mine * (bn + 96) + (tiles - mine) * (left + 96);
-            if (cost > most) most = cost;
-        }
+        // whole tiles first, tile t to pair t mod pairs; then a tile of the rows that are left for each of W's.  The first pair has no fewer than any
+        // of either, and a whole tile costs no less than one of what is left: it has most to do.
+        const long long mine = (whole + pairs - 1) / pairs, tiles = (whole + (left ? tiles_w : 0) + pairs - 1) / pairs;
+        const long long most = mine * (bn + 96) + (tiles - mine) * (left + 96);
         if (best < 0 || most < best) { best = most; rows = bn; }
     }
     return rows;

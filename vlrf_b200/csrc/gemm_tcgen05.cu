@@ -522,9 +522,9 @@ extern "C" int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias
     // pairs, float32 with a residual: 512 x 768 x 768 5.8 -> 5.1 us, 2,048 x 768 x 768 7.3 -> 7.0, 2,050 x 1,600 x 1,600 17.0 -> 14.8, 2,050 x 1,600 x 6,400 43.3 ->
     // 40.6, 1,928 x 4,096 x 2,048 37.4 -> 31.5, 4,096 cubed 125 -> 111 (2,048 x 768 x 3,072 13.0 -> 13.4); bfloat16: 1,928 x 11,264 x 2,048 74.0 -> 67.9, 4,096
     // cubed 104 -> 97, 2,050 x 1,600 x 6,400 37.0 -> 37.3, but 2,048 x 2,304 x 768 9.2 -> 10.2, 2,048 x 768 x 3,072 11.1 -> 12.8.
-    if (g_forced_width == 0) {
+    if (g_forced_width == 0 && (out_dtype == VLRF_F32 || K >= 2048)) {
         const int rows = vlrf_gemm_pair_rows(M, N, vlrf_sm_count());
-        if (out_dtype == VLRF_F32 || (K >= 2048 && rows >= 192))
+        if (out_dtype == VLRF_F32 || rows >= 192)
             return vlrf_gemm_pair(X, W, bias, residual, Y, M, N, K, ldx, ldy, out_dtype, act, rows, Kc, Vc, block_table, max_blocks, tok_slot,
                                   tok_pos, k_off, v_off, Hkv, dh, BT, dev_err, stream);
     }
