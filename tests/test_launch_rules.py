@@ -67,6 +67,21 @@ def test_rows_of_a_tile_of_a_pair_cost_the_same_to_find_on_any_gpu():
     assert time.perf_counter() - t0 < 0.1
 
 
+@pytest.mark.parametrize("M,N,K,dtype,rows", [
+    # measured faster by pairs of SMs …
+    (2048, 768, 768, 0, 96), (2048, 768, 3072, 0, 96), (512, 768, 768, 0, 64), (2050, 1600, 1600, 0, 224), (2050, 1600, 6400, 0, 224), (4096, 4096, 4096, 0, 256),
+    (1024, 11264, 2048, 0, 224), (65, 16, 1024, 0, 64), (128, 6144, 2048, 0, 64), (1928, 11264, 2048, 1, 256), (4096, 4096, 4096, 1, 256), (512, 4096, 4096, 1, 128), (777, 8192, 3072, 1, 224),
+    (512, 8192, 3072, 1, 256), (2050, 11264, 2048, 1, 256), (777, 2048, 4096, 1, 96),
+    # … and by one CTA a tile: little work for 2-byte columns, tiles of 160 to 224 rows along a long K, rows that fill no tile of 192
+    (2048, 2304, 768, 1, 0), (512, 4096, 1024, 1, 0), (1928, 4096, 1024, 1, 0), (2048, 3072, 1024, 1, 0), (2050, 4800, 1600, 1, 0), (1024, 6144, 2048, 1, 0), (2048, 1600, 6400, 1, 0), (3000, 2048, 2048, 1, 0),
+    (128, 11264, 2048, 1, 0), (240, 11264, 2048, 1, 0), (240, 11264, 2048, 0, 0), (2048, 1280, 5120, 0, 0), (1500, 1600, 6400, 0, 0), (2048, 1600, 6400, 0, 0)])
+def test_products_by_pairs_only_where_they_gain(M, N, K, dtype, rows):
+    """Float32 (0) and bfloat16 (1) results; the rows of a pair's tile, 0 for one CTA a tile."""
+    from vlrf_b200.csrc import library, ops
+    assert (ops.F32, ops.BF16) == (0, 1)
+    assert library().vlrf_gemm_tcgen05_pair_rows(M, N, K, dtype, 148) == rows
+
+
 @pytest.mark.parametrize("M,N,K,then,exchanged", [
     # alone: wide products from four rows on, a vocabulary always
     (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),

@@ -59,6 +59,7 @@ _SIGNATURES = {
                           _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,
                           _c_int, _c_int, _c_int, _c_void_p, _c_void_p],
     "vlrf_gemm_pair_rows": [_c_int] * 3,
+    "vlrf_gemm_tcgen05_pair_rows": [_c_int] * 5,
     "vlrf_gemm_pair_wait_polls": [_c_int],
     "vlrf_gemm_pair": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                        _c_int, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int,

@@ -485,6 +485,56 @@ extern "C" int vlrf_gemm_tcgen05_force_width(int bn) {
     return VLRF_OK;
 }
 
+namespace {
+// Columns of a tile: the fewest rounds of the persistent CTAs, each weighted by the bytes a tile's stage pulls through L2 (128 rows of one operand and the
+// tile's width of the other): that, not the MMAs, is what a round's time follows when all SMs run (measured over the products of
+// GPT-2 small to XL at 512 to 8,192 rows)
+int tc_width(int M, int N, int sms) {
+    int best_bn = 128;
+    long long best = -1;
+    for (int bn : {256, 224, 192, 160, 128, 96, 64}) {
+        if (bn > 64 && N <= bn / 2) continue;
+        const long long tiles = (long long)((N + bn - 1) / bn) * ((M + 127) / 128);
+        const long long rounds = (tiles + sms - 1) / sms;
+        if (bn == 96 && rounds > 1) continue;      // the odd width only where it puts every tile on an SM of its own
+        const long long cost = rounds * (bn + 128);
+        if (best < 0 || cost < best) { best = cost; best_bn = bn; }
+    }
+    return best_bn;
+}
+}  // namespace
+
+// Rows of a tile where a product goes by pairs of SMs (gemm_pair.cu), 0 where a CTA takes a tile: by the rounds of the SM or pair that has most to do, each
+// at the cycles that K takes it there and, with float32 results, 4,000 more of a CTA of its own (whose lanes have a row each and store to 32
+// lines at once), with bfloat16 ones 1,000 more of a pair (whose lanes have a column each, 2 bytes of a row).  The cycles are those of 64 of K for
+// tiles of 64 to 256 columns (a CTA) or rows (a pair) in steps of 32, from products that differ in K alone (K = 1,600 and 6,400 of 2,048 x 1,600 and the
+// like).  A pair's stage holds two of K's atoms up to 128 rows and one beyond, and costs it some 590 cycles at least, whatever the rows.
+// With bfloat16 results the two lie closer than this tells: pairs where they come to less than 0.92 of it, or, along a long K in tiles of 192
+// rows or more, where the stages of many rounds pull half the bytes of an operand through L2, to less than 1.1.  One CTA a tile against pairs, us, over 453
+// products of 65 to 8,192 rows and K = 768 to 8,192.  float32 with a residual: 512 x 768 x 768 6.7, 5.8; 2,048 x 768 x 768 9.2, 8.4; 2,048 x 768 x
+// 3,072 15.2, 14.8; 2,050 x 1,600 x 1,600 19.9, 17.2; 2,050 x 1,600 x 6,400 44.4, 40.8, but 2,048 rows of it 38.4, 40.6 and 1,500 rows 32.6, 38.2; 2,048 x
+// 1,280 x 5,120 28.5, 32.0; 4,096 cubed 118, 108.  bfloat16: 1,928 x 11,264 x 2,048 75.3, 71.1, but 128 rows of it 13.1, 15.3; 777 x 8,192 x 3,072 40.9, 37.6;
+// 4,096 cubed 103, 100; 1,024 x 6,144 x 2,048 24.3, 27.2; 2,048 x 2,304 x 768 11.8, 12.3; 2,048 x 3,072 x 1,024 14.5, 17.4; 2,048 x 5,120 x 1,280 25.0, 27.8;
+// 2,048 x 6,400 x 1,600 36.6, 35.8; 777 x 2,048 x 4,096 18.6, 16.6.
+extern "C" int vlrf_gemm_tcgen05_pair_rows(int M, int N, int K, int out_dtype, int sms) {
+    constexpr int ONE[7] = {305, 307, 428, 450, 548, 630, 703}, PAIR[7] = {323, 343, 364, 590, 610, 640, 670};
+    const bool f32 = out_dtype == VLRF_F32;
+    const int width = tc_width(M, N, sms);
+    const long long rounds = ((long long)((N + width - 1) / width) * ((M + 127) / 128) + sms - 1) / sms;
+    const long long one = rounds * ((long long)ONE[(width - 64) / 32] * K / 64 + (f32 ? 4000 : 0));
+    int rows = vlrf_gemm_pair_rows(M, N, sms);
+    if (M < rows) rows = M <= 64 ? 64 : (M + 31) & ~31;          // (no wider than the rows that there are)
+    const int pairs = sms / 2 > 0 ? sms / 2 : 1, left = (M % rows + 31) & ~31;
+    const long long tiles_w = (N + 255) / 256, whole = M / rows * tiles_w, all = whole + (left ? tiles_w : 0);
+    const long long mine = (whole + pairs - 1) / pairs, tiles = (all + pairs - 1) / pairs;
+    auto cost = [&](int r) {
+        const int c = PAIR[r < 64 ? 0 : (r - 64) / 32];
+        return (long long)(rows > 128 && c < PAIR[3] ? PAIR[3] : c) * K / 64 + (f32 ? 0 : 1000);
+    };
+    const long long pair = mine * cost(rows) + (tiles - mine) * cost(left);
+    return 100 * pair < (f32 ? 100 : K >= 2048 && rows >= 192 ? 110 : 92) * one ? rows : 0;
+}
+
 // Whether this kernel takes the shape (bfloat16 only): rows must start on 16-byte boundaries for TMA.
 extern "C" int vlrf_gemm_tcgen05_takes(int M, int N, int K, int ldx) {
     return (M >= 1 && N >= 1 && K >= 8 && K % 8 == 0 && ldx % 8 == 0) ? 1 : 0;
@@ -517,36 +567,14 @@ extern "C" int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias
         return SWAPPED(64);
 #undef SWAPPED
     }
-    // By pairs of SMs (gemm_pair.cu): float32 results, which its whole-line stores finish sooner at every size; bfloat16 results where K is long and
-    // tiles are wide, so that half the bytes of an operand a stage count for more than 2-byte columns to store.  One CTA a tile against
-    // pairs, float32 with a residual: 512 x 768 x 768 5.8 -> 5.1 us, 2,048 x 768 x 768 7.3 -> 7.0, 2,050 x 1,600 x 1,600 17.0 -> 14.8, 2,050 x 1,600 x 6,400 43.3 ->
-    // 40.6, 1,928 x 4,096 x 2,048 37.4 -> 31.5, 4,096 cubed 125 -> 111 (2,048 x 768 x 3,072 13.0 -> 13.4); bfloat16: 1,928 x 11,264 x 2,048 74.0 -> 67.9, 4,096
-    // cubed 104 -> 97, 2,050 x 1,600 x 6,400 37.0 -> 37.3, but 2,048 x 2,304 x 768 9.2 -> 10.2, 2,048 x 768 x 3,072 11.1 -> 12.8.
-    if (g_forced_width == 0 && (out_dtype == VLRF_F32 || K >= 2048)) {
-        const int rows = vlrf_gemm_pair_rows(M, N, vlrf_sm_count());
-        if (out_dtype == VLRF_F32 || rows >= 192)
+    const int sms = vlrf_sm_count();
+    if (g_forced_width == 0) {
+        const int rows = vlrf_gemm_tcgen05_pair_rows(M, N, K, out_dtype, sms);
+        if (rows > 0)
             return vlrf_gemm_pair(X, W, bias, residual, Y, M, N, K, ldx, ldy, out_dtype, act, rows, Kc, Vc, block_table, max_blocks, tok_slot,
                                   tok_pos, k_off, v_off, Hkv, dh, BT, dev_err, stream);
     }
-    // tile width: the fewest rounds of the persistent CTAs, each weighted by the bytes a tile's stage pulls through
-    // L2 (128 rows of one operand and the tile's width of the other): that, not the MMAs, is what a round's time
-    // follows when all SMs run (measured over the products of GPT-2 small to XL at 512 to 8,192 rows)
-    int best_bn = 128;
-    {
-        const int sms = vlrf_sm_count();
-        long long best = -1;
-        const int widths[7] = {256, 224, 192, 160, 128, 96, 64};
-        for (int i = 0; i < 7; ++i) {
-            const int bn = widths[i];
-            if (bn > 64 && N <= bn / 2) continue;
-            const long long tiles = (long long)((N + bn - 1) / bn) * ((M + 127) / 128);
-            const long long rounds = (tiles + sms - 1) / sms;
-            if (bn == 96 && rounds > 1) continue;      // the odd width only where it puts every tile on an SM of its own
-            const long long cost = rounds * (bn + 128);
-            if (best < 0 || cost < best) { best = cost; best_bn = bn; }
-        }
-        if (g_forced_width > 0) best_bn = g_forced_width;
-    }
+    const int best_bn = g_forced_width > 0 ? g_forced_width : tc_width(M, N, sms);
 #define TILED(BNV, ST) (out_dtype == VLRF_BF16 ? launch_tc<BNV, ST, __nv_bfloat16>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, kv, dev_err, stream) \
                                               : launch_tc<BNV, ST, float>(X, W, bias, residual, Y, M, N, K, ldx, ldy, act, kv, dev_err, stream))
     VLRF_REQUIRE(out_dtype == VLRF_BF16 || out_dtype == VLRF_F32, "gemm_tcgen05: unknown output dtype %d", out_dtype);

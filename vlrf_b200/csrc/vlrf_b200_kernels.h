@@ -97,8 +97,9 @@ int vlrf_gemm_tcgen05(const void* X, const void* W, const float* bias, const flo
                       int max_blocks, const int* tok_slot, const int* tok_pos, int k_off, int v_off, int Hkv, int dh,
                       int BT, int* dev_err, cudaStream_t stream);
 // The same product by pairs of SMs (`cta_group::2`), tiles of 256 columns by bn rows (a multiple of 32 up to 256); vlrf_gemm_tcgen05 chooses it by
-// size, with the rows that vlrf_gemm_pair_rows gives.
+// size, with the rows that vlrf_gemm_tcgen05_pair_rows gives.
 int vlrf_gemm_pair_rows(int M, int N, int sms);
+int vlrf_gemm_tcgen05_pair_rows(int M, int N, int K, int out_dtype, int sms);      // 0: one CTA a tile
 // How often a wait of the calling thread's next launches by pairs polls before it gives up (negative: as ever); for tests.
 int vlrf_gemm_pair_wait_polls(int polls);
 int vlrf_gemm_pair(const void* X, const void* W, const float* bias, const float* residual, void* Y, int M, int N, int K, int ldx,
