@@ -82,6 +82,16 @@ def test_products_by_pairs_only_where_they_gain(M, N, K, dtype, rows):
     assert library().vlrf_gemm_tcgen05_pair_rows(M, N, K, dtype, 148) == rows
 
 
+@pytest.mark.parametrize("M,N,K,gains", [
+    # measured faster with the norm ahead: GPT-2 small up to 8 rows, medium up to 4 (and 1 row of its feed-forward) …
+    (1, 2304, 768, True), (4, 3072, 768, True), (8, 2304, 768, True), (8, 3072, 768, True), (1, 3072, 1024, True), (4, 3072, 1024, True), (1, 4096, 1024, True),
+    # … and slower, or no faster, where a second round of CTAs is needed; nine rows and 1,280 columns are not taken
+    (5, 3072, 1024, False), (8, 3072, 1024, False), (2, 4096, 1024, False), (4, 4096, 1024, False), (8, 4096, 1024, False), (9, 768, 768, False), (1, 3840, 1280, False)])
+def test_float32_norm_ahead_of_a_product_only_where_its_ctas_find_room(M, N, K, gains):
+    from vlrf_b200.csrc import library
+    assert bool(library().vlrf_gemm_f32_norm_gains(M, N, K, 148)) == gains
+
+
 @pytest.mark.parametrize("M,N,K,then,exchanged", [
     # alone: wide products from four rows on, a vocabulary always
     (4, 7296, 1024, "kernels", True), (3, 7296, 1024, "kernels", False), (8, 8192, 2048, "kernels", False), (1, 50257, 768, "product", True),

@@ -33,6 +33,7 @@ _SIGNATURES = {
     "vlrf_gemm_simt": [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
                        _c_int, _c_int, _c_int, _c_int, _c_void_p],
     "vlrf_gemm_f32_norm_takes": [_c_int, _c_int],
+    "vlrf_gemm_f32_norm_gains": [_c_int] * 4,
     "vlrf_gemm_f32_norm": [_c_void_p, _c_void_p, _c_void_p, _c_float, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int,
                            _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p, _c_void_p, _c_int, _c_int, _c_int, _c_int, _c_int,
                            _c_void_p, _c_void_p],

@@ -11,7 +11,7 @@
 // one order.  In float32 that order is: K in PARTS = 8 runs of equal length (`part_length`), each a chain of FMAs in the
 // order of k, the eight sums added in their order.  The parts are what a few rows are spread over the GPU by (a chain of
 // all K terms in one thread took 104 us a product at 4 rows, whatever its size):
-//   up to 8 rows     gemm_f32_norm_kernel: the next, with a LayerNorm ahead and a cache write behind
+//   up to 8 rows     gemm_f32_norm_kernel: the next, with a LayerNorm ahead and a cache write behind, where all its CTAs find room at once
 //   up to 16 rows    gemm_f32_rows_kernel: a thread per (column, part); bound by streaming W once
 //   more rows        gemm_f32_tile_kernel: 64 x 64 tiles, the eight parts of a tile one CTA each of a cluster; bound by FMAs
 // bfloat16 operands take gemm_simt_kernel (shapes outside the tensor-core kernels' rules: rare and small).
@@ -194,7 +194,7 @@ gemm_f32_rows_kernel(const float* __restrict__ X, const float* __restrict__ W, c
     }
 }
 
-// Up to R rows with a LayerNorm ahead and, for a q/k/v projection, the write of its k and v columns into one layer's paged cache behind:
+// Up to R rows with a LayerNorm ahead (vlrf_gemm_f32_norm_gains says where that pays) and, for a q/k/v projection, the write of its k and v columns into one layer's paged cache behind:
 // the norm's kernel and the append's are launches of their own otherwise, 2.5 us each inside a decode step for rows that every CTA here
 // has read and normed in 1.  The sums are those of gemm_f32_rows_kernel, the norm is that of embed_norm.cu (a warp a row, the row in
 // registers), so the same bits come out.  The whole rows lie in shared memory, each part's run 16 bytes further than its place
@@ -204,7 +204,7 @@ struct F32Scatter {
     const int* block_table; const int* tok_slot; const int* tok_pos;
     int max_blocks, k_off, v_off, width, dh, Hkv, BT;      // width = Hkv·dh
 };
-constexpr int NORM_MAX_K = 1024, NORM_NV = NORM_MAX_K / 128;
+constexpr int NORM_MAX_K = 1024, NORM_NV = NORM_MAX_K / 128, NORM_STAGES = 4;
 template <int R, int C, int STAGES> __host__ __device__ constexpr size_t norm_smem(int K) {
     return ((size_t)STAGES * PARTS * C * KPITCH + (size_t)R * (K + 4 * PARTS) + 2 * (size_t)K) * 4;
 }
@@ -428,7 +428,7 @@ int launch_f32_rows(const float* X, const float* W, const float* bias, const flo
 template <int R, int C>
 int launch_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y, int M, int N, int K,
                     int act, const F32Scatter& kv, int* dev_err, cudaStream_t stream) {
-    constexpr int STAGES = 4;
+    constexpr int STAGES = NORM_STAGES;
     static_assert((size_t)STAGES * C * KPITCH >= (size_t)R * C, "the sums take the ring's place");
     const size_t smem = norm_smem<R, C, STAGES>(K);
     auto kern = gemm_f32_norm_kernel<R, C, STAGES>;
@@ -500,9 +500,23 @@ extern "C" int vlrf_gemm_simt(const void* X, const void* W, const float* bias, c
     return vlrf_check_launch("gemm_simt");
 }
 
-// Whether the product with a LayerNorm ahead takes these rows: up to 8 (beyond, a norm of its own costs less than every CTA's), as many
-// columns as the norm keeps in registers.
+// Whether the product with a LayerNorm ahead takes these rows: up to 8, as many columns as the norm keeps in registers.  (With rows for 16 a
+// launch took 1.15 to 1.8 times what norm, product and append take one after the other: 9 rows of 768 x 2,304 11.8, 13.5 us, of 768 x 3,072 13.6, 24.4.
+// With registers for 1,664 columns GPT-2's sizes were 3 to 10 % slower, and of those with 1,280 and 1,600 columns half gained, half lost.)
 extern "C" int vlrf_gemm_f32_norm_takes(int M, int K) { return M >= 1 && M <= 8 && K >= 4 && K % 4 == 0 && K <= NORM_MAX_K ? 1 : 0; }
+
+// Whether it also gains: where all its CTAs find room on the GPU at once, by their shared memory (the rows, the norm's weight and bias and the ring).  A
+// CTA of a second round norms all rows again, behind what it could have hidden that behind.  Norm and product apart (with the append for q/k/v) against
+// together, us: 1 row of 768 x 2,304 7.6, 5.7, of 1,024 x 4,096 7.1, 5.9; 4 rows of 768 x 3,072 7.3, 6.1, of 1,024 x 3,072 11.9, 7.9, of 1,024 x 4,096
+// (512 CTAs, room for 444) 12.1, 12.2; 8 rows of 768 x 3,072 (384 CTAs, room for 444) 10.2, 8.8, of 1,024 x 3,072 (384, 296) 15.4, 19.0, of 1,024 x 4,096 13.0, 17.2.
+extern "C" int vlrf_gemm_f32_norm_gains(int M, int N, int K, int sms) {
+    if (!vlrf_gemm_f32_norm_takes(M, K)) return 0;
+    const bool wide = N >= 8 * sms;                        // (as launch_f32_norm_for)
+    const size_t smem = wide ? (M == 1 ? norm_smem<1, 8, NORM_STAGES>(K) : M <= 4 ? norm_smem<4, 8, NORM_STAGES>(K) : norm_smem<8, 8, NORM_STAGES>(K))
+                             : (M == 1 ? norm_smem<1, 4, NORM_STAGES>(K) : M <= 4 ? norm_smem<4, 4, NORM_STAGES>(K) : norm_smem<8, 4, NORM_STAGES>(K));
+    const int ctas = wide ? (N + 7) / 8 : (N + 3) / 4;
+    return ctas <= (int)(228 * 1024 / (smem + 1024)) * sms ? 1 : 0;      // (an SM's 228 KiB; a CTA has 1 KiB beside what it asks for)
+}
 
 // Y = act(LayerNorm(X) · Wᵀ + bias) in float32, X [M][K], Y [M][N]; Kc != null: columns k_off … and v_off … also into the cache.
 extern "C" int vlrf_gemm_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y,

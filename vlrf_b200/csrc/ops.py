@@ -342,12 +342,16 @@ def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, s
 
 
 def can_fuse_layernorm(n_rows: int, width: int, w_dtype: torch.dtype, *tensors) -> bool:
-    """Whether `linear_layernorm` takes this many rows of this width; `tensors`: the rows, the norm's weight and bias and the
-    product's weights, which in float32 must begin on 16 bytes."""
+    """Whether `linear_layernorm` takes this many rows of this width, and gains by it; `tensors`: the rows, the norm's weight and bias and the
+    product's weights, which in float32 must begin on 16 bytes (and say whether it gains)."""
     # with more rows, every CTA repeating the norm costs more than a norm kernel of its own
     if w_dtype == torch.float32:
         from . import library
-        return all(t.data_ptr() % 16 == 0 for t in tensors) and bool(library().vlrf_gemm_f32_norm_takes(n_rows, width))
+        if not all(t.data_ptr() % 16 == 0 for t in tensors):
+            return False
+        if len(tensors) == 4:
+            return bool(library().vlrf_gemm_f32_norm_gains(n_rows, tensors[3].shape[0], width, sm_count()))
+        return bool(library().vlrf_gemm_f32_norm_takes(n_rows, width))
     if w_dtype != torch.bfloat16 or n_rows > FUSED_NORM_MAX_ROWS or n_rows < 1 or width % 32 != 0:
         return False
     from . import library

@@ -85,6 +85,7 @@ int vlrf_gemm_simt(const void* X, const void* W, const float* bias, const float*
 // act(LayerNorm(X) · Wᵀ + bias) in float32 for up to 8 rows, the norm in the product's prologue; Kc != null: columns k_off … and v_off … of
 // the result also into one layer's paged cache.  The bits of vlrf_layernorm, vlrf_gemm_simt and vlrf_kv_append one after the other.
 int vlrf_gemm_f32_norm_takes(int M, int K);
+int vlrf_gemm_f32_norm_gains(int M, int N, int K, int sms);      // takes them, and faster than the three do
 int vlrf_gemm_f32_norm(const float* X, const float* gamma, const float* beta, float eps, const float* W, const float* bias, float* Y, int M,
                        int N, int K, int act, float* Kc, float* Vc, const int* block_table, int max_blocks, const int* tok_slot,
                        const int* tok_pos, int k_off, int v_off, int Hkv, int dh, int BT, int* dev_err, cudaStream_t stream);
