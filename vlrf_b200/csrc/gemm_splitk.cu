@@ -579,33 +579,14 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             };
             if (whole) write(std::true_type{});
             else write(std::false_type{});
-            if (stats_out != nullptr && seg0 < N) {
+            if (RP == 1 && stats_out != nullptr && seg0 < N) {
                 // what a LayerNorm of these rows will need: this segment's sum and squared deviation from its
-                // own mean (of the values as stored; statistics are kept of float32 rows only)
-                const int n_seg = min(32, N - seg0);
-                float sum[RP], m2[RP];
-#pragma unroll
-                for (int e = 0; e < RP; ++e) sum[e] = n < N ? y[e] : 0.f;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                    for (int e = 0; e < RP; ++e) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
-#pragma unroll
-                for (int e = 0; e < RP; ++e) {
-                    const float d = n < N ? y[e] - sum[e] / (float)n_seg : 0.f;
-                    m2[e] = d * d;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                    for (int e = 0; e < RP; ++e) m2[e] += __shfl_xor_sync(0xffffffffu, m2[e], o);
+                // own mean (of the values as stored; statistics are kept of float32 rows only, and of no more than a norm ahead takes)
+                const float sum = warp_sum(n < N ? y[0] : 0.f), d = n < N ? y[0] - sum / (float)min(32, N - seg0) : 0.f;
+                const float m2 = warp_sum(d * d);
                 if (lane == 0) {
-#pragma unroll
-                    for (int e = 0; e < RP; ++e)
-                        if (m0 + e < M) {
-                            float* so = stats_out + ((size_t)(m0 + e) * ((N + 31) >> 5) + (seg0 >> 5)) * 2;
-                            so[0] = sum[e]; so[1] = m2[e];
-                        }
+                    float* so = stats_out + ((size_t)m0 * ((N + 31) >> 5) + (seg0 >> 5)) * 2;
+                    so[0] = sum; so[1] = m2;
                 }
             }
         }
@@ -760,8 +741,8 @@ extern "C" int vlrf_gemm_splitk(const void* X, int x_is_f32_ln, const void* W, c
     VLRF_REQUIRE(ldx >= K && ldy >= N && act >= 0 && act <= VLRF_ACT_LAST_FUSED, "gemm_splitk: bad arguments");
     VLRF_REQUIRE(dev_err != nullptr, "gemm_splitk: needs the device error word");
     VLRF_REQUIRE(!x_is_f32_ln || (gamma && beta && stats_in), "gemm_splitk: the fused LayerNorm needs weight, bias and the rows' statistics");
-    VLRF_REQUIRE(stats_out == nullptr || ((N + 31) / 32 <= SP_STAT_SEGS && out_dtype == VLRF_F32),
-                 "gemm_splitk: statistics are kept of float32 rows of at most %d columns", SP_STAT_SEGS * 32);
+    VLRF_REQUIRE(stats_out == nullptr || (M <= 16 && (N + 31) / 32 <= SP_STAT_SEGS && out_dtype == VLRF_F32),
+                 "gemm_splitk: statistics are kept of at most 16 float32 rows of at most %d columns", SP_STAT_SEGS * 32);
     VLRF_REQUIRE(out_dtype == VLRF_BF16 || out_dtype == VLRF_F32, "gemm_splitk: unknown output dtype %d", out_dtype);
     SpKvScatter kv{};
     if (Kc != nullptr) {

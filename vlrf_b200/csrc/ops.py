@@ -171,7 +171,7 @@ SPLITK_NORM_MIN_WEIGHT_BYTES = 0
 _DEV_ERR = None
 
 
-ROW_STATS_MAX_ROWS, ROW_STATS_MAX_WIDTH = 64, 8192
+ROW_STATS_MAX_ROWS, ROW_STATS_MAX_WIDTH = FUSED_NORM_MAX_ROWS, 8192      # (with more rows no norm reads them)
 
 
 class RowStats:
@@ -316,7 +316,7 @@ def _linear_dispatch(x, w, bias, out, act, residual, M, N, K, kv_scatter=None, s
     if x.dtype == torch.bfloat16 and M <= SKINNY_MAX_ROWS and _splitk_takes(M, N, K, K, False):
         # few rows, a large matrix: tiles of w on the tensor cores, the sum over k cut into parts
         scatter = kv_scatter is not None and bf16_out
-        keep = stats is not None and not bf16_out and M <= FUSED_NORM_MAX_ROWS and stats.takes(M, N)      # (with more rows no norm reads them)
+        keep = stats is not None and not bf16_out and stats.takes(M, N)
         call("vlrf_gemm_splitk", _ptr(x), 0, _ptr(w), _ptr(bias), _ptr(residual), _ptr(out), dtype_code(out.dtype),
              M, N, K, K, N, act, 0, 0, 0.0, *_kv_args(kv_scatter if scatter else None, N), 0,
              _ptr(stats.buffer()) if keep else 0, _ptr(_dev_err()), _stream())
