@@ -157,3 +157,14 @@ def test_warps_that_go_on_together_wait_with_one_answer(name):
                 alone = any(re.search(r"elect_one\(\)|\b(lane|threadIdx\.x) == 0", s) for s in scopes + [statement])
                 assert alone, f"{name}: {' '.join(statement.split())}"
     assert not scopes and "tbar_wait_warp(" in text
+
+
+@pytest.mark.parametrize("name", ["attention_prefill_tc.cu", "gemm_pair.cu"])
+def test_kernels_that_give_up_wait_for_what_is_under_way(name):
+    """Whichever role gave up: behind the place where all roles meet, and ahead of giving tensor memory back; nowhere inside a role."""
+    import re
+    text = re.sub(r"//[^\n]*", "", (SRC / name).read_text())
+    calls = [m.start() for m in re.finditer(r"if \(\*?s_abort\)\s+\w+_drain\(", text)]
+    given_back = [m.start() for m in re.finditer(r"tcgen05\.dealloc", text)]
+    assert len(calls) == len(given_back) == 1 and calls[0] < given_back[0]
+    assert re.search(r"(__syncthreads|cluster_sync_all)\(\);[^{}]*$", text[:calls[0]])
